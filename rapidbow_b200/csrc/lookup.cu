@@ -1,7 +1,9 @@
 // Vocabulary-tree descent kernels (reference semantics: vocTreeLookUp.cu:82-155 -- exact
 // squared L2 over 16 centers per node, lowest branch index on ties, idx = idx*B + b).
 //
-// Two implementations behind launchLookup():
+// Three implementations, launchLookupDirect() and two behind launchLookup():
+//   * lookupDirect  : a warp per descriptor, every level in one launch, dp4a dot products (exact);
+//                     for few descriptors, where launches and the regroup cost more than the work.
 //   * lookupPassTc  : tcgen05 kind::i8 (u8 x u8 -> s32, exact) over level pairs.  A pass takes
 //                     the descriptors grouped by their node at level 2p, stages 128-row tiles in
 //                     shared memory (a TMA tiled load in input order for the first pass, a 16-byte
@@ -1321,6 +1323,60 @@ __global__ void __launch_bounds__(kSimtThreads, 8) lookupSimtF32(const uint8_t* 
     if (base + threadIdx.x < n) out[base + threadIdx.x] = static_cast<uint32_t>(idx);
 }
 
+// ------------------------------------------------------------------ few descriptors: one launch
+// A warp per descriptor, all levels in one kernel.  Lane l keeps chunk l % 8 of the row and reads
+// chunk l % 8 of centers 4 k + l / 8 (k = 0..3), so each 16-byte load instruction of the warp
+// covers 512 contiguous bytes of the node; the dot products are dp4a sums (exact).  A level is
+// four such loads, 16 dp4a per lane, four shuffles and one warp-wide minimum: bound by the node
+// reads (2 KB per row and level, 31 cycles per SM).  731 rows of a 65,536-word tree: 43 us by the
+// tensor passes (six launches), 11 us here, the host's share of a call.
+constexpr uint32_t kDirectThreads = 128;
+
+__global__ void __launch_bounds__(kDirectThreads) lookupDirect(const uint8_t* __restrict__ centers,
+                                                               const int32_t* __restrict__ cnorm, uint32_t B,
+                                                               uint32_t L, const uint8_t* __restrict__ desc,
+                                                               uint64_t n, uint32_t* __restrict__ out)
+{
+    const uint64_t row = uint64_t(blockIdx.x) * (kDirectThreads / 32) + threadIdx.x / 32;
+    if (row >= n) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint4 x = __ldg(reinterpret_cast<const uint4*>(desc + row * kDims) + (lane & 7u));
+    // after the reduction over the eight lanes of a chunk group, this lane holds the dot product
+    // of center 4 (2 bit2(lane) + bit1(lane)) + lane / 8 (two lanes hold each)
+    const bool hi2 = (lane & 4u) != 0, hi1 = (lane & 2u) != 0;
+    const uint32_t b = 4u * ((hi2 ? 2u : 0u) + (hi1 ? 1u : 0u)) + (lane >> 3);
+    uint64_t idx = 0, lb = 0;
+    for (uint32_t level = 0; level < L; level++) {
+        const uint64_t node = lb + idx;
+        const uint4* c4 = reinterpret_cast<const uint4*>(centers + node * kMaxBranch * kDims) + lane;
+        uint4 v[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) v[k] = 4u * k < B ? __ldg(c4 + 32u * k) : make_uint4(0, 0, 0, 0);
+        const int32_t cn = __ldg(cnorm + node * kMaxBranch + b);
+        uint32_t d[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) {
+            d[k] = __dp4a(x.x, v[k].x, 0u);
+            d[k] = __dp4a(x.y, v[k].y, d[k]);
+            d[k] = __dp4a(x.z, v[k].z, d[k]);
+            d[k] = __dp4a(x.w, v[k].w, d[k]);
+        }
+        // sums over the eight lanes, halving the centers a lane keeps in each of two steps
+        const uint32_t s0 = __shfl_xor_sync(0xFFFFFFFFu, hi2 ? d[0] : d[2], 4);
+        const uint32_t s1 = __shfl_xor_sync(0xFFFFFFFFu, hi2 ? d[1] : d[3], 4);
+        const uint32_t e0 = (hi2 ? d[2] : d[0]) + s0, e1 = (hi2 ? d[3] : d[1]) + s1;
+        uint32_t f = (hi1 ? e1 : e0) + __shfl_xor_sync(0xFFFFFFFFu, hi1 ? e0 : e1, 2);
+        f += __shfl_xor_sync(0xFFFFFFFFu, f, 1);
+        // |c|^2 - 2 x.c lies in (-2^24, 2^23], so 16 times it plus the branch fits 32 bits and its
+        // minimum is the lowest branch of the lowest score (vocTreeLookUp.cu:108-125)
+        const int32_t key = b < B ? (cn - 2 * static_cast<int32_t>(f)) * 16 + static_cast<int32_t>(b) : 0x7FFFFFFF;
+        const uint32_t bi = static_cast<uint32_t>(__reduce_min_sync(0xFFFFFFFFu, key)) & 15u;
+        idx = idx * B + bi;
+        lb = lb * B + 1;
+    }
+    if (lane == 0) out[row] = static_cast<uint32_t>(idx);
+}
+
 // ------------------------------------------------------------------ host side
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1407,6 +1463,27 @@ LookupScratch carveLookupScratch(void* base, uint32_t B, uint32_t L, uint64_t n)
     p += a((n / kTileRows + bins + 1) * sizeof(TileInfo));
     s.ctaHist = reinterpret_cast<uint32_t*>(p);
     return s;
+}
+
+// Where lookupDirect ends.  It is bound by the L1's load path (a node is 2 KB per row and level,
+// 0.11 ns per row and level whatever the tree) above the ~11 us a call takes on the host; the
+// tensor-core path starts at one pass (12 us) up to L = 2, two passes and a regroup (41-43 us) up
+// to L = 4, and three of more bins above.  Measured, direct against tensor, us per call: B=16 L=4:
+// 731 rows 11 / 43, 64,000 29 / 49, 100,000 43 / 54, 150,000 64 / 60; B=16 L=2: 32,000 11 / 13,
+// 48,000 14 / 13; B=10 L=6: 16,000 14 / 155, 200,000 123 / 213, 400,000 240 / 239; B=2 L=8:
+// 200,000 142 / 135.
+uint64_t directLookupRows(uint32_t, uint32_t L) { return L <= 2 ? 32768 : L <= 4 ? 100000 : 200000; }
+
+uint32_t launchLookupDirect(const DeviceTree& tree, const uint8_t* desc, uint64_t n, uint32_t* leaf,
+                            cudaStream_t stream)
+{
+    if (n == 0) return 0;
+    const uint64_t perBlock = kDirectThreads / 32;
+    ScopedKernelTimer timer(kTimedLookupPass, stream);
+    lookupDirect<<<static_cast<uint32_t>((n + perBlock - 1) / perBlock), kDirectThreads, 0, stream>>>(
+        tree.centers, tree.cnorm, tree.B, tree.L, desc, n, leaf);
+    RBW_CUDA(cudaGetLastError());
+    return 1;
 }
 
 uint32_t launchLookup(const DeviceTree& tree, const uint8_t* desc, uint64_t n, uint32_t* leaf, LookupAlgo algo,

@@ -16,7 +16,7 @@ struct DeviceTree {
 };
 
 enum LookupAlgo : int {
-    kLookupAuto = 0,     // fastest exact path (tensor cores)
+    kLookupAuto = 0,     // fastest exact path (lookupDirect for few rows, else tensor cores)
     kLookupTensorU8 = 1, // tcgen05 kind::i8, level pairs + counting-sort regroup
     kLookupSimtF32 = 2,  // plain FP32 SIMT kernel (the comparison baseline)
     kLookupTensorU8WarpNode = 3, // as kLookupTensorU8, the node level of each pair by warp-level MMAs
@@ -42,6 +42,12 @@ struct LookupScratch {
 size_t lookupScratchBytes(uint32_t B, uint32_t L, uint64_t n);
 // Carves `base` (256-B aligned, lookupScratchBytes bytes) into a LookupScratch.
 LookupScratch carveLookupScratch(void* base, uint32_t B, uint32_t L, uint64_t n);
+
+// Largest number of descriptors that kLookupAuto descends with lookupDirect.
+uint64_t directLookupRows(uint32_t B, uint32_t L);
+// One launch, no scratch: every warp takes one descriptor down the whole tree (dp4a, exact).
+uint32_t launchLookupDirect(const DeviceTree& tree, const uint8_t* desc, uint64_t n, uint32_t* leaf,
+                            cudaStream_t stream);
 
 // Stream-ordered lookup of n descriptors (16-B aligned device rows of 128 B) into leaf indices.
 // Returns the number of kernels launched.

@@ -310,6 +310,7 @@ uint32_t Vocabulary::lookup(const uint8_t* devDesc, uint64_t n, uint32_t* devLea
         if (algo == kLookupSimtF32) throw Error(kUnsupported, "the FP32 SIMT lookup reads uint8 centers");
         return lookupFloat(devDesc, n, devLeaf, stream);
     }
+    if (algo == kLookupAuto && n <= directLookupRows(mB, mL)) return launchLookupDirect(mTree, devDesc, n, devLeaf, stream);
     if (algo == kLookupAuto)
         algo = tunedValue(kTuneLookupSchedule, mB, mL, n) == 2 ? kLookupTensorU8Ring : kLookupTensorU8;
     LookupScratch s{};

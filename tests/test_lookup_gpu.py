@@ -140,3 +140,18 @@ def test_lookup_repeated_large_batches_are_exact():
             torch.cuda.synchronize()
             assert voc.device_errors() == (0, 0)
             assert int((got != want).sum()) == 0, algo
+
+
+@pytest.mark.parametrize("B,L", [(2, 8), (3, 2), (5, 4), (9, 3), (10, 6), (12, 1), (13, 4), (16, 3), (16, 4)])
+def test_auto_lookup_matches_oracle_on_both_sides_of_the_direct_limit(oracle, B, L):
+    """Few rows go down the tree in one launch (a warp per row, ragged last block), more through
+    the tensor-core passes: the same words, ties included, and as many launches as that path has."""
+    centers, masks, weights = random_tree(B, L, seed=B + L, dup_rate=0.3)
+    voc = rbw.vocabulary_from_host(B, L, centers, masks, weights)
+    limit = 32768 if L <= 2 else 100000 if L <= 4 else 200000
+    for n in (1, 2, 3, 4, 5, 31, 733, limit, limit + 1):
+        desc = edge_descriptors(centers, n, seed=n)
+        got = _lookup(voc, desc, "auto")
+        assert (voc.last_kernels == 1) == (n <= limit or L <= 2)
+        want = oracle.lookup(centers, B, L, desc, threads=8)
+        assert np.array_equal(got, want), f"n={n}: {np.count_nonzero(got != want)} mismatches"
