@@ -381,8 +381,8 @@ enum {
                                             while those tables stay small (default), 2 one CSR */
     RBW_TUNE_LOOKUP_SCHEDULE = 4,        /* the tensor-core schedule RBW_LOOKUP_AUTO runs: 1 level
                                             pairs in two buffers (default), 2 the three-slot ring */
-    RBW_TUNE_ASSIGN_SUMS = 5             /* uint8 k-means center sums: 1 shared-memory atomics
-                                            (default), 2 a second MMA per tile (at most 4 CTAs/SM) */
+    RBW_TUNE_ASSIGN_SUMS = 5             /* 1 or 2, accepted for saved tuning files: the uint8 k-means
+                                            center sums always come from a second MMA per tile */
 };
 /* value 0 removes the entry; RBW_ERR_INVALID_ARG for a value the parameter cannot take. */
 RBW_API int rbw_tuning_set(uint32_t param, uint32_t branch_factor, uint32_t nb_levels, uint32_t bucket,

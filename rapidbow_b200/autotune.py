@@ -5,14 +5,14 @@ candidates of each tunable parameter are timed on the caller's own workload (CUD
 the library's kernels, rbw_timing_*) and the fastest is kept, per (parameter, branch factor,
 tree levels, descriptor-count bucket = floor(log2(n))):
 
-    assign_ctas_per_sm      uint8 k-means assign, CTAs per SM: 2..8         (default 6)
+    assign_ctas_per_sm      uint8 k-means assign, CTAs per SM: 2..8 (default 6; 5 fit)
     assign_f32_ctas_per_sm  float-center assign, CTAs per SM: 1..3          (default 3)
     scatter_rows            lookup regroup scatter of more than 1,024 bins, rows per thread:
                             8|16|32 (default 16)
     lookup_schedule         tensor-core lookup schedule of algo "auto": 1 level pairs in two
                             accumulator buffers, 2 the three-slot ring (default 1)
-    assign_sums             uint8 k-means center sums: 1 shared atomics, 2 a second MMA per
-                            tile (default 1; with 2 at most 4 CTAs per SM)
+    assign_sums             1 or 2, kept for saved files: the uint8 k-means center sums have one
+                            form (a second MMA per tile) whatever the value
     db_shard_tables         DataBase inverted file: 1 one CSR per 2,560-document shard while
                             small, 2 one CSR (default 1; its bucket counts documents)
 

@@ -355,43 +355,49 @@ __global__ void __launch_bounds__(kPPSample, kPPCtasPerSm) kmeansPPKernel(KMeans
 
 // ------------------------------------------------------------------ assign
 // One step handles one 128-member tile of one node (the reference's DescTile groups,
-// kmeans.cu:62-211, on the tensor core):
-//   1. the members' rows are gathered into shared memory in the 128-byte swizzled K-major layout
-//      (eight threads per row), next to the node's 16 centers in the same layout;
-//   2. one thread issues four tcgen05.mma.kind::i8 (M = 128 members, N = 16 centers, K = 4 x 32
-//      dims, u8 x u8 -> s32, exact) into this CTA's TMEM columns;
-//   3. warp w reads the dot products of rows 32w..32w+31 (its TMEM lane quarter) and takes the
-//      argmin of |c_b|^2 - 2 x.c_b, lowest index on ties (kmeans.cu:131-135), updating the
-//      assignment, the per-center counts and the changed count;
-//   4. the same warp adds its rows into the node's per-CTA center sums: lane l owns dims
-//      4l..4l+3 and adds each row's four bytes with shared atomics, the sums stored
-//      dim-interleaved so that the 32 lanes hit 32 banks.
-// Counts and sums go to global memory when the CTA moves to another node.  Several CTAs per SM
-// overlap one another's gathers, MMAs and sums.
+// kmeans.cu:62-211), both contractions on the tensor core:
+//   1. the members' rows are gathered into shared memory in the 128-byte swizzled layout (eight
+//      threads per row), next to the node's 16 centers in the same layout;
+//   2. distances: one thread issues four tcgen05.mma.kind::i8 (M = 128 members, N = 16 centers,
+//      K = 4 x 32 dims, u8 x u8 -> s32, exact) into TMEM columns [0, 16); warp w reads rows
+//      32 w .. 32 w + 31 and takes the argmin of |c_b|^2 - 2 x.c_b, lowest index on ties
+//      (kmeans.cu:131-135);
+//   3. center sums: D[dim][center] += X[member][dim] * OH[member][center] over the tile's
+//      members, four more MMAs (M = 128 dims, N = 16, K = 4 x 32 members) into columns [16, 32),
+//      accumulated over the node's tiles in this CTA.  X is the gathered tile as it lies (read
+//      MN-major: K = members), OH one 16-byte row per member, a single 1 at its center (zeros
+//      for rows past the tile's count).
+// Counts, change counts and sums go to global memory when the CTA moves to another node (or every
+// kAssignFlushTiles tiles, which keeps each s32 below 2^31: 65,536 x 128 x 255 < 2^31).
+//
+// A tile costs the SM 8 x 45 cycles of tensor pipe and its 16 KB of gathered rows, which is more
+// (0.37 us per tile at HBM speed); the wait -> MMA -> read -> MMA chain of a tile (~1 us) is hidden
+// by five CTAs per SM, each gathering its next tile while one is scored.  The 60 steps of a
+// 10M-member build (B = 10, L = 6): 18.2 ms, 0.30 ms per step against 0.20 ms to read the rows;
+// 39.6 ms with the sums by shared atomics (128 per member), 35.3 ms by MMAs over a tile
+// transposed in shared memory.
 constexpr uint32_t kAssignThreads = 128;
 constexpr uint32_t kAssignRows = 128;
-constexpr uint32_t kAssignTmemCols = 32; // the smallest allocation; the MMA writes 16 columns
-constexpr uint32_t kAssignCtasPerSm = 8; // by registers (<= 64) and shared memory; 256 TMEM columns
+constexpr uint32_t kAssignTmemCols = 32; // the smallest allocation: distances | sums
+constexpr uint32_t kAssignCtasPerSm = 5; // by shared memory (~40 KB each)
+constexpr uint32_t kAssignFlushTiles = 65536;
+constexpr uint32_t kTileWindow = kAssignThreads; // one tile entry per thread per refill
+constexpr uint32_t kTileFrozen = 0x80000000u;
 
 struct AssignSmem {
-    uint8_t tile[kAssignRows * kDims];   // member rows, 128-byte swizzle (1024-byte aligned)
-    uint8_t cen[kMaxBranch * kDims];     // node centers, same layout
-    uint32_t acc[kMaxBranch * kDims];    // center sums of the current node, see accIndex
-    int32_t cn[kMaxBranch];
+    uint8_t tile[2][kAssignRows * kDims]; // member rows, 128-byte swizzle (1024-byte aligned)
+    uint8_t cen[kMaxBranch * kDims];      // node centers, same layout
+    uint8_t oh[kAssignRows * kMaxBranch]; // [member][center] one-hot
+    NodeTile win[kTileWindow];            // tiles [winBase, winBase + kTileWindow) of the CTA's
+                                          // range, count | kTileFrozen for a frozen node
+    int32_t cnk[kMaxBranch];              // 16 |c_b|^2 + b, INT_MAX for padding slots
     uint32_t cnt[kMaxBranch];
-    uint8_t bsel[kAssignRows];
-    uint64_t mmaBar;
+    uint64_t mmaBar, sumBar;
     uint32_t tmemBase;
     uint32_t chg;
     uint32_t abortFlag;
 };
 constexpr size_t kAssignSmemBytes = sizeof(AssignSmem) + 1024;
-
-// Position of (center b, dim d = 4 l + k) in AssignSmem::acc: b * 128 + 32 k + l.
-__device__ __forceinline__ uint32_t accIndex(uint32_t b, uint32_t d)
-{
-    return b * kDims + (d & 3u) * 32u + (d >> 2);
-}
 
 __global__ void __launch_bounds__(kAssignThreads, kAssignCtasPerSm) assignKernel(KMeansLevel lv, const NodeTile* tiles,
                                                                   const uint32_t* nTilesDev)
@@ -402,190 +408,7 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignCtasPerSm) assignKernel
     const uint32_t T = *nTilesDev;
     const uint32_t t0 = static_cast<uint32_t>(uint64_t(T) * blockIdx.x / gridDim.x);
     const uint32_t t1 = static_cast<uint32_t>(uint64_t(T) * (blockIdx.x + 1) / gridDim.x);
-    volatile uint32_t* abortFlag = &S.abortFlag;
-    if (tid == 0) {
-        mbarInit(&S.mmaBar, 1);
-        S.abortFlag = 0;
-        fenceMbarInit();
-    }
-    if (warp == 0) {
-        tmemAlloc(&S.tmemBase, kAssignTmemCols);
-        tmemRelinquish();
-    }
-    tcFenceBefore();
-    __syncthreads();
-    tcFenceAfter();
-    const uint32_t tmem = S.tmemBase;
-    uint32_t curNode = 0xFFFFFFFFu, phase = 0;
-    bool curExclusive = false; // every tile of the current node is in this CTA's range
-    auto flush = [&]() {
-        __syncthreads();
-        if (curNode != 0xFFFFFFFFu) {
-            // A node no other CTA touches in this launch is written with plain stores (its
-            // global accumulators are zero on entry); a shared node is added atomically.
-            for (uint32_t i = tid; i < kMaxBranch * kDims; i += kAssignThreads) {
-                const uint32_t b = i / kDims, d = i % kDims;
-                const uint32_t v = S.acc[accIndex(b, d)];
-                unsigned long long* dst = lv.sums + (uint64_t(curNode) * kMaxBranch + b) * kDims + d;
-                if (v) {
-                    if (curExclusive) *dst = v;
-                    else atomicAdd(dst, (unsigned long long)v);
-                }
-            }
-            if (tid < kMaxBranch && S.cnt[tid]) {
-                uint32_t* dst = lv.counts + uint64_t(curNode) * kMaxBranch + tid;
-                if (curExclusive) *dst = S.cnt[tid];
-                else atomicAdd(dst, S.cnt[tid]);
-            }
-            if (tid == 0 && S.chg) {
-                if (curExclusive) lv.changed[curNode] = S.chg;
-                else atomicAdd(lv.changed + curNode, S.chg);
-            }
-        }
-        __syncthreads();
-    };
-    for (uint32_t t = t0; t < t1; t++) {
-        const NodeTile ti = tiles[t];
-        if (lv.lastChanged[ti.node] == 0) continue; // frozen node (kmeans.cu:238-240)
-        if (ti.node != curNode) {
-            flush();
-            curNode = ti.node;
-            curExclusive = ti.first >= t0 && uint64_t(ti.first) + (lv.nodeCnt[curNode] + kAssignRows - 1) / kAssignRows <= t1;
-            {
-                // thread i copies chunk i % 8 of center i / 8 (16 centers x 8 chunks)
-                const uint32_t b = tid / 8, c = tid % 8;
-                const uint4 v = reinterpret_cast<const uint4*>(lv.centers + (uint64_t(curNode) * kMaxBranch + b) * kDims)[c];
-                *reinterpret_cast<uint4*>(S.cen + b * kDims + ((c ^ (b & 7u)) << 4)) = v;
-            }
-            if (tid < kMaxBranch) {
-                S.cn[tid] = lv.cnorm[uint64_t(curNode) * kMaxBranch + tid];
-                S.cnt[tid] = 0;
-            }
-            for (uint32_t i = tid; i < kMaxBranch * kDims; i += kAssignThreads) S.acc[i] = 0;
-            if (tid == 0) S.chg = 0;
-        }
-        {
-            // eight threads per row, 16 rows per round; rows past the tile's count repeat its
-            // first member (their results are not used)
-            const uint32_t c = tid % 8;
-            uint32_t m[kAssignRows / 16];
-#pragma unroll
-            for (uint32_t k = 0; k < kAssignRows / 16; k++) {
-                const uint32_t row = 16u * k + tid / 8;
-                m[k] = lv.members[uint64_t(ti.start) + (row < ti.count ? row : 0u)];
-            }
-#pragma unroll
-            for (uint32_t k = 0; k < kAssignRows / 16; k++) {
-                const uint32_t row = 16u * k + tid / 8;
-                cpAsync16(S.tile + row * kDims + ((c ^ (row & 7u)) << 4), lv.desc + uint64_t(m[k]) * kDims + (c << 4));
-            }
-            cpAsyncCommit();
-            cpAsyncWait<0>();
-        }
-        // the copies and the center stores are generic-proxy writes read by the tensor core
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            tcFenceAfter();
-            const uint32_t aBase = smemAddr(S.tile), bBase = smemAddr(S.cen);
-#pragma unroll
-            for (uint32_t q4 = 0; q4 < 4; q4++)
-                mmaU8(tmem, smemDescSw128(aBase + 32u * q4), smemDescSw128(bBase + 32u * q4), idescU8(16),
-                      q4 > 0 ? 1u : 0u);
-            mmaCommit(&S.mmaBar);
-        }
-        if (!mbarWait(&S.mmaBar, phase, abortFlag, lv.err, 40)) break;
-        phase ^= 1u;
-        tcFenceAfter();
-        const uint32_t row = tid; // warp w reads TMEM lanes 32w .. 32w + 31
-        uint32_t r[16];
-        tmemLoad16(tmem + ((warp * 32u) << 16), r);
-        tmemWaitTie(r);
-        tcFenceBefore(); // the next step's MMA overwrites these columns after the barriers below
-        int32_t best = S.cn[0] - 2 * static_cast<int32_t>(r[0]);
-        uint32_t bi = 0;
-#pragma unroll
-        for (uint32_t b = 1; b < kMaxBranch; b++) {
-            const int32_t sc = S.cn[b] - 2 * static_cast<int32_t>(r[b]);
-            if (sc < best) {
-                best = sc;
-                bi = b;
-            }
-        }
-        if (row < ti.count) {
-            const uint64_t at = uint64_t(ti.start) + row;
-            if (lv.assign[at] != bi) atomicAdd(&S.chg, 1u);
-            lv.assign[at] = static_cast<uint8_t>(bi);
-            atomicAdd(&S.cnt[bi], 1u);
-        }
-        S.bsel[row] = static_cast<uint8_t>(bi);
-        __syncwarp();
-        const uint32_t rEnd = ti.count < 32u * warp + 32u ? ti.count : 32u * warp + 32u;
-        for (uint32_t rr = 32u * warp; rr < rEnd; rr++) {
-            const uint32_t b = S.bsel[rr];
-            const uint32_t x = *reinterpret_cast<const uint32_t*>(S.tile + rr * kDims + (((lane >> 2) ^ (rr & 7u)) << 4) +
-                                                                  ((lane & 3u) << 2));
-            uint32_t* a = S.acc + b * kDims + lane;
-            atomicAdd(a, x & 0xFFu);
-            atomicAdd(a + 32, (x >> 8) & 0xFFu);
-            atomicAdd(a + 64, (x >> 16) & 0xFFu);
-            atomicAdd(a + 96, x >> 24);
-        }
-        __syncthreads(); // the tile and bsel are rewritten by the next step
-    }
-    flush();
-    if (warp == 0) {
-        tcFenceAfter();
-        tmemDealloc(tmem, kAssignTmemCols);
-    }
-}
-
-// ------------------------------------------------------------------ assign, sums on the tensor core
-// The same assignment as assignKernel; the center sums come from a second MMA per tile instead of
-// 128 shared atomics per member: D[dim][center] += XT[dim][member] * OH[center][member], with XT
-// the tile transposed in shared memory (4 x 4 byte blocks through byte permutes) and OH the
-// one-hot of the members' centers built from ballots.  Both operands are K-major with K =
-// members, u8 x u8 -> s32 (exact); D lives in TMEM columns [16, 32) and accumulates over the
-// node's tiles in this CTA, read and written out when the CTA moves to another node (or every
-// kTsFlushTiles tiles, which keeps each s32 below 2^31: 65,536 x 128 x 255 < 2^31).
-constexpr uint32_t kAssignTsCtasPerSm = 4;     // by shared memory (~54 KB each)
-constexpr uint32_t kTsFlushTiles = 65536;
-constexpr uint32_t kTsTileWindow = kAssignThreads; // one tile entry per thread per refill
-constexpr uint32_t kTsFrozen = 0x80000000u;
-
-struct AssignTsSmem {
-    uint8_t tile[2][kAssignRows * kDims]; // member rows, K-major (dims), 128-byte swizzle; the
-                                          // next tile's rows are gathered while this one is scored
-    uint8_t xt[kDims * kAssignRows];     // the rows transposed: [dim][member], same layout
-    uint8_t oh[kMaxBranch * kAssignRows]; // [center][member]: 1 where the member chose the center
-    uint8_t cen[kMaxBranch * kDims];     // node centers
-    NodeTile win[kTsTileWindow];         // tiles [winBase, winBase + kTsTileWindow) of the CTA's
-                                         // range, count | kTsFrozen for a frozen node
-    int32_t cn[kMaxBranch];
-    uint32_t cnt[kMaxBranch];
-    uint64_t mmaBar, sumBar;
-    uint32_t tmemBase;
-    uint32_t chg;
-    uint32_t abortFlag;
-};
-constexpr size_t kAssignTsSmemBytes = sizeof(AssignTsSmem) + 1024;
-
-// Byte (row, col) of a 128-column, 128-byte-swizzled K-major operand.
-__device__ __forceinline__ uint32_t sw128(uint32_t row, uint32_t col)
-{
-    return row * 128u + ((((col >> 4) ^ row) & 7u) << 4) + (col & 15u);
-}
-
-__global__ void __launch_bounds__(kAssignThreads, kAssignTsCtasPerSm)
-    assignKernelTs(KMeansLevel lv, const NodeTile* tiles, const uint32_t* nTilesDev)
-{
-    extern __shared__ uint8_t smemRaw[];
-    AssignTsSmem& S =
-        *reinterpret_cast<AssignTsSmem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
-    const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    const uint32_t T = *nTilesDev;
-    const uint32_t t0 = static_cast<uint32_t>(uint64_t(T) * blockIdx.x / gridDim.x);
-    const uint32_t t1 = static_cast<uint32_t>(uint64_t(T) * (blockIdx.x + 1) / gridDim.x);
+    if (t0 == t1) return; // uniform: fewer tiles than CTAs
     volatile uint32_t* abortFlag = &S.abortFlag;
     if (tid == 0) {
         mbarInit(&S.mmaBar, 1);
@@ -602,8 +425,10 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignTsCtasPerSm)
     tcFenceAfter();
     const uint32_t tmem = S.tmemBase;
     uint32_t curNode = 0xFFFFFFFFu, phase = 0, sumPhase = 0, accTiles = 0, buf = 0;
-    bool curExclusive = false, sumInFlight = false, ok = true;
-    // The tile list and the frozen flags are read a window of kTsTileWindow tiles at a time (one
+    uint32_t myCnt = 0, myChg = 0; // lane c < 16: members of this warp's rows that chose center c
+    bool curExclusive = false;     // every tile of the current node is in this CTA's range
+    bool ok = true;
+    // The tile list and the frozen flags are read a window of kTileWindow tiles at a time (one
     // load per thread, all in flight together), so that finding the next live tile costs no
     // global round trip; the member indices of the next tile are loaded into registers one
     // tile ahead of its row copies.  Every thread runs the same window refills (uniform).
@@ -612,20 +437,20 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignTsCtasPerSm)
         __syncthreads(); // nobody reads the old window any more
         if (base + tid < t1) {
             NodeTile x = tiles[base + tid];
-            if (lv.lastChanged[x.node] == 0) x.count |= kTsFrozen; // frozen node (kmeans.cu:238-240)
+            if (lv.lastChanged[x.node] == 0) x.count |= kTileFrozen; // frozen node (kmeans.cu:238-240)
             S.win[tid] = x;
         }
         winBase = base;
         __syncthreads();
     };
     auto entry = [&](uint32_t t) -> NodeTile {
-        if (t - winBase >= kTsTileWindow) refill(t);
+        if (t - winBase >= kTileWindow) refill(t);
         return S.win[t - winBase];
     };
     // the first live tile at or after t, or t1
     auto nextLive = [&](uint32_t t) -> uint32_t {
         for (; t < t1; t++)
-            if (!(entry(t).count & kTsFrozen)) return t;
+            if (!(entry(t).count & kTileFrozen)) return t;
         return t1;
     };
     auto loadIndices = [&](const NodeTile& tn, uint32_t (&m)[kAssignRows / 16]) {
@@ -646,23 +471,23 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignTsCtasPerSm)
         }
         cpAsyncCommit();
     };
-    auto waitSums = [&]() {
-        if (!sumInFlight) return;
-        ok = ok && mbarWait(&S.sumBar, sumPhase, abortFlag, lv.err, 42);
-        sumPhase ^= 1u;
-        sumInFlight = false;
-        tcFenceAfter();
-    };
     // writes the node's partial sums (TMEM), counts and change count
     auto flush = [&]() {
-        __syncthreads();
         if (curNode != 0xFFFFFFFFu) {
+            if (lane < kMaxBranch && myCnt) atomicAdd(&S.cnt[lane], myCnt);
+            if (lane == 0 && myChg) atomicAdd(&S.chg, myChg);
             if (accTiles > 0) {
-                waitSums();
+                // the last sums MMA was issued by thread 0; nothing was committed for it yet
+                if (tid == 0) mmaCommit(&S.sumBar);
+                ok = ok && mbarWait(&S.sumBar, sumPhase, abortFlag, lv.err, 42);
+                sumPhase ^= 1u;
+                tcFenceAfter();
                 uint32_t r[16];
                 tmemLoad16(tmem + 16u + ((warp * 32u) << 16), r); // lane = dimension tid
                 tmemWaitTie(r);
                 tcFenceBefore();
+                // A node no other CTA touches in this launch is written with plain stores (its
+                // global accumulators are zero on entry); a shared node is added atomically.
 #pragma unroll
                 for (uint32_t b = 0; b < kMaxBranch; b++) {
                     if (r[b] == 0) continue;
@@ -671,6 +496,7 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignTsCtasPerSm)
                     else atomicAdd(dst, (unsigned long long)r[b]);
                 }
             }
+            __syncthreads(); // S.cnt and S.chg complete
             if (tid < kMaxBranch && S.cnt[tid]) {
                 uint32_t* dst = lv.counts + uint64_t(curNode) * kMaxBranch + tid;
                 if (curExclusive) *dst = S.cnt[tid];
@@ -682,9 +508,11 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignTsCtasPerSm)
             }
         }
         accTiles = 0;
+        myCnt = 0;
+        myChg = 0;
         __syncthreads();
     };
-    if (t0 < t1) refill(t0);
+    refill(t0);
     uint32_t t = nextLive(t0);
     NodeTile ti{}, tn1{};
     uint32_t mNext[kAssignRows / 16];
@@ -704,49 +532,36 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignTsCtasPerSm)
             curNode = ti.node;
             curExclusive = ti.first >= t0 && uint64_t(ti.first) + (lv.nodeCnt[curNode] + kAssignRows - 1) / kAssignRows <= t1;
             {
+                // thread i copies chunk i % 8 of center i / 8 (16 centers x 8 chunks)
                 const uint32_t b = tid / 8, c = tid % 8;
                 const uint4 v = reinterpret_cast<const uint4*>(lv.centers + (uint64_t(curNode) * kMaxBranch + b) * kDims)[c];
                 *reinterpret_cast<uint4*>(S.cen + b * kDims + ((c ^ (b & 7u)) << 4)) = v;
             }
             if (tid < kMaxBranch) {
-                S.cn[tid] = lv.cnorm[uint64_t(curNode) * kMaxBranch + tid];
+                S.cnk[tid] = tid < lv.B ? lv.cnorm[uint64_t(curNode) * kMaxBranch + tid] * 16 + int32_t(tid) : 0x7FFFFFFF;
                 S.cnt[tid] = 0;
             }
             if (tid == 0) S.chg = 0;
-        } else if (accTiles == kTsFlushTiles) {
+        } else if (accTiles == kAssignFlushTiles) {
             // keep each s32 sum below 2^31: add this node's partial results to global memory and
             // go on from zero (its later flushes add too)
             curExclusive = false;
             flush();
             if (tid < kMaxBranch) S.cnt[tid] = 0;
             if (tid == 0) S.chg = 0;
-            __syncthreads();
         }
-        // the next live tile's rows go into the other buffer (its indices were loaded one tile
-        // ago), the indices of the one after it into registers; then this tile's rows must be in
-        uint32_t n2 = t1;
-        NodeTile tn2{};
-        if (n1 < t1) {
-            gatherRows(mNext, buf ^ 1u);
-            n2 = nextLive(n1 + 1);
-            if (n2 < t1) {
-                tn2 = entry(n2);
-                loadIndices(tn2, mNext);
-            }
-            cpAsyncWait<1>();
-        } else {
-            cpAsyncWait<0>();
-        }
-        const uint32_t row = tid;
+        const uint32_t row = tid; // warp w reads TMEM lanes 32w .. 32w + 31
         const bool valid = row < ti.count;
         const uint64_t at = uint64_t(ti.start) + row;
         const uint32_t prevAssign = valid ? lv.assign[at] : 0u;
+        cpAsyncWait<0>(); // this tile's rows
+        // the copies, the center stores and the one-hot rows are generic-proxy writes read by the
+        // tensor core
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        const uint8_t* tileBuf = S.tile[buf];
         if (tid == 0) {
             tcFenceAfter();
-            const uint32_t aBase = smemAddr(tileBuf), bBase = smemAddr(S.cen);
+            const uint32_t aBase = smemAddr(S.tile[buf]), bBase = smemAddr(S.cen);
 #pragma unroll
             for (uint32_t q4 = 0; q4 < 4; q4++)
                 mmaU8(tmem, smemDescSw128(aBase + 32u * q4), smemDescSw128(bBase + 32u * q4), idescU8(16),
@@ -759,79 +574,57 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignTsCtasPerSm)
         }
         phase ^= 1u;
         tcFenceAfter();
+        // The commit also covers the previous tile's sums MMAs: the other tile buffer and the
+        // one-hot rows are free.  The next live tile's rows go into that buffer (its indices were
+        // loaded one tile ago), the indices of the one after it into registers.
+        uint32_t n2 = t1;
+        NodeTile tn2{};
+        if (n1 < t1) {
+            gatherRows(mNext, buf ^ 1u);
+            n2 = nextLive(n1 + 1);
+            if (n2 < t1) {
+                tn2 = entry(n2);
+                loadIndices(tn2, mNext);
+            }
+        }
         uint32_t r[16];
         tmemLoad16(tmem + ((warp * 32u) << 16), r);
         tmemWaitTie(r);
-        tcFenceBefore();
-        int32_t best = S.cn[0] - 2 * static_cast<int32_t>(r[0]);
-        uint32_t bi = 0;
+        tcFenceBefore(); // the next tile's MMA overwrites these columns after the barriers below
+        // |c|^2 - 2 x.c lies in (-2^24, 2^23]: 16 times it plus the center fits 32 bits, and the
+        // minimum is the lowest center of the lowest score
+        int32_t best = 0x7FFFFFFF;
 #pragma unroll
-        for (uint32_t b = 1; b < kMaxBranch; b++) {
-            const int32_t sc = S.cn[b] - 2 * static_cast<int32_t>(r[b]);
-            if (sc < best) {
-                best = sc;
-                bi = b;
-            }
-        }
-        if (valid) {
-            if (prevAssign != bi) atomicAdd(&S.chg, 1u);
-            lv.assign[at] = static_cast<uint8_t>(bi);
-            atomicAdd(&S.cnt[bi], 1u);
-        }
-        // the previous tile's sums MMA must be done reading xt and oh before they are rewritten
-        waitSums();
-        if (!ok) break;
-        // one-hot: lane c writes row c's 32 bytes of this warp's members (bit i = member 32 w + i)
-        uint32_t mine = 0;
-#pragma unroll
-        for (uint32_t c = 0; c < kMaxBranch; c++) {
-            const uint32_t bits = __ballot_sync(0xFFFFFFFFu, valid && bi == c);
-            if (lane == c) mine = bits;
-        }
-        if (lane < kMaxBranch) {
-#pragma unroll
-            for (uint32_t half = 0; half < 2; half++) {
-                uint32_t w4[4];
-#pragma unroll
-                for (uint32_t q = 0; q < 4; q++) {
-                    const uint32_t nib = (mine >> (16u * half + 4u * q)) & 0xFu;
-                    w4[q] = (nib & 1u) | ((nib & 2u) << 7) | ((nib & 4u) << 14) | ((nib & 8u) << 21);
-                }
-                const uint32_t col = 32u * warp + 16u * half;
-                *reinterpret_cast<uint4*>(S.oh + sw128(lane, col)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-            }
-        }
-        // transpose this warp's 32 rows into xt columns 32 w .. 32 w + 31, 4 x 4 byte blocks:
-        // lane = (dimension quad dq0 = lane / 8, member quad mq = lane % 8), eight dimension quads
+        for (uint32_t b = 0; b < kMaxBranch; b++) best = min(best, S.cnk[b] - 32 * static_cast<int32_t>(r[b]));
+        const uint32_t bi = static_cast<uint32_t>(best) & 15u;
+        if (valid) lv.assign[at] = static_cast<uint8_t>(bi);
         {
-            const uint32_t m0 = 32u * warp + 4u * (lane & 7u);
+            const uint32_t word = valid ? 1u << (8u * (bi & 3u)) : 0u;
+            const uint32_t q = bi >> 2;
+            *reinterpret_cast<uint4*>(S.oh + row * kMaxBranch) =
+                make_uint4(q == 0 ? word : 0u, q == 1 ? word : 0u, q == 2 ? word : 0u, q == 3 ? word : 0u);
+        }
+        {
+            const uint32_t live = __ballot_sync(0xFFFFFFFFu, valid);
+            uint32_t mask = live;
 #pragma unroll
-            for (uint32_t k = 0; k < 8; k++) {
-                const uint32_t d0 = 4u * ((lane >> 3) + 4u * k);
-                const uint32_t w0 = *reinterpret_cast<const uint32_t*>(tileBuf + sw128(m0, d0));
-                const uint32_t w1 = *reinterpret_cast<const uint32_t*>(tileBuf + sw128(m0 + 1, d0));
-                const uint32_t w2 = *reinterpret_cast<const uint32_t*>(tileBuf + sw128(m0 + 2, d0));
-                const uint32_t w3 = *reinterpret_cast<const uint32_t*>(tileBuf + sw128(m0 + 3, d0));
-                const uint32_t a = __byte_perm(w0, w1, 0x5140), b = __byte_perm(w2, w3, 0x5140);
-                const uint32_t c = __byte_perm(w0, w1, 0x7362), d = __byte_perm(w2, w3, 0x7362);
-                *reinterpret_cast<uint32_t*>(S.xt + sw128(d0, m0)) = __byte_perm(a, b, 0x5410);
-                *reinterpret_cast<uint32_t*>(S.xt + sw128(d0 + 1, m0)) = __byte_perm(a, b, 0x7632);
-                *reinterpret_cast<uint32_t*>(S.xt + sw128(d0 + 2, m0)) = __byte_perm(c, d, 0x5410);
-                *reinterpret_cast<uint32_t*>(S.xt + sw128(d0 + 3, m0)) = __byte_perm(c, d, 0x7632);
+            for (uint32_t k = 0; k < 4; k++) {
+                const uint32_t bits = __ballot_sync(0xFFFFFFFFu, (bi >> k) & 1u);
+                mask &= (lane >> k) & 1u ? bits : ~bits;
             }
+            myCnt += __popc(mask); // used of lanes below kMaxBranch
+            myChg += __popc(__ballot_sync(0xFFFFFFFFu, valid && prevAssign != bi));
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads(); // xt, oh complete; the tile is rewritten by the next gather
+        __syncthreads(); // every row's one-hot is in, every warp has read its distances
         if (tid == 0) {
             tcFenceAfter();
-            const uint32_t aBase = smemAddr(S.xt), bBase = smemAddr(S.oh);
+            const uint32_t aBase = smemAddr(S.tile[buf]), bBase = smemAddr(S.oh);
 #pragma unroll
             for (uint32_t q4 = 0; q4 < 4; q4++)
-                mmaU8(tmem + 16u, smemDescSw128(aBase + 32u * q4), smemDescSw128(bBase + 32u * q4), idescU8(16),
-                      (accTiles > 0 || q4 > 0) ? 1u : 0u);
-            mmaCommit(&S.sumBar);
+                mmaU8(tmem + 16u, smemDescSw128(aBase + 4096u * q4), smemDescMn16(bBase + 512u * q4),
+                      idescU8(16) | kIdescMnMajorAB, (accTiles > 0 || q4 > 0) ? 1u : 0u);
         }
-        sumInFlight = true;
         accTiles++;
         buf ^= 1u;
         t = n1;
@@ -840,8 +633,14 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignTsCtasPerSm)
         tn1 = tn2;
     }
     cpAsyncWait<0>(); // a prefetch of a tile that was not scored (abort) must land before exit
-    if (ok) flush();
-    else waitSums();
+    if (ok) {
+        flush();
+    } else {
+        // MMAs may still be in flight: the TMEM is freed after them (a bounded wait)
+        if (tid == 0) mmaCommit(&S.sumBar);
+        mbarWait(&S.sumBar, sumPhase, abortFlag, lv.err, 43);
+        __syncthreads();
+    }
     if (warp == 0) {
         tcFenceAfter();
         tmemDealloc(tmem, kAssignTmemCols);
@@ -981,22 +780,15 @@ void launchAssign(const KMeansLevel& lv, const NodeTile* tiles, const uint32_t* 
     RBW_CUDA(cudaGetDevice(&dev));
     RBW_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     // A fixed grid (the occupancy query gave one CTA per SM on some launches, 3-4x slower) of
-    // up to kAssignCtasPerSm CTAs per SM, the count the autotuner chose for this workload.
+    // up to kAssignCtasPerSm CTAs per SM, or fewer where the autotuner chose so for this workload.
     static_assert(kAssignCtasPerSm * kAssignTmemCols <= 512, "TMEM columns of the resident CTAs");
-    static_assert(kAssignCtasPerSm * kAssignSmemBytes <= 227 * 1024, "shared memory of the resident CTAs");
-    static_assert(kAssignTsCtasPerSm * kAssignTsSmemBytes <= 227 * 1024, "shared memory of the resident CTAs");
-    const bool tensorSums = tunedValue(kTuneAssignSums, lv.B, 0, lv.nbMembers) == 2;
-    const uint32_t cap = tensorSums ? kAssignTsCtasPerSm : kAssignCtasPerSm;
-    const uint32_t perSm = std::min(cap, tunedValue(kTuneAssignCtasPerSm, lv.B, 0, lv.nbMembers));
+    static_assert(kAssignCtasPerSm * (kAssignSmemBytes + 1024) <= 228 * 1024, "shared memory of the resident CTAs");
+    const uint32_t perSm = std::min(kAssignCtasPerSm, tunedValue(kTuneAssignCtasPerSm, lv.B, 0, lv.nbMembers));
     const uint32_t grid = std::max(1u, std::min<uint32_t>(maxTiles, static_cast<uint32_t>(sms) * perSm));
     ScopedKernelTimer timer(kTimedAssign, s);
-    if (tensorSums) {
-        static std::atomic<uint64_t> attr{0};
-        setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(assignKernelTs), int(kAssignTsSmemBytes), attr);
-        assignKernelTs<<<grid, kAssignThreads, kAssignTsSmemBytes, s>>>(lv, tiles, nTilesDev);
-    } else {
-        assignKernel<<<grid, kAssignThreads, kAssignSmemBytes, s>>>(lv, tiles, nTilesDev);
-    }
+    static std::atomic<uint64_t> attr{0};
+    setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(assignKernel), int(kAssignSmemBytes), attr);
+    assignKernel<<<grid, kAssignThreads, kAssignSmemBytes, s>>>(lv, tiles, nTilesDev);
     RBW_CUDA(cudaGetLastError());
 }
 

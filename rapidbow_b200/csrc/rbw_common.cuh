@@ -299,6 +299,23 @@ __device__ __forceinline__ uint64_t smemDescSw128(uint32_t addr)
     return d;
 }
 
+// Shared-memory matrix descriptor of an MN-major operand 16 bytes wide (N = 16 elements of one
+// byte) without swizzle: K rows of 16 bytes back to back, core matrices of 8 rows 128 B apart
+// (LBO; SBO would step along N, unused), descriptor version 1, layout type 0.
+__device__ __forceinline__ uint64_t smemDescMn16(uint32_t addr)
+{
+    uint64_t d = 0;
+    d |= uint64_t((addr >> 4) & 0x3FFFu);
+    d |= uint64_t(128u >> 4) << 16;       // LBO (16 B units)
+    d |= uint64_t(128u >> 4) << 32;       // SBO (16 B units)
+    d |= uint64_t(1u) << 46;              // version
+    return d;
+}
+// Both operands MN-major (bits 15 and 16 of the instruction descriptor).  A 128-byte-swizzled
+// tile of 128-byte rows read this way has M = its 128 columns and K = its rows: smemDescSw128
+// describes it too (SBO = 1024 B steps eight rows along K), advanced by 4,096 B per K = 32.
+constexpr uint32_t kIdescMnMajorAB = (1u << 15) | (1u << 16);
+
 // Instruction descriptor (M = 128, K-major A and B, uint8 x uint8 -> s32).
 __host__ __device__ constexpr uint32_t idescU8(uint32_t n)
 {

@@ -109,3 +109,15 @@ def test_build_rejects_bad_input():
     with pytest.raises(rbw.RbwError) as e:
         rbw.build_vocabulary(d, 17, nb_doc=1, nb_levels=2)
     assert e.value.status == rbw.RBW_ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("B,n", [(2, 127), (3, 128), (16, 129), (10, 255), (16, 257), (7, 94_721), (16, 189_440 + 33)])
+def test_build_tile_edges_match_oracle(oracle, B, n):
+    """Nodes of one tile, one row more or less, and one node over every CTA (one and two tiles per
+    CTA of five on each SM, ragged): assignment, change counts and center sums of the two MMAs."""
+    desc = sift_like(n, seed=n).numpy()
+    for level_members in (desc, np.repeat(desc[: max(B, n // 50)], 7, axis=0)):  # distinct, duplicated rows
+        voc = rbw.build_vocabulary(torch.from_numpy(np.ascontiguousarray(level_members)).cuda(), B, nb_doc=50,
+                                   nb_levels=2, init="kmeans++", seed=4, max_iterations=6, ieee_division=True)
+        ref = oracle.build_vocabulary(level_members, 50, B, 2, max_iter=6, init=INIT_KMEANSPP, seed=4)
+        _tree_equal(voc, ref)
