@@ -23,8 +23,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden", "-I", INCLUDE, "-I", CSRC]
 # Per-file extra flags: the center update must divide exactly like the reference's
 # --use_fast_math kernels.
-EXTRA = {"kmeans_update.cu": ["--use_fast_math"]}
-SOURCES = ["lookup.cu", "kmeans.cu", "kmeans_update.cu", "kmeans_f32.cu", "vocabulary.cu", "database.cu", "capi.cpp", "facade.cpp",
+EXTRA = {"kmeans_update.cu": ["--use_fast_math"], "kmeans_lloyd.cu": ["--use_fast_math"]}
+SOURCES = ["lookup.cu", "kmeans.cu", "kmeans_update.cu", "kmeans_lloyd.cu", "kmeans_f32.cu", "vocabulary.cu", "database.cu", "capi.cpp", "facade.cpp",
            "timing.cpp", "noalloc.cu", "server.cpp", "tuning.cpp", "kmeans_shard.cu"]
 
 

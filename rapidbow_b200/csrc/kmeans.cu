@@ -404,7 +404,8 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignCtasPerSm) assignKernel
 {
     extern __shared__ uint8_t smemRaw[];
     AssignSmem& S = *reinterpret_cast<AssignSmem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
-    const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const uint32_t tid = threadIdx.x, lane = tid % 32;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid / 32, 0); // uniform
     const uint32_t T = *nTilesDev;
     const uint32_t t0 = static_cast<uint32_t>(uint64_t(T) * blockIdx.x / gridDim.x);
     const uint32_t t1 = static_cast<uint32_t>(uint64_t(T) * (blockIdx.x + 1) / gridDim.x);
@@ -424,6 +425,7 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignCtasPerSm) assignKernel
     __syncthreads();
     tcFenceAfter();
     const uint32_t tmem = S.tmemBase;
+    const bool issuer = warp == 0 && electOne(); // one thread issues and commits every MMA
     uint32_t curNode = 0xFFFFFFFFu, phase = 0, sumPhase = 0, accTiles = 0, buf = 0;
     uint32_t myCnt = 0, myChg = 0; // lane c < 16: members of this warp's rows that chose center c
     bool curExclusive = false;     // every tile of the current node is in this CTA's range
@@ -477,8 +479,8 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignCtasPerSm) assignKernel
             if (lane < kMaxBranch && myCnt) atomicAdd(&S.cnt[lane], myCnt);
             if (lane == 0 && myChg) atomicAdd(&S.chg, myChg);
             if (accTiles > 0) {
-                // the last sums MMA was issued by thread 0; nothing was committed for it yet
-                if (tid == 0) mmaCommit(&S.sumBar);
+                // nothing was committed yet for the last sums MMA
+                if (issuer) mmaCommit(&S.sumBar);
                 ok = ok && mbarWait(&S.sumBar, sumPhase, abortFlag, lv.err, 42);
                 sumPhase ^= 1u;
                 tcFenceAfter();
@@ -559,14 +561,11 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignCtasPerSm) assignKernel
         // tensor core
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0) {
             tcFenceAfter();
-            const uint32_t aBase = smemAddr(S.tile[buf]), bBase = smemAddr(S.cen);
-#pragma unroll
-            for (uint32_t q4 = 0; q4 < 4; q4++)
-                mmaU8(tmem, smemDescSw128(aBase + 32u * q4), smemDescSw128(bBase + 32u * q4), idescU8(16),
-                      q4 > 0 ? 1u : 0u);
-            mmaCommit(&S.mmaBar);
+            mmaU8x4(issuer, tmem, smemDescSw128(smemAddr(S.tile[buf])), 32u, smemDescSw128(smemAddr(S.cen)), 32u,
+                    idescU8(16), 0u);
+            if (issuer) mmaCommit(&S.mmaBar);
         }
         if (!mbarWait(&S.mmaBar, phase, abortFlag, lv.err, 41)) {
             ok = false;
@@ -617,13 +616,10 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignCtasPerSm) assignKernel
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads(); // every row's one-hot is in, every warp has read its distances
-        if (tid == 0) {
+        if (warp == 0) {
             tcFenceAfter();
-            const uint32_t aBase = smemAddr(S.tile[buf]), bBase = smemAddr(S.oh);
-#pragma unroll
-            for (uint32_t q4 = 0; q4 < 4; q4++)
-                mmaU8(tmem + 16u, smemDescSw128(aBase + 4096u * q4), smemDescMn16(bBase + 512u * q4),
-                      idescU8(16) | kIdescMnMajorAB, (accTiles > 0 || q4 > 0) ? 1u : 0u);
+            mmaU8x4(issuer, tmem + 16u, smemDescSw128(smemAddr(S.tile[buf])), 4096u, smemDescMn16(smemAddr(S.oh)), 512u,
+                    idescU8(16) | kIdescMnMajorAB, accTiles);
         }
         accTiles++;
         buf ^= 1u;
@@ -637,7 +633,7 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignCtasPerSm) assignKernel
         flush();
     } else {
         // MMAs may still be in flight: the TMEM is freed after them (a bounded wait)
-        if (tid == 0) mmaCommit(&S.sumBar);
+        if (issuer) mmaCommit(&S.sumBar);
         mbarWait(&S.sumBar, sumPhase, abortFlag, lv.err, 43);
         __syncthreads();
     }

@@ -62,6 +62,26 @@ void launchAssign(const KMeansLevel& lv, const NodeTile* tiles, const uint32_t* 
 // changed, activeCount = number of nodes updated.
 void launchUpdate(const KMeansLevel& lv, cudaStream_t s);
 
+// Nodes small enough to stay in shared memory run their whole Lloyd loop in one CTA
+// (lloydResidentKernel), in classes by the 128-member tiles they need; larger ones are streamed by
+// launchAssign / launchUpdate in every step.
+constexpr uint32_t kLloydClasses = 4;
+__host__ __device__ constexpr uint32_t lloydTiles(uint32_t c) { return c == 0 ? 1u : c == 1 ? 2u : c == 2 ? 6u : 12u; }
+constexpr uint32_t kLloydCursor = kLloydClasses + 1;        // counters: nodes per class, streamed nodes,
+constexpr uint32_t kLloydMaxSteps = 2 * kLloydClasses + 1;  // the classes' work cursors, most steps run
+constexpr uint32_t kLloydCounters = 2 * kLloydClasses + 2;
+struct LloydClasses {
+    uint32_t* lists;     // [kLloydClasses][nbNodes] nodes of each class
+    uint32_t* counters;  // [kLloydCounters], zero on entry
+    uint32_t* streamCnt; // [nbNodes] members of streamed nodes, 0 for all others
+};
+// Fills the lists and counters, and lastChanged (0 for nodes that are not streamed).
+void launchClassifyNodes(const KMeansLevel& lv, const LloydClasses& cls, cudaStream_t s);
+// Every resident node's Lloyd loop: assign, centers, cnorm and counters[kLloydMaxSteps].
+// hostCounts: counters[0, kLloydClasses) on the host (grid sizes; empty classes are not launched).
+void launchLloydResident(const KMeansLevel& lv, const LloydClasses& cls, const uint32_t* hostCounts,
+                         uint32_t maxIterations, cudaStream_t s);
+
 // ------------------------------------------------------------------ float-center mode
 // fp32 centers (the FP64 quotient of the exact integer sums, rounded once), distances from the
 // tensor core in bf16 with each center split into hi + lo bf16 parts and fp32 accumulation, and

@@ -1,0 +1,365 @@
+// Lloyd loops of small nodes, whole in one CTA: the node's rows stay in shared memory from its
+// first assignment to its last center update (kmeans.cpp:118-133, kmeans.cu:62-384).  This
+// translation unit is compiled with --use_fast_math like kmeans_update.cu, so that
+// float(sum) / float(count) is the reference's quotient (kmeans.cu:367); everything else here is
+// integer arithmetic.
+#include "kmeans.cuh"
+#include "timing.h"
+
+#include <algorithm>
+
+namespace rbw {
+namespace {
+
+constexpr uint32_t kRows = 128;     // members per tile
+constexpr uint32_t kTileBytes = kRows * kDims;
+constexpr uint32_t kOneHotBytes = kRows * kMaxBranch;
+
+// Sorts the level's nodes by the room they need: lists of nodes of at most lloydTiles(c) tiles
+// for each resident class c, and streamCnt / lastChanged for the nodes that stay with the
+// streaming assign (0 members, frozen, for all others).
+__global__ void __launch_bounds__(256) classifyNodesKernel(const uint32_t* nodeCnt, uint32_t nbNodes,
+                                                           LloydClasses cls, uint32_t* lastChanged)
+{
+    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    const uint32_t n = g < nbNodes ? nodeCnt[g] : 0u;
+    uint32_t c = kLloydClasses + 1; // empty: nothing to do
+    if (n > 0) {
+        c = kLloydClasses;          // streamed
+#pragma unroll
+        for (uint32_t k = kLloydClasses; k-- > 0;)
+            if (n <= lloydTiles(k) * kRows) c = k;
+    }
+    if (g < nbNodes) {
+        cls.streamCnt[g] = c == kLloydClasses ? n : 0u;
+        lastChanged[g] = c == kLloydClasses ? 0xFFFFFFFFu : 0u;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k <= kLloydClasses; k++) {
+        const uint32_t mask = __ballot_sync(0xFFFFFFFFu, c == k);
+        if (mask == 0) continue;
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(cls.counters + k, uint32_t(__popc(mask)));
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        if (k < kLloydClasses && c == k) cls.lists[uint64_t(k) * nbNodes + base + __popc(mask & ((1u << lane) - 1u))] = g;
+    }
+}
+
+// One CTA per node at a time, kTiles x 128 rows of shared memory, kGroups groups of 128 threads.
+// Per step:
+//   1. group q takes tiles q, q + kGroups, ...: its first warp issues their distance MMAs (M = 128
+//      members, N = 16 centers, see assignKernel), one commit per tile;
+//   2. a thread per row takes the argmin of |c|^2 - 2 x.c (lowest center on ties) and writes the
+//      row's one-hot; then the group's first warp issues the tile's sums MMAs (A = the tile read
+//      MN-major) into the group's own 16 TMEM columns;
+//   3. the thread of dimension d adds the groups' sums and writes the new byte of each center
+//      with members (kmeans.cu:356-372), and the norms follow by warp sums.
+// A node stops after the step that changes no assignment (kmeans.cu:238-240, 341-343).
+//
+// The streaming assign reads a node's rows from memory in every step and passes its sums through
+// global memory to the update; for nodes of about 100 members those sums are as many bytes as the
+// rows.  Here a step is bound by its chain (MMA -> argmin -> MMA -> update, ~2 us) with as many
+// nodes in flight per SM as fit.
+template <uint32_t kTiles, uint32_t kGroups>
+struct LloydSmem {
+    uint8_t tile[kTiles][kTileBytes];  // member rows, 128-byte swizzle
+    uint8_t cen[kMaxBranch * kDims];   // centers, same layout
+    uint8_t oh[kTiles][kOneHotBytes];  // [member][center] one-hot
+    int32_t cnk[kMaxBranch];           // 16 |c_b|^2 + b, INT_MAX for padding slots
+    uint32_t cnt[kMaxBranch];
+    uint32_t normPart[4][kMaxBranch];
+    uint64_t distBar[kTiles];
+    uint64_t sumBar;
+    uint32_t tmemBase, abortFlag, chg, slot;
+};
+template <uint32_t kTiles, uint32_t kGroups>
+constexpr size_t lloydSmemBytes() { return sizeof(LloydSmem<kTiles, kGroups>) + 1024; }
+
+template <uint32_t kTiles, uint32_t kGroups>
+__host__ __device__ constexpr uint32_t lloydTmemCols()
+{
+    const uint32_t need = 16 * (kTiles + kGroups);
+    return need <= 32 ? 32 : need <= 64 ? 64 : need <= 128 ? 128 : 256;
+}
+
+// 32 lanes x N columns of 32-bit accumulators, waited for.
+template <uint32_t N>
+__device__ __forceinline__ void tmemLoadN(uint32_t taddr, uint32_t (&r)[N])
+{
+    if constexpr (N == 16) {
+        tmemLoad16(taddr, r);
+        tmemWaitTie(r);
+    } else if constexpr (N == 8) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+                     "tcgen05.wait::ld.sync.aligned;"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr)
+                     : "memory");
+    } else {
+        static_assert(N == 4, "4, 8 or 16 columns");
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n\t"
+                     "tcgen05.wait::ld.sync.aligned;"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(taddr)
+                     : "memory");
+    }
+}
+
+// Barrier of one group's 128 threads.  Barrier numbers are constants: with a number in a register
+// the compiler reserves all 16 of the CTA, and an SM has barriers for four such CTAs only.
+template <uint32_t kGroups>
+__device__ __forceinline__ void groupBarrier(uint32_t group)
+{
+    static_assert(kGroups == 1 || kGroups == 2 || kGroups == 4, "one, two or four groups");
+    if (kGroups == 1 || group == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+    else if (kGroups == 2 || group == 1) asm volatile("bar.sync 2, 128;" ::: "memory");
+    else if (group == 2) asm volatile("bar.sync 3, 128;" ::: "memory");
+    else asm volatile("bar.sync 4, 128;" ::: "memory");
+}
+
+template <uint32_t kTiles, uint32_t kGroups, uint32_t kCtasPerSm>
+__global__ void __launch_bounds__(kRows * kGroups, kCtasPerSm)
+    lloydResidentKernel(KMeansLevel lv, const uint32_t* list, const uint32_t* listCount, uint32_t* cursor,
+                        uint32_t maxIterations, uint32_t* maxSteps)
+{
+    using Smem = LloydSmem<kTiles, kGroups>;
+    constexpr uint32_t kThreads = kRows * kGroups;
+    constexpr uint32_t kPerGroup = kTiles / kGroups;    // tiles of a group
+    constexpr uint32_t kOwnCenters = kMaxBranch / kGroups; // centers a group updates
+    constexpr uint32_t kSumCol = 16 * kTiles;
+    static_assert(kTiles % kGroups == 0 && kMaxBranch % kGroups == 0, "whole tiles and centers per group");
+    extern __shared__ uint8_t smemRaw[];
+    Smem& S = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
+    const uint32_t tid = threadIdx.x, lane = tid % 32;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid / 32, 0); // uniform
+    const uint32_t group = warp / 4, row = tid % kRows;          // row of a tile; dimension in the update
+    const uint32_t laneQuarter = ((warp % 4) * 32u) << 16;
+    volatile uint32_t* abortFlag = &S.abortFlag;
+    if (tid == 0) {
+        for (uint32_t i = 0; i < kTiles; i++) mbarInit(&S.distBar[i], 1);
+        mbarInit(&S.sumBar, kGroups);
+        S.abortFlag = 0;
+        fenceMbarInit();
+    }
+    if (warp == 0) {
+        tmemAlloc(&S.tmemBase, lloydTmemCols<kTiles, kGroups>());
+        tmemRelinquish();
+    }
+    tcFenceBefore();
+    __syncthreads();
+    tcFenceAfter();
+    const uint32_t tmem = S.tmemBase;
+    const bool issuer = warp % 4 == 0 && electOne(); // one thread per group issues and commits its MMAs
+    const uint32_t nList = *listCount;
+    uint32_t distPhase = 0, sumPhase = 0; // distPhase: bit j for this group's tile j
+    bool failed = false;
+    while (!failed) {
+        if (tid == 0) S.slot = atomicAdd(cursor, 1u);
+        __syncthreads(); // the previous node's shared memory is no longer read
+        const uint32_t slot = S.slot;
+        if (slot >= nList) break;
+        const uint32_t g = list[slot];
+        const uint32_t n = lv.nodeCnt[g], off = lv.nodeOff[g];
+        const uint32_t T = (n + kRows - 1) / kRows;
+        // rows: eight threads per row; rows past n keep whatever the buffer holds (their one-hot is
+        // zero and their assignment is not written)
+        for (uint32_t r0 = tid / 8; r0 < n; r0 += 8 * (kThreads / 8)) {
+            uint32_t m[8];
+#pragma unroll
+            for (uint32_t u = 0; u < 8; u++) {
+                const uint32_t r = r0 + u * (kThreads / 8);
+                m[u] = r < n ? lv.members[uint64_t(off) + r] : 0u;
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 8; u++) {
+                const uint32_t r = r0 + u * (kThreads / 8), c = tid % 8;
+                if (r < n)
+                    cpAsync16(&S.tile[0][0] + r * kDims + ((c ^ (r & 7u)) << 4),
+                              lv.desc + uint64_t(m[u]) * kDims + (c << 4));
+            }
+        }
+        cpAsyncCommit();
+        if (tid < kMaxBranch * 8) {
+            const uint32_t b = tid / 8, c = tid % 8;
+            *reinterpret_cast<uint4*>(S.cen + b * kDims + ((c ^ (b & 7u)) << 4)) =
+                reinterpret_cast<const uint4*>(lv.centers + (uint64_t(g) * kMaxBranch + b) * kDims)[c];
+        }
+        if (tid < kMaxBranch) {
+            S.cnk[tid] = tid < lv.B ? lv.cnorm[uint64_t(g) * kMaxBranch + tid] * 16 + int32_t(tid) : 0x7FFFFFFF;
+            S.cnt[tid] = 0;
+        }
+        if (tid == 0) S.chg = 0;
+        cpAsyncWait<0>();
+        uint32_t mine[kPerGroup]; // this thread's rows' centers (zero at first, as fresh assignment memory)
+#pragma unroll
+        for (uint32_t j = 0; j < kPerGroup; j++) mine[j] = 0;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        uint32_t step = 0;
+        for (;;) {
+            if (warp % 4 == 0) {
+                tcFenceAfter();
+                for (uint32_t i = group; i < T; i += kGroups) {
+                    mmaU8x4(issuer, tmem + 16u * i, smemDescSw128(smemAddr(S.tile[i])), 32u,
+                            smemDescSw128(smemAddr(S.cen)), 32u, idescU8(16), 0u);
+                    if (issuer) mmaCommit(&S.distBar[i]);
+                }
+            }
+            uint32_t myCnt = 0, myChg = 0; // lane c < 16: rows of this warp that chose center c
+#pragma unroll
+            for (uint32_t j = 0; j < kPerGroup; j++) {
+                const uint32_t i = group + kGroups * j;
+                if (i < T) { // uniform in the group
+                    failed |= !mbarWait(&S.distBar[i], (distPhase >> j) & 1u, abortFlag, lv.err, 50);
+                    distPhase ^= 1u << j;
+                    tcFenceAfter();
+                    uint32_t r[16];
+                    tmemLoad16(tmem + 16u * i + laneQuarter, r);
+                    tmemWaitTie(r);
+                    // 16 (|c|^2 - 2 x.c) + b fits 32 bits: the minimum is the lowest center of the
+                    // lowest score
+                    int32_t best = 0x7FFFFFFF;
+#pragma unroll
+                    for (uint32_t b = 0; b < kMaxBranch; b++)
+                        best = min(best, S.cnk[b] - 32 * static_cast<int32_t>(r[b]));
+                    const uint32_t bi = static_cast<uint32_t>(best) & 15u;
+                    const bool valid = kRows * i + row < n;
+                    const uint32_t word = valid ? 1u << (8u * (bi & 3u)) : 0u, q = bi >> 2;
+                    *reinterpret_cast<uint4*>(S.oh[i] + row * kMaxBranch) =
+                        make_uint4(q == 0 ? word : 0u, q == 1 ? word : 0u, q == 2 ? word : 0u, q == 3 ? word : 0u);
+                    uint32_t mask = __ballot_sync(0xFFFFFFFFu, valid);
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; k++) {
+                        const uint32_t bits = __ballot_sync(0xFFFFFFFFu, (bi >> k) & 1u);
+                        mask &= (lane >> k) & 1u ? bits : ~bits;
+                    }
+                    myCnt += __popc(mask);
+                    myChg += __popc(__ballot_sync(0xFFFFFFFFu, valid && mine[j] != bi));
+                    mine[j] = bi;
+                    tcFenceBefore();
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    groupBarrier<kGroups>(group);
+                    if (warp % 4 == 0) {
+                        tcFenceAfter();
+                        mmaU8x4(issuer, tmem + kSumCol + 16u * group, smemDescSw128(smemAddr(S.tile[i])), 4096u,
+                                smemDescMn16(smemAddr(S.oh[i])), 512u, idescU8(16) | kIdescMnMajorAB, j);
+                    }
+                }
+            }
+            if (issuer) {
+                if (group < T) mmaCommit(&S.sumBar);
+                else mbarArrive(&S.sumBar);
+            }
+            if (lane < kMaxBranch && myCnt) atomicAdd(&S.cnt[lane], myCnt);
+            if (lane == 0 && myChg) atomicAdd(&S.chg, myChg);
+            failed |= !mbarWait(&S.sumBar, sumPhase, abortFlag, lv.err, 51);
+            sumPhase ^= 1u;
+            tcFenceAfter();
+            failed = __syncthreads_or(failed) != 0; // and cnt, chg are complete
+            step++;
+            const bool changed = S.chg != 0;
+            if (failed || !changed) break; // uniform
+            // centers b0 .. b0 + kOwnCenters - 1, dimension `row`
+            const uint32_t b0 = group * kOwnCenters;
+            uint32_t sum[kOwnCenters];
+            tmemLoadN<kOwnCenters>(tmem + kSumCol + b0 + laneQuarter, sum);
+#pragma unroll
+            for (uint32_t q = 1; q < kGroups; q++) {
+                if (q < T) {
+                    uint32_t more[kOwnCenters];
+                    tmemLoadN<kOwnCenters>(tmem + kSumCol + 16u * q + b0 + laneQuarter, more);
+#pragma unroll
+                    for (uint32_t k = 0; k < kOwnCenters; k++) sum[k] += more[k];
+                }
+            }
+            tcFenceBefore();
+#pragma unroll
+            for (uint32_t k = 0; k < kOwnCenters; k++) {
+                const uint32_t b = b0 + k, c = S.cnt[b];
+                uint8_t* at = S.cen + b * kDims + (((row >> 4) ^ (b & 7u)) << 4) + (row & 15u);
+                uint32_t v = *at;
+                if (c != 0) {
+                    const float quot =
+                        lv.ieeeDivision ? __fdiv_rn(float(sum[k]), float(c)) : float(sum[k]) / float(c);
+                    v = static_cast<uint8_t>(roundf(quot));
+                    *at = static_cast<uint8_t>(v);
+                }
+                const uint32_t part = __reduce_add_sync(0xFFFFFFFFu, v * v);
+                if (lane == 0) S.normPart[warp % 4][b] = part;
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads(); // centers and norm parts written, cnt read
+            if (tid < kMaxBranch) {
+                if (tid < lv.B)
+                    S.cnk[tid] = int32_t(S.normPart[0][tid] + S.normPart[1][tid] + S.normPart[2][tid] +
+                                         S.normPart[3][tid]) * 16 + int32_t(tid);
+                S.cnt[tid] = 0;
+            }
+            if (tid == 0) S.chg = 0;
+            if (step >= maxIterations) break; // uniform
+            __syncthreads();
+        }
+        __syncthreads(); // cnk is final
+#pragma unroll
+        for (uint32_t j = 0; j < kPerGroup; j++) {
+            const uint32_t r = kRows * (group + kGroups * j) + row;
+            if (r < n) lv.assign[uint64_t(off) + r] = static_cast<uint8_t>(mine[j]);
+        }
+        if (tid < kMaxBranch * 8) {
+            const uint32_t b = tid / 8, c = tid % 8;
+            reinterpret_cast<uint4*>(lv.centers + (uint64_t(g) * kMaxBranch + b) * kDims)[c] =
+                *reinterpret_cast<const uint4*>(S.cen + b * kDims + ((c ^ (b & 7u)) << 4));
+        }
+        if (tid < lv.B) lv.cnorm[uint64_t(g) * kMaxBranch + tid] = S.cnk[tid] >> 4;
+        if (tid == 0) atomicMax(maxSteps, step);
+    }
+    if (failed) {
+        // a wait ran out: MMAs may still be in flight, the TMEM is freed after them (bounded)
+        if (issuer) mmaCommit(&S.sumBar);
+        mbarWait(&S.sumBar, sumPhase, abortFlag, lv.err, 52);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        tcFenceAfter();
+        tmemDealloc(tmem, lloydTmemCols<kTiles, kGroups>());
+    }
+}
+
+template <uint32_t kTiles, uint32_t kGroups, uint32_t kCtasPerSm>
+void launchClass(const KMeansLevel& lv, const LloydClasses& cls, uint32_t c, uint32_t count, uint32_t maxIterations,
+                 cudaStream_t s)
+{
+    if (count == 0) return;
+    constexpr size_t smem = lloydSmemBytes<kTiles, kGroups>();
+    static_assert(kCtasPerSm * (smem + 1024) <= 228 * 1024, "shared memory of the resident CTAs");
+    static_assert(kCtasPerSm * lloydTmemCols<kTiles, kGroups>() <= 512, "TMEM columns of the resident CTAs");
+    static std::atomic<uint64_t> attr{0};
+    const auto kernel = lloydResidentKernel<kTiles, kGroups, kCtasPerSm>;
+    setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(kernel), int(smem), attr);
+    const uint32_t grid = std::min(count, uint32_t(currentSmCount()) * kCtasPerSm);
+    kernel<<<grid, kRows * kGroups, smem, s>>>(lv, cls.lists + uint64_t(c) * lv.nbNodes, cls.counters + c,
+                                               cls.counters + kLloydCursor + c, maxIterations,
+                                               cls.counters + kLloydMaxSteps);
+    RBW_CUDA(cudaGetLastError());
+}
+
+} // namespace
+
+void launchClassifyNodes(const KMeansLevel& lv, const LloydClasses& cls, cudaStream_t s)
+{
+    classifyNodesKernel<<<(lv.nbNodes + 255) / 256, 256, 0, s>>>(lv.nodeCnt, lv.nbNodes, cls, lv.lastChanged);
+    RBW_CUDA(cudaGetLastError());
+}
+
+void launchLloydResident(const KMeansLevel& lv, const LloydClasses& cls, const uint32_t* hostCounts,
+                         uint32_t maxIterations, cudaStream_t s)
+{
+    ScopedKernelTimer timer(kTimedAssign, s);
+    // the longest nodes first, so that the short ones fill the last wave
+    launchClass<lloydTiles(3), 4, 1>(lv, cls, 3, hostCounts[3], maxIterations, s);
+    launchClass<lloydTiles(2), 2, 2>(lv, cls, 2, hostCounts[2], maxIterations, s);
+    launchClass<lloydTiles(1), 1, 5>(lv, cls, 1, hostCounts[1], maxIterations, s);
+    launchClass<lloydTiles(0), 1, 8>(lv, cls, 0, hostCounts[0], maxIterations, s);
+}
+
+} // namespace rbw

@@ -242,6 +242,24 @@ __device__ __forceinline__ void mmaU8(uint32_t dTmem, uint64_t aDesc, uint64_t b
         "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate), "r"(z), "r"(z), "r"(z), "r"(z)
         : "memory");
 }
+// True in one lane of the warp; all lanes call it.
+__device__ __forceinline__ bool electOne()
+{
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+// The four K steps of one tile's product, by the elected lane of a warp whose lanes all call this
+// with the same operands.  With warp-uniform control flow the descriptors stay in uniform
+// registers: four MMAs issue in 84 cycles, 232 from one lane of a diverged warp.
+__device__ __forceinline__ void mmaU8x4(bool elected, uint32_t dTmem, uint64_t aDesc, uint32_t aStep, uint64_t bDesc,
+                                        uint32_t bStep, uint32_t idesc, uint32_t accumulate)
+{
+#pragma unroll
+    for (uint32_t q4 = 0; q4 < 4; q4++)
+        if (elected)
+            mmaU8(dTmem, aDesc + q4 * (aStep >> 4), bDesc + q4 * (bStep >> 4), idesc, (accumulate || q4 > 0) ? 1u : 0u);
+}
 // D[tmem] (+)= A[smem] * B[smem]^T, bf16 x bf16 -> fp32, M = 128, N from idesc.
 __device__ __forceinline__ void mmaBf16(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc,
                                         uint32_t accumulate)

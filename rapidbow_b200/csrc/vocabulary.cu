@@ -464,6 +464,11 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
     StreamBuffer tileHist(uint64_t(B) * maxTiles32 * 4, st), tileScan(uint64_t(B) * maxTiles32 * 4, st);
     uint32_t* totals = small.as<uint32_t>();
     uint32_t* activeCount = small.as<uint32_t>() + 4;
+    // uint8 centers: the nodes by how their Lloyd loop runs (kmeans.cuh)
+    StreamBuffer lloyd(opts.floatCenters ? 0 : (uint64_t(kLloydClasses + 1) * maxLevelNodes + kLloydCounters * L) * 4, st);
+    uint32_t hostLloyd[kLloydCounters] = {};
+    std::vector<uint32_t> hostLloydAll(kLloydCounters * size_t(L), 0u);
+    if (lloyd.get()) RBW_CUDA(cudaMemsetAsync(lloyd.get(), 0, kLloydCounters * 4 * L, stream));
     // float centers: member |x|^2 sums, per-node inertia, the level's inertia per step, counters
     StreamBuffer qSums(fl ? maxLevelNodes * kMaxBranch * 8 : 0, st), inertiaNode(fl ? maxLevelNodes * 8 : 0, st);
     StreamBuffer inertiaTrace(fl ? uint64_t(opts.maxIterations) * 8 : 0, st), counters(fl ? uint64_t(L) * 16 : 0, st);
@@ -525,6 +530,15 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
             lvf.lookupOnly = 0;
         }
 
+        LloydClasses cls{};
+        if (!fl) {
+            // the counters reach the host with the initial centers' copies and synchronisation below
+            cls.counters = lloyd.as<uint32_t>() + kLloydCounters * level;
+            cls.streamCnt = lloyd.as<uint32_t>() + kLloydCounters * L;
+            cls.lists = cls.streamCnt + maxLevelNodes;
+            launchClassifyNodes(lv, cls, stream);
+            RBW_CUDA(cudaMemcpyAsync(hostLloyd, cls.counters, sizeof(hostLloyd), cudaMemcpyDeviceToHost, stream));
+        }
         // ---- initial centers
         if (opts.initMode == kInitReference) {
             hostCnt.resize(nbLv);
@@ -570,12 +584,16 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
         }
 
         // ---- Lloyd iterations (kmeans.cpp:118-133)
-        buildNodeTiles(lv.nodeCnt, lv.nodeOff, nbLv, 128, tileOff.as<uint32_t>(), scanTmp.as<uint32_t>(),
-                       tiles128.as<NodeTile>(), maxTiles128, totals, stream);
-        RBW_CUDA(cudaMemsetAsync(assign.get(), 0, n, stream)); // fresh (zeroed) assignment memory
-        RBW_CUDA(cudaMemsetAsync(lastChanged.get(), 0xFF, uint64_t(nbLv) * 4, stream));
+        const bool streamed = fl || hostLloyd[kLloydClasses] != 0;
+        if (streamed) {
+            buildNodeTiles(fl ? lv.nodeCnt : cls.streamCnt, lv.nodeOff, nbLv, 128, tileOff.as<uint32_t>(),
+                           scanTmp.as<uint32_t>(), tiles128.as<NodeTile>(), maxTiles128, totals, stream);
+            RBW_CUDA(cudaMemsetAsync(assign.get(), 0, n, stream)); // fresh (zeroed) assignment memory
+        }
+        if (fl) RBW_CUDA(cudaMemsetAsync(lastChanged.get(), 0xFF, uint64_t(nbLv) * 4, stream));
+        else launchLloydResident(lv, cls, hostLloyd, opts.maxIterations, stream);
         uint32_t iters = 0;
-        for (uint32_t it = 0; it < opts.maxIterations; it++) {
+        for (uint32_t it = 0; streamed && it < opts.maxIterations; it++) {
             if (fl) {
                 launchAssignF(lvf, tiles128.as<NodeTile>(), totals, maxTiles128, stream);
                 RBW_CUDA(cudaMemsetAsync(activeCount, 0, 4, stream));
@@ -629,6 +647,9 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
     float* w = voc->mWeights.data();
     const size_t nw = voc->mWeights.size();
     RBW_CUDA(cudaMemcpyAsync(w, occDev.get(), nw * 4, cudaMemcpyDeviceToHost, stream));
+    if (lloyd.get())
+        RBW_CUDA(cudaMemcpyAsync(hostLloydAll.data(), lloyd.get(), hostLloydAll.size() * 4, cudaMemcpyDeviceToHost,
+                                 stream));
     // the weights of every count below kIdfMemo, computed once (the same expression, so the same
     // float), while the copy runs
     constexpr uint32_t kIdfMemo = 1u << 12;
@@ -652,6 +673,12 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
         throw Error(kTimeout, "a bounded device wait gave up during the build (site " + std::to_string(e.where) + ")");
     bs.levels = L;
     for (uint32_t level = 0; level < L && level < 16; level++) {
+        if (lloyd.get()) {
+            // resident nodes count their own steps; a loop over all nodes is left at its polls
+            const uint64_t steps = hostLloydAll[kLloydCounters * level + kLloydMaxSteps];
+            const uint64_t polled = std::min<uint64_t>(opts.maxIterations, (steps + check - 1) / check * check);
+            bs.iterations[level] = std::max(bs.iterations[level], static_cast<uint32_t>(polled));
+        }
         bs.inertiaFirst[level] = hostFirst[level];
         bs.inertiaLast[level] = hostLast[level];
         bs.refined[level] = hostCounters[2 * level];

@@ -121,3 +121,18 @@ def test_build_tile_edges_match_oracle(oracle, B, n):
                                    nb_levels=2, init="kmeans++", seed=4, max_iterations=6, ieee_division=True)
         ref = oracle.build_vocabulary(level_members, 50, B, 2, max_iter=6, init=INIT_KMEANSPP, seed=4)
         _tree_equal(voc, ref)
+
+
+@pytest.mark.parametrize("n", [16, 128, 129, 256, 257, 767, 768, 769, 1535, 1536, 1537])
+@pytest.mark.parametrize("B,iters,check", [(16, 1000, 4), (5, 7, 3)])
+def test_build_resident_node_sizes_match_oracle(oracle, n, B, iters, check):
+    """Nodes at the edges of the classes whose whole Lloyd loop runs in one CTA, and one row above
+    the largest (streamed); the level's step count is the one of a loop polled every `check` steps."""
+    desc = sift_like(n, seed=n + B).numpy()
+    voc = rbw.build_vocabulary(torch.from_numpy(desc).cuda(), B, nb_doc=30, nb_levels=2, max_iterations=iters,
+                               check_interval=check, ieee_division=True)
+    ref = oracle.build_vocabulary(desc, 30, B, 2, max_iter=iters, init=INIT_REFERENCE)
+    _tree_equal(voc, ref)
+    stops = [ref["iters"][:1].max(), ref["iters"][1:].max()]  # the step that changed nothing, per level
+    want = [min(iters, -(-int(s) // check) * check) for s in stops]
+    assert voc.build_stats()["iterations"] == want
