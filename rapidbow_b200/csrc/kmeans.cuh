@@ -69,9 +69,10 @@ constexpr uint32_t kLloydClasses = 4;
 __host__ __device__ constexpr uint32_t lloydTiles(uint32_t c) { return c == 0 ? 1u : c == 1 ? 2u : c == 2 ? 6u : 12u; }
 constexpr uint32_t kLloydCursor = kLloydClasses + 1;        // counters: nodes per class, streamed nodes,
 constexpr uint32_t kLloydMaxSteps = 2 * kLloydClasses + 1;  // the classes' work cursors, most steps run
-constexpr uint32_t kLloydCounters = 2 * kLloydClasses + 2;
+constexpr uint32_t kLloydShareCtas = 2 * kLloydClasses + 2; // CTAs that hold all streamed rows
+constexpr uint32_t kLloydCounters = 2 * kLloydClasses + 3;
 struct LloydClasses {
-    uint32_t* lists;     // [kLloydClasses][nbNodes] nodes of each class
+    uint32_t* lists;     // [kLloydClasses + 1][nbNodes] nodes of each class, then the streamed ones
     uint32_t* counters;  // [kLloydCounters], zero on entry
     uint32_t* streamCnt; // [nbNodes] members of streamed nodes, 0 for all others
 };
@@ -81,6 +82,13 @@ void launchClassifyNodes(const KMeansLevel& lv, const LloydClasses& cls, cudaStr
 // hostCounts: counters[0, kLloydClasses) on the host (grid sizes; empty classes are not launched).
 void launchLloydResident(const KMeansLevel& lv, const LloydClasses& cls, const uint32_t* hostCounts,
                          uint32_t maxIterations, cudaStream_t s);
+
+// The Lloyd loops of the nbShared streamed nodes of a level whose rows fit the SMs' shared memory
+// together (counters[kLloydShareCtas] <= SMs), each node spread over several CTAs, and with `tail`
+// those of the resident nodes too.  shareMem: lloydShareBytes(nbShared).
+size_t lloydShareBytes(uint32_t nbShared);
+void launchLloydShared(const KMeansLevel& lv, const LloydClasses& cls, uint32_t nbShared, void* shareMem, bool tail,
+                       uint32_t maxIterations, cudaStream_t s);
 
 // ------------------------------------------------------------------ float-center mode
 // fp32 centers (the FP64 quotient of the exact integer sums, rounded once), distances from the

@@ -465,7 +465,7 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
     uint32_t* totals = small.as<uint32_t>();
     uint32_t* activeCount = small.as<uint32_t>() + 4;
     // uint8 centers: the nodes by how their Lloyd loop runs (kmeans.cuh)
-    StreamBuffer lloyd(opts.floatCenters ? 0 : (uint64_t(kLloydClasses + 1) * maxLevelNodes + kLloydCounters * L) * 4, st);
+    StreamBuffer lloyd(opts.floatCenters ? 0 : (uint64_t(kLloydClasses + 2) * maxLevelNodes + kLloydCounters * L) * 4, st);
     uint32_t hostLloyd[kLloydCounters] = {};
     std::vector<uint32_t> hostLloydAll(kLloydCounters * size_t(L), 0u);
     if (lloyd.get()) RBW_CUDA(cudaMemsetAsync(lloyd.get(), 0, kLloydCounters * 4 * L, stream));
@@ -584,14 +584,25 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
         }
 
         // ---- Lloyd iterations (kmeans.cpp:118-133)
-        const bool streamed = fl || hostLloyd[kLloydClasses] != 0;
+        // One cooperative launch runs the whole level when its larger nodes fit the SMs together and
+        // its small ones are too few to fill the GPU in classes of several CTAs per SM.
+        uint32_t resident = 0;
+        for (uint32_t c = 0; c < kLloydClasses; c++) resident += hostLloyd[c];
+        const uint32_t sms = static_cast<uint32_t>(currentSmCount()), nbShared = hostLloyd[kLloydClasses];
+        const bool tail = resident <= 2 * sms;
+        const bool shared = !fl && hostLloyd[kLloydShareCtas] <= sms && (nbShared != 0 || tail);
+        const bool streamed = fl || (nbShared != 0 && !shared);
         if (streamed) {
             buildNodeTiles(fl ? lv.nodeCnt : cls.streamCnt, lv.nodeOff, nbLv, 128, tileOff.as<uint32_t>(),
                            scanTmp.as<uint32_t>(), tiles128.as<NodeTile>(), maxTiles128, totals, stream);
             RBW_CUDA(cudaMemsetAsync(assign.get(), 0, n, stream)); // fresh (zeroed) assignment memory
         }
         if (fl) RBW_CUDA(cudaMemsetAsync(lastChanged.get(), 0xFF, uint64_t(nbLv) * 4, stream));
-        else launchLloydResident(lv, cls, hostLloyd, opts.maxIterations, stream);
+        else if (!shared || !tail) launchLloydResident(lv, cls, hostLloyd, opts.maxIterations, stream);
+        if (shared) {
+            StreamBuffer shareMem(lloydShareBytes(nbShared), st);
+            launchLloydShared(lv, cls, nbShared, shareMem.get(), tail, opts.maxIterations, stream);
+        }
         uint32_t iters = 0;
         for (uint32_t it = 0; streamed && it < opts.maxIterations; it++) {
             if (fl) {

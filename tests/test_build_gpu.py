@@ -136,3 +136,17 @@ def test_build_resident_node_sizes_match_oracle(oracle, n, B, iters, check):
     stops = [ref["iters"][:1].max(), ref["iters"][1:].max()]  # the step that changed nothing, per level
     want = [min(iters, -(-int(s) // check) * check) for s in stops]
     assert voc.build_stats()["iterations"] == want
+
+
+@pytest.mark.parametrize("rows_per_sm,extra,L", [(12, -1, 2), (1536, 0, 1), (1536, 1, 1), (400, 77, 2)])
+def test_build_shared_level_edges_match_oracle(oracle, rows_per_sm, extra, L):
+    """Levels whose streamed rows fit the SMs together run in one cooperative launch, nodes spread
+    over the CTAs (up to 1,536 rows per SM); one row more is streamed step by step."""
+    n = torch.cuda.get_device_properties(0).multi_processor_count * rows_per_sm + extra
+    desc = sift_like(n, seed=rows_per_sm).numpy()
+    B = 6
+    voc = rbw.build_vocabulary(torch.from_numpy(desc).cuda(), B, nb_doc=30, nb_levels=L, max_iterations=9,
+                               ieee_division=True)
+    ref = oracle.build_vocabulary(desc, 30, B, L, max_iter=9, init=INIT_REFERENCE)
+    _tree_equal(voc, ref)
+    assert voc.build_stats()["iterations"][0] == min(9, -(-int(ref["iters"][0]) // 4) * 4)
