@@ -128,8 +128,7 @@ int rbw_voc_get_centers_f32(const rbw_vocabulary* voc, float* host_centers)
 {
     return guard([&] {
         if (host_centers == nullptr) throw rbw::Error(rbw::kInvalidArg, "null output");
-        const auto c = vocOf(voc).centersF32Host();
-        std::memcpy(host_centers, c.data(), c.size() * sizeof(float));
+        vocOf(voc).copyCentersF32(host_centers);
     });
 }
 
@@ -238,10 +237,7 @@ int rbw_voc_get_tree(const rbw_vocabulary* voc, uint8_t* host_centers, uint32_t*
 {
     return guard([&] {
         const auto& v = vocOf(voc);
-        if (host_centers) {
-            const auto c = v.centersHost();
-            std::memcpy(host_centers, c.data(), c.size());
-        }
+        if (host_centers) v.copyCenters(host_centers);
         if (host_masks) std::memcpy(host_masks, v.masks().data(), v.masks().size() * 4);
         if (host_weights) std::memcpy(host_weights, v.weights().data(), v.weights().size() * 4);
     });

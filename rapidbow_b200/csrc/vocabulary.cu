@@ -148,7 +148,49 @@ float idfWeight(uint32_t nbDoc, uint32_t occ)
                     : std::max(std::numeric_limits<float>::min(), std::log(float(nbDoc) / float(occ)));
 }
 
-void Vocabulary::allocate(uint32_t B, uint32_t L)
+namespace {
+cudaMemPool_t vocabularyPool(int dev)
+{
+    static cudaMemPool_t pools[kMaxDevices] = {};
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    if (pools[dev] == nullptr) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        RBW_CUDA(cudaMemPoolCreate(&pools[dev], &props));
+        uint64_t keep = VocabularyMemory::kPooledBytes;
+        RBW_CUDA(cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    return pools[dev];
+}
+} // namespace
+
+void VocabularyMemory::allocate(size_t bytes, cudaStream_t s)
+{
+    mDevice = currentDevice();
+    mPooled = bytes <= kPooledBytes;
+    if (mPooled) RBW_CUDA(cudaMallocFromPoolAsync(&mPtr, bytes, vocabularyPool(mDevice), s));
+    else RBW_CUDA(cudaMalloc(&mPtr, bytes));
+}
+
+VocabularyMemory::~VocabularyMemory()
+{
+    if (mPtr == nullptr) return;
+    if (!mPooled) {
+        cudaFree(mPtr);
+        return;
+    }
+    int cur = mDevice;
+    cudaGetDevice(&cur);
+    if (cur != mDevice) cudaSetDevice(mDevice);
+    cudaDeviceSynchronize();
+    cudaFreeAsync(mPtr, nullptr);
+    if (cur != mDevice) cudaSetDevice(cur);
+}
+
+void Vocabulary::allocate(uint32_t B, uint32_t L, bool floatCenters, cudaStream_t stream)
 {
     if (B < 2 || B > kMaxBranch) throw Error(kUnsupported, "branch factor must be in [2, 16]");
     if (L < 1 || L > 8) throw Error(kUnsupported, "number of levels must be in [1, 8]");
@@ -157,11 +199,32 @@ void Vocabulary::allocate(uint32_t B, uint32_t L)
     mB = B;
     mL = L;
     mNbNodes = nodes;
-    mCenters.reset(nodes * kMaxBranch * kDims);
-    mCentersSw.reset(nodes * kMaxBranch * kDims);
-    mCnorm.reset(nodes * kMaxBranch * sizeof(int32_t));
-    mErrors.reset(sizeof(DeviceErrors));
-    RBW_CUDA(cudaMemset(mErrors.get(), 0, sizeof(DeviceErrors)));
+    mFloat = floatCenters;
+    struct Part {
+        DeviceArray* array;
+        size_t bytes;
+    };
+    const uint64_t fl = floatCenters ? 1 : 0;
+    const Part parts[] = {{&mCenters, nodes * kMaxBranch * kDims},
+                          {&mCentersSw, nodes * kMaxBranch * kDims},
+                          {&mCnorm, nodes * kMaxBranch * sizeof(int32_t)},
+                          {&mErrors, sizeof(DeviceErrors)},
+                          {&mCentersF, fl * nodes * kMaxBranch * kDims * sizeof(float)},
+                          {&mSplit, fl * nodes * kSplitBytes},
+                          {&mCnF, fl * nodes * kMaxBranch * sizeof(float)},
+                          {&mBound, fl * nodes * sizeof(float2)},
+                          {&mRefined, fl * 2 * sizeof(unsigned long long)}};
+    auto padded = [](size_t b) { return (b + 1023) / 1024 * 1024; };
+    size_t total = 0;
+    for (const Part& p : parts) total += padded(p.bytes);
+    mMemory.allocate(total, stream);
+    uint8_t* at = mMemory.get();
+    for (const Part& p : parts) {
+        if (p.bytes) *p.array = DeviceArray(at, p.bytes);
+        at += padded(p.bytes);
+    }
+    RBW_CUDA(cudaMemsetAsync(mErrors.get(), 0, mErrors.bytes(), stream));
+    if (fl) RBW_CUDA(cudaMemsetAsync(mRefined.get(), 0, mRefined.bytes(), stream));
     mTree = DeviceTree{B, L, nodes, mCenters.as<uint8_t>(), mCentersSw.as<uint8_t>(), mCnorm.as<int32_t>()};
 }
 
@@ -173,18 +236,6 @@ void Vocabulary::finalizeDevice(cudaStream_t stream)
     normsKernel<<<blocksFor(mNbNodes * kMaxBranch, 256), 256, 0, stream>>>(mCenters.as<uint8_t>(),
                                                                            mCnorm.as<int32_t>(), mNbNodes, mB);
     RBW_CUDA(cudaGetLastError());
-}
-
-void Vocabulary::allocateFloat()
-{
-    const uint64_t nodes = mNbNodes;
-    mCentersF.reset(nodes * kMaxBranch * kDims * sizeof(float));
-    mSplit.reset(nodes * kSplitBytes);
-    mCnF.reset(nodes * kMaxBranch * sizeof(float));
-    mBound.reset(nodes * sizeof(float2));
-    mRefined.reset(2 * sizeof(unsigned long long));
-    RBW_CUDA(cudaMemset(mRefined.get(), 0, 2 * sizeof(unsigned long long)));
-    mFloat = true;
 }
 
 void Vocabulary::roundFloatCenters(cudaStream_t stream)
@@ -199,8 +250,7 @@ std::unique_ptr<Vocabulary> Vocabulary::fromHostF32(uint32_t B, uint32_t L, cons
                                                     const uint32_t* masks, const float* weights)
 {
     std::unique_ptr<Vocabulary> v{new Vocabulary};
-    v->allocate(B, L);
-    v->allocateFloat();
+    v->allocate(B, L, true, nullptr);
     const uint64_t nodes = v->mNbNodes;
     DeviceBuffer canon(nodes * B * kDims * sizeof(float));
     RBW_CUDA(cudaMemcpy(canon.get(), centers, canon.bytes(), cudaMemcpyHostToDevice));
@@ -217,15 +267,54 @@ std::unique_ptr<Vocabulary> Vocabulary::fromHostF32(uint32_t B, uint32_t L, cons
     return v;
 }
 
-std::vector<float> Vocabulary::centersF32Host() const
+namespace {
+// The first B of the 16 slots of nodes [node0, node0 + count), back to back, in 16-byte words.
+__global__ void packKernel(const uint4* __restrict__ padded, uint4* __restrict__ canon, uint64_t node0, uint64_t count,
+                           uint32_t B, uint32_t wordsPerCenter)
+{
+    const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint64_t perNode = uint64_t(B) * wordsPerCenter;
+    if (i >= count * perNode) return;
+    canon[i] = padded[(node0 + i / perNode) * kMaxBranch * wordsPerCenter + i % perNode];
+}
+
+// Canonical host copy of a padded device array ([nodes][16][bytesPerCenter]): straight from the
+// device for B = 16, else packed there a piece at a time first.
+void copyUnpadded(const void* padded, void* host, uint64_t nodes, uint32_t B, size_t bytesPerCenter)
+{
+    if (B == kMaxBranch) {
+        RBW_CUDA(cudaMemcpy(host, padded, nodes * kMaxBranch * bytesPerCenter, cudaMemcpyDeviceToHost));
+        return;
+    }
+    const size_t nodeBytes = B * bytesPerCenter;
+    const uint64_t piece = std::min<uint64_t>(nodes, (size_t(32) << 20) / nodeBytes);
+    void* tmp = nullptr;
+    RBW_CUDA(cudaMallocFromPoolAsync(&tmp, piece * nodeBytes, libraryPool(), nullptr));
+    cudaError_t e = cudaSuccess;
+    for (uint64_t n0 = 0; n0 < nodes && e == cudaSuccess; n0 += piece) {
+        const uint64_t count = std::min(piece, nodes - n0);
+        packKernel<<<blocksFor(count * nodeBytes / 16, 256), 256>>>(static_cast<const uint4*>(padded),
+                                                                    static_cast<uint4*>(tmp), n0, count, B,
+                                                                    static_cast<uint32_t>(bytesPerCenter / 16));
+        e = cudaGetLastError();
+        if (e == cudaSuccess)
+            e = cudaMemcpy(static_cast<uint8_t*>(host) + n0 * nodeBytes, tmp, count * nodeBytes, cudaMemcpyDeviceToHost);
+    }
+    cudaFreeAsync(tmp, nullptr);
+    RBW_CUDA(e);
+}
+} // namespace
+
+void Vocabulary::copyCentersF32(float* host) const
 {
     if (!mFloat) throw Error(kUnsupported, "the vocabulary has uint8 centers");
-    std::vector<float> padded(mNbNodes * kMaxBranch * kDims);
-    RBW_CUDA(cudaMemcpy(padded.data(), mCentersF.get(), padded.size() * sizeof(float), cudaMemcpyDeviceToHost));
+    copyUnpadded(mCentersF.get(), host, mNbNodes, mB, kDims * sizeof(float));
+}
+
+std::vector<float> Vocabulary::centersF32Host() const
+{
     std::vector<float> out(mNbNodes * mB * kDims);
-    for (uint64_t n = 0; n < mNbNodes; n++)
-        std::memcpy(out.data() + n * mB * kDims, padded.data() + n * kMaxBranch * kDims,
-                    size_t(mB) * kDims * sizeof(float));
+    copyCentersF32(out.data());
     return out;
 }
 
@@ -242,7 +331,7 @@ std::unique_ptr<Vocabulary> Vocabulary::fromHost(uint32_t B, uint32_t L, const u
                                                  const float* weights)
 {
     std::unique_ptr<Vocabulary> v{new Vocabulary};
-    v->allocate(B, L);
+    v->allocate(B, L, false, nullptr);
     const uint64_t nodes = v->mNbNodes;
     DeviceBuffer canon(nodes * B * kDims);
     RBW_CUDA(cudaMemcpy(canon.get(), centers, nodes * B * kDims, cudaMemcpyHostToDevice));
@@ -255,13 +344,12 @@ std::unique_ptr<Vocabulary> Vocabulary::fromHost(uint32_t B, uint32_t L, const u
     return v;
 }
 
+void Vocabulary::copyCenters(uint8_t* host) const { copyUnpadded(mCenters.get(), host, mNbNodes, mB, kDims); }
+
 std::vector<uint8_t> Vocabulary::centersHost() const
 {
-    std::vector<uint8_t> padded(mNbNodes * kMaxBranch * kDims);
-    RBW_CUDA(cudaMemcpy(padded.data(), mCenters.get(), padded.size(), cudaMemcpyDeviceToHost));
     std::vector<uint8_t> out(mNbNodes * mB * kDims);
-    for (uint64_t n = 0; n < mNbNodes; n++)
-        std::memcpy(out.data() + n * mB * kDims, padded.data() + n * kMaxBranch * kDims, size_t(mB) * kDims);
+    copyCenters(out.data());
     return out;
 }
 
@@ -441,9 +529,8 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
     if (opts.maxIterations == 0) throw Error(kInvalidArg, "maxIterations must be positive");
     const uint32_t check = std::max(1u, opts.checkInterval);
     std::unique_ptr<Vocabulary> voc{new Vocabulary};
-    voc->allocate(B, L);
     const bool fl = opts.floatCenters;
-    if (fl) voc->allocateFloat();
+    voc->allocate(B, L, fl, stream);
     RBW_CUDA(cudaMemsetAsync(voc->mCenters.get(), 0, voc->mCenters.bytes(), stream));
     const uint64_t n = nbDesc;
     const uint64_t maxLevelNodes = ipow(B, L - 1);
@@ -658,6 +745,8 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
     float* w = voc->mWeights.data();
     const size_t nw = voc->mWeights.size();
     RBW_CUDA(cudaMemcpyAsync(w, occDev.get(), nw * 4, cudaMemcpyDeviceToHost, stream));
+    DeviceErrors e{};
+    RBW_CUDA(cudaMemcpyAsync(&e, voc->mErrors.get(), sizeof(e), cudaMemcpyDeviceToHost, stream));
     if (lloyd.get())
         RBW_CUDA(cudaMemcpyAsync(hostLloydAll.data(), lloyd.get(), hostLloydAll.size() * 4, cudaMemcpyDeviceToHost,
                                  stream));
@@ -679,7 +768,6 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
     for (size_t k = 1; k < nThreads; k++) helpers.emplace_back(weigh, nw * k / nThreads, nw * (k + 1) / nThreads);
     weigh(0, nw / nThreads);
     for (auto& h : helpers) h.join();
-    const DeviceErrors e = voc->takeDeviceErrors();
     if (e.code != 0)
         throw Error(kTimeout, "a bounded device wait gave up during the build (site " + std::to_string(e.where) + ")");
     bs.levels = L;

@@ -155,3 +155,25 @@ def test_auto_lookup_matches_oracle_on_both_sides_of_the_direct_limit(oracle, B,
         assert (voc.last_kernels == 1) == (n <= limit or L <= 2)
         want = oracle.lookup(centers, B, L, desc, threads=8)
         assert np.array_equal(got, want), f"n={n}: {np.count_nonzero(got != want)} mismatches"
+
+
+@pytest.mark.parametrize("B,L,float_centers", [(16, 3, False), (10, 6, False), (3, 7, False), (16, 2, True), (9, 4, True)])
+def test_centers_come_back_as_they_went_in(B, L, float_centers):
+    """Trees above and below one 32 MiB piece of the packed copy, with and without padded slots, and
+    the memory of a freed tree used again."""
+    rng = np.random.default_rng(B * L)
+    nodes = sum(B ** i for i in range(L))
+    masks = np.full(nodes, (1 << B) - 1, np.uint32)
+    weights = rng.random((nodes, B), np.float32)
+    for _ in range(2):
+        if float_centers:
+            centers = (rng.random((nodes, B, 128), np.float32) * 255).astype(np.float32)
+            voc = rbw.vocabulary_from_host_f32(B, L, centers, masks, weights)
+            assert np.array_equal(voc.centers_f32(), centers)
+            assert np.array_equal(voc.tree()[0], np.rint(centers).astype(np.uint8))
+        else:
+            centers = rng.integers(0, 256, (nodes, B, 128), dtype=np.uint8)
+            voc = rbw.vocabulary_from_host(B, L, centers, masks, weights)
+            assert np.array_equal(voc.tree()[0], centers)
+        assert voc.device_errors() == (0, 0)
+        del voc
