@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 {
     extern __shared__ uint8_t smemRaw[];
     TcSmem& S = *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
-    const uint32_t warp = threadIdx.x / 32;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x / 32, 0); // uniform
     const uint32_t lane = threadIdx.x % 32;
     const uint32_t T = p.tiles == nullptr ? static_cast<uint32_t>((p.nRows + kTileRows - 1) / kTileRows)
                                           : *p.nTilesDev;
@@ -490,7 +490,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         // waits; commits track only the committing thread's MMAs, so each buffer's barriers see
         // exactly its own tiles.  Both issuers pass every tile and commit once per centre group
         // on the producer's "centre block free" barrier.
-        if (lane == 0) {
+        {
+            const bool issuer = electOne();
             const uint32_t jm = warp == 1 ? 0u : 1u;
             const uint32_t idescA = idescU8(16);
             const uint32_t idescB = idescU8(16 * p.B);
@@ -512,15 +513,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         if (!mbarWait(&S.aFull[s], (t / kStages) & 1u, abortFlag, p.err, 21)) break;
                         if (t >= 2 && !mbarWait(&S.bufFree[jm], ((t >> 1) - 1u) & 1u, abortFlag, p.err, 25)) break;
                         tcFenceAfter();
-                        const uint32_t aBase = smemAddr(S.a[s]);
-                        const uint32_t bBase = smemAddr(S.b[slot]);
-#pragma unroll
-                        for (uint32_t q4 = 0; q4 < 4; q4++) {
-                            mmaU8(tmem + kTmemBuf * jm, smemDescSw128(aBase + 32u * q4),
-                                  smemDescSw128(bBase + kNodeBytes + 32u * q4), idescB, q4 > 0 ? 1u : 0u);
+                        mmaU8x4(issuer, tmem + kTmemBuf * jm, smemDescSw128(smemAddr(S.a[s])), 32u,
+                                smemDescSw128(smemAddr(S.b[slot]) + kNodeBytes), 32u, idescB, 0u);
+                        if (issuer) {
+                            mmaCommit(&S.accB[jm]);
+                            mmaCommit(&S.aEmpty[s]);
                         }
-                        mmaCommit(&S.accB[jm]);
-                        mmaCommit(&S.aEmpty[s]);
                     }
                 } else if ((t & 1u) == jm) {
                     const uint32_t j = jm;
@@ -530,30 +528,23 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                             p.err, 22))
                         break;
                     tcFenceAfter();
-                    const uint32_t aBase = smemAddr(S.a[s]);
-                    const uint32_t bBase = smemAddr(S.b[slot]);
-#pragma unroll
-                    for (uint32_t q4 = 0; q4 < 4; q4++) {
-                        mmaU8(tmem + kTmemBuf * j, smemDescSw128(aBase + 32u * q4),
-                              smemDescSw128(bBase + 32u * q4), idescA, q4 > 0 ? 1u : 0u);
-                    }
-                    mmaCommit(&S.accA[j]);
+                    const uint64_t aDesc = smemDescSw128(smemAddr(S.a[s]));
+                    mmaU8x4(issuer, tmem + kTmemBuf * j, aDesc, 32u, smemDescSw128(smemAddr(S.b[slot])), 32u, idescA,
+                            0u);
+                    if (issuer) mmaCommit(&S.accA[j]);
                     if (two) {
                         if (!mbarWait(&S.aRead[j], (t >> 1) & 1u, abortFlag, p.err, 23)) break;
                         if (t >= 2 && !mbarWait(&S.bufFree[j], ((t >> 1) - 1u) & 1u, abortFlag, p.err, 25)) break;
                         tcFenceAfter();
-#pragma unroll
-                        for (uint32_t q4 = 0; q4 < 4; q4++) {
-                            mmaU8(tmem + kTmemBuf * j, smemDescSw128(aBase + 32u * q4),
-                                  smemDescSw128(bBase + kNodeBytes + 32u * q4), idescB, q4 > 0 ? 1u : 0u);
-                        }
-                        mmaCommit(&S.accB[j]);
+                        mmaU8x4(issuer, tmem + kTmemBuf * j, aDesc, 32u,
+                                smemDescSw128(smemAddr(S.b[slot]) + kNodeBytes), 32u, idescB, 0u);
+                        if (issuer) mmaCommit(&S.accB[j]);
                     }
-                    mmaCommit(&S.aEmpty[s]);
+                    if (issuer) mmaCommit(&S.aEmpty[s]);
                 }
-                if (lastOfGroupSmem(S, p, t0, nT, t, ti.group)) mmaCommit(&S.bEmpty[slot]);
+                if (lastOfGroupSmem(S, p, t0, nT, t, ti.group) && issuer) mmaCommit(&S.bEmpty[slot]);
             }
-            mmaCommit(&S.mmaDone);
+            if (issuer) mmaCommit(&S.mmaDone);
             mbarWait(&S.mmaDone, 0, abortFlag, p.err, 24);
         }
         __syncwarp();
