@@ -20,7 +20,7 @@
 // Queries (any number per launch, uneven sizes):
 //   * queryPrepKernel, one CTA per query: sort, query L1 norm (same order as documents), and
 //     the (level, word, run) entries that survive the skip rule;
-//   * scoreKernel, one CTA per query: warps take entries and add, for every document in the
+//   * scoreKernel, one or more CTAs per query and range of documents: warps take entries and add, for every document in the
 //     entry's postings, the reference's term |q - d| - (q + d), q = run*w*qRcp and
 //     d = tf*w*dRcp in float (DataBase.cpp:117,127-131; d read from the pair at the leaf
 //     level, formed from the summed tf at upper levels).  Each document's terms are summed in
@@ -35,6 +35,8 @@
 #include "timing.h"
 #include "tuning.h"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -42,16 +44,26 @@
 #include <optional>
 #include <shared_mutex>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 namespace rbw {
 namespace {
 
 constexpr uint32_t kMaxDocDesc = 32768;   // descriptors sorted in shared memory; larger ones in global memory
-constexpr uint32_t kPrepThreads = 512;
-constexpr uint32_t kScoreThreads = 1024;
-constexpr uint32_t kFlatList = 256;        // leaf lists shorter than this are walked flattened per warp batch
-constexpr uint32_t kFlatDepth = 8;         // pairs per lane in flight in the flattened walk
+constexpr uint32_t kPrepThreads = 512;      // documents, and queries of large batches
+constexpr uint32_t kPrepThreadsFew = 1024; // queries, when there are fewer than SMs
+constexpr uint32_t kMaxLevels = 8;         // Vocabulary::allocate
+constexpr uint32_t kScoreThreads = 1024;   // one inverted file per segment, and the merge
+constexpr uint32_t kScoreThreadsGrouped = 512; // grouped segments: two CTAs per SM
+constexpr uint32_t kScoreBatch = 4;        // entries a warp takes at a time
+constexpr uint32_t kListsAtOnce = 4;       // lists whose first pairs are loaded together
+constexpr uint32_t kUnionPairs = 256;      // pairs of an upper-level word gathered per warp
+constexpr uint32_t kUnionTfBits = 17;      // ... as local document (15 bits: kSmemDocs) and tf
+constexpr uint32_t kUnionTfMax = (1u << kUnionTfBits) - 1u;
+constexpr uint32_t kUnionDepth = 4;        // loads in flight per lane while gathering
+constexpr uint32_t kMaxParts = 8;          // CTAs that share a query's range of documents (a cluster)
+constexpr uint32_t kGroupedShards = 4;     // shards per CTA at most (80 KB of accumulators: two CTAs per SM)
 constexpr uint32_t kSegThreads = 256;
 constexpr uint32_t kSmemDocs = 20480;     // per-document accumulators kept in shared memory
 constexpr uint32_t kShardDocs = 2560;     // documents per inverted-file shard
@@ -66,7 +78,7 @@ struct Entry {
     uint32_t level;
     uint32_t word;   // index of the word within its level (= node index at level + 1)
     uint32_t run;    // query descriptors under this word
-    uint32_t widx;   // index into the weight table: levelBeg(level) * B + word
+    float weight;    // of the word
 };
 
 __host__ __device__ inline uint64_t levelBegDev(uint32_t B, uint32_t level)
@@ -81,6 +93,14 @@ __host__ __device__ inline uint64_t ipowDev(uint32_t b, uint32_t e)
     uint64_t r = 1;
     for (uint32_t i = 0; i < e; i++) r *= b;
     return r;
+}
+
+// v / B for any 32-bit v, from inverseB = ceil(2^64 / B): the error v (inverseB B - 2^64) / (B 2^64)
+// is below 1 / B, so the quotient is exact.
+__host__ __device__ inline uint64_t inverseOf(uint32_t B) { return ~0ull / B + 1; }
+__device__ __forceinline__ uint32_t divBranch(uint32_t v, uint64_t inverseB)
+{
+    return static_cast<uint32_t>((v * (inverseB >> 32) + __umulhi(v, static_cast<uint32_t>(inverseB))) >> 32);
 }
 
 uint32_t nextPow2(uint32_t n)
@@ -126,12 +146,90 @@ __device__ __forceinline__ uint32_t warpSlot(bool take, uint32_t* counter)
     return base + __popc(mask & ((1u << lane) - 1u));
 }
 
+// Ascending sort of nPow2 >= kSortSegment keys (shared or global memory), all threads of the CTA
+// taking part: the bitonic network, its strides below kSortSegment run in the registers of one warp
+// (lane l holds four consecutive keys: strides 1 and 2 in registers, 4 .. 64 by shuffles), so that
+// 2,048 keys take 15 barriers instead of 66.
+constexpr uint32_t kSortSegment = 128;
+__device__ __forceinline__ void keepOrdered(uint32_t& a, uint32_t& b, bool up)
+{
+    const uint32_t lo = min(a, b), hi = max(a, b);
+    a = up ? lo : hi;
+    b = up ? hi : lo;
+}
+__device__ __forceinline__ void sortSegmentStrides(uint32_t (&v)[4], uint32_t lane, uint32_t firstStride, bool up)
+{
+#pragma unroll
+    for (uint32_t j = kSortSegment / 2; j >= 4; j >>= 1) {
+        if (j > firstStride) continue;
+        const bool low = (lane & (j / 4)) == 0; // this lane holds the lower indices of its pairs
+#pragma unroll
+        for (uint32_t c = 0; c < 4; c++) {
+            const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, v[c], j / 4);
+            v[c] = low == up ? min(v[c], o) : max(v[c], o);
+        }
+    }
+    if (firstStride >= 2) {
+        keepOrdered(v[0], v[2], up);
+        keepOrdered(v[1], v[3], up);
+    }
+    keepOrdered(v[0], v[1], up);
+    keepOrdered(v[2], v[3], up);
+}
+__device__ void sortKeys(uint32_t* keys, uint32_t nPow2)
+{
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x / 32, nWarps = blockDim.x / 32;
+    uint4* quads = reinterpret_cast<uint4*>(keys);
+    for (uint32_t seg = warp; seg < nPow2 / kSortSegment; seg += nWarps) {
+        uint4 q = quads[seg * 32 + lane];
+        uint32_t v[4] = {q.x, q.y, q.z, q.w};
+        // k = 2: pairs (0, 1) ascending, (2, 3) descending
+        keepOrdered(v[0], v[1], true);
+        keepOrdered(v[2], v[3], false);
+#pragma unroll
+        for (uint32_t k = 4; k < kSortSegment; k <<= 1) sortSegmentStrides(v, lane, k / 2, (lane & (k / 4)) == 0);
+        sortSegmentStrides(v, lane, kSortSegment / 2, (seg & 1u) == 0 || nPow2 == kSortSegment);
+        quads[seg * 32 + lane] = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+    for (uint32_t k = 2 * kSortSegment; k <= nPow2; k <<= 1) {
+        for (uint32_t j = k / 2; j >= kSortSegment; j >>= 1) {
+            __syncthreads();
+            // four consecutive pairs (i, i | j) at a time
+            for (uint32_t t = threadIdx.x; t < nPow2 / 8; t += blockDim.x) {
+                const uint32_t t4 = 4 * t, i = ((t4 & ~(j - 1)) << 1) | (t4 & (j - 1));
+                const bool up = (i & k) == 0;
+                uint4 x = quads[i / 4], y = quads[(i | j) / 4];
+                keepOrdered(x.x, y.x, up);
+                keepOrdered(x.y, y.y, up);
+                keepOrdered(x.z, y.z, up);
+                keepOrdered(x.w, y.w, up);
+                quads[i / 4] = x;
+                quads[(i | j) / 4] = y;
+            }
+        }
+        __syncthreads();
+        for (uint32_t seg = warp; seg < nPow2 / kSortSegment; seg += nWarps) {
+            uint4 q = quads[seg * 32 + lane];
+            uint32_t v[4] = {q.x, q.y, q.z, q.w};
+            sortSegmentStrides(v, lane, kSortSegment / 2, ((seg * kSortSegment) & k) == 0);
+            quads[seg * 32 + lane] = make_uint4(v[0], v[1], v[2], v[3]);
+        }
+    }
+    __syncthreads();
+}
+// Keys a sort of n needs room for.
+__host__ __device__ inline uint32_t sortRoom(uint32_t n)
+{
+    uint32_t p = kSortSegment;
+    while (p < n) p <<= 1;
+    return p;
+}
+
 // Loads n leaf indices, sorts them and returns how many are valid (< nbLeaves): leaves out of
 // range sort to the end and are ignored, so a bad index never reaches a table lookup.
 __device__ uint32_t loadAndSort(const uint32_t* src, uint32_t n, uint32_t* keys, uint64_t nbLeaves, uint32_t* nValid)
 {
-    uint32_t nPow2 = 1;
-    while (nPow2 < n) nPow2 <<= 1;
+    const uint32_t nPow2 = sortRoom(n);
     if (threadIdx.x == 0) *nValid = 0;
     __syncthreads();
     uint32_t mine = 0;
@@ -140,9 +238,10 @@ __device__ uint32_t loadAndSort(const uint32_t* src, uint32_t n, uint32_t* keys,
         keys[i] = v;
         mine += v < nbLeaves ? 1u : 0u;
     }
-    atomicAdd(nValid, mine);
+    mine = __reduce_add_sync(0xFFFFFFFFu, mine);
+    if ((threadIdx.x & 31u) == 0 && mine) atomicAdd(nValid, mine);
     __syncthreads();
-    bitonicSortShared(keys, nPow2);
+    sortKeys(keys, nPow2);
     return *nValid;
 }
 
@@ -196,9 +295,11 @@ __device__ double l1NormWarp(const uint32_t* sorted, uint32_t n, const float* we
 // Call from every thread.  Returns false when this cannot be shown; the caller then adds the
 // terms in order (l1NormWarp) in one warp while the others go on.
 __device__ bool l1NormBlockExact(const uint32_t* sorted, uint32_t n, const float* weights, uint32_t B, uint32_t L,
-                                 double* norm)
+                                 uint64_t inverseB, double* norm)
 {
     constexpr uint32_t kTinyBits = uint32_t(127 - 70) << 23; // float bits of 2^-70
+    __shared__ uint64_t sBase[kMaxLevels]; // first weight of the level it above the leaves
+    if (threadIdx.x < L) sBase[threadIdx.x] = levelBegDev(B, L - 1 - threadIdx.x) * B;
     __shared__ int32_t sLsb;
     __shared__ uint32_t sBad, sMinBig, sMaxTiny, sTiny;
     __shared__ unsigned long long sTotal;
@@ -219,36 +320,54 @@ __device__ bool l1NormBlockExact(const uint32_t* sorted, uint32_t n, const float
     };
     int32_t lsb = 0x7FFFFFFF;
     uint32_t bad = 0, minBig = 0xFFFFFFFFu, maxTiny = 0, tiny = 0;
-    uint32_t span = 1;
-    for (uint32_t it = 0; it < L; it++) {
-        const float* lw = weights + levelBegDev(B, L - 1 - it) * B;
+    // f(bits) for the weight of every (level, descriptor), four levels' loads in flight at a time
+    auto forEachWeight = [&](auto f) {
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            const uint32_t bits = __float_as_uint(lw[sorted[i] / span]);
-            if ((bits & 0x7FFFFFFFu) == 0) continue; // +-0 adds nothing
-            if ((bits >> 31) != 0 || ((bits >> 23) & 0xFFu) == 0xFFu) {
-                bad = 1;                              // negative, infinite or NaN
-                continue;
+            uint32_t word = sorted[i];
+            for (uint32_t it0 = 0; it0 < L; it0 += 4) {
+                uint32_t bits[4];
+#pragma unroll
+                for (uint32_t u = 0; u < 4; u++) {
+                    bits[u] = 0; // adds nothing
+                    if (it0 + u < L) bits[u] = __float_as_uint(weights[sBase[it0 + u] + word]);
+                    word = divBranch(word, inverseB);
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < 4; u++) f(bits[u]);
             }
-            if (bits < kTinyBits) {                   // positive floats order like their bits
-                tiny++;
-                maxTiny = max(maxTiny, bits);
-                continue;
-            }
-            minBig = min(minBig, bits);
-            int32_t e0;
-            uint32_t m;
-            split(bits, e0, m);
-            lsb = min(lsb, e0 + int32_t(__ffs(m)) - 1);
         }
-        span *= B;
+    };
+    forEachWeight([&](uint32_t b) {
+        if ((b & 0x7FFFFFFFu) == 0) return; // +-0 adds nothing
+        if ((b >> 31) != 0 || ((b >> 23) & 0xFFu) == 0xFFu) {
+            bad = 1;                         // negative, infinite or NaN
+            return;
+        }
+        if (b < kTinyBits) {                 // positive floats order like their bits
+            tiny++;
+            maxTiny = max(maxTiny, b);
+            return;
+        }
+        minBig = min(minBig, b);
+        int32_t e0;
+        uint32_t m;
+        split(b, e0, m);
+        lsb = min(lsb, e0 + int32_t(__ffs(m)) - 1);
+    });
+    lsb = __reduce_min_sync(0xFFFFFFFFu, lsb);
+    minBig = __reduce_min_sync(0xFFFFFFFFu, minBig);
+    tiny = __reduce_add_sync(0xFFFFFFFFu, tiny);
+    maxTiny = __reduce_max_sync(0xFFFFFFFFu, maxTiny);
+    const bool anyBad = __any_sync(0xFFFFFFFFu, bad);
+    if ((threadIdx.x & 31u) == 0) {
+        atomicMin(&sLsb, lsb);
+        if (anyBad) atomicOr(&sBad, 1u);
+        if (tiny) {
+            atomicAdd(&sTiny, tiny);
+            atomicMax(&sMaxTiny, maxTiny);
+        }
+        atomicMin(&sMinBig, minBig);
     }
-    atomicMin(&sLsb, lsb);
-    if (bad) atomicOr(&sBad, 1u);
-    if (tiny) {
-        atomicAdd(&sTiny, tiny);
-        atomicMax(&sMaxTiny, maxTiny);
-    }
-    atomicMin(&sMinBig, minBig);
     __syncthreads();
     const int32_t e = sLsb;
     bool ok = !sBad;
@@ -267,32 +386,29 @@ __device__ bool l1NormBlockExact(const uint32_t* sorted, uint32_t n, const float
     }
     constexpr unsigned long long kLimit = 1ull << 53;
     unsigned long long total = 0;
-    span = 1;
-    for (uint32_t it = 0; it < L && !bad; it++) {
-        const float* lw = weights + levelBegDev(B, L - 1 - it) * B;
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            const uint32_t bits = __float_as_uint(lw[sorted[i] / span]);
-            if ((bits & 0x7FFFFFFFu) == 0 || bits < kTinyBits) continue;
-            int32_t e0;
-            uint32_t m;
-            split(bits, e0, m);
-            const int32_t tz = __ffs(m) - 1;
-            m >>= tz;                          // odd significand, lowest set bit 2^(e0 + tz)
-            const int32_t shift = e0 + tz - e; // >= 0: e is the lowest of those bits
-            if (shift + 32 - int32_t(__clz(m)) > 53) {
-                bad = 1;                       // the term alone reaches 2^(e + 53)
-                break;
-            }
-            total += static_cast<unsigned long long>(m) << shift;
-            if (total >= kLimit) {
-                bad = 1;
-                break;
-            }
+    forEachWeight([&](uint32_t b) {
+        if (bad || (b & 0x7FFFFFFFu) == 0 || b < kTinyBits) return;
+        int32_t e0;
+        uint32_t m;
+        split(b, e0, m);
+        const int32_t tz = __ffs(m) - 1;
+        m >>= tz;                          // odd significand, lowest set bit 2^(e0 + tz)
+        const int32_t shift = e0 + tz - e; // >= 0: e is the lowest of those bits
+        if (shift + 32 - int32_t(__clz(m)) > 53) {
+            bad = 1;                       // the term alone reaches 2^(e + 53)
+            return;
         }
-        span *= B;
+        total += static_cast<unsigned long long>(m) << shift;
+        if (total >= kLimit) bad = 1;
+    });
+    // one 64-bit shared atomic (a compare-and-swap loop) per warp; < blockDim * 2^53: no overflow
+#pragma unroll
+    for (uint32_t off = 16; off > 0; off >>= 1) total += __shfl_xor_sync(0xFFFFFFFFu, total, off);
+    const bool nowBad = __any_sync(0xFFFFFFFFu, bad);
+    if ((threadIdx.x & 31u) == 0) {
+        if (nowBad) atomicOr(&sBad, 1u);
+        atomicAdd(&sTotal, total);
     }
-    if (bad) atomicOr(&sBad, 1u);
-    atomicAdd(&sTotal, total); // < blockDim * 2^53: no overflow
     __syncthreads();
     if (sBad || sTotal >= kLimit) return false;
     *norm = ldexp(static_cast<double>(sTotal), e);
@@ -307,10 +423,10 @@ __device__ bool l1NormBlockExact(const uint32_t* sorted, uint32_t n, const float
 __global__ void __launch_bounds__(kPrepThreads) docPrepKernel(const uint32_t* newLeaves, const uint64_t* docOff,
                                                               uint32_t s0, const uint32_t* slotList, uint32_t* gkeys,
                                                               uint32_t gstride, const float* weights, uint32_t B,
-                                                              uint32_t L, uint64_t nbLeaves, float* rcpF,
-                                                              uint64_t* docPairs, uint32_t* pairCount)
+                                                              uint32_t L, uint64_t nbLeaves, uint64_t inverseB,
+                                                              float* rcpF, uint64_t* docPairs, uint32_t* pairCount)
 {
-    extern __shared__ uint32_t skeys[];
+    extern __shared__ __align__(16) uint32_t skeys[];
     __shared__ uint32_t cnt, nValid;
     const uint32_t slot = gkeys ? slotList[blockIdx.x] : s0 + blockIdx.x;
     const uint64_t beg = docOff[slot];
@@ -320,7 +436,7 @@ __global__ void __launch_bounds__(kPrepThreads) docPrepKernel(const uint32_t* ne
     if (threadIdx.x == 0) cnt = 0;
     const uint32_t n = loadAndSort(newLeaves + (beg - docOff[s0]), nAll, keys, nbLeaves, &nValid);
     double norm = 0;
-    if (l1NormBlockExact(keys, n, weights, B, L, &norm)) {
+    if (l1NormBlockExact(keys, n, weights, B, L, inverseB, &norm)) {
         if (threadIdx.x == 0) rcpF[slot] = float(1 / norm); // DataBase.cpp:68
     } else if (threadIdx.x < 32) {
         norm = l1NormWarp(keys, n, weights, B, L);
@@ -417,18 +533,21 @@ __global__ void wordPostKernel(unsigned long long* wordPost, uint32_t B, uint32_
 }
 
 // ------------------------------------------------------------------ queries
-// One CTA per query: without gkeys CTA i prepares query i in shared memory (skipping queries
+// One CTA per query (a query of 1,733 leaves: 26 us, of which a third is the sort; 56 us with the sort's
+// strides all through shared memory, a division per weight and 64-bit shared atomics, which are
+// compare-and-swap loops, from every thread): without gkeys CTA i prepares query i in shared memory (skipping queries
 // above kMaxDocDesc descriptors); with gkeys CTA i prepares query qList[i] in its gstride-word
 // slice of gkeys.
-__global__ void __launch_bounds__(kPrepThreads) queryPrepKernel(const uint32_t* qLeaves, const uint64_t* qOff,
+__global__ void __launch_bounds__(kPrepThreadsFew) queryPrepKernel(const uint32_t* qLeaves, const uint64_t* qOff,
                                                                 const uint32_t* qList, uint32_t* gkeys,
                                                                 uint32_t gstride, const float* weights,
                                                                 const unsigned long long* wordPost, uint32_t B,
-                                                                uint32_t L, uint64_t nbLeaves, uint32_t k,
+                                                                uint32_t L, uint64_t nbLeaves, uint64_t inverseB,
+                                                                uint32_t k,
                                                                 float* qRcpF, Entry* entries, uint32_t* entryCount,
                                                                 unsigned long long* work)
 {
-    extern __shared__ uint32_t skeys[];
+    extern __shared__ __align__(16) uint32_t skeys[];
     __shared__ uint32_t cnt, nValid;
     __shared__ unsigned long long workSum;
     const uint32_t q = gkeys ? qList[blockIdx.x] : blockIdx.x;
@@ -443,7 +562,7 @@ __global__ void __launch_bounds__(kPrepThreads) queryPrepKernel(const uint32_t* 
     }
     const uint32_t n = loadAndSort(qLeaves + beg, nAll, keys, nbLeaves, &nValid);
     double norm = 0;
-    if (l1NormBlockExact(keys, n, weights, B, L, &norm)) {
+    if (l1NormBlockExact(keys, n, weights, B, L, inverseB, &norm)) {
         if (threadIdx.x == 0) qRcpF[q] = float(1 / norm); // DataBase.cpp:77-94
     } else if (threadIdx.x < 32) {
         norm = l1NormWarp(keys, n, weights, B, L); // while the other warps build the entries
@@ -455,29 +574,46 @@ __global__ void __launch_bounds__(kPrepThreads) queryPrepKernel(const uint32_t* 
     for (uint32_t it = 0; it < L; it++) {
         const uint32_t level = L - 1 - it;
         const uint64_t base = levelBegDev(B, level) * B;
-        for (uint32_t i0 = 0; i0 < n; i0 += blockDim.x) {
-            const uint32_t i = i0 + threadIdx.x;
-            const uint32_t word = i < n ? keys[i] / span : 0u;
-            bool keep = false;
-            uint32_t run = 0;
-            uint64_t widx = 0;
-            if (i < n && (i == 0 || keys[i - 1] / span != word)) {
-                // the run of `word` ends at the first key >= (word + 1) * span (keys are sorted)
-                const uint64_t end = (uint64_t(word) + 1) * span;
-                uint32_t lo = i + 1, hi = n;
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (keys[mid] < end) lo = mid + 1;
-                    else hi = mid;
+        // two descriptors per thread at a time: their searches and count reads overlap
+        constexpr uint32_t kAtOnce = 2;
+        for (uint32_t i0 = 0; i0 < n; i0 += kAtOnce * blockDim.x) {
+            uint32_t word[kAtOnce], lo[kAtOnce], hi[kAtOnce];
+            bool head[kAtOnce];
+#pragma unroll
+            for (uint32_t u = 0; u < kAtOnce; u++) {
+                const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
+                word[u] = i < n ? keys[i] : 0u;
+                uint32_t before = i < n && i > 0 ? keys[i - 1] : 0u;
+                for (uint32_t up = 0; up < it; up++) {
+                    word[u] = divBranch(word[u], inverseB);
+                    before = divBranch(before, inverseB);
                 }
-                run = lo - i;
-                widx = base + word;
-                const unsigned long long post = wordPost[widx];
-                keep = it == 0 || post < limit;
-                if (keep) myWork += post + 1ull;
+                head[u] = i < n && (i == 0 || before != word[u]);
+                lo[u] = i + 1;
+                hi[u] = head[u] ? n : i + 1;
             }
-            const uint32_t p = warpSlot(keep, &cnt);
-            if (keep) out[p] = Entry{level, word, run, static_cast<uint32_t>(widx)};
+            // the run of `word` ends at the first key >= (word + 1) * span (keys are sorted)
+            for (uint32_t left = n; left > 0; left >>= 1) {
+#pragma unroll
+                for (uint32_t u = 0; u < kAtOnce; u++) {
+                    if (lo[u] < hi[u]) {
+                        const uint32_t mid = (lo[u] + hi[u]) >> 1;
+                        if (keys[mid] < (uint64_t(word[u]) + 1) * span) lo[u] = mid + 1;
+                        else hi[u] = mid;
+                    }
+                }
+            }
+            unsigned long long post[kAtOnce];
+#pragma unroll
+            for (uint32_t u = 0; u < kAtOnce; u++) post[u] = head[u] ? wordPost[base + word[u]] : 0ull;
+#pragma unroll
+            for (uint32_t u = 0; u < kAtOnce; u++) {
+                const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
+                const bool keep = head[u] && (it == 0 || post[u] < limit);
+                if (keep) myWork += post[u] + 1ull;
+                const uint32_t p = warpSlot(keep, &cnt);
+                if (keep) out[p] = Entry{level, word[u], lo[u] - i, weights[base + word[u]]};
+            }
         }
         span *= B;
     }
@@ -552,9 +688,13 @@ __device__ __forceinline__ float termOf(float q, float d) { return fabsf(q - d) 
 __device__ __forceinline__ void addTerm(unsigned long long* acc, uint32_t i, float term)
 {
     // term * 2^56 is exact in fp32 (|term| <= 2, a power-of-two scale), so rounding it to the
-    // nearest integer in fp32 gives the value llrint(double(term) * 2^56) would, without FP64
-    const long long fx = __float2ll_rn(term * 0x1p56f);
-    atomicAdd(&acc[i], static_cast<unsigned long long>(fx < 0 ? fx : -1ll));
+    // nearest integer in fp32 gives the value llrint(double(term) * 2^56) would, without FP64;
+    // terms above -1 unit count as -1 (min.NaN keeps a NaN, which the conversion turns into the
+    // lowest integer)
+    float scaled;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(scaled) : "f"(term * 0x1p56f), "f"(-1.0f));
+    const long long fx = __float2ll_rn(scaled);
+    atomicAdd(&acc[i], static_cast<unsigned long long>(fx));
 }
 
 // Float bits mapped so that unsigned order is numeric order (negative scores included).
@@ -568,27 +708,60 @@ __device__ __forceinline__ float fromOrderedBits(uint32_t o)
     return __uint_as_float((o & 0x80000000u) ? (o & 0x7FFFFFFFu) : ~o);
 }
 
-// The `want` smallest of n distinct keys (~0 = no key), ascending, into sel[0, want): radix
-// select of the want-th smallest key, 8 bits at a time, then a bitonic sort of the winners.
-// All threads of the CTA call it; keys and sel may live in shared or global memory; selCap is a
-// power of two >= want.
+// The `want` smallest of n distinct keys (~0 = no key), ascending, into sel[0, want): radix select of
+// the want-th smallest key, then a sort of the winners.  The digits (8 bits) start at the highest bit
+// in which the keys differ -- scores share their sign, exponent and leading bits, so digits from bit 63
+// down would put every key into one counter twice -- and stop when every key of the digit found is
+// wanted.  All threads of the CTA call it; keys and sel may live in shared or global memory; selCap is
+// a power of two >= want.
+constexpr uint32_t kRankSort = 256; // winners sorted by counting the smaller ones; more by the bitonic network
 __device__ __forceinline__ void selectSmallest(const unsigned long long* keys, uint32_t n, uint32_t want,
                                                unsigned long long* sel, uint32_t selCap)
 {
     __shared__ uint32_t hist[256];
-    __shared__ unsigned long long prefix;
-    __shared__ uint32_t need, nSel;
+    __shared__ unsigned long long prefix, warpMin[32], warpMax[32];
+    __shared__ uint32_t need, nSel, done;
+    const uint32_t lane = threadIdx.x & 31u;
     if (threadIdx.x == 0) {
-        prefix = 0;
         nSel = 0;
         need = want;
+        done = 0;
     }
     __syncthreads();
     if (want > 0) {
-        for (int shift = 56; shift >= 0; shift -= 8) {
+        unsigned long long lo = ~0ull, hi = 0;
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+            const unsigned long long key = keys[i];
+            if (key != ~0ull) {
+                lo = min(lo, key);
+                hi = max(hi, key);
+            }
+        }
+#pragma unroll
+        for (uint32_t off = 16; off > 0; off >>= 1) {
+            lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, off));
+            hi = max(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, off));
+        }
+        // (64-bit shared atomics are compare-and-swap loops: one value per warp instead)
+        if (lane == 0) {
+            warpMin[threadIdx.x / 32] = lo;
+            warpMax[threadIdx.x / 32] = hi;
+        }
+        __syncthreads();
+        lo = lane < blockDim.x / 32 ? warpMin[lane] : ~0ull;
+        hi = lane < blockDim.x / 32 ? warpMax[lane] : 0ull;
+#pragma unroll
+        for (uint32_t off = 16; off > 0; off >>= 1) {
+            lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, off));
+            hi = max(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, off));
+        }
+        // bits above `shift` + 8 are the same in every key
+        int shift = max(0, 63 - __clzll((lo ^ hi) | 1ull) - 7);
+        unsigned long long hiMask = shift + 8 >= 64 ? 0ull : ~0ull << (shift + 8);
+        if (threadIdx.x == 0) prefix = lo & hiMask;
+        for (;;) {
             for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
             __syncthreads();
-            const unsigned long long hiMask = shift == 56 ? 0ull : (~0ull << (shift + 8));
             for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
                 const unsigned long long key = keys[i];
                 if (key != ~0ull && (key & hiMask) == prefix) atomicAdd(&hist[(key >> shift) & 0xFFu], 1u);
@@ -597,7 +770,6 @@ __device__ __forceinline__ void selectSmallest(const unsigned long long* keys, u
             if (threadIdx.x < 32) {
                 // d = the first digit below 255 whose inclusive count reaches `need`, else 255;
                 // c = the count of the digits before d.  Lane l holds digits 8l .. 8l + 7.
-                const uint32_t lane = threadIdx.x;
                 uint32_t h[8], incl[8], run = 0;
 #pragma unroll
                 for (uint32_t j = 0; j < 8; j++) {
@@ -613,11 +785,12 @@ __device__ __forceinline__ void selectSmallest(const unsigned long long* keys, u
                 }
                 before -= run; // digits of the lower lanes
                 const uint32_t nd = need;
-                uint32_t jHit = 8, cHit = 0;
+                uint32_t jHit = 8, cHit = 0, hHit = 0;
 #pragma unroll
                 for (int j = 7; j >= 0; j--) {
                     if (8 * lane + j < 255 && before + incl[j] >= nd) {
                         jHit = j;
+                        hHit = h[j];
                         cHit = before + incl[j] - h[j];
                     }
                 }
@@ -628,11 +801,20 @@ __device__ __forceinline__ void selectSmallest(const unsigned long long* keys, u
                     const uint32_t c = hitLanes ? cHit : before + incl[6]; // else digits 0 .. 254
                     need = nd - c;
                     prefix |= static_cast<unsigned long long>(d) << shift;
+                    // every key of this digit is wanted: the bound is the digit's last value
+                    if ((hitLanes ? hHit : h[7]) == nd - c) {
+                        prefix |= (1ull << shift) - 1ull;
+                        done = 1;
+                    }
                 }
             }
             __syncthreads();
+            if (done || shift == 0) break;
+            const int next = max(0, shift - 8);
+            hiMask = ~0ull << shift;
+            shift = next;
         }
-        // prefix is the want-th smallest key; keys are distinct, so exactly `want` are <= prefix
+        // `prefix` bounds the want-th smallest key; keys are distinct, so exactly `want` are <= prefix
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
             const unsigned long long key = keys[i];
             if (key <= prefix) {
@@ -643,6 +825,18 @@ __device__ __forceinline__ void selectSmallest(const unsigned long long* keys, u
     }
     __syncthreads();
     const uint32_t m = nSel < selCap ? nSel : selCap;
+    if (m <= kRankSort && m <= blockDim.x) {
+        unsigned long long mine = 0;
+        uint32_t rank = 0;
+        if (threadIdx.x < m) {
+            mine = sel[threadIdx.x];
+            for (uint32_t j = 0; j < m; j++) rank += sel[j] < mine ? 1u : 0u;
+        }
+        __syncthreads();
+        if (threadIdx.x < m) sel[rank] = mine;
+        __syncthreads();
+        return;
+    }
     uint32_t mPow2 = 1;
     while (mPow2 < m) mPow2 <<= 1;
     for (uint32_t i = m + threadIdx.x; i < mPow2; i += blockDim.x) sel[i] = ~0ull;
@@ -664,14 +858,26 @@ __device__ __forceinline__ void writeResults(const ScoreParams& P, uint32_t q, c
 // csrPerCta shards only (one range per leaf word); upper-level words read their group's range
 // and keep the CTA's documents.  A single-layout segment is walked by every CTA of the query,
 // each keeping the postings of its range.  kSharded = false: one range holds every document and
-// no posting needs the range test.
-template <bool kSharded, uint32_t kThreads>
+// no posting needs the range test.  kParts: the blockIdx.z CTAs of a cluster take the entries in
+// turn, each into its own accumulators; their sums are added through distributed shared memory
+// (integers, so in any order) and the first CTA selects.
+//
+// A large batch is bound by the 64-bit shared atomics: 7.7 cycles per warp of random addresses in
+// isolation, 8.8 per 32 pairs here (256 queries against 20,000 images whose longest lists hold a
+// third of the documents: 1.17 ms, 1.35 ms with one CTA of 1,024 threads per query, where the
+// longest query's CTA ran alone at the end).  A single query is bound by load latency, so it is
+// spread over up to 64 CTAs per 20,480 documents: 39 us, 141 us with one CTA per 2,560.
+template <bool kSharded, bool kGrouped, uint32_t kThreads, bool kParts>
 __global__ void __launch_bounds__(kThreads, kThreads >= 1024 ? 1 : 1024 / kThreads) scoreKernel(ScoreParams P)
 {
     extern __shared__ unsigned long long dyn[];
     __shared__ uint32_t nTouched;
     __shared__ uint32_t nextBatch; // entry batches are handed to warps as they finish
-    __shared__ unsigned long long sel[kMaxK];
+    __shared__ union {
+        uint32_t unionBuf[kThreads / 32][kUnionPairs]; // while the entries are walked
+        unsigned long long sel[kMaxK];                 // while the results are selected
+    } u;
+    unsigned long long* sel = u.sel;
     const uint32_t q = P.order ? P.order[blockIdx.x] : blockIdx.x;
     const uint32_t shard = blockIdx.y;
     const uint32_t docBeg = kSharded ? shard * P.shardDocs : 0u;
@@ -714,117 +920,188 @@ __global__ void __launch_bounds__(kThreads, kThreads >= 1024 ? 1 : 1024 / kThrea
             b = t[hi * kGroupShards];
         }
     };
-    auto addPair = [&](uint64_t pr, float qv) {
-        const uint32_t i = static_cast<uint32_t>(pr >> 32) - docBeg;
-        if (!kSharded || i < nLocal) addTerm(acc, i, termOf(qv, __uint_as_float(static_cast<uint32_t>(pr))));
+    // Two pairs of a leaf word's list [a, b), at positions `at` (even) and at + 1.  A grouped range
+    // holds documents of this CTA only.
+    auto addPair = [&](uint32_t slot, uint32_t d, float qv) {
+        const uint32_t i = slot - docBeg;
+        if (!kSharded || kGrouped || i < nLocal) addTerm(acc, i, termOf(qv, __uint_as_float(d)));
     };
-    // A leaf word's list [a, b) by the whole warp, eight pairs per lane in flight.
-    auto leafList = [&](const uint64_t* pairs, uint32_t a, uint32_t b, float qv) {
-        uint32_t p = a + lane;
-        for (; p + 224 < b; p += 256) {
-            uint64_t pr[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) pr[u] = pairs[p + 32 * u];
-#pragma unroll
-            for (int u = 0; u < 8; u++) addPair(pr[u], qv);
-        }
-        for (; p < b; p += 32) addPair(pairs[p], qv);
+    auto addPairs = [&](const uint4& v, uint32_t at, uint32_t a, uint32_t b, float qv) {
+        if (at >= a && at < b) addPair(v.y, v.x, qv);
+        if (at + 1 < b) addPair(v.w, v.z, qv);
+    };
+    auto loadPairs = [&](const uint64_t* pairs, uint32_t at, uint32_t b) {
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (at < b)
+            asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                         : "l"(pairs + at));
+        return v;
     };
     // Virtual inverted file of a non-leaf word: the union of the leaf lists below it, counted
     // per document (DataBase.cpp:150-164).  A document lives in one segment only, and the skip
-    // rule keeps the union short, so each lane scans the range for the documents of this shard
-    // whose first pair it holds.
+    // rule keeps the union short.  The pairs of this CTA's documents are gathered into the warp's
+    // buffer as (local document, tf), and each lane adds up the tf of the documents whose first
+    // entry it holds there.
+    auto virtualTerm = [&](uint32_t i, uint32_t tf, float w, float qv) {
+        const float d = float(tf) * w * P.rcpF[docBeg + i];
+        addTerm(acc, i, termOf(qv, d));
+    };
     auto virtualList = [&](int s, uint32_t a, uint32_t b, float w, float qv) {
         const uint64_t* pairs = P.seg[s].pairs;
+        const uint32_t* tfs = P.seg[s].tf;
+        uint32_t* buf = u.unionBuf[threadIdx.x / 32];
+        uint32_t m = 0;
+        bool fits = true;
+        for (uint32_t p0 = a; p0 < b && fits; p0 += 32u * kUnionDepth) {
+            uint32_t local[kUnionDepth], tf[kUnionDepth];
+#pragma unroll
+            for (uint32_t c = 0; c < kUnionDepth; c++) {
+                const uint32_t p = p0 + 32u * c + lane;
+                local[c] = p < b ? static_cast<uint32_t>(pairs[p] >> 32) - docBeg : 0xFFFFFFFFu;
+            }
+#pragma unroll
+            for (uint32_t c = 0; c < kUnionDepth; c++) tf[c] = local[c] < nLocal ? tfs[p0 + 32u * c + lane] : 0u;
+#pragma unroll
+            for (uint32_t c = 0; c < kUnionDepth; c++) {
+                const bool in = local[c] < nLocal;
+                const uint32_t mask = __ballot_sync(0xFFFFFFFFu, in);
+                const uint32_t at = m + __popc(mask & ((1u << lane) - 1u));
+                m += __popc(mask);
+                fits = fits && m <= kUnionPairs && !__any_sync(0xFFFFFFFFu, tf[c] > kUnionTfMax);
+                if (in && fits) buf[at] = (local[c] << kUnionTfBits) | tf[c];
+            }
+        }
+        if (fits) {
+            __syncwarp();
+            for (uint32_t i0 = 0; i0 < m; i0 += 32) {
+                const uint32_t i = i0 + lane;
+                const uint32_t mine = i < m ? buf[i] : 0xFFFFFFFFu;
+                uint32_t tf = 0;
+                bool first = i < m;
+#pragma unroll 4
+                for (uint32_t j = 0; j < m; j++) {
+                    const uint32_t v = buf[j];
+                    const bool same = ((v ^ mine) >> kUnionTfBits) == 0;
+                    tf += same ? v & kUnionTfMax : 0u;
+                    first = first && !(same && j < i);
+                }
+                if (first) virtualTerm(mine >> kUnionTfBits, tf, w, qv);
+            }
+            __syncwarp(); // the buffer is reused by the next word
+            return;
+        }
+        // more pairs of this CTA's documents than the buffer holds (large k), or a huge tf: each
+        // lane scans the range for the documents whose first pair it holds
         for (uint32_t p = a + lane; p < b; p += 32) {
             const uint32_t slot = static_cast<uint32_t>(pairs[p] >> 32);
-            if (kSharded && slot - docBeg >= nLocal) continue;
+            if (slot - docBeg >= nLocal) continue;
             bool first = true;
             for (uint32_t r = a; r < p && first; r++) first = static_cast<uint32_t>(pairs[r] >> 32) != slot;
             if (!first) continue;
             uint32_t tf = 0;
             for (uint32_t r = p; r < b; r++)
-                if (static_cast<uint32_t>(pairs[r] >> 32) == slot) tf += P.seg[s].tf[r];
-            const float d = float(tf) * w * P.rcpF[slot];
-            addTerm(acc, slot - docBeg, termOf(qv, d));
+                if (static_cast<uint32_t>(pairs[r] >> 32) == slot) tf += tfs[r];
+            virtualTerm(slot - docBeg, tf, w, qv);
         }
+        __syncwarp();
     };
-    // Entries in batches of 32 per warp: lane j fetches entry base + j, its weight and its
-    // offsets in both segments, so these loads overlap instead of chaining entry after entry.
-    // Leaf lists shorter than kFlatList are then walked as one range over the batch (lane t of
-    // a round takes pair t of the concatenated lists, kFlatDepth pairs per lane in flight);
-    // longer lists and non-leaf words go one at a time with the whole warp.
-    for (;;) {
+    // Entries in batches of kScoreBatch per warp, lane j holding entry j's weight and its pair ranges
+    // in both segments; the next batch's are loaded while the current one's lists are walked.  (The
+    // longest lists hold a third of the documents: with 32 entries per batch, 53 batches of a query
+    // of 1,700 words, the last warps to finish held up the CTA.)
+    struct Batch {
+        float qv, w;
+        uint32_t a0, b0, a1, b1;
+        bool live, leaf;
+    };
+    auto fetch = [&](Batch& f) -> bool {
         uint32_t batch = 0;
         if (lane == 0) batch = atomicAdd(&nextBatch, 1u);
-        const uint32_t base = __shfl_sync(0xFFFFFFFFu, batch, 0) * 32u;
-        if (base >= ne) break;
-        const uint32_t e = base + lane;
-        const bool valid = e < ne;
-        float qv = 0.f, w = 0.f;
-        bool leaf = false;
-        uint32_t a0 = 0, b0 = 0, a1 = 0, b1 = 0;
-        if (valid) {
-            const Entry en = ent[e];
-            w = P.weights[en.widx];
-            qv = float(en.run) * w * qRcp;
-            leaf = en.level == P.L - 1;
+        batch = __shfl_sync(0xFFFFFFFFu, batch, 0);
+        if (kParts) batch = batch * gridDim.z + blockIdx.z;
+        const uint32_t base = batch * kScoreBatch;
+        f = Batch{0.f, 0.f, 0u, 0u, 0u, 0u, false, false};
+        if (base >= ne) return false;
+        if (lane < kScoreBatch && base + lane < ne) {
+            const Entry en = ent[base + lane];
+            f.live = true;
+            f.w = en.weight;
+            f.qv = float(en.run) * en.weight * qRcp;
+            f.leaf = en.level == P.L - 1;
             const uint64_t span = ipowDev(P.B, P.L - 1 - en.level);
             const uint64_t lo = uint64_t(en.word) * span;
-            wordRange(0, lo, lo + span, leaf, a0, b0);
-            wordRange(1, lo, lo + span, leaf, a1, b1);
+            wordRange(0, lo, lo + span, f.leaf, f.a0, f.b0);
+            wordRange(1, lo, lo + span, f.leaf, f.a1, f.b1);
         }
-        const uint32_t len = (b0 - a0) + (b1 - a1);
-        const bool flat = valid && leaf && len < kFlatList;
-        for (uint32_t one = __ballot_sync(0xFFFFFFFFu, valid && !flat); one != 0; one &= one - 1) {
-            const uint32_t j = __ffs(one) - 1;
-            const uint32_t ja0 = __shfl_sync(0xFFFFFFFFu, a0, j), jb0 = __shfl_sync(0xFFFFFFFFu, b0, j);
-            const uint32_t ja1 = __shfl_sync(0xFFFFFFFFu, a1, j), jb1 = __shfl_sync(0xFFFFFFFFu, b1, j);
-            const float jq = __shfl_sync(0xFFFFFFFFu, qv, j), jw = __shfl_sync(0xFFFFFFFFu, w, j);
-            if (__shfl_sync(0xFFFFFFFFu, leaf, j)) {
-                leafList(P.seg[0].pairs, ja0, jb0, jq);
-                leafList(P.seg[1].pairs, ja1, jb1, jq);
-            } else {
-                virtualList(0, ja0, jb0, jw, jq);
-                virtualList(1, ja1, jb1, jw, jq);
+        return true;
+    };
+    Batch cur, next;
+    for (bool have = fetch(cur); have;) {
+        const bool more = fetch(next);
+#pragma unroll 1
+        for (int s = 0; s < 2; s++) {
+            const uint32_t a = s ? cur.a1 : cur.a0, b = s ? cur.b1 : cur.b0;
+            if (!__any_sync(0xFFFFFFFFu, a < b)) continue;
+            const uint64_t* pairs = P.seg[s].pairs;
+            // upper-level words one at a time
+            for (uint32_t one = __ballot_sync(0xFFFFFFFFu, cur.live && !cur.leaf); one != 0; one &= one - 1) {
+                const uint32_t j = __ffs(one) - 1;
+                virtualList(s, __shfl_sync(0xFFFFFFFFu, a, j), __shfl_sync(0xFFFFFFFFu, b, j),
+                            __shfl_sync(0xFFFFFFFFu, cur.w, j), __shfl_sync(0xFFFFFFFFu, cur.qv, j));
             }
-        }
-        const uint32_t c0 = flat ? b0 - a0 : 0u;
-        const uint32_t cnt = flat ? len : 0u;
-        uint32_t incl = cnt;
+            // Leaf lists by the whole warp, two pairs per lane and load: the first 64 pairs of
+            // kListsAtOnce lists together (short lists), then the rest of each, 256 pairs at a time.
+            const uint32_t endOf = cur.leaf ? b : a; // empty unless a leaf word
+#pragma unroll 1
+            for (uint32_t j0 = 0; j0 < kScoreBatch; j0 += kListsAtOnce) {
+                uint32_t la[kListsAtOnce], lb[kListsAtOnce];
+                float lq[kListsAtOnce];
+                uint4 v[kListsAtOnce];
 #pragma unroll
-        for (uint32_t off = 1; off < 32; off <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, off);
-            if (lane >= off) incl += v;
-        }
-        const uint32_t excl = incl - cnt;
-        const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        for (uint32_t f0 = 0; f0 < total; f0 += 32u * kFlatDepth) {
-            uint64_t pr[kFlatDepth];
-            float pq[kFlatDepth];
-#pragma unroll
-            for (uint32_t u = 0; u < kFlatDepth; u++) {
-                const uint32_t t = f0 + 32u * u + lane;
-                // owner lane: the last j with excl_j <= t (excl is non-decreasing; it holds pairs)
-                uint32_t j = 0;
-#pragma unroll
-                for (uint32_t step = 16; step > 0; step >>= 1) {
-                    const uint32_t v = __shfl_sync(0xFFFFFFFFu, excl, j + step);
-                    if (v <= t) j += step;
+                for (uint32_t k = 0; k < kListsAtOnce; k++) {
+                    la[k] = __shfl_sync(0xFFFFFFFFu, a, j0 + k);
+                    lb[k] = __shfl_sync(0xFFFFFFFFu, endOf, j0 + k);
+                    lq[k] = __shfl_sync(0xFFFFFFFFu, cur.qv, j0 + k);
+                    v[k] = loadPairs(pairs, (la[k] & ~1u) + 2 * lane, lb[k]);
                 }
-                const uint32_t off = t - __shfl_sync(0xFFFFFFFFu, excl, j);
-                const uint32_t jc0 = __shfl_sync(0xFFFFFFFFu, c0, j);
-                const uint32_t ja0 = __shfl_sync(0xFFFFFFFFu, a0, j), ja1 = __shfl_sync(0xFFFFFFFFu, a1, j);
-                pq[u] = __shfl_sync(0xFFFFFFFFu, qv, j);
-                pr[u] = 0;
-                if (t < total) pr[u] = off < jc0 ? P.seg[0].pairs[ja0 + off] : P.seg[1].pairs[ja1 + off - jc0];
-            }
 #pragma unroll
-            for (uint32_t u = 0; u < kFlatDepth; u++)
-                if (f0 + 32u * u + lane < total) addPair(pr[u], pq[u]);
+                for (uint32_t k = 0; k < kListsAtOnce; k++)
+                    addPairs(v[k], (la[k] & ~1u) + 2 * lane, la[k], lb[k], lq[k]);
+#pragma unroll
+                for (uint32_t k = 0; k < kListsAtOnce; k++) {
+#pragma unroll 1
+                    for (uint32_t p0 = (la[k] & ~1u) + 64; p0 < lb[k]; p0 += 256) {
+                        uint4 w[4];
+#pragma unroll
+                        for (uint32_t c = 0; c < 4; c++) w[c] = loadPairs(pairs, p0 + 64 * c + 2 * lane, lb[k]);
+#pragma unroll
+                        for (uint32_t c = 0; c < 4; c++)
+                            addPairs(w[c], p0 + 64 * c + 2 * lane, la[k], lb[k], lq[k]);
+                    }
+                }
+            }
         }
+        cur = next;
+        have = more;
     }
     __syncthreads();
+    if (kParts) {
+        namespace cg = cooperative_groups;
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync(); // every part's sums are complete
+        const uint32_t parts = gridDim.z, rank = blockIdx.z;
+        unsigned long long* first = cluster.map_shared_rank(dyn, 0);
+        // this CTA adds up the documents [d0, d1); the first CTA's sums receive them
+        const uint32_t d0 = uint32_t(uint64_t(nLocal) * rank / parts), d1 = uint32_t(uint64_t(nLocal) * (rank + 1) / parts);
+        for (uint32_t i = d0 + threadIdx.x; i < d1; i += blockDim.x) {
+            unsigned long long sum = 0;
+            for (uint32_t r = 0; r < parts; r++) sum += cluster.map_shared_rank(dyn, r)[i];
+            first[i] = sum;
+        }
+        cluster.sync(); // the sums have arrived, and no CTA's memory is read any more
+        if (rank != 0) return;
+    }
 
     // Keys: ordered score bits << 32 | document id.  Ties in score go to the lower document id;
     // untouched documents get ~0.
@@ -839,7 +1116,8 @@ __global__ void __launch_bounds__(kThreads, kThreads >= 1024 ? 1 : 1024 / kThrea
         }
         acc[i] = key;
     }
-    atomicAdd(&nTouched, myTouched);
+    myTouched = __reduce_add_sync(0xFFFFFFFFu, myTouched);
+    if (lane == 0 && myTouched) atomicAdd(&nTouched, myTouched);
     __syncthreads();
     const uint32_t want = P.k < nTouched ? P.k : nTouched;
     unsigned long long* selp = P.selGlobal ? P.selGlobal + (uint64_t(q) * gridDim.y + shard) * P.selStride : sel;
@@ -864,7 +1142,8 @@ __global__ void __launch_bounds__(kScoreThreads) mergeKernel(ScoreParams P, uint
     __syncthreads();
     uint32_t mine = 0;
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) mine += c[i] != ~0ull ? 1u : 0u;
-    atomicAdd(&nValid, mine);
+    mine = __reduce_add_sync(0xFFFFFFFFu, mine);
+    if ((threadIdx.x & 31u) == 0 && mine) atomicAdd(&nValid, mine);
     __syncthreads();
     const uint32_t want = P.k < nValid ? P.k : nValid;
     unsigned long long* selp = P.selGlobal ? P.selGlobal + uint64_t(q) * shards * P.selStride : sel;
@@ -926,19 +1205,40 @@ struct Segment {
 constexpr int kPrepSmemMax = int(kMaxDocDesc) * 4;
 constexpr int kScoreSmemMax = int(kSmemDocs) * 8;
 
-template <uint32_t kThreads>
-void launchScore(bool sharded, dim3 grid, size_t smem, cudaStream_t stream, const ScoreParams& P)
+template <bool kSharded, bool kGrouped, uint32_t kThreads, bool kParts>
+void launchScoreAs(dim3 grid, size_t smem, cudaStream_t stream, const ScoreParams& P)
 {
-    static std::atomic<uint64_t> setS{0}, setU{0};
-    if (sharded) {
-        setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(scoreKernel<true, kThreads>), kScoreSmemMax, setS);
-        scoreKernel<true, kThreads><<<grid, kThreads, smem, stream>>>(P);
+    static std::atomic<uint64_t> set{0};
+    const auto kernel = scoreKernel<kSharded, kGrouped, kThreads, kParts>;
+    setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(kernel), kScoreSmemMax, set);
+    if (kParts) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = 1;
+        at.val.clusterDim.y = 1;
+        at.val.clusterDim.z = grid.z;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        RBW_CUDA(cudaLaunchKernelEx(&cfg, kernel, P));
     } else {
-        setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(scoreKernel<false, kThreads>), kScoreSmemMax,
-                                       setU);
-        scoreKernel<false, kThreads><<<grid, kThreads, smem, stream>>>(P);
+        kernel<<<grid, kThreads, smem, stream>>>(P);
     }
     RBW_CUDA(cudaGetLastError());
+}
+
+template <bool kGrouped>
+void launchScore(dim3 grid, size_t smem, cudaStream_t stream, const ScoreParams& P)
+{
+    constexpr uint32_t kThreads = kGrouped ? kScoreThreadsGrouped : kScoreThreads;
+    // CTAs that share a range are about one per SM: as many threads as fit, for loads in flight
+    if (grid.z > 1) launchScoreAs<true, kGrouped, kScoreThreads, true>(grid, smem, stream, P);
+    else if (grid.y > 1) launchScoreAs<true, kGrouped, kThreads, false>(grid, smem, stream, P);
+    else launchScoreAs<false, kGrouped, kThreads, false>(grid, smem, stream, P);
 }
 
 } // namespace
@@ -960,7 +1260,7 @@ public:
         // empty index: zero offsets in both segments, zero word counts
         for (Segment* sg : {&mMain, &mDelta}) {
             sg->leafOff.reserve((mNbLeaves + 1) * 4, 0, mStream);
-            sg->pairs.reserve(8, 0, mStream);
+            sg->pairs.reserve(16, 0, mStream);
             sg->tf.reserve(4, 0, mStream);
             RBW_CUDA(cudaMemsetAsync(sg->leafOff.get(), 0, (mNbLeaves + 1) * 4, mStream));
         }
@@ -1014,35 +1314,44 @@ public:
         if (k == 0) return 0;
         const uint64_t off[2] = {0, n};
         cudaStream_t s = mStream;
-        void* din = nullptr;
-        void* dout = nullptr;
-        RBW_CUDA(cudaMallocFromPoolAsync(&din, 16 + size_t(n) * 4, libraryPool(), s));
-        RBW_CUDA(cudaMallocFromPoolAsync(&dout, size_t(k) * 8 + 16, libraryPool(), s));
-        uint32_t got = 0;
+        // offsets and leaves go in one copy; documents, scores and their count come back in one
+        // unless the room for them is large (the count first, then what there is)
+        constexpr uint32_t kOneCopy = 65536;
+        const size_t outWords = 2 * size_t(k) + 1;
+        std::vector<uint32_t> in(4 + size_t(n)), out(k <= kOneCopy ? outWords : 0);
+        std::memcpy(in.data(), off, sizeof(off));
+        if (n) std::memcpy(in.data() + 4, leaves, size_t(n) * 4);
+        void* block = nullptr;
+        RBW_CUDA(cudaMallocFromPoolAsync(&block, (in.size() + outWords) * 4, libraryPool(), s));
+        uint32_t* dIn = static_cast<uint32_t*>(block);
+        uint32_t* dOut = dIn + in.size();
         try {
-            uint64_t* dOff = static_cast<uint64_t*>(din);
-            uint32_t* dLeaves = reinterpret_cast<uint32_t*>(dOff + 2);
-            RBW_CUDA(cudaMemcpyAsync(dOff, off, 16, cudaMemcpyHostToDevice, s));
-            if (n) RBW_CUDA(cudaMemcpyAsync(dLeaves, leaves, size_t(n) * 4, cudaMemcpyHostToDevice, s));
-            uint32_t* dDocs = static_cast<uint32_t*>(dout);
-            float* dScores = reinterpret_cast<float*>(dDocs + k);
-            uint32_t* dCount = reinterpret_cast<uint32_t*>(dScores + k);
-            queryBatched(dLeaves, dOff, 1, k, dDocs, dScores, dCount, s, off);
-            RBW_CUDA(cudaMemcpyAsync(&got, dCount, 4, cudaMemcpyDeviceToHost, s));
-            RBW_CUDA(cudaStreamSynchronize(s));
-            if (got) {
-                RBW_CUDA(cudaMemcpyAsync(docs, dDocs, size_t(got) * 4, cudaMemcpyDeviceToHost, s));
-                if (scores) RBW_CUDA(cudaMemcpyAsync(scores, dScores, size_t(got) * 4, cudaMemcpyDeviceToHost, s));
+            RBW_CUDA(cudaMemcpyAsync(dIn, in.data(), in.size() * 4, cudaMemcpyHostToDevice, s));
+            queryBatched(dIn + 4, reinterpret_cast<const uint64_t*>(dIn), 1, k, dOut, reinterpret_cast<float*>(dOut + k),
+                         dOut + 2 * size_t(k), s, off);
+            if (k <= kOneCopy) {
+                RBW_CUDA(cudaMemcpyAsync(out.data(), dOut, outWords * 4, cudaMemcpyDeviceToHost, s));
+            } else {
+                uint32_t got = 0;
+                RBW_CUDA(cudaMemcpyAsync(&got, dOut + 2 * size_t(k), 4, cudaMemcpyDeviceToHost, s));
+                RBW_CUDA(cudaStreamSynchronize(s));
+                if (got) RBW_CUDA(cudaMemcpyAsync(docs, dOut, size_t(got) * 4, cudaMemcpyDeviceToHost, s));
+                if (got && scores)
+                    RBW_CUDA(cudaMemcpyAsync(scores, dOut + k, size_t(got) * 4, cudaMemcpyDeviceToHost, s));
+                RBW_CUDA(cudaFreeAsync(std::exchange(block, nullptr), s));
+                RBW_CUDA(cudaStreamSynchronize(s));
+                return got;
             }
         } catch (...) {
-            cudaFreeAsync(din, s);
-            cudaFreeAsync(dout, s);
+            if (block) cudaFreeAsync(block, s);
             cudaStreamSynchronize(s);
             throw;
         }
-        RBW_CUDA(cudaFreeAsync(din, s));
-        RBW_CUDA(cudaFreeAsync(dout, s));
+        RBW_CUDA(cudaFreeAsync(block, s));
         RBW_CUDA(cudaStreamSynchronize(s));
+        const uint32_t got = out[2 * size_t(k)];
+        std::memcpy(docs, out.data(), size_t(got) * 4);
+        if (scores) std::memcpy(scores, out.data() + k, size_t(got) * 4);
         return got;
     }
 
@@ -1084,58 +1393,62 @@ public:
             return;
         }
         const uint32_t nDocs = mIndexed;
-        cudaMemPool_t pool = libraryPool();
-        int dev = 0, sms = 0;
-        RBW_CUDA(cudaGetDevice(&dev));
-        RBW_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        const int sms = currentSmCount();
         // Document range per scoring CTA.  With grouped inverted files it is csrPerCta shards of
-        // kShardDocs documents: the most (up to a group of kSmemDocs documents) that still gives
-        // one CTA per SM, so a small batch spreads over the GPU; with one inverted file per
-        // segment, kSmemDocs documents (every CTA of a query walks the whole list).
+        // kShardDocs documents: the most (up to kGroupedShards) that still gives two CTAs per SM, so
+        // a small batch spreads over the GPU; with one inverted file per segment, kSmemDocs
+        // documents (every CTA of a query walks the whole list).
         uint32_t csrPerCta = 1, shardDocs = std::min(std::max(nDocs, 1u), kSmemDocs);
-        if (groupedIndex()) {
-            csrPerCta = kSmemDocs / kShardDocs;
+        const bool grouped = groupedIndex();
+        const uint64_t wanted = 2 * uint64_t(sms);
+        if (grouped) {
+            csrPerCta = kGroupedShards;
             while (csrPerCta > 1 &&
-                   uint64_t(nq) * ((nDocs + csrPerCta * kShardDocs - 1) / (csrPerCta * kShardDocs)) < uint64_t(sms))
+                   uint64_t(nq) * ((nDocs + csrPerCta * kShardDocs - 1) / (csrPerCta * kShardDocs)) < wanted)
                 csrPerCta /= 2;
             shardDocs = std::min(std::max(nDocs, 1u), csrPerCta * kShardDocs);
         }
         const uint32_t shards = std::max(1u, (nDocs + shardDocs - 1) / shardDocs);
+        // fewer CTAs than that: several share a range, each taking part of the query's entries
+        uint32_t parts = 1;
+        while (parts < kMaxParts && uint64_t(nq) * shards * parts * 2 <= wanted) parts *= 2;
         const size_t entBytes = std::max<uint64_t>(totalLeaves, 1) * mL * sizeof(Entry);
         const size_t candBytes = shards > 1 ? size_t(nq) * shards * k * 8 : 16;
         const uint32_t selStride = k > kMaxK ? nextPow2(k) : 0u;
         const size_t selBytes = k > kMaxK ? size_t(nq) * shards * selStride * 8 : 16;
-        const uint32_t bigStride = maxBig ? nextPow2(maxBig) : 0u;
+        const uint32_t bigStride = maxBig ? sortRoom(maxBig) : 0u;
         const size_t bigBytes = bigQ.empty() ? 16 : bigQ.size() * (size_t(bigStride) + 1) * 4;
-        void *ent = nullptr, *cnt = nullptr, *qr = nullptr, *cand = nullptr, *selG = nullptr, *big = nullptr;
-        void* wk = nullptr;
-        RBW_CUDA(cudaMallocFromPoolAsync(&wk, size_t(nq) * 12, pool, stream));
-        unsigned long long* work = static_cast<unsigned long long*>(wk);
+        // one block of working memory, its parts 256 bytes apart
+        const size_t parted[] = {size_t(nq) * 12, entBytes, size_t(nq) * 4, size_t(nq) * 4, candBytes, selBytes, bigBytes};
+        constexpr size_t kParted = sizeof(parted) / sizeof(parted[0]);
+        size_t at[kParted + 1] = {0};
+        for (size_t i = 0; i < kParted; i++) at[i + 1] = at[i] + (parted[i] + 255) / 256 * 256;
+        void* block = nullptr;
+        RBW_CUDA(cudaMallocFromPoolAsync(&block, at[kParted], libraryPool(), stream));
+        auto part = [&](size_t i) { return static_cast<void*>(static_cast<uint8_t*>(block) + at[i]); };
+        unsigned long long* work = static_cast<unsigned long long*>(part(0));
         uint32_t* order = reinterpret_cast<uint32_t*>(work + nq);
-        RBW_CUDA(cudaMallocFromPoolAsync(&ent, entBytes, pool, stream));
-        RBW_CUDA(cudaMallocFromPoolAsync(&cnt, size_t(nq) * 4, pool, stream));
-        RBW_CUDA(cudaMallocFromPoolAsync(&qr, size_t(nq) * 4, pool, stream));
-        RBW_CUDA(cudaMallocFromPoolAsync(&cand, candBytes, pool, stream));
-        RBW_CUDA(cudaMallocFromPoolAsync(&selG, selBytes, pool, stream));
-        RBW_CUDA(cudaMallocFromPoolAsync(&big, bigBytes, pool, stream));
+        void *ent = part(1), *cnt = part(2), *qr = part(3), *cand = part(4), *selG = part(5), *big = part(6);
         {
             ScopedKernelTimer timer(kTimedScore, stream);
             std::optional<ScopedKernelTimer> prepTimer(std::in_place, kTimedScorePrep, stream);
-            const size_t prepSmem = size_t(nextPow2(std::max(maxN, 1u))) * 4;
+            const size_t prepSmem = size_t(sortRoom(maxN)) * 4;
+            // 1,024 threads while the queries leave SMs idle, 512 (two queries per SM) above
+            const uint32_t prepThreads = nq <= uint32_t(sms) ? kPrepThreadsFew : kPrepThreads;
             static std::atomic<uint64_t> setPrep{0};
             setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(queryPrepKernel), kPrepSmemMax, setPrep);
-            queryPrepKernel<<<nq, kPrepThreads, prepSmem, stream>>>(
+            queryPrepKernel<<<nq, prepThreads, prepSmem, stream>>>(
                 dLeaves, dOff, nullptr, nullptr, 0u, mWeights.as<float>(), skipCounts(), mB, mL,
-                mNbLeaves, k, static_cast<float*>(qr), static_cast<Entry*>(ent), static_cast<uint32_t*>(cnt), work);
+                mNbLeaves, inverseOf(mB), k, static_cast<float*>(qr), static_cast<Entry*>(ent), static_cast<uint32_t*>(cnt), work);
             RBW_CUDA(cudaGetLastError());
             if (!bigQ.empty()) {
                 // queries above kMaxDocDesc descriptors: one CTA each, sorted in global memory
-                uint32_t* qList = static_cast<uint32_t*>(big);
-                uint32_t* gkeys = qList + bigQ.size();
+                uint32_t* gkeys = static_cast<uint32_t*>(big); // 16-byte rows for the sort, so first
+                uint32_t* qList = gkeys + bigQ.size() * size_t(bigStride);
                 RBW_CUDA(cudaMemcpyAsync(qList, bigQ.data(), bigQ.size() * 4, cudaMemcpyHostToDevice, stream));
                 queryPrepKernel<<<static_cast<uint32_t>(bigQ.size()), kPrepThreads, 0, stream>>>(
                     dLeaves, dOff, qList, gkeys, bigStride, mWeights.as<float>(), skipCounts(),
-                    mB, mL, mNbLeaves, k, static_cast<float*>(qr), static_cast<Entry*>(ent),
+                    mB, mL, mNbLeaves, inverseOf(mB), k, static_cast<float*>(qr), static_cast<Entry*>(ent),
                     static_cast<uint32_t*>(cnt), work);
                 RBW_CUDA(cudaGetLastError());
             }
@@ -1169,23 +1482,16 @@ public:
             P.outDocs = dDocs;
             P.outScores = dScores;
             P.outCount = dCount;
-            // 1,024 threads per CTA whatever its document range: the pair walk is bound by load
-            // latency, so a query split over few CTAs needs every warp an SM can hold
             const size_t smem = size_t(shardDocs) * 8;
-            launchScore<kScoreThreads>(shards > 1, dim3(nq, shards), smem, stream, P);
+            if (grouped) launchScore<true>(dim3(nq, shards, parts), smem, stream, P);
+            else launchScore<false>(dim3(nq, shards, parts), smem, stream, P);
             if (shards > 1) {
                 ScopedKernelTimer mergeTimer(kTimedScoreMerge, stream);
                 mergeKernel<<<nq, kScoreThreads, 0, stream>>>(P, shards);
                 RBW_CUDA(cudaGetLastError());
             }
         }
-        RBW_CUDA(cudaFreeAsync(ent, stream));
-        RBW_CUDA(cudaFreeAsync(cnt, stream));
-        RBW_CUDA(cudaFreeAsync(qr, stream));
-        RBW_CUDA(cudaFreeAsync(cand, stream));
-        RBW_CUDA(cudaFreeAsync(selG, stream));
-        RBW_CUDA(cudaFreeAsync(big, stream));
-        RBW_CUDA(cudaFreeAsync(wk, stream));
+        RBW_CUDA(cudaFreeAsync(block, stream));
         recordQuery(stream);
     }
 
@@ -1355,7 +1661,7 @@ private:
         }
         const uint64_t entries = sg.grouped ? uint64_t(sg.nGroups) * mNbLeaves * kGroupShards : mNbLeaves;
         sg.leafOff.reserve((entries + 1) * 4, 0, mStream);
-        sg.pairs.reserve(std::max<uint64_t>(pairsUpper, 1) * 8, 0, mStream);
+        sg.pairs.reserve((pairsUpper + 2) * 8, 0, mStream); // lists are read two pairs at a time
         sg.tf.reserve(std::max<uint64_t>(pairsUpper, 1) * 4, 0, mStream);
         void* tmp = nullptr;
         const size_t cntBytes = entries * 4;
@@ -1415,12 +1721,12 @@ private:
         RBW_CUDA(cudaMallocFromPoolAsync(&newLeaves, std::max<uint64_t>(p1 - p0, 1) * 4, libraryPool(), mStream));
         if (p1 > p0)
             RBW_CUDA(cudaMemcpyAsync(newLeaves, mStage.data(), (p1 - p0) * 4, cudaMemcpyHostToDevice, mStream));
-        const size_t smem = size_t(nextPow2(std::max(mStageMaxN, 1u))) * 4;
+        const size_t smem = size_t(sortRoom(mStageMaxN)) * 4;
         static std::atomic<uint64_t> setDoc{0};
         setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(docPrepKernel), kPrepSmemMax, setDoc);
         docPrepKernel<<<s1 - s0, kPrepThreads, smem, mStream>>>(
             static_cast<const uint32_t*>(newLeaves), mDocOff.as<uint64_t>(), s0, nullptr, nullptr, 0u,
-            mWeights.as<float>(), mB, mL, mNbLeaves, mRcpF.as<float>(), mDocPairs.as<uint64_t>(),
+            mWeights.as<float>(), mB, mL, mNbLeaves, inverseOf(mB), mRcpF.as<float>(), mDocPairs.as<uint64_t>(),
             mPairCount.as<uint32_t>());
         RBW_CUDA(cudaGetLastError());
         // documents above kMaxDocDesc descriptors: one CTA each, sorted in global memory
@@ -1434,14 +1740,15 @@ private:
             }
         }
         if (!bigSlots.empty()) {
-            const uint32_t stride = nextPow2(static_cast<uint32_t>(maxBig));
+            const uint32_t stride = sortRoom(static_cast<uint32_t>(maxBig));
             void* big = nullptr;
             RBW_CUDA(cudaMallocFromPoolAsync(&big, bigSlots.size() * (size_t(stride) + 1) * 4, libraryPool(), mStream));
-            uint32_t* slotList = static_cast<uint32_t*>(big);
+            uint32_t* gkeys = static_cast<uint32_t*>(big); // 16-byte rows for the sort, so first
+            uint32_t* slotList = gkeys + bigSlots.size() * size_t(stride);
             RBW_CUDA(cudaMemcpyAsync(slotList, bigSlots.data(), bigSlots.size() * 4, cudaMemcpyHostToDevice, mStream));
             docPrepKernel<<<static_cast<uint32_t>(bigSlots.size()), kPrepThreads, 0, mStream>>>(
                 static_cast<const uint32_t*>(newLeaves), mDocOff.as<uint64_t>(), s0, slotList,
-                slotList + bigSlots.size(), stride, mWeights.as<float>(), mB, mL, mNbLeaves, mRcpF.as<float>(),
+                gkeys, stride, mWeights.as<float>(), mB, mL, mNbLeaves, inverseOf(mB), mRcpF.as<float>(),
                 mDocPairs.as<uint64_t>(), mPairCount.as<uint32_t>());
             RBW_CUDA(cudaGetLastError());
             RBW_CUDA(cudaFreeAsync(big, mStream));

@@ -503,3 +503,41 @@ def test_batched_queries_interleaved_with_adds(oracle):
     for (d, s, c), want in outs:
         assert int(c[0]) == want.size
         assert set(d[0, : want.size].cpu().numpy().view(np.uint32).tolist()) == set(want.tolist())
+
+
+@pytest.mark.parametrize("layout", [1, 2])
+@pytest.mark.parametrize("B,L,n_docs", [(7, 3, 90), (16, 3, 2600), (3, 6, 5200)])
+def test_ranges_shared_by_several_ctas_match_oracle(oracle, B, L, n_docs, layout):
+    """Few queries: a range of documents is shared by up to eight CTAs, and the database has one to
+    three such ranges; queries at the edges of the sort's segments; selections above and below the
+    sorted sizes; upper-level words with more pairs than a warp gathers (large k)."""
+    from rapidbow_b200 import autotune as at
+
+    n_leaves = B ** L
+    docs = make_docs(n_docs, n_leaves, seed=n_docs, lo=5, hi=60)
+    at.set_value("db_shard_tables", B, L, at.bucket(n_docs), layout)
+    try:
+        centers, masks, weights = random_tree(B, L, 5, dup_rate=0.0)
+        voc = rbw.vocabulary_from_host(B, L, centers, masks, weights)
+        db, odb = rbw.DataBase(voc), oracle.db(B, L, weights)
+        off = np.concatenate([[0], np.cumsum([d.size for d in docs])]).astype(np.uint64)
+        db.add_docs(np.arange(n_docs, dtype=np.uint32), np.concatenate(docs), off)
+        for i, d in enumerate(docs):
+            odb.add(i, d)
+        rng = np.random.default_rng(3)
+        for m, k in [(1, 5), (2, 257), (127, 100), (128, 1024), (129, 20), (256, 300), (257, 1300), (2047, 100), (2049, 50)]:
+            check_query(db, odb, rng.integers(0, n_leaves, size=m, dtype=np.uint32), k)
+    finally:
+        at.clear()
+
+
+def test_upper_level_word_with_a_huge_tf_matches_oracle(oracle):
+    """A document with more descriptors of one word than the gathered (document, tf) pair can hold,
+    under an upper-level word that a very large k does not skip."""
+    B, L = 4, 3
+    rng = np.random.default_rng(8)
+    docs = [np.full(140_000, 5, np.uint32), rng.integers(0, 64, 300, dtype=np.uint32),
+            rng.integers(0, 8, 50, dtype=np.uint32)]
+    _, db, odb, _ = build_pair(oracle, B, L, docs, range(3), seed=4)
+    for k in (20, 40_000, 70_000):
+        check_query(db, odb, np.array([4, 5, 6, 7, 7, 20], np.uint32), k)
