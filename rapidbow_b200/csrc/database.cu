@@ -1255,6 +1255,7 @@ public:
         mWeights.reset(mNbWords * 4);
         RBW_CUDA(cudaMemcpy(mWeights.get(), v.weights().data(), mNbWords * 4, cudaMemcpyHostToDevice));
         mHostDocOff.push_back(0);
+        mDevice = currentDevice();
         RBW_CUDA(cudaStreamCreateWithFlags(&mStream, cudaStreamNonBlocking));
         RBW_CUDA(cudaEventCreateWithFlags(&mIndexReady, cudaEventDisableTiming));
         // empty index: zero offsets in both segments, zero word counts
@@ -1276,7 +1277,7 @@ public:
     ~DataBase()
     {
         waitQueriesOnStream();
-        for (PoolBuffer* b : {&mDocOff, &mDocPairs, &mPairCount, &mRcpF, &mSlotDoc, &mMainLeafPost, &mWordPost,
+        for (PoolBuffer* b : {&mNewLeaves, &mDocOff, &mDocPairs, &mPairCount, &mRcpF, &mSlotDoc, &mMainLeafPost, &mWordPost,
                               &mMain.leafOff, &mMain.pairs, &mMain.tf, &mDelta.leafOff, &mDelta.pairs, &mDelta.tf})
             b->release(mStream);
         cudaStreamSynchronize(mStream);
@@ -1289,21 +1290,27 @@ public:
     {
         std::unique_lock<std::shared_mutex> lk(mMu);
         checkDoc(id, leaves, n);
-        stageLocked(id, leaves, n);
+        checkLeaves(leaves, n);
+        registerDoc(id, leaves, n);
     }
     void addDocs(const uint32_t* ids, const uint32_t* leaves, const uint64_t* off, uint32_t nDocs)
     {
         std::unique_lock<std::shared_mutex> lk(mMu);
         // validate the whole batch first: a failed call adds nothing
         std::unordered_map<uint32_t, uint32_t> seen;
+        seen.reserve(nDocs);
+        const bool direct = nDocs && uploadsDirectly(leaves, off[0], off[nDocs]);
         for (uint32_t d = 0; d < nDocs; d++) {
             if (off[d + 1] < off[d] || off[d + 1] - off[d] > 0xFFFFFFFFull)
                 throw Error(kInvalidArg, "bad document offsets");
-            checkDoc(ids[d], leaves + off[d], static_cast<uint32_t>(off[d + 1] - off[d]));
+            const uint32_t n = static_cast<uint32_t>(off[d + 1] - off[d]);
+            checkDoc(ids[d], leaves + off[d], n);
+            if (!direct) checkLeaves(leaves + off[d], n);
             if (!seen.emplace(ids[d], d).second) throw Error(kDuplicate, "Duplicate document index");
         }
+        const bool uploaded = direct && uploadChecked(leaves + off[0], off[nDocs] - off[0]);
         for (uint32_t d = 0; d < nDocs; d++)
-            stageLocked(ids[d], leaves + off[d], static_cast<uint32_t>(off[d + 1] - off[d]));
+            registerDoc(ids[d], uploaded ? nullptr : leaves + off[d], static_cast<uint32_t>(off[d + 1] - off[d]));
     }
 
     // Host leaves in, host results out (the reference's query).  Synchronous.
@@ -1601,17 +1608,86 @@ private:
     {
         if (mSlotOf.count(id)) throw Error(kDuplicate, "Duplicate document index"); // DataBase.cpp:41-43
         if (n && leaves == nullptr) throw Error(kInvalidArg, "null leaves");
-        for (uint32_t i = 0; i < n; i++)
-            if (leaves[i] >= mNbLeaves) throw Error(kInvalidArg, "leaf index out of range");
+    }
+    void checkLeaves(const uint32_t* leaves, uint64_t n) const
+    {
+        const uint32_t limit = static_cast<uint32_t>(mNbLeaves); // below 2^32 - 1 (constructor)
+        uint32_t bad = 0;
+        for (uint64_t i = 0; i < n; i++) bad |= leaves[i] >= limit ? 1u : 0u; // no exit: vectorised
+        if (bad) throw Error(kInvalidArg, "leaf index out of range");
     }
 
-    void stageLocked(uint32_t id, const uint32_t* leaves, uint32_t n)
+    // A document's host record; its leaves go to the host staging area unless already uploaded.
+    void registerDoc(uint32_t id, const uint32_t* leaves, uint32_t n)
     {
         mSlotOf.emplace(id, static_cast<uint32_t>(mHostIds.size()));
         mHostIds.push_back(id);
-        mStage.insert(mStage.end(), leaves, leaves + n);
+        if (leaves) mStage.insert(mStage.end(), leaves, leaves + n);
         mHostDocOff.push_back(mHostDocOff.back() + n);
         if (n <= kMaxDocDesc) mStageMaxN = std::max(mStageMaxN, n);
+    }
+
+    // Large batches of documents are copied to the device when they are added, instead of through
+    // the host staging area: 5.1M leaves took 25 ms there, most of it faulting in fresh pages and
+    // checking one leaf at a time, 3 ms here.  Only from pageable memory, whose copy has been read
+    // when the call returns, and only while the database's stream is idle, so that adding never
+    // waits for the GPU.
+    bool uploadsDirectly(const uint32_t* leaves, uint64_t beg, uint64_t end) const
+    {
+        constexpr uint64_t kDirectLeaves = 65536;
+        if (leaves == nullptr || end < beg || end - beg < kDirectLeaves) return false;
+        int dev = -1;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev != mDevice) return false; // the pool is the current device's
+        if (cudaStreamQuery(mStream) != cudaSuccess) {
+            cudaGetLastError(); // not ready: no error of ours
+            return false;
+        }
+        for (const uint32_t* p : {leaves + beg, leaves + end - 1}) {
+            cudaPointerAttributes at{};
+            if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            if (at.type != cudaMemoryTypeUnregistered) return false;
+        }
+        return true;
+    }
+    // Checks and uploads n leaves after those already staged; throws (staging nothing more) if one
+    // is out of range.  False: the copy failed, the caller stages the leaves on the host instead.
+    bool uploadChecked(const uint32_t* leaves, uint64_t n)
+    {
+        try {
+            uploadStage(n);
+        } catch (const Error&) {
+            cudaGetLastError();
+            checkLeaves(leaves, n);
+            return false;
+        }
+        constexpr uint64_t kChunk = uint64_t(1) << 18; // checked while it is read into the cache
+        bool copied = true;
+        for (uint64_t i = 0; i < n; i += kChunk) {
+            const uint64_t m = std::min(kChunk, n - i);
+            checkLeaves(leaves + i, m);
+            if (copied)
+                copied = cudaMemcpyAsync(mNewLeaves.as<uint32_t>() + mUploaded + i, leaves + i, m * 4,
+                                         cudaMemcpyHostToDevice, mStream) == cudaSuccess;
+        }
+        if (!copied) {
+            cudaGetLastError();
+            return false;
+        }
+        mUploaded += n;
+        return true;
+    }
+    // Moves the host staging area to the device, with room for `more` leaves after it.
+    void uploadStage(uint64_t more)
+    {
+        mNewLeaves.reserve(std::max<uint64_t>(mUploaded + mStage.size() + more, 1) * 4, mUploaded * 4, mStream);
+        if (mStage.empty()) return;
+        RBW_CUDA(cudaMemcpyAsync(mNewLeaves.as<uint32_t>() + mUploaded, mStage.data(), mStage.size() * 4,
+                                 cudaMemcpyHostToDevice, mStream));
+        mUploaded += mStage.size();
+        mStage.clear();
     }
 
     // Makes the stream wait for every query launched since the last index update.
@@ -1717,15 +1793,13 @@ private:
                                  uint64_t(s1 - s0) * 8, cudaMemcpyHostToDevice, mStream));
         RBW_CUDA(cudaMemcpyAsync(mSlotDoc.as<uint32_t>() + s0, mHostIds.data() + s0, uint64_t(s1 - s0) * 4,
                                  cudaMemcpyHostToDevice, mStream));
-        void* newLeaves = nullptr;
-        RBW_CUDA(cudaMallocFromPoolAsync(&newLeaves, std::max<uint64_t>(p1 - p0, 1) * 4, libraryPool(), mStream));
-        if (p1 > p0)
-            RBW_CUDA(cudaMemcpyAsync(newLeaves, mStage.data(), (p1 - p0) * 4, cudaMemcpyHostToDevice, mStream));
+        uploadStage(0);
+        const uint32_t* newLeaves = mNewLeaves.as<uint32_t>();
         const size_t smem = size_t(sortRoom(mStageMaxN)) * 4;
         static std::atomic<uint64_t> setDoc{0};
         setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(docPrepKernel), kPrepSmemMax, setDoc);
         docPrepKernel<<<s1 - s0, kPrepThreads, smem, mStream>>>(
-            static_cast<const uint32_t*>(newLeaves), mDocOff.as<uint64_t>(), s0, nullptr, nullptr, 0u,
+            newLeaves, mDocOff.as<uint64_t>(), s0, nullptr, nullptr, 0u,
             mWeights.as<float>(), mB, mL, mNbLeaves, inverseOf(mB), mRcpF.as<float>(), mDocPairs.as<uint64_t>(),
             mPairCount.as<uint32_t>());
         RBW_CUDA(cudaGetLastError());
@@ -1747,14 +1821,14 @@ private:
             uint32_t* slotList = gkeys + bigSlots.size() * size_t(stride);
             RBW_CUDA(cudaMemcpyAsync(slotList, bigSlots.data(), bigSlots.size() * 4, cudaMemcpyHostToDevice, mStream));
             docPrepKernel<<<static_cast<uint32_t>(bigSlots.size()), kPrepThreads, 0, mStream>>>(
-                static_cast<const uint32_t*>(newLeaves), mDocOff.as<uint64_t>(), s0, slotList,
+                newLeaves, mDocOff.as<uint64_t>(), s0, slotList,
                 gkeys, stride, mWeights.as<float>(), mB, mL, mNbLeaves, inverseOf(mB), mRcpF.as<float>(),
                 mDocPairs.as<uint64_t>(), mPairCount.as<uint32_t>());
             RBW_CUDA(cudaGetLastError());
             RBW_CUDA(cudaFreeAsync(big, mStream));
         }
-        RBW_CUDA(cudaFreeAsync(newLeaves, mStream));
-        mStage.clear();
+        mNewLeaves.release(mStream);
+        mUploaded = 0;
         mStageMaxN = 0;
 
         // 2. segments: compact everything into main when the delta outgrows its share
@@ -1808,11 +1882,14 @@ private:
     std::vector<uint32_t> mHostIds;        // slot -> document id
     std::vector<uint64_t> mHostDocOff;     // slot -> first posting (prefix sums of sizes)
     std::unordered_map<uint32_t, uint32_t> mSlotOf;
-    std::vector<uint32_t> mStage;          // leaves of documents [mIndexed, nSlots)
+    std::vector<uint32_t> mStage;          // leaves of documents [mIndexed, nSlots) not yet in mNewLeaves
     uint32_t mStageMaxN = 0;
     uint32_t mIndexed = 0;                 // documents in the device index
     // device state (library pool, ordered on mStream)
     PoolBuffer mDocOff, mDocPairs, mPairCount, mRcpF, mSlotDoc;
+    PoolBuffer mNewLeaves;                 // the first mUploaded leaves of documents [mIndexed, nSlots)
+    uint64_t mUploaded = 0;
+    int mDevice = 0;
     Segment mMain, mDelta;
     PoolBuffer mMainLeafPost, mWordPost;
     cudaStream_t mStream = nullptr;

@@ -541,3 +541,53 @@ def test_upper_level_word_with_a_huge_tf_matches_oracle(oracle):
     _, db, odb, _ = build_pair(oracle, B, L, docs, range(3), seed=4)
     for k in (20, 40_000, 70_000):
         check_query(db, odb, np.array([4, 5, 6, 7, 7, 20], np.uint32), k)
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+def test_large_batches_added_between_small_ones_match_oracle(oracle, pinned):
+    """Batches of 65,536 leaves and more go to the device when they are added (pageable memory; not
+    page-locked arrays, whose copy could outlast the call), after what the host still holds; a batch
+    with a leaf out of range adds nothing, wherever that leaf is."""
+    import torch
+
+    B, L, n_docs = 16, 3, 700
+    n_leaves = B ** L
+    docs = make_docs(n_docs, n_leaves, seed=17, lo=150, hi=400)
+    centers, masks, weights = random_tree(B, L, 18, dup_rate=0.0)
+    voc = rbw.vocabulary_from_host(B, L, centers, masks, weights)
+    db, odb = rbw.DataBase(voc), oracle.db(B, L, weights)
+    for i, d in enumerate(docs):
+        odb.add(i, d)
+
+    def batch(i0, i1, bad_at=None):
+        leaves = np.concatenate(docs[i0:i1])
+        if pinned:
+            leaves = torch.from_numpy(leaves.astype(np.int32)).pin_memory().numpy().view(np.uint32)
+        if bad_at is not None:
+            leaves[bad_at] = n_leaves
+        off = np.concatenate([[0], np.cumsum([d.size for d in docs[i0:i1]])]).astype(np.uint64)
+        db.add_docs(np.arange(i0, i1, dtype=np.uint32), leaves, off)
+        leaves[:] = 0  # the caller's again once the call has returned
+        return off[-1]
+
+    def posted():
+        return sum(d.size for d in docs[: db.info()[0]])
+
+    db.add_doc(0, docs[0])
+    db.add_doc(1, docs[1])
+    assert batch(2, 320) >= 65536
+    for bad_at in (0, 40_000, -1):
+        with pytest.raises(rbw.RbwError):
+            batch(320, 640, bad_at)
+        assert db.info() == (320, posted())
+    batch(320, 330)
+    db.query(docs[5], 10)
+    assert batch(330, 650) >= 65536
+    db.add_doc(650, docs[650])
+    batch(651, 700)
+    assert db.info() == (700, posted())
+    rng = np.random.default_rng(2)
+    for leaf in rng.integers(0, n_leaves, 60):
+        assert np.array_equal(db.postings(int(leaf)), odb.postings(int(leaf)))
+    for q in make_queries(docs, n_leaves, 6, seed=4):
+        check_query(db, odb, q, 30)
