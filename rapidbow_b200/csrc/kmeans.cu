@@ -409,6 +409,7 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignCtasPerSm) assignKernel
     const uint32_t T = *nTilesDev;
     const uint32_t t0 = static_cast<uint32_t>(uint64_t(T) * blockIdx.x / gridDim.x);
     const uint32_t t1 = static_cast<uint32_t>(uint64_t(T) * (blockIdx.x + 1) / gridDim.x);
+    if (lv.activeCount && blockIdx.x == 0 && tid == 0) *lv.activeCount = 0; // counted by the update that follows
     if (t0 == t1) return; // uniform: fewer tiles than CTAs
     volatile uint32_t* abortFlag = &S.abortFlag;
     if (tid == 0) {

@@ -104,7 +104,9 @@ __global__ void __launch_bounds__(256) prepareNodesKernel(const float* centers, 
 // ------------------------------------------------------------------ assign
 constexpr uint32_t kAfThreads = 128;
 constexpr uint32_t kAfRows = 128;
-constexpr uint32_t kAfTmemCols = 32;
+constexpr uint32_t kAfTmemCols = 64; // distances to the hi and lo parts | sums
+constexpr uint32_t kAfSumCol = 32;
+constexpr uint32_t kAfFlushTiles = 65536; // 65,536 x 128 x 255 < 2^31
 constexpr uint32_t kAfCtasPerSm = 3;
 constexpr uint32_t kAfTileWindow = kAfThreads; // one tile entry per thread per refill
 constexpr uint32_t kAfFrozen = 0x80000000u;
@@ -112,17 +114,16 @@ constexpr uint32_t kAfFrozen = 0x80000000u;
 struct AssignFSmem {
     uint8_t a[2][kAfRows * 128];     // members as bf16, two K-blocks of 64 dims, 128-byte swizzle
     uint8_t b[2][32 * 128];          // the node's hi (rows 0-15) and lo (rows 16-31) centers
-    uint8_t x8[kAfRows * kDims];     // members as uint8, row-major (sums and FP64 re-score)
+    uint8_t x8[kAfRows * kDims];     // members as uint8, 128-byte swizzle (sums and FP64 re-score)
+    uint8_t oh[kAfRows * kMaxBranch]; // [member][center] one-hot
     NodeTile win[kAfTileWindow];     // tiles [winBase, winBase + kAfTileWindow) of the CTA's range,
                                      // count | kAfFrozen for a frozen node
-    uint32_t acc[kMaxBranch * kDims]; // center sums of the current node (accIndex layout)
     unsigned long long q[kMaxBranch];
     float cn[kMaxBranch];
     uint32_t xn[kAfRows];
     uint32_t cnt[kMaxBranch];
-    uint8_t bsel[kAfRows];
     float2 bnd;
-    uint64_t mmaBar;
+    uint64_t mmaBar, sumBar;
     uint32_t tmemBase;
     uint32_t chg;
     uint32_t abortFlag;
@@ -130,11 +131,6 @@ struct AssignFSmem {
     uint32_t visited;
 };
 constexpr size_t kAfSmemBytes = sizeof(AssignFSmem) + 1024;
-
-__device__ __forceinline__ uint32_t accIndexF(uint32_t b, uint32_t d)
-{
-    return b * kDims + (d & 3u) * 32u + (d >> 2);
-}
 
 // bf16 of the four bytes of w (exact: integers below 256), packed in two bf16x2 words.
 __device__ __forceinline__ void bytesToBf16(uint32_t w, uint32_t& lo2, uint32_t& hi2)
@@ -154,15 +150,18 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
     extern __shared__ uint8_t smemRaw[];
     AssignFSmem& S = *reinterpret_cast<AssignFSmem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
     const KMeansLevel& L0 = lv.base;
-    const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const uint32_t tid = threadIdx.x, lane = tid % 32;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid / 32, 0); // uniform
     const uint32_t B = L0.B;
     const bool build = lv.lookupOnly == 0;
+    if (build && blockIdx.x == 0 && tid == 0) *L0.activeCount = 0; // counted by the update that follows
     const uint32_t T = *nTilesDev;
     const uint32_t t0 = static_cast<uint32_t>(uint64_t(T) * blockIdx.x / gridDim.x);
     const uint32_t t1 = static_cast<uint32_t>(uint64_t(T) * (blockIdx.x + 1) / gridDim.x);
     volatile uint32_t* abortFlag = &S.abortFlag;
     if (tid == 0) {
         mbarInit(&S.mmaBar, 1);
+        mbarInit(&S.sumBar, 1);
         S.abortFlag = 0;
         S.refined = 0;
         S.visited = 0;
@@ -176,21 +175,43 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
     __syncthreads();
     tcFenceAfter();
     const uint32_t tmem = S.tmemBase;
-    uint32_t curNode = 0xFFFFFFFFu, phase = 0;
-    bool curExclusive = false; // every tile of the current node is in this CTA's range
+    const bool issuer = warp == 0 && electOne(); // one thread issues and commits every MMA
+    uint32_t curNode = 0xFFFFFFFFu, phase = 0, sumPhase = 0, accTiles = 0;
+    uint32_t myCnt = 0, myChg = 0;   // lane c < 16: this warp's rows that chose center c, and the
+    unsigned long long myQ = 0;      // sum of their |x|^2
+    bool curExclusive = false;       // every tile of the current node is in this CTA's range
+    bool sumsInFlight = false;
+    // the last sums MMA has read the tile and the one-hot rows
+    auto waitSums = [&]() -> bool {
+        if (!sumsInFlight) return true;
+        sumsInFlight = false;
+        const bool ok = mbarWait(&S.sumBar, sumPhase, abortFlag, L0.err, 55);
+        sumPhase ^= 1u;
+        tcFenceAfter();
+        return ok;
+    };
     auto flush = [&]() {
-        __syncthreads();
         if (curNode != 0xFFFFFFFFu && build) {
-            // plain stores for a node no other CTA touches (its accumulators are zero on entry)
-            for (uint32_t i = tid; i < kMaxBranch * kDims; i += kAfThreads) {
-                const uint32_t b = i / kDims, d = i % kDims;
-                const uint32_t v = S.acc[accIndexF(b, d)];
-                unsigned long long* dst = L0.sums + (uint64_t(curNode) * kMaxBranch + b) * kDims + d;
-                if (v) {
-                    if (curExclusive) *dst = v;
-                    else atomicAdd(dst, (unsigned long long)v);
+            if (lane < kMaxBranch && myCnt) {
+                atomicAdd(&S.cnt[lane], myCnt);
+                atomicAdd(&S.q[lane], myQ);
+            }
+            if (lane == 0 && myChg) atomicAdd(&S.chg, myChg);
+            if (accTiles > 0 && waitSums()) {
+                uint32_t r[16];
+                tmemLoad16(tmem + kAfSumCol + ((warp * 32u) << 16), r); // lane = dimension tid
+                tmemWaitTie(r);
+                tcFenceBefore();
+                // plain stores for a node no other CTA touches (its accumulators are zero on entry)
+#pragma unroll
+                for (uint32_t b = 0; b < kMaxBranch; b++) {
+                    if (r[b] == 0) continue;
+                    unsigned long long* dst = L0.sums + (uint64_t(curNode) * kMaxBranch + b) * kDims + tid;
+                    if (curExclusive) *dst = r[b];
+                    else atomicAdd(dst, (unsigned long long)r[b]);
                 }
             }
+            __syncthreads(); // S.cnt, S.q and S.chg complete
             if (tid < kMaxBranch && S.cnt[tid]) {
                 uint32_t* c = L0.counts + uint64_t(curNode) * kMaxBranch + tid;
                 unsigned long long* qd = lv.q + uint64_t(curNode) * kMaxBranch + tid;
@@ -207,6 +228,10 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
                 else atomicAdd(L0.changed + curNode, S.chg);
             }
         }
+        accTiles = 0;
+        myCnt = 0;
+        myChg = 0;
+        myQ = 0;
         __syncthreads();
     };
     // The tile list and the frozen flags are read a window of kAfTileWindow tiles at a time (one
@@ -281,9 +306,17 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
                 S.bnd = lv.bound[curNode];
                 S.chg = 0;
             }
-            if (build)
-                for (uint32_t i = tid; i < kMaxBranch * kDims; i += kAfThreads) S.acc[i] = 0;
+        } else if (accTiles == kAfFlushTiles) {
+            // keep each s32 sum below 2^31: this node's partial results go out, later flushes add
+            curExclusive = false;
+            flush();
+            if (tid < kMaxBranch) {
+                S.cnt[tid] = 0;
+                S.q[tid] = 0;
+            }
+            if (tid == 0) S.chg = 0;
         }
+        if (!waitSums()) break; // the tile below is read by the previous tile's sums MMA
         {
             // Eight threads per row, 16 rows per round: thread c8 = tid % 8 stages dims
             // 16 c8 .. 16 c8 + 15 of its row as uint8 and as bf16 (K-block c8 / 4, 16-byte chunks
@@ -292,7 +325,7 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
 #pragma unroll
             for (uint32_t k = 0; k < kAfRows / 16; k++) {
                 const uint32_t row = 16u * k + tid / 8;
-                *reinterpret_cast<uint4*>(S.x8 + row * kDims + c8 * 16) = v[k];
+                *reinterpret_cast<uint4*>(S.x8 + row * kDims + ((c8 ^ (row & 7u)) << 4)) = v[k];
                 uint32_t w[8];
                 bytesToBf16(v[k].x, w[0], w[1]);
                 bytesToBf16(v[k].y, w[2], w[3]);
@@ -331,15 +364,15 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
         // generic-proxy shared-memory writes read by the tensor core
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0) {
             tcFenceAfter();
-            const uint32_t aBase = smemAddr(&S.a[0][0]), bBase = smemAddr(&S.b[0][0]);
+            const uint64_t aDesc = smemDescSw128(smemAddr(&S.a[0][0])), bDesc = smemDescSw128(smemAddr(&S.b[0][0]));
 #pragma unroll
-            for (uint32_t k = 0; k < 8; k++) {
-                mmaBf16(tmem, smemDescSw128(aBase + (k >> 2) * (kAfRows * 128) + 32u * (k & 3u)),
-                        smemDescSw128(bBase + (k >> 2) * (32 * 128) + 32u * (k & 3u)), idescBf16(32), k > 0 ? 1u : 0u);
-            }
-            mmaCommit(&S.mmaBar);
+            for (uint32_t k = 0; k < 8; k++)
+                if (issuer)
+                    mmaBf16(tmem, aDesc + (((k >> 2) * (kAfRows * 128) + 32u * (k & 3u)) >> 4),
+                            bDesc + (((k >> 2) * (32 * 128) + 32u * (k & 3u)) >> 4), idescBf16(32), k > 0 ? 1u : 0u);
+            if (issuer) mmaCommit(&S.mmaBar);
         }
         if (!mbarWait(&S.mmaBar, phase, abortFlag, L0.err, 50)) break;
         phase ^= 1u;
@@ -371,31 +404,58 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
         uint32_t mask = __ballot_sync(0xFFFFFFFFu, refine);
         if (mask != 0) {
             // FP64 re-score of the flagged rows of this warp, one row at a time, every lane on
-            // dims 4 lane .. 4 lane + 3 of every center (the oracle's orc_dist64 order).
+            // dims 4 lane .. 4 lane + 3 (the oracle's orc_dist64 order) -- of the centers whose
+            // score is within the margin of the best, two at a time: by the margin's definition
+            // every other center is farther than the best in FP64 too.
+            uint32_t near = 0;
+#pragma unroll
+            for (uint32_t b = 0; b < kMaxBranch; b++) {
+                const float dot = __fadd_rn(__uint_as_float(rh[b]), __uint_as_float(rl[b]));
+                const float s = __fmaf_rn(-2.f, dot, S.cn[b]);
+                if (b < B && !(s - best > thr)) near |= 1u << b;
+            }
             if (lane == 0) atomicAdd(&S.refined, uint32_t(__popc(mask)));
             const float* cBase = lv.centers + uint64_t(curNode) * kMaxBranch * kDims + 4u * lane;
             while (mask != 0) {
                 const uint32_t src = __ffs(mask) - 1;
                 mask &= mask - 1;
-                const uint32_t xw = *reinterpret_cast<const uint32_t*>(S.x8 + (warp * 32u + src) * kDims + 4u * lane);
+                uint32_t cand = __shfl_sync(0xFFFFFFFFu, near, src);
+                const uint32_t xw = *reinterpret_cast<const uint32_t*>(
+                    S.x8 + (warp * 32u + src) * kDims + (((lane >> 2) ^ (src & 7u)) << 4) + ((lane & 3u) << 2));
+                const double x0 = double(xw & 0xFFu), x1 = double((xw >> 8) & 0xFFu);
+                const double x2 = double((xw >> 16) & 0xFFu), x3 = double(xw >> 24);
+                auto partial = [&](const float4& c4) {
+                    double e = __dsub_rn(x0, double(c4.x));
+                    double p = __fma_rn(e, e, 0.0);
+                    e = __dsub_rn(x1, double(c4.y));
+                    p = __fma_rn(e, e, p);
+                    e = __dsub_rn(x2, double(c4.z));
+                    p = __fma_rn(e, e, p);
+                    e = __dsub_rn(x3, double(c4.w));
+                    return __fma_rn(e, e, p);
+                };
                 double bestD = 0.0;
-                uint32_t bb = 0;
-                for (uint32_t b = 0; b < B; b++) {
-                    const float4 c4 = __ldg(reinterpret_cast<const float4*>(cBase + b * kDims));
-                    double p = 0.0;
-                    double e = __dsub_rn(double(xw & 0xFFu), double(c4.x));
-                    p = __fma_rn(e, e, p);
-                    e = __dsub_rn(double((xw >> 8) & 0xFFu), double(c4.y));
-                    p = __fma_rn(e, e, p);
-                    e = __dsub_rn(double((xw >> 16) & 0xFFu), double(c4.z));
-                    p = __fma_rn(e, e, p);
-                    e = __dsub_rn(double(xw >> 24), double(c4.w));
-                    p = __fma_rn(e, e, p);
+                uint32_t bb = kMaxBranch;
+                while (cand != 0) {
+                    const uint32_t b0 = __ffs(cand) - 1;
+                    cand &= cand - 1;
+                    const uint32_t b1 = cand ? __ffs(cand) - 1 : b0; // the same again if there is no other
+                    cand &= cand - 1;
+                    const float4 c0 = __ldg(reinterpret_cast<const float4*>(cBase + b0 * kDims));
+                    const float4 c1 = __ldg(reinterpret_cast<const float4*>(cBase + b1 * kDims));
+                    double p0 = partial(c0), p1 = partial(c1);
 #pragma unroll
-                    for (uint32_t off = 16; off > 0; off >>= 1) p = __dadd_rn(p, __shfl_xor_sync(0xFFFFFFFFu, p, off));
-                    if (b == 0 || p < bestD) {
-                        bestD = p;
-                        bb = b;
+                    for (uint32_t off = 16; off > 0; off >>= 1) {
+                        p0 = __dadd_rn(p0, __shfl_xor_sync(0xFFFFFFFFu, p0, off));
+                        p1 = __dadd_rn(p1, __shfl_xor_sync(0xFFFFFFFFu, p1, off));
+                    }
+                    if (bb == kMaxBranch || p0 < bestD) {
+                        bestD = p0;
+                        bb = b0;
+                    }
+                    if (p1 < bestD) {
+                        bestD = p1;
+                        bb = b1;
                     }
                 }
                 if (lane == src) bi = bb;
@@ -404,32 +464,44 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
         if (!build) {
             if (valid) L0.assign[uint64_t(ti.start) + row] = static_cast<uint8_t>(bi);
         } else {
-            if (valid) {
-                if (prevAssign != bi) atomicAdd(&S.chg, 1u);
-                L0.assign[at] = static_cast<uint8_t>(bi);
-                atomicAdd(&S.cnt[bi], 1u);
-                atomicAdd(&S.q[bi], (unsigned long long)S.xn[row]);
+            if (valid) L0.assign[at] = static_cast<uint8_t>(bi);
+            const uint32_t word = valid ? 1u << (8u * (bi & 3u)) : 0u, quad = bi >> 2;
+            *reinterpret_cast<uint4*>(S.oh + row * kMaxBranch) =
+                make_uint4(quad == 0 ? word : 0u, quad == 1 ? word : 0u, quad == 2 ? word : 0u, quad == 3 ? word : 0u);
+            uint32_t chose = __ballot_sync(0xFFFFFFFFu, valid);
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+                const uint32_t bits = __ballot_sync(0xFFFFFFFFu, (bi >> k) & 1u);
+                chose &= (lane >> k) & 1u ? bits : ~bits;
             }
-            S.bsel[row] = static_cast<uint8_t>(bi);
-            __syncwarp();
-            const uint32_t rEnd = ti.count < 32u * warp + 32u ? ti.count : 32u * warp + 32u;
-            for (uint32_t rr = 32u * warp; rr < rEnd; rr++) {
-                const uint32_t b = S.bsel[rr];
-                const uint32_t x = *reinterpret_cast<const uint32_t*>(S.x8 + rr * kDims + 4u * lane);
-                uint32_t* a = S.acc + b * kDims + lane;
-                atomicAdd(a, x & 0xFFu);
-                atomicAdd(a + 32, (x >> 8) & 0xFFu);
-                atomicAdd(a + 64, (x >> 16) & 0xFFu);
-                atomicAdd(a + 96, x >> 24);
+            myCnt += __popc(chose); // used of lanes below kMaxBranch
+            myChg += __popc(__ballot_sync(0xFFFFFFFFu, valid && prevAssign != bi));
+            const uint32_t xn = valid ? S.xn[row] : 0u; // below 2^23: 32 of them fit 32 bits
+            for (uint32_t b = 0; b < B; b++) {
+                const uint32_t part = __reduce_add_sync(0xFFFFFFFFu, bi == b ? xn : 0u);
+                if (lane == b) myQ += part;
             }
+            // center sums: x8 read MN-major (K = members) against the one-hot rows, as in assignKernel
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+            if (warp == 0) {
+                tcFenceAfter();
+                mmaU8x4(issuer, tmem + kAfSumCol, smemDescSw128(smemAddr(S.x8)), 4096u, smemDescMn16(smemAddr(S.oh)), 512u,
+                        idescU8(16) | kIdescMnMajorAB, accTiles);
+                if (issuer) mmaCommit(&S.sumBar);
+            }
+            sumsInFlight = true;
+            accTiles++;
         }
-        __syncthreads(); // the tiles, bsel and xn are rewritten by the next step
+        __syncthreads(); // the tiles and xn are rewritten by the next step
         t = n1;
         ti = tn1;
         n1 = n2;
         tn1 = tn2;
     }
-    flush();
+    if (t >= t1) flush();
+    waitSums(); // after a wait that ran out: MMAs in flight (bounded)
+    __syncthreads();
     if (tid == 0) {
         if (S.refined) atomicAdd(lv.refined, (unsigned long long)S.refined);
         if (S.visited) atomicAdd(lv.refined + 1, (unsigned long long)S.visited);

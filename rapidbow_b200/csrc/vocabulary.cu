@@ -694,12 +694,10 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
         for (uint32_t it = 0; streamed && it < opts.maxIterations; it++) {
             if (fl) {
                 launchAssignF(lvf, tiles128.as<NodeTile>(), totals, maxTiles128, stream);
-                RBW_CUDA(cudaMemsetAsync(activeCount, 0, 4, stream));
                 launchUpdateF(lvf, stream);
                 launchInertiaSum(inertiaNode.as<double>(), nbLv, inertiaTrace.as<double>() + it, stream);
             } else {
                 launchAssign(lv, tiles128.as<NodeTile>(), totals, maxTiles128, stream);
-                RBW_CUDA(cudaMemsetAsync(activeCount, 0, 4, stream));
                 launchUpdate(lv, stream);
             }
             iters = it + 1;
