@@ -25,6 +25,7 @@ struct KMeansLevel {
     uint8_t* centers;           // [nbNodes][16][128] (this level's slice of the tree)
     int32_t* cnorm;             // [nbNodes][16]
     uint8_t* assign;            // [nbMembers]
+    uint32_t* leaf;             // float lookups, last level: leaf per descriptor instead of `assign`
     uint32_t* counts;           // [nbNodes][16]
     unsigned long long* sums;   // [nbNodes][16][128]
     uint32_t* changed;          // [nbNodes] this iteration
@@ -91,11 +92,12 @@ void launchLloydShared(const KMeansLevel& lv, const LloydClasses& cls, uint32_t 
                        uint32_t maxIterations, cudaStream_t s);
 
 // ------------------------------------------------------------------ float-center mode
-// fp32 centers (the FP64 quotient of the exact integer sums, rounded once), distances from the
-// tensor core in bf16 with each center split into hi + lo bf16 parts and fp32 accumulation, and
-// an FP64 re-score of every member whose best-versus-second margin is within the error bound.
-// Per node, `split` holds the MMA B operand: [2 K-blocks of 64 dims][32 rows][128 B] bf16 in the
-// 128-byte swizzled K-major layout, rows 0-15 the hi parts and rows 16-31 the lo parts.
+// fp32 centers (the FP64 quotient of the exact integer sums, rounded once), approximate distances
+// from the tensor core, and an FP64 re-score of every member whose best-versus-second margin is
+// within the error bound.  Per node, `split` holds the MMA B operand, rows of 128 bytes in the
+// 128-byte swizzled K-major layout:
+//   limbs: round(c * 2^16) of centers in [0, 256), [48 rows]: high, middle and low byte of the 16;
+//   else:  bf16 hi + lo parts, [2 K-blocks of 64 dims][32 rows], rows 0-15 hi and 16-31 lo.
 constexpr uint32_t kSplitBytes = 2 * 32 * 128;
 constexpr float kPadNormF = 3.0e38f; // |c|^2 of padding slots: never the argmin
 
@@ -109,13 +111,14 @@ struct KMeansLevelF {
     double* inertiaNode;          // [nbNodes] FP64 inertia of the node's last assignment
     unsigned long long* refined;  // [2] members re-scored in FP64, members assigned (accumulated)
     uint32_t lookupOnly;          // 1: assignment only (lookup through a float tree)
+    uint32_t limbs;               // split holds the fixed-point operand
 };
 
 // fp32 centers from this level's uint8 initial centers (base.centers), then split, norms, bound.
 void launchCentersToFloat(const KMeansLevelF& lv, cudaStream_t s);
 // Split, norms and bound of nbNodes nodes of fp32 centers (tree upload / deserialisation).
 void launchPrepareFloatNodes(const float* centers, uint8_t* split, float* cn, float2* bound, uint64_t nbNodes,
-                             uint32_t B, cudaStream_t s);
+                             uint32_t B, bool limbs, cudaStream_t s);
 // One assign step (build) or one level of a lookup (lookupOnly) over 128-member node tiles.
 void launchAssignF(const KMeansLevelF& lv, const NodeTile* tiles, const uint32_t* nTilesDev, uint32_t maxTiles,
                    cudaStream_t s);

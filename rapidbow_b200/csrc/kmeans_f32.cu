@@ -3,18 +3,19 @@
 //
 //   * centers are fp32: c = float(double(sum) / double(count)) from the exact integer sums,
 //     kept when a center has no member (kmeans.cu:360-362);
-//   * distances: score_b = |c_b|^2 - 2 x.c_b with x.c_b from the tensor core.  x (uint8) is
-//     exact in bf16; every center is split into hi = bf16(c) and lo = bf16(c - hi), and one
-//     tcgen05.mma.kind::f16 (M = 128 members, N = 32 = 16 hi + 16 lo rows, fp32 accumulation)
-//     gives x.hi and x.lo, added in fp32;
-//   * error bound: |score error| <= 4e-5 (|x||c| + |c|^2) (the split leaves |c - hi - lo| <=
-//     2^-18 |c|; the products are exact in fp32; at most 127 accumulation roundings of <= 2^-23
-//     each; |c|^2 and the final subtraction round once more), so a member whose best-versus-
-//     second margin is at most kMarginScale (|x| max|c| + max|c|^2) -- six times the bound for
-//     both scores together -- is re-scored in FP64: the warp computes its squared distance to
-//     every center in the oracle's fixed order (lane partials of four fused multiply-adds, then
-//     a butterfly of pairwise sums) and keeps the lowest index on ties (kmeans.cu:131-135);
-//     every other member's fp32 argmin is the FP64 argmin by a margin;
+//   * distances: score_b = |c_b|^2 - 2 x.c_b with x.c_b from the tensor core, in one of two forms:
+//     centers in [0, 256) -- every build's, and most uploaded ones -- as 24-bit fixed point in three
+//     bytes (assignKernelX, exact integer products); any others as hi = bf16(c) and lo = bf16(c - hi)
+//     with x exact in bf16 (assignKernelF, fp32 accumulation);
+//   * error bound: of the bf16 form, |score error| <= 4e-5 (|x||c| + |c|^2) (the split leaves
+//     |c - hi - lo| <= 2^-18 |c|; the products are exact in fp32; at most 127 accumulation roundings
+//     of <= 2^-23 each; |c|^2 and the final subtraction round once more); of the fixed-point form, see
+//     assignKernelX.  A member whose best-versus-second margin is at most
+//     kMarginScale (|x| max|c| + max|c|^2) -- six times the bound for both scores together -- is
+//     re-scored in FP64: the warp computes its squared distance to every center within that margin of
+//     the best in the oracle's fixed order (lane partials of four fused multiply-adds, then a
+//     butterfly of pairwise sums) and keeps the lowest index on ties (kmeans.cu:131-135); every other
+//     center and member is decided by more than the error;
 //   * inertia: per node, sum_b (Q_b - 2 c_b.S_b + n_b |c_b|^2) in FP64 from the exact member
 //     sums S_b, counts n_b and sums of squared norms Q_b, with the centers of the assignment.
 #include "kmeans.cuh"
@@ -45,27 +46,46 @@ __device__ __forceinline__ void splitPair(float a, float b, uint32_t& hi, uint32
 }
 
 // Split, |c|^2 and bound of one node (256 threads: thread t handles dims 8 (t % 16) .. +7 of
-// center t / 16).  `red` is 16 floats of shared memory.
+// center t / 16).  `red` is 16 floats of shared memory.  limbs: the fixed-point operand (centers in
+// [0, 256)), else the bf16 one.
 __device__ void prepareNode(const float* __restrict__ c, uint8_t* __restrict__ split, float* __restrict__ cn,
-                            float2* __restrict__ bound, uint32_t B, float* red)
+                            float2* __restrict__ bound, uint32_t B, bool limbs, float* red)
 {
     const uint32_t t = threadIdx.x;
     const uint32_t j = t / 16, part = t % 16, d0 = part * 8;
-    uint32_t hi[4], lo[4];
+    float v[8];
     double nrm = 0.0;
 #pragma unroll
-    for (uint32_t k = 0; k < 4; k++) {
-        const float a = j < B ? c[j * kDims + d0 + 2 * k] : 0.f;
-        const float b = j < B ? c[j * kDims + d0 + 2 * k + 1] : 0.f;
-        splitPair(a, b, hi[k], lo[k]);
-        nrm = __fma_rn(double(a), double(a), nrm);
-        nrm = __fma_rn(double(b), double(b), nrm);
+    for (uint32_t k = 0; k < 8; k++) {
+        v[k] = j < B ? c[j * kDims + d0 + k] : 0.f;
+        nrm = __fma_rn(double(v[k]), double(v[k]), nrm);
     }
-    const uint32_t kb = d0 / 64, ch = (d0 % 64) / 8;
-    uint8_t* base = split + kb * 4096;
-    *reinterpret_cast<uint4*>(base + j * 128 + ((ch ^ (j & 7u)) << 4)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    const uint32_t r = 16 + j;
-    *reinterpret_cast<uint4*>(base + r * 128 + ((ch ^ (r & 7u)) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    if (limbs) {
+        // round(c * 2^16) in three bytes, the highest in rows 0-15, then 16-31 and 32-47; dims
+        // 8 part .. + 7 are half of 16-byte chunk part / 2
+        uint32_t w[3][2] = {};
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++) {
+            const uint32_t q = min(__float2uint_rn(v[k] * 65536.0f), 0xFFFFFFu);
+#pragma unroll
+            for (uint32_t l = 0; l < 3; l++) w[l][k / 4] |= ((q >> (16 - 8 * l)) & 0xFFu) << (8 * (k % 4));
+        }
+#pragma unroll
+        for (uint32_t l = 0; l < 3; l++) {
+            const uint32_t r = 16 * l + j;
+            *reinterpret_cast<uint2*>(split + r * 128 + (((part / 2) ^ (r & 7u)) << 4) + (part % 2) * 8) =
+                make_uint2(w[l][0], w[l][1]);
+        }
+    } else {
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) splitPair(v[2 * k], v[2 * k + 1], hi[k], lo[k]);
+        const uint32_t kb = d0 / 64, ch = (d0 % 64) / 8;
+        uint8_t* base = split + kb * 4096;
+        *reinterpret_cast<uint4*>(base + j * 128 + ((ch ^ (j & 7u)) << 4)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        const uint32_t r = 16 + j;
+        *reinterpret_cast<uint4*>(base + r * 128 + ((ch ^ (r & 7u)) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
 #pragma unroll
     for (uint32_t off = 8; off > 0; off >>= 1) nrm = __dadd_rn(nrm, __shfl_xor_sync(0xFFFFFFFFu, nrm, off));
     if (part == 0) {
@@ -90,42 +110,81 @@ __global__ void __launch_bounds__(256) centersToFloatKernel(KMeansLevelF lv)
         c[i] = i / kDims < lv.base.B ? float(u[i]) : 0.f;
     __syncthreads();
     prepareNode(c, lv.split + uint64_t(g) * kSplitBytes, lv.cn + uint64_t(g) * kMaxBranch, lv.bound + g, lv.base.B,
-                red);
+                true, red);
 }
 
 __global__ void __launch_bounds__(256) prepareNodesKernel(const float* centers, uint8_t* split, float* cn,
-                                                          float2* bound, uint32_t B)
+                                                          float2* bound, uint32_t B, bool limbs)
 {
     __shared__ float red[kMaxBranch];
     const uint64_t g = blockIdx.x;
-    prepareNode(centers + g * kMaxBranch * kDims, split + g * kSplitBytes, cn + g * kMaxBranch, bound + g, B, red);
+    prepareNode(centers + g * kMaxBranch * kDims, split + g * kSplitBytes, cn + g * kMaxBranch, bound + g, B, limbs,
+                red);
 }
 
-// ------------------------------------------------------------------ assign
+// The nearest of the centers in `cand` to the row whose dims 4 lane .. 4 lane + 3 are x0 .. x3, in FP64
+// in the oracle's order (orc_dist64: lane partials of four fused multiply-adds, then a butterfly of
+// pairwise sums), the lowest index on ties.  All lanes of the warp call it; cBase is their dims of
+// center 0.
+__device__ __forceinline__ uint32_t nearestFp64(const float* cBase, uint32_t cand, double x0, double x1, double x2,
+                                                double x3)
+{
+    auto partial = [&](const float4& c4) {
+        double e = __dsub_rn(x0, double(c4.x));
+        double p = __fma_rn(e, e, 0.0);
+        e = __dsub_rn(x1, double(c4.y));
+        p = __fma_rn(e, e, p);
+        e = __dsub_rn(x2, double(c4.z));
+        p = __fma_rn(e, e, p);
+        e = __dsub_rn(x3, double(c4.w));
+        return __fma_rn(e, e, p);
+    };
+    double bestD = 0.0;
+    uint32_t bb = kMaxBranch;
+    while (cand != 0) {
+        const uint32_t b0 = __ffs(cand) - 1;
+        cand &= cand - 1;
+        const uint32_t b1 = cand ? __ffs(cand) - 1 : b0; // the same again if there is no other
+        cand &= cand - 1;
+        const float4 c0 = __ldg(reinterpret_cast<const float4*>(cBase + b0 * kDims));
+        const float4 c1 = __ldg(reinterpret_cast<const float4*>(cBase + b1 * kDims));
+        double p0 = partial(c0), p1 = partial(c1);
+#pragma unroll
+        for (uint32_t off = 16; off > 0; off >>= 1) {
+            p0 = __dadd_rn(p0, __shfl_xor_sync(0xFFFFFFFFu, p0, off));
+            p1 = __dadd_rn(p1, __shfl_xor_sync(0xFFFFFFFFu, p1, off));
+        }
+        if (bb == kMaxBranch || p0 < bestD) {
+            bestD = p0;
+            bb = b0;
+        }
+        if (p1 < bestD) {
+            bestD = p1;
+            bb = b1;
+        }
+    }
+    return bb;
+}
+
+// ------------------------------------------------------------------ assign, any fp32 centers
+// Lookups through trees with centers outside [0, 256) (uploaded ones: centers of a build are means of
+// bytes), for which the fixed-point operand of assignKernelX does not exist.
 constexpr uint32_t kAfThreads = 128;
 constexpr uint32_t kAfRows = 128;
-constexpr uint32_t kAfTmemCols = 64; // distances to the hi and lo parts | sums
-constexpr uint32_t kAfSumCol = 32;
-constexpr uint32_t kAfFlushTiles = 65536; // 65,536 x 128 x 255 < 2^31
+constexpr uint32_t kAfTmemCols = 32;
 constexpr uint32_t kAfCtasPerSm = 3;
 constexpr uint32_t kAfTileWindow = kAfThreads; // one tile entry per thread per refill
-constexpr uint32_t kAfFrozen = 0x80000000u;
 
 struct AssignFSmem {
     uint8_t a[2][kAfRows * 128];     // members as bf16, two K-blocks of 64 dims, 128-byte swizzle
     uint8_t b[2][32 * 128];          // the node's hi (rows 0-15) and lo (rows 16-31) centers
-    uint8_t x8[kAfRows * kDims];     // members as uint8, 128-byte swizzle (sums and FP64 re-score)
-    uint8_t oh[kAfRows * kMaxBranch]; // [member][center] one-hot
-    NodeTile win[kAfTileWindow];     // tiles [winBase, winBase + kAfTileWindow) of the CTA's range,
-                                     // count | kAfFrozen for a frozen node
-    unsigned long long q[kMaxBranch];
+    uint8_t x8[kAfRows * kDims];     // members as uint8, 128-byte swizzle (FP64 re-score)
+    NodeTile win[kAfTileWindow];     // tiles [winBase, winBase + kAfTileWindow) of the CTA's range
     float cn[kMaxBranch];
     uint32_t xn[kAfRows];
-    uint32_t cnt[kMaxBranch];
     float2 bnd;
-    uint64_t mmaBar, sumBar;
+    uint64_t mmaBar;
     uint32_t tmemBase;
-    uint32_t chg;
     uint32_t abortFlag;
     uint32_t refined;
     uint32_t visited;
@@ -153,15 +212,12 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
     const uint32_t tid = threadIdx.x, lane = tid % 32;
     const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid / 32, 0); // uniform
     const uint32_t B = L0.B;
-    const bool build = lv.lookupOnly == 0;
-    if (build && blockIdx.x == 0 && tid == 0) *L0.activeCount = 0; // counted by the update that follows
     const uint32_t T = *nTilesDev;
     const uint32_t t0 = static_cast<uint32_t>(uint64_t(T) * blockIdx.x / gridDim.x);
     const uint32_t t1 = static_cast<uint32_t>(uint64_t(T) * (blockIdx.x + 1) / gridDim.x);
     volatile uint32_t* abortFlag = &S.abortFlag;
     if (tid == 0) {
         mbarInit(&S.mmaBar, 1);
-        mbarInit(&S.sumBar, 1);
         S.abortFlag = 0;
         S.refined = 0;
         S.visited = 0;
@@ -176,65 +232,8 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
     tcFenceAfter();
     const uint32_t tmem = S.tmemBase;
     const bool issuer = warp == 0 && electOne(); // one thread issues and commits every MMA
-    uint32_t curNode = 0xFFFFFFFFu, phase = 0, sumPhase = 0, accTiles = 0;
-    uint32_t myCnt = 0, myChg = 0;   // lane c < 16: this warp's rows that chose center c, and the
-    unsigned long long myQ = 0;      // sum of their |x|^2
-    bool curExclusive = false;       // every tile of the current node is in this CTA's range
-    bool sumsInFlight = false;
-    // the last sums MMA has read the tile and the one-hot rows
-    auto waitSums = [&]() -> bool {
-        if (!sumsInFlight) return true;
-        sumsInFlight = false;
-        const bool ok = mbarWait(&S.sumBar, sumPhase, abortFlag, L0.err, 55);
-        sumPhase ^= 1u;
-        tcFenceAfter();
-        return ok;
-    };
-    auto flush = [&]() {
-        if (curNode != 0xFFFFFFFFu && build) {
-            if (lane < kMaxBranch && myCnt) {
-                atomicAdd(&S.cnt[lane], myCnt);
-                atomicAdd(&S.q[lane], myQ);
-            }
-            if (lane == 0 && myChg) atomicAdd(&S.chg, myChg);
-            if (accTiles > 0 && waitSums()) {
-                uint32_t r[16];
-                tmemLoad16(tmem + kAfSumCol + ((warp * 32u) << 16), r); // lane = dimension tid
-                tmemWaitTie(r);
-                tcFenceBefore();
-                // plain stores for a node no other CTA touches (its accumulators are zero on entry)
-#pragma unroll
-                for (uint32_t b = 0; b < kMaxBranch; b++) {
-                    if (r[b] == 0) continue;
-                    unsigned long long* dst = L0.sums + (uint64_t(curNode) * kMaxBranch + b) * kDims + tid;
-                    if (curExclusive) *dst = r[b];
-                    else atomicAdd(dst, (unsigned long long)r[b]);
-                }
-            }
-            __syncthreads(); // S.cnt, S.q and S.chg complete
-            if (tid < kMaxBranch && S.cnt[tid]) {
-                uint32_t* c = L0.counts + uint64_t(curNode) * kMaxBranch + tid;
-                unsigned long long* qd = lv.q + uint64_t(curNode) * kMaxBranch + tid;
-                if (curExclusive) {
-                    *c = S.cnt[tid];
-                    *qd = S.q[tid];
-                } else {
-                    atomicAdd(c, S.cnt[tid]);
-                    atomicAdd(qd, S.q[tid]);
-                }
-            }
-            if (tid == 0 && S.chg) {
-                if (curExclusive) L0.changed[curNode] = S.chg;
-                else atomicAdd(L0.changed + curNode, S.chg);
-            }
-        }
-        accTiles = 0;
-        myCnt = 0;
-        myChg = 0;
-        myQ = 0;
-        __syncthreads();
-    };
-    // The tile list and the frozen flags are read a window of kAfTileWindow tiles at a time (one
+    uint32_t curNode = 0xFFFFFFFFu, phase = 0;
+    // The tile list is read a window of kAfTileWindow tiles at a time (one
     // load per thread, all in flight together), the member indices two tiles ahead and the member
     // rows one tile ahead of their use, into registers, so that no tile waits on a chain of
     // dependent global loads.  Every thread runs the same window refills (uniform).
@@ -242,9 +241,7 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
     auto refill = [&](uint32_t base) {
         __syncthreads(); // nobody reads the old window any more
         if (base + tid < t1) {
-            NodeTile x = tiles[base + tid];
-            if (build && L0.lastChanged[x.node] == 0) x.count |= kAfFrozen; // frozen node (kmeans.cu:238-240)
-            S.win[tid] = x;
+            S.win[tid] = tiles[base + tid];
         }
         winBase = base;
         __syncthreads();
@@ -252,11 +249,6 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
     auto entry = [&](uint32_t t) -> NodeTile {
         if (t - winBase >= kAfTileWindow) refill(t);
         return S.win[t - winBase];
-    };
-    auto nextLive = [&](uint32_t t) -> uint32_t {
-        for (; t < t1; t++)
-            if (!(entry(t).count & kAfFrozen)) return t;
-        return t1;
     };
     // rows past a tile's count repeat its first member (their results are not used)
     auto loadIndices = [&](const NodeTile& tn, uint32_t (&m)[kAfRows / 16]) {
@@ -273,7 +265,7 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
             v[k] = __ldg(reinterpret_cast<const uint4*>(L0.desc + uint64_t(m[k]) * kDims) + c8);
     };
     if (t0 < t1) refill(t0);
-    uint32_t t = nextLive(t0);
+    uint32_t t = t0;
     NodeTile ti{}, tn1{};
     uint32_t mNext[kAfRows / 16];
     uint4 v[kAfRows / 16];
@@ -282,7 +274,7 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
         loadIndices(ti, mNext);
         loadRows(mNext, v);
     }
-    uint32_t n1 = t < t1 ? nextLive(t + 1) : t1;
+    uint32_t n1 = min(t + 1, t1);
     if (n1 < t1) {
         tn1 = entry(n1);
         loadIndices(tn1, mNext);
@@ -290,33 +282,17 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
     while (t < t1) {
         if (tid == 0) S.visited += ti.count;
         if (ti.node != curNode) {
-            flush();
+            __syncthreads(); // the previous node's centers are no longer read
             curNode = ti.node;
-            curExclusive = ti.first >= t0 && uint64_t(ti.first) + (L0.nodeCnt[curNode] + kAfRows - 1) / kAfRows <= t1;
             const uint4* src = reinterpret_cast<const uint4*>(lv.split + uint64_t(curNode) * kSplitBytes);
 #pragma unroll
             for (uint32_t k = 0; k < kSplitBytes / 16 / kAfThreads; k++)
                 reinterpret_cast<uint4*>(&S.b[0][0])[tid + kAfThreads * k] = src[tid + kAfThreads * k];
             if (tid < kMaxBranch) {
                 S.cn[tid] = lv.cn[uint64_t(curNode) * kMaxBranch + tid];
-                S.cnt[tid] = 0;
-                S.q[tid] = 0;
             }
-            if (tid == 0) {
-                S.bnd = lv.bound[curNode];
-                S.chg = 0;
-            }
-        } else if (accTiles == kAfFlushTiles) {
-            // keep each s32 sum below 2^31: this node's partial results go out, later flushes add
-            curExclusive = false;
-            flush();
-            if (tid < kMaxBranch) {
-                S.cnt[tid] = 0;
-                S.q[tid] = 0;
-            }
-            if (tid == 0) S.chg = 0;
+            if (tid == 0) S.bnd = lv.bound[curNode];
         }
-        if (!waitSums()) break; // the tile below is read by the previous tile's sums MMA
         {
             // Eight threads per row, 16 rows per round: thread c8 = tid % 8 stages dims
             // 16 c8 .. 16 c8 + 15 of its row as uint8 and as bf16 (K-block c8 / 4, 16-byte chunks
@@ -351,7 +327,7 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
         NodeTile tn2{};
         if (n1 < t1) {
             loadRows(mNext, v);
-            n2 = nextLive(n1 + 1);
+            n2 = n1 + 1;
             if (n2 < t1) {
                 tn2 = entry(n2);
                 loadIndices(tn2, mNext);
@@ -359,8 +335,6 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
         }
         const uint32_t row = tid;
         const bool valid = row < ti.count;
-        const uint64_t at = uint64_t(ti.start) + row;
-        const uint32_t prevAssign = build && valid ? L0.assign[at] : 0u; // lands during the MMA
         // generic-proxy shared-memory writes read by the tensor core
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
@@ -419,79 +393,19 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
             while (mask != 0) {
                 const uint32_t src = __ffs(mask) - 1;
                 mask &= mask - 1;
-                uint32_t cand = __shfl_sync(0xFFFFFFFFu, near, src);
+                const uint32_t cand = __shfl_sync(0xFFFFFFFFu, near, src);
                 const uint32_t xw = *reinterpret_cast<const uint32_t*>(
                     S.x8 + (warp * 32u + src) * kDims + (((lane >> 2) ^ (src & 7u)) << 4) + ((lane & 3u) << 2));
                 const double x0 = double(xw & 0xFFu), x1 = double((xw >> 8) & 0xFFu);
                 const double x2 = double((xw >> 16) & 0xFFu), x3 = double(xw >> 24);
-                auto partial = [&](const float4& c4) {
-                    double e = __dsub_rn(x0, double(c4.x));
-                    double p = __fma_rn(e, e, 0.0);
-                    e = __dsub_rn(x1, double(c4.y));
-                    p = __fma_rn(e, e, p);
-                    e = __dsub_rn(x2, double(c4.z));
-                    p = __fma_rn(e, e, p);
-                    e = __dsub_rn(x3, double(c4.w));
-                    return __fma_rn(e, e, p);
-                };
-                double bestD = 0.0;
-                uint32_t bb = kMaxBranch;
-                while (cand != 0) {
-                    const uint32_t b0 = __ffs(cand) - 1;
-                    cand &= cand - 1;
-                    const uint32_t b1 = cand ? __ffs(cand) - 1 : b0; // the same again if there is no other
-                    cand &= cand - 1;
-                    const float4 c0 = __ldg(reinterpret_cast<const float4*>(cBase + b0 * kDims));
-                    const float4 c1 = __ldg(reinterpret_cast<const float4*>(cBase + b1 * kDims));
-                    double p0 = partial(c0), p1 = partial(c1);
-#pragma unroll
-                    for (uint32_t off = 16; off > 0; off >>= 1) {
-                        p0 = __dadd_rn(p0, __shfl_xor_sync(0xFFFFFFFFu, p0, off));
-                        p1 = __dadd_rn(p1, __shfl_xor_sync(0xFFFFFFFFu, p1, off));
-                    }
-                    if (bb == kMaxBranch || p0 < bestD) {
-                        bestD = p0;
-                        bb = b0;
-                    }
-                    if (p1 < bestD) {
-                        bestD = p1;
-                        bb = b1;
-                    }
-                }
+                const uint32_t bb = nearestFp64(cBase, cand, x0, x1, x2, x3);
                 if (lane == src) bi = bb;
             }
         }
-        if (!build) {
-            if (valid) L0.assign[uint64_t(ti.start) + row] = static_cast<uint8_t>(bi);
-        } else {
-            if (valid) L0.assign[at] = static_cast<uint8_t>(bi);
-            const uint32_t word = valid ? 1u << (8u * (bi & 3u)) : 0u, quad = bi >> 2;
-            *reinterpret_cast<uint4*>(S.oh + row * kMaxBranch) =
-                make_uint4(quad == 0 ? word : 0u, quad == 1 ? word : 0u, quad == 2 ? word : 0u, quad == 3 ? word : 0u);
-            uint32_t chose = __ballot_sync(0xFFFFFFFFu, valid);
-#pragma unroll
-            for (uint32_t k = 0; k < 4; k++) {
-                const uint32_t bits = __ballot_sync(0xFFFFFFFFu, (bi >> k) & 1u);
-                chose &= (lane >> k) & 1u ? bits : ~bits;
-            }
-            myCnt += __popc(chose); // used of lanes below kMaxBranch
-            myChg += __popc(__ballot_sync(0xFFFFFFFFu, valid && prevAssign != bi));
-            const uint32_t xn = valid ? S.xn[row] : 0u; // below 2^23: 32 of them fit 32 bits
-            for (uint32_t b = 0; b < B; b++) {
-                const uint32_t part = __reduce_add_sync(0xFFFFFFFFu, bi == b ? xn : 0u);
-                if (lane == b) myQ += part;
-            }
-            // center sums: x8 read MN-major (K = members) against the one-hot rows, as in assignKernel
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncthreads();
-            if (warp == 0) {
-                tcFenceAfter();
-                mmaU8x4(issuer, tmem + kAfSumCol, smemDescSw128(smemAddr(S.x8)), 4096u, smemDescMn16(smemAddr(S.oh)), 512u,
-                        idescU8(16) | kIdescMnMajorAB, accTiles);
-                if (issuer) mmaCommit(&S.sumBar);
-            }
-            sumsInFlight = true;
-            accTiles++;
+        if (valid) {
+            const uint64_t at = uint64_t(ti.start) + row;
+            if (L0.leaf) L0.leaf[L0.members[at]] = curNode * B + bi;
+            else L0.assign[at] = static_cast<uint8_t>(bi);
         }
         __syncthreads(); // the tiles and xn are rewritten by the next step
         t = n1;
@@ -499,9 +413,6 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
         n1 = n2;
         tn1 = tn2;
     }
-    if (t >= t1) flush();
-    waitSums(); // after a wait that ran out: MMAs in flight (bounded)
-    __syncthreads();
     if (tid == 0) {
         if (S.refined) atomicAdd(lv.refined, (unsigned long long)S.refined);
         if (S.visited) atomicAdd(lv.refined + 1, (unsigned long long)S.visited);
@@ -509,6 +420,425 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
     if (warp == 0) {
         tcFenceAfter();
         tmemDealloc(tmem, kAfTmemCols);
+    }
+}
+
+// ------------------------------------------------------------------ assign, centers in [0, 256)
+// The build's Lloyd step and lookups: assignKernel's tiles with fp32 centers.  A center is
+// round(c * 2^16), three bytes, so the distances are one u8 x u8 -> s32 product of the tile as it was
+// gathered (no conversion of the rows) with N = 48: x.c = 2^-16 (65536 D2 + 256 D1 + D0), D exact.
+//   * |x.c - that| <= 2^-17 sum(x) <= 8.7e-5 |x|; forming D2 + 2^-8 (D1 + floor(D0 / 2^8)) loses less
+//     than 2^-8 and rounds once, |c|^2 and the score round once: two scores are off by less than
+//     2^-21 (|x||c| + |c|^2) + 3.6e-4 |x| + 0.02 together, which the margin covers twice
+//     (kMarginScale's part alone: 256 times the first term).
+//   * Members within the margin go to a queue; the warps settle them in FP64 together, each row's
+//     near centers two at a time (oracle's orc_dist64 order), when the queue fills and at the end of
+//     the CTA's tiles: about 1 % of the rows, whose 1,200-cycle chains would otherwise hold up
+//     nearly every tile.  Their counts and sums go to global memory directly.
+// 300,007 members, one Lloyd step: 23-28 us, 33-40 us by bf16 halves (rows converted to bf16 in shared
+// memory, two K-blocks, the queue's work inside each tile); a lookup level of 200,003: 15.6, 21.5 us.
+constexpr uint32_t kAxThreads = 128;
+constexpr uint32_t kAxRows = 128;
+constexpr uint32_t kAxTmemCols = 64;    // three limbs' distances | sums
+constexpr uint32_t kAxSumCol = 48;
+constexpr uint32_t kAxCtasPerSm = 4;    // by shared memory (~49 KB each)
+constexpr uint32_t kAxFlushTiles = 65536; // 65,536 x 128 x 255 < 2^31
+constexpr uint32_t kAxQueue = 256;      // queued members; a tile adds at most 128
+constexpr uint32_t kAxFrozen = 0x80000000u;
+
+struct AssignXSmem {
+    uint8_t tile[2][kAxRows * kDims];     // member rows, 128-byte swizzle
+    uint8_t cen[48 * kDims];              // the node's limbs, same layout
+    uint8_t oh[kAxRows * kMaxBranch];     // [member][center] one-hot
+    NodeTile win[kAxThreads];             // tiles [winBase, winBase + 128) of the CTA's range
+    uint4 queue[kAxQueue];                // member position, node, near centers | previous << 16, |x|^2
+    unsigned long long q[kMaxBranch];
+    float cn[kMaxBranch];
+    uint32_t cnt[kMaxBranch];
+    float2 bnd;
+    uint64_t mmaBar, sumBar;
+    uint32_t tmemBase, abortFlag, chg, nQueue, nFold, refined, visited;
+};
+constexpr size_t kAxSmemBytes = sizeof(AssignXSmem) + 1024;
+
+__global__ void __launch_bounds__(kAxThreads, kAxCtasPerSm) assignKernelX(KMeansLevelF lv, const NodeTile* tiles,
+                                                                         const uint32_t* nTilesDev)
+{
+    extern __shared__ uint8_t smemRaw[];
+    AssignXSmem& S = *reinterpret_cast<AssignXSmem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
+    const KMeansLevel& L0 = lv.base;
+    const uint32_t tid = threadIdx.x, lane = tid % 32;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid / 32, 0); // uniform
+    const uint32_t B = L0.B;
+    const bool build = lv.lookupOnly == 0;
+    if (build && blockIdx.x == 0 && tid == 0) *L0.activeCount = 0; // counted by the update that follows
+    const uint32_t T = *nTilesDev;
+    const uint32_t t0 = static_cast<uint32_t>(uint64_t(T) * blockIdx.x / gridDim.x);
+    const uint32_t t1 = static_cast<uint32_t>(uint64_t(T) * (blockIdx.x + 1) / gridDim.x);
+    if (t0 == t1) return; // uniform: fewer tiles than CTAs
+    volatile uint32_t* abortFlag = &S.abortFlag;
+    if (tid == 0) {
+        mbarInit(&S.mmaBar, 1);
+        mbarInit(&S.sumBar, 1);
+        S.abortFlag = 0;
+        S.nQueue = 0;
+        S.refined = 0;
+        S.visited = 0;
+        fenceMbarInit();
+    }
+    if (warp == 0) {
+        tmemAlloc(&S.tmemBase, kAxTmemCols);
+        tmemRelinquish();
+    }
+    tcFenceBefore();
+    __syncthreads();
+    tcFenceAfter();
+    const uint32_t tmem = S.tmemBase;
+    const bool issuer = warp == 0 && electOne(); // one thread issues and commits every MMA
+    uint32_t curNode = 0xFFFFFFFFu, phase = 0, sumPhase = 0, accTiles = 0, buf = 0;
+    uint32_t myCnt = 0, myChg = 0;   // lane c < 16: this warp's rows that chose center c, and the
+    unsigned long long myQ = 0;      // sum of their |x|^2
+    bool curExclusive = false;       // every tile of the current node is in this CTA's range
+    bool ok = true;
+    uint32_t winBase = t0;
+    auto refill = [&](uint32_t base) {
+        __syncthreads(); // nobody reads the old window any more
+        if (base + tid < t1) {
+            NodeTile x = tiles[base + tid];
+            if (build && L0.lastChanged[x.node] == 0) x.count |= kAxFrozen; // frozen node (kmeans.cu:238-240)
+            S.win[tid] = x;
+        }
+        winBase = base;
+        __syncthreads();
+    };
+    auto entry = [&](uint32_t t) -> NodeTile {
+        if (t - winBase >= kAxThreads) refill(t);
+        return S.win[t - winBase];
+    };
+    auto nextLive = [&](uint32_t t) -> uint32_t {
+        for (; t < t1; t++)
+            if (!(entry(t).count & kAxFrozen)) return t;
+        return t1;
+    };
+    auto loadIndices = [&](const NodeTile& tn, uint32_t (&m)[kAxRows / 16]) {
+#pragma unroll
+        for (uint32_t k = 0; k < kAxRows / 16; k++) {
+            const uint32_t row = 16u * k + tid / 8;
+            m[k] = L0.members[uint64_t(tn.start) + (row < tn.count ? row : 0u)];
+        }
+    };
+    auto gatherRows = [&](const uint32_t (&m)[kAxRows / 16], uint32_t b) {
+        const uint32_t c = tid % 8;
+#pragma unroll
+        for (uint32_t k = 0; k < kAxRows / 16; k++) {
+            const uint32_t row = 16u * k + tid / 8;
+            cpAsync16(S.tile[b] + row * kDims + ((c ^ (row & 7u)) << 4), L0.desc + uint64_t(m[k]) * kDims + (c << 4));
+        }
+        cpAsyncCommit();
+    };
+    // Settles the queued members, one per warp at a time; their counts and sums go to global memory
+    // atomically.  At the end of the CTA's tiles (`last`) those of the current node, which are all of
+    // them where a node has many tiles, form one more tile for the sums MMA instead: 4,000 queued
+    // members of one node are half a million atomics on 1,280 addresses.
+    auto drain = [&](bool last) {
+        const bool fold = last && build && accTiles > 0;
+        if (fold) {
+            if (issuer) mmaCommit(&S.sumBar);
+            ok = mbarWait(&S.sumBar, sumPhase, abortFlag, L0.err, 57) && ok;
+            sumPhase ^= 1u;
+            tcFenceAfter();
+            *reinterpret_cast<uint4*>(S.oh + tid * kMaxBranch) = make_uint4(0, 0, 0, 0);
+            if (tid == 0) S.nFold = 0;
+        }
+        __syncthreads(); // the queue is complete
+        const uint32_t nq = S.nQueue;
+        for (uint32_t e = warp; e < nq; e += kAxThreads / 32) {
+            const uint4 en = S.queue[e];
+            const uint32_t member = L0.members[en.x];
+            const uint32_t xw = __ldg(reinterpret_cast<const uint32_t*>(L0.desc + uint64_t(member) * kDims) + lane);
+            const float* cBase = lv.centers + uint64_t(en.y) * kMaxBranch * kDims + 4u * lane;
+            const double x0 = double(xw & 0xFFu), x1 = double((xw >> 8) & 0xFFu);
+            const double x2 = double((xw >> 16) & 0xFFu), x3 = double(xw >> 24);
+            const uint32_t bi = nearestFp64(cBase, en.z & 0xFFFFu, x0, x1, x2, x3);
+            if (!build) {
+                if (lane == 0) {
+                    if (L0.leaf) L0.leaf[member] = en.y * B + bi;
+                    else L0.assign[en.x] = static_cast<uint8_t>(bi);
+                    if (L0.counts) atomicAdd(L0.counts + uint64_t(en.y) * kMaxBranch + bi, 1u);
+                }
+                continue;
+            }
+            if (lane == 0) L0.assign[en.x] = static_cast<uint8_t>(bi);
+            uint32_t slot = kAxRows;
+            if (fold && en.y == curNode) {
+                if (lane == 0) slot = atomicAdd(&S.nFold, 1u);
+                slot = __shfl_sync(0xFFFFFFFFu, slot, 0);
+            }
+            if (slot < kAxRows) {
+                *reinterpret_cast<uint32_t*>(S.tile[buf] + slot * kDims + (((lane >> 2) ^ (slot & 7u)) << 4) +
+                                             ((lane & 3u) << 2)) = xw;
+                if (lane == 0) {
+                    S.oh[slot * kMaxBranch + bi] = 1;
+                    atomicAdd(&S.cnt[bi], 1u);
+                    atomicAdd(&S.q[bi], (unsigned long long)en.w);
+                    if (en.z >> 16 != bi) atomicAdd(&S.chg, 1u);
+                }
+            } else {
+                if (en.y == curNode) curExclusive = false; // a plain-store flush would overwrite these
+                unsigned long long* sum = L0.sums + (uint64_t(en.y) * kMaxBranch + bi) * kDims + 4u * lane;
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++) atomicAdd(sum + k, (unsigned long long)((xw >> (8 * k)) & 0xFFu));
+                if (lane == 0) {
+                    atomicAdd(L0.counts + uint64_t(en.y) * kMaxBranch + bi, 1u);
+                    atomicAdd(lv.q + uint64_t(en.y) * kMaxBranch + bi, (unsigned long long)en.w);
+                    if (en.z >> 16 != bi) atomicAdd(L0.changed + en.y, 1u);
+                }
+            }
+        }
+        if (fold) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        curExclusive = __syncthreads_and(curExclusive) != 0; // and the queue has been read
+        if (fold && warp == 0) {
+            tcFenceAfter();
+            mmaU8x4(issuer, tmem + kAxSumCol, smemDescSw128(smemAddr(S.tile[buf])), 4096u, smemDescMn16(smemAddr(S.oh)),
+                    512u, idescU8(16) | kIdescMnMajorAB, 1u);
+        }
+        if (tid == 0) {
+            S.refined += nq;
+            S.nQueue = 0;
+        }
+        __syncthreads();
+    };
+    auto flush = [&]() {
+        if (curNode != 0xFFFFFFFFu && (build || L0.counts)) {
+            if (lane < kMaxBranch && myCnt) atomicAdd(&S.cnt[lane], myCnt);
+            if (build && lane < kMaxBranch && myQ) atomicAdd(&S.q[lane], myQ);
+            if (lane == 0 && myChg) atomicAdd(&S.chg, myChg);
+            if (accTiles > 0) {
+                if (issuer) mmaCommit(&S.sumBar); // nothing was committed yet for the last sums MMA
+                ok = ok && mbarWait(&S.sumBar, sumPhase, abortFlag, L0.err, 55);
+                sumPhase ^= 1u;
+                tcFenceAfter();
+                uint32_t r[16];
+                tmemLoad16(tmem + kAxSumCol + ((warp * 32u) << 16), r); // lane = dimension tid
+                tmemWaitTie(r);
+                tcFenceBefore();
+#pragma unroll
+                for (uint32_t b = 0; b < kMaxBranch; b++) {
+                    if (r[b] == 0) continue;
+                    unsigned long long* dst = L0.sums + (uint64_t(curNode) * kMaxBranch + b) * kDims + tid;
+                    if (curExclusive) *dst = r[b];
+                    else atomicAdd(dst, (unsigned long long)r[b]);
+                }
+            }
+            __syncthreads(); // S.cnt, S.q and S.chg complete
+            if (tid < kMaxBranch && S.cnt[tid]) {
+                uint32_t* c = L0.counts + uint64_t(curNode) * kMaxBranch + tid;
+                unsigned long long* qd = lv.q + uint64_t(curNode) * kMaxBranch + tid;
+                if (build && curExclusive) {
+                    *c = S.cnt[tid];
+                    *qd = S.q[tid];
+                } else {
+                    atomicAdd(c, S.cnt[tid]);
+                    if (build) atomicAdd(qd, S.q[tid]);
+                }
+            }
+            if (build && tid == 0 && S.chg) {
+                if (curExclusive) L0.changed[curNode] = S.chg;
+                else atomicAdd(L0.changed + curNode, S.chg);
+            }
+        }
+        accTiles = 0;
+        myCnt = 0;
+        myChg = 0;
+        myQ = 0;
+        __syncthreads();
+    };
+    refill(t0);
+    uint32_t t = nextLive(t0);
+    NodeTile ti{}, tn1{};
+    uint32_t mNext[kAxRows / 16];
+    if (t < t1) {
+        ti = entry(t);
+        loadIndices(ti, mNext);
+        gatherRows(mNext, buf);
+    }
+    uint32_t n1 = t < t1 ? nextLive(t + 1) : t1;
+    if (n1 < t1) {
+        tn1 = entry(n1);
+        loadIndices(tn1, mNext);
+    }
+    while (ok && t < t1) {
+        if (tid == 0) S.visited += ti.count;
+        if (ti.node != curNode) {
+            flush();
+            curNode = ti.node;
+            curExclusive = ti.first >= t0 && uint64_t(ti.first) + (L0.nodeCnt[curNode] + kAxRows - 1) / kAxRows <= t1;
+            const uint4* src = reinterpret_cast<const uint4*>(lv.split + uint64_t(curNode) * kSplitBytes);
+#pragma unroll
+            for (uint32_t k = 0; k < 3; k++) reinterpret_cast<uint4*>(S.cen)[tid + kAxThreads * k] = src[tid + kAxThreads * k];
+            if (tid < kMaxBranch) {
+                S.cn[tid] = lv.cn[uint64_t(curNode) * kMaxBranch + tid];
+                S.cnt[tid] = 0;
+                S.q[tid] = 0;
+            }
+            if (tid == 0) {
+                S.bnd = lv.bound[curNode];
+                S.chg = 0;
+            }
+        } else if (accTiles == kAxFlushTiles) {
+            // keep each s32 sum below 2^31: this node's partial results go out, later flushes add
+            curExclusive = false;
+            flush();
+            if (tid < kMaxBranch) {
+                S.cnt[tid] = 0;
+                S.q[tid] = 0;
+            }
+            if (tid == 0) S.chg = 0;
+        }
+        const uint32_t row = tid;
+        const bool valid = row < ti.count;
+        const uint64_t at = uint64_t(ti.start) + row;
+        const uint32_t prevAssign = build && valid ? L0.assign[at] : 0u;
+        cpAsyncWait<0>(); // this tile's rows
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (warp == 0) {
+            tcFenceAfter();
+            mmaU8x4(issuer, tmem, smemDescSw128(smemAddr(S.tile[buf])), 32u, smemDescSw128(smemAddr(S.cen)), 32u,
+                    idescU8(48), 0u);
+            if (issuer) mmaCommit(&S.mmaBar);
+        }
+        // |x|^2 of this thread's row while the product runs
+        uint32_t xn = 0;
+#pragma unroll
+        for (uint32_t c = 0; c < 8; c++) {
+            const uint4 x = *reinterpret_cast<const uint4*>(S.tile[buf] + row * kDims + ((c ^ (row & 7u)) << 4));
+            xn = __dp4a(x.x, x.x, xn);
+            xn = __dp4a(x.y, x.y, xn);
+            xn = __dp4a(x.z, x.z, xn);
+            xn = __dp4a(x.w, x.w, xn);
+        }
+        const float xLen = __fsqrt_ru(float(xn));
+        const float thr = __fmaf_rn(kMarginScale, __fmaf_rn(xLen, S.bnd.x, S.bnd.y), __fmaf_rn(xLen, 7.2e-4f, 0.04f));
+        if (!mbarWait(&S.mmaBar, phase, abortFlag, L0.err, 54)) {
+            ok = false;
+            break;
+        }
+        phase ^= 1u;
+        tcFenceAfter();
+        // The commit also covers the previous tile's sums MMAs: the other tile buffer and the one-hot
+        // rows are free.
+        uint32_t n2 = t1;
+        NodeTile tn2{};
+        if (n1 < t1) {
+            gatherRows(mNext, buf ^ 1u);
+            n2 = nextLive(n1 + 1);
+            if (n2 < t1) {
+                tn2 = entry(n2);
+                loadIndices(tn2, mNext);
+            }
+        }
+        float score[kMaxBranch];
+        {
+            uint32_t d2[16], d1[16], d0[16];
+            const uint32_t at0 = tmem + ((warp * 32u) << 16);
+            tmemLoad16(at0, d2);
+            tmemLoad16(at0 + 16u, d1);
+            tmemLoad16(at0 + 32u, d0);
+            tmemWaitTie(d2);
+            tmemWaitTie(d1);
+            tmemWaitTie(d0);
+            tcFenceBefore(); // the next tile's MMA overwrites these columns after the barriers below
+#pragma unroll
+            for (uint32_t b = 0; b < kMaxBranch; b++) {
+                // both integers are below 2^23: placed in the mantissa of 2^23 and freed of it
+                const float hi = __uint_as_float(d2[b] | 0x4B000000u) - 8388608.0f;
+                const float lo = __uint_as_float((d1[b] + (d0[b] >> 8)) | 0x4B000000u) - 8388608.0f;
+                score[b] = __fmaf_rn(-2.f, __fmaf_rn(lo, 0x1p-8f, hi), S.cn[b]);
+            }
+        }
+        float best = __int_as_float(0x7F800000), second = best;
+        uint32_t bi = 0;
+#pragma unroll
+        for (uint32_t b = 0; b < kMaxBranch; b++) {
+            if (b < B) {
+                const float s = score[b];
+                if (s < best) {
+                    second = best;
+                    best = s;
+                    bi = b;
+                } else if (s < second) {
+                    second = s;
+                }
+            }
+        }
+        const bool refine = valid && !(second - best > thr);
+        if (refine) {
+            uint32_t near = 0;
+#pragma unroll
+            for (uint32_t b = 0; b < kMaxBranch; b++)
+                if (b < B && !(score[b] - best > thr)) near |= 1u << b;
+            S.queue[atomicAdd(&S.nQueue, 1u)] = make_uint4(static_cast<uint32_t>(at), curNode, near | (prevAssign << 16), xn);
+        }
+        const bool settled = valid && !refine;
+        if (settled) {
+            if (L0.leaf) L0.leaf[L0.members[at]] = curNode * B + bi;
+            else L0.assign[at] = static_cast<uint8_t>(bi);
+        }
+        if (build || L0.counts) {
+            uint32_t chose = __ballot_sync(0xFFFFFFFFu, settled);
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+                const uint32_t bits = __ballot_sync(0xFFFFFFFFu, (bi >> k) & 1u);
+                chose &= (lane >> k) & 1u ? bits : ~bits;
+            }
+            myCnt += __popc(chose); // used of lanes below kMaxBranch
+        }
+        if (build) {
+            const uint32_t word = settled ? 1u << (8u * (bi & 3u)) : 0u, quad = bi >> 2;
+            *reinterpret_cast<uint4*>(S.oh + row * kMaxBranch) =
+                make_uint4(quad == 0 ? word : 0u, quad == 1 ? word : 0u, quad == 2 ? word : 0u, quad == 3 ? word : 0u);
+            myChg += __popc(__ballot_sync(0xFFFFFFFFu, settled && prevAssign != bi));
+            const uint32_t xs = settled ? xn : 0u; // below 2^23: 32 of them fit 32 bits
+            for (uint32_t b = 0; b < B; b++) {
+                const uint32_t part = __reduce_add_sync(0xFFFFFFFFu, bi == b ? xs : 0u);
+                if (lane == b) myQ += part;
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        __syncthreads(); // one-hot rows and queue entries are in, every warp has read its distances
+        if (build) {
+            if (warp == 0) {
+                tcFenceAfter();
+                mmaU8x4(issuer, tmem + kAxSumCol, smemDescSw128(smemAddr(S.tile[buf])), 4096u, smemDescMn16(smemAddr(S.oh)),
+                        512u, idescU8(16) | kIdescMnMajorAB, accTiles);
+            }
+            accTiles++;
+        }
+        if (S.nQueue > kAxQueue - kAxRows) drain(false); // uniform
+        buf ^= 1u;
+        t = n1;
+        ti = tn1;
+        n1 = n2;
+        tn1 = tn2;
+    }
+    cpAsyncWait<0>(); // a prefetch of a tile that was not scored (abort) must land before exit
+    if (ok) {
+        drain(true);
+        flush();
+    } else {
+        // MMAs may still be in flight: the TMEM is freed after them (a bounded wait)
+        if (issuer) mmaCommit(&S.sumBar);
+        mbarWait(&S.sumBar, sumPhase, abortFlag, L0.err, 56);
+        __syncthreads();
+    }
+    if (tid == 0) {
+        if (S.refined) atomicAdd(lv.refined, (unsigned long long)S.refined);
+        if (S.visited) atomicAdd(lv.refined + 1, (unsigned long long)S.visited);
+    }
+    if (warp == 0) {
+        tcFenceAfter();
+        tmemDealloc(tmem, kAxTmemCols);
     }
 }
 
@@ -576,7 +906,7 @@ __global__ void __launch_bounds__(256) updateKernelF(KMeansLevelF lv)
         q[t] = 0ull;
     }
     if (ch != 0)
-        prepareNode(c, lv.split + uint64_t(g) * kSplitBytes, lv.cn + uint64_t(g) * kMaxBranch, lv.bound + g, B, red);
+        prepareNode(c, lv.split + uint64_t(g) * kSplitBytes, lv.cn + uint64_t(g) * kMaxBranch, lv.bound + g, B, true, red);
 }
 
 __global__ void __launch_bounds__(1024) inertiaSumKernel(const double* in, uint32_t n, double* out)
@@ -618,13 +948,13 @@ void launchCentersToFloat(const KMeansLevelF& lv, cudaStream_t s)
 }
 
 void launchPrepareFloatNodes(const float* centers, uint8_t* split, float* cn, float2* bound, uint64_t nbNodes,
-                             uint32_t B, cudaStream_t s)
+                             uint32_t B, bool limbs, cudaStream_t s)
 {
     for (uint64_t off = 0; off < nbNodes; off += 0x7FFFFFFFull) {
         const uint64_t m = std::min<uint64_t>(nbNodes - off, 0x7FFFFFFFull);
         prepareNodesKernel<<<static_cast<uint32_t>(m), 256, 0, s>>>(centers + off * kMaxBranch * kDims,
                                                                      split + off * kSplitBytes, cn + off * kMaxBranch,
-                                                                     bound + off, B);
+                                                                     bound + off, B, limbs);
         RBW_CUDA(cudaGetLastError());
     }
 }
@@ -632,17 +962,24 @@ void launchPrepareFloatNodes(const float* centers, uint8_t* split, float* cn, fl
 void launchAssignF(const KMeansLevelF& lv, const NodeTile* tiles, const uint32_t* nTilesDev, uint32_t maxTiles,
                    cudaStream_t s)
 {
-    static std::atomic<uint64_t> attrSet{0};
-    setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(assignKernelF), static_cast<int>(kAfSmemBytes),
-                                   attrSet);
-    static_assert(kAfCtasPerSm * kAfTmemCols <= 512, "TMEM columns of the resident CTAs");
+    static_assert(kAfCtasPerSm * kAfTmemCols <= 512 && kAxCtasPerSm * kAxTmemCols <= 512, "TMEM columns");
     static_assert(kAfCtasPerSm * kAfSmemBytes <= 227 * 1024, "shared memory of the resident CTAs");
-    const uint32_t perSm =
-        std::min(kAfCtasPerSm, tunedValue(kTuneAssignFCtasPerSm, lv.base.B, 0, lv.base.nbMembers));
-    const uint32_t grid =
-        std::max(1u, std::min<uint32_t>(maxTiles, static_cast<uint32_t>(currentSmCount()) * perSm));
+    static_assert(kAxCtasPerSm * (kAxSmemBytes + 1024) <= 228 * 1024, "shared memory of the resident CTAs");
+    static std::atomic<uint64_t> attrF{0}, attrX{0};
+    const uint32_t tuned = tunedValue(kTuneAssignFCtasPerSm, lv.base.B, 0, lv.base.nbMembers);
+    const uint32_t sms = static_cast<uint32_t>(currentSmCount());
     ScopedKernelTimer timer(kTimedAssign, s);
-    assignKernelF<<<grid, kAfThreads, kAfSmemBytes, s>>>(lv, tiles, nTilesDev);
+    if (lv.limbs) {
+        // the tunable's largest value, also its default, stands for all that fit
+        const uint32_t perSm = tuned >= kAfCtasPerSm ? kAxCtasPerSm : tuned;
+        setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(assignKernelX), int(kAxSmemBytes), attrX);
+        assignKernelX<<<std::max(1u, std::min(maxTiles, sms * perSm)), kAxThreads, kAxSmemBytes, s>>>(lv, tiles, nTilesDev);
+    } else {
+        if (lv.lookupOnly == 0) throw Error(kInternal, "builds use fixed-point centers");
+        setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(assignKernelF), int(kAfSmemBytes), attrF);
+        assignKernelF<<<std::max(1u, std::min(maxTiles, sms * std::min(kAfCtasPerSm, tuned))), kAfThreads, kAfSmemBytes,
+                        s>>>(lv, tiles, nTilesDev);
+    }
     RBW_CUDA(cudaGetLastError());
 }
 

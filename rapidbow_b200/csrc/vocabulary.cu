@@ -90,14 +90,18 @@ __global__ void padKernel(const uint8_t* __restrict__ canon, uint8_t* __restrict
     reinterpret_cast<uint4*>(padded)[i] = v;
 }
 
-__global__ void padFloatKernel(const float* __restrict__ canon, float* __restrict__ padded, uint64_t nbNodes, uint32_t B)
+// *outside becomes non-zero if a center is not in [0, 256).
+__global__ void padFloatKernel(const float* __restrict__ canon, float* __restrict__ padded, uint64_t nbNodes, uint32_t B,
+                               unsigned long long* outside)
 {
     const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; // (node, slot, dim)
     if (i >= nbNodes * kMaxBranch * kDims) return;
     const uint32_t d = i % kDims;
     const uint32_t b = (i / kDims) % kMaxBranch;
     const uint64_t node = i / (uint64_t(kDims) * kMaxBranch);
-    padded[i] = b < B ? canon[(node * B + b) * kDims + d] : 0.f;
+    const float v = b < B ? canon[(node * B + b) * kDims + d] : 0.f;
+    padded[i] = v;
+    if (!(v >= 0.f && v < 256.f)) *outside = 1;
 }
 
 __global__ void roundCentersKernel(const float* __restrict__ f, uint8_t* __restrict__ u, uint64_t count, uint32_t B)
@@ -254,11 +258,17 @@ std::unique_ptr<Vocabulary> Vocabulary::fromHostF32(uint32_t B, uint32_t L, cons
     const uint64_t nodes = v->mNbNodes;
     DeviceBuffer canon(nodes * B * kDims * sizeof(float));
     RBW_CUDA(cudaMemcpy(canon.get(), centers, canon.bytes(), cudaMemcpyHostToDevice));
+    unsigned long long* outside = v->mRefined.as<unsigned long long>(); // zero, and again below
     padFloatKernel<<<blocksFor(nodes * kMaxBranch * kDims, 256), 256>>>(canon.as<float>(), v->mCentersF.as<float>(),
-                                                                        nodes, B);
+                                                                        nodes, B, outside);
     RBW_CUDA(cudaGetLastError());
+    // centers of a build are means of bytes; these may be any values
+    unsigned long long any = 0;
+    RBW_CUDA(cudaMemcpy(&any, outside, sizeof(any), cudaMemcpyDeviceToHost));
+    RBW_CUDA(cudaMemsetAsync(outside, 0, sizeof(any), nullptr));
+    v->mLimbs = any == 0;
     launchPrepareFloatNodes(v->mCentersF.as<float>(), v->mSplit.as<uint8_t>(), v->mCnF.as<float>(),
-                            v->mBound.as<float2>(), nodes, B, nullptr);
+                            v->mBound.as<float2>(), nodes, B, v->mLimbs, nullptr);
     v->roundFloatCenters(nullptr);
     v->mMasks.assign(masks, masks + nodes);
     v->mWeights.assign(weights, weights + nodes * B);
@@ -558,13 +568,13 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
     if (lloyd.get()) RBW_CUDA(cudaMemsetAsync(lloyd.get(), 0, kLloydCounters * 4 * L, stream));
     // float centers: member |x|^2 sums, per-node inertia, the level's inertia per step, counters
     StreamBuffer qSums(fl ? maxLevelNodes * kMaxBranch * 8 : 0, st), inertiaNode(fl ? maxLevelNodes * 8 : 0, st);
-    StreamBuffer inertiaTrace(fl ? uint64_t(opts.maxIterations) * 8 : 0, st), counters(fl ? uint64_t(L) * 16 : 0, st);
+    StreamBuffer inertiaLevel(fl ? uint64_t(L) * 16 : 0, st), counters(fl ? uint64_t(L) * 16 : 0, st);
     if (fl) {
         RBW_CUDA(cudaMemsetAsync(qSums.get(), 0, qSums.bytes(), stream));
         RBW_CUDA(cudaMemsetAsync(inertiaNode.get(), 0, inertiaNode.bytes(), stream));
         RBW_CUDA(cudaMemsetAsync(counters.get(), 0, counters.bytes(), stream));
     }
-    std::vector<double> hostFirst(L, 0.0), hostLast(L, 0.0);
+    std::vector<double> hostInertia(2 * size_t(L), 0.0);
     std::vector<unsigned long long> hostCounters(2 * size_t(L), 0ull);
 
     iotaKernel<<<blocksFor(n, 256), 256, 0, stream>>>(members.as<uint32_t>(), n);
@@ -609,6 +619,7 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
             lvf.base = lv;
             lvf.centers = voc->mCentersF.as<float>() + lb * kMaxBranch * kDims;
             lvf.split = voc->mSplit.as<uint8_t>() + lb * kSplitBytes;
+            lvf.limbs = 1;
             lvf.cn = voc->mCnF.as<float>() + lb * kMaxBranch;
             lvf.bound = voc->mBound.as<float2>() + lb;
             lvf.q = qSums.as<unsigned long long>();
@@ -692,16 +703,20 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
         }
         uint32_t iters = 0;
         for (uint32_t it = 0; streamed && it < opts.maxIterations; it++) {
+            const bool poll = (it + 1) % check == 0 || it + 1 == opts.maxIterations;
             if (fl) {
                 launchAssignF(lvf, tiles128.as<NodeTile>(), totals, maxTiles128, stream);
                 launchUpdateF(lvf, stream);
-                launchInertiaSum(inertiaNode.as<double>(), nbLv, inertiaTrace.as<double>() + it, stream);
+                // a level is left at a poll: the first step's sum and each poll's are all that is reported
+                if (it == 0) launchInertiaSum(inertiaNode.as<double>(), nbLv, inertiaLevel.as<double>() + 2 * level, stream);
+                if (poll)
+                    launchInertiaSum(inertiaNode.as<double>(), nbLv, inertiaLevel.as<double>() + 2 * level + 1, stream);
             } else {
                 launchAssign(lv, tiles128.as<NodeTile>(), totals, maxTiles128, stream);
                 launchUpdate(lv, stream);
             }
             iters = it + 1;
-            if ((it + 1) % check == 0 || it + 1 == opts.maxIterations) {
+            if (poll) {
                 // the host-side weight array is touched (its pages faulted in) while the device
                 // runs the level's first Lloyd steps, not after the last level
                 if (voc->mWeights.empty()) voc->mWeights.assign(voc->mNbNodes * B, 0.0f);
@@ -712,11 +727,6 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
             }
         }
         if (level < 16) bs.iterations[level] = iters;
-        if (fl) {
-            RBW_CUDA(cudaMemcpyAsync(&hostFirst[level], inertiaTrace.get(), 8, cudaMemcpyDeviceToHost, stream));
-            RBW_CUDA(cudaMemcpyAsync(&hostLast[level], inertiaTrace.as<double>() + (iters - 1), 8,
-                                     cudaMemcpyDeviceToHost, stream));
-        }
 
         // ---- stable regroup into the next level's nodes (Vocabulary.cpp:83-98)
         RegroupScratch rs{tileHist.as<uint32_t>(), tileScan.as<uint32_t>(), scanTmp.as<uint32_t>(),
@@ -733,6 +743,8 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
     voc->finalizeDevice(stream);
     if (fl) {
         RBW_CUDA(cudaMemcpyAsync(hostCounters.data(), counters.get(), hostCounters.size() * 8, cudaMemcpyDeviceToHost,
+                                 stream));
+        RBW_CUDA(cudaMemcpyAsync(hostInertia.data(), inertiaLevel.get(), hostInertia.size() * 8, cudaMemcpyDeviceToHost,
                                  stream));
     }
     // The counts land in the weights' own storage (one host buffer instead of two) and are
@@ -776,8 +788,8 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
             const uint64_t polled = std::min<uint64_t>(opts.maxIterations, (steps + check - 1) / check * check);
             bs.iterations[level] = std::max(bs.iterations[level], static_cast<uint32_t>(polled));
         }
-        bs.inertiaFirst[level] = hostFirst[level];
-        bs.inertiaLast[level] = hostLast[level];
+        bs.inertiaFirst[level] = hostInertia[2 * level];
+        bs.inertiaLast[level] = hostInertia[2 * level + 1];
         bs.refined[level] = hostCounters[2 * level];
         bs.assignments[level] = hostCounters[2 * level + 1];
     }
@@ -831,6 +843,7 @@ uint32_t Vocabulary::lookupFloat(const uint8_t* devDesc, uint64_t nTotal, uint32
             lvf.base = lv;
             lvf.centers = mCentersF.as<float>() + lb * kMaxBranch * kDims;
             lvf.split = mSplit.as<uint8_t>() + lb * kSplitBytes;
+            lvf.limbs = mLimbs ? 1u : 0u;
             lvf.cn = mCnF.as<float>() + lb * kMaxBranch;
             lvf.bound = mBound.as<float2>() + lb;
             lvf.refined = mRefined.as<unsigned long long>();

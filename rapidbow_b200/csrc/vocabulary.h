@@ -165,8 +165,9 @@ private:
     DeviceTree mTree;
     // float-center vocabularies
     bool mFloat = false;
+    bool mLimbs = true;      // every center is in [0, 256): fixed-point MMA operand
     DeviceArray mCentersF;  // [nbNodes][16][128] float
-    DeviceArray mSplit;     // [nbNodes][kSplitBytes] bf16 hi/lo MMA operand
+    DeviceArray mSplit;     // [nbNodes][kSplitBytes] MMA operand
     DeviceArray mCnF;       // [nbNodes][16] float |c|^2
     DeviceArray mBound;     // [nbNodes] float2
     DeviceArray mRefined;   // u64: lookup descriptors re-scored in FP64

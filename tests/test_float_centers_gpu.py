@@ -168,3 +168,42 @@ def test_uint8_build_injected_init_matches_oracle(oracle):
     assert np.array_equal(m, ref["masks"])
     assert np.array_equal(w, ref["weights"])
     assert np.array_equal(_lookup(voc, desc), oracle.lookup(ref["centers"], B, L, desc, threads=THREADS))
+
+
+@pytest.mark.parametrize("scale,shift", [(1.0, 0.0), (255.99 / 255, 0.0), (3.0, -100.0), (1.0, -0.001), (1.01, 0.0)])
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 30_011])
+def test_float_lookup_inside_and_outside_the_fixed_point_range(oracle, scale, shift, n):
+    """Centers in [0, 256) take the fixed-point operand, any other value the bf16 one; both equal FP64,
+    near ties (copies of rows among the centers) included."""
+    rng = np.random.default_rng(n)
+    B, L = 10, 3
+    nodes = level_beg(B, L)
+    data = sift_like(3000, seed=61).numpy()
+    centers = data[rng.integers(0, data.shape[0], nodes * B)].reshape(nodes, B, 128).astype(np.float32)
+    centers[:, 1::2] += rng.uniform(0, 0.02, centers[:, 1::2].shape).astype(np.float32)
+    centers[0, 0, 0] = 255.0
+    centers = (centers * np.float32(scale) + np.float32(shift)).astype(np.float32)
+    voc = rbw.vocabulary_from_host_f32(B, L, centers, np.full(nodes, 1023, np.uint32), np.ones((nodes, B), np.float32))
+    desc = np.concatenate([data, edge_descriptors(np.clip(centers, 0, 255).astype(np.uint8), 30_011, 62)])[-n:]
+    assert np.array_equal(_lookup(voc, np.ascontiguousarray(desc)), oracle.lookup_f32(centers, B, L, desc, threads=THREADS))
+
+
+@pytest.mark.parametrize("n_distinct,n", [(3, 700), (40, 30_000), (500, 9_000)])
+def test_float_build_of_duplicated_rows_matches_fp64_oracle(oracle, n_distinct, n):
+    """Few distinct rows: exact ties in most tiles, so the queue of members to settle in FP64 fills
+    within a node and at its end, in one node over many CTAs and in small ones."""
+    base = sift_like(n_distinct, seed=71 + n_distinct).numpy()
+    base[1] = base[0]
+    base[1, :2] += 1
+    desc = np.ascontiguousarray(base[np.random.default_rng(n).integers(0, n_distinct, n)])
+    B, L = 10, 2
+    rng = np.random.default_rng(n + 1)
+    injected = rng.integers(0, n, (level_beg(B, L), B)).astype(np.uint32)
+    voc = rbw.build_vocabulary(torch.from_numpy(desc).cuda(), B, nb_doc=30, nb_levels=L, init="injected",
+                               injected=injected, max_iterations=5, check_interval=2, float_centers=True)
+    ref = oracle.build_vocabulary_f32(desc, 30, B, L, max_iter=5, init=INIT_INJECTED, injected=injected, threads=THREADS)
+    assert np.array_equal(voc.centers_f32(), ref["centers"])
+    assert np.array_equal(voc.tree()[2], ref["weights"])
+    st = voc.build_stats()
+    for lv in range(L):
+        assert abs(st["inertia_last"][lv] - ref["inertia_last"][lv]) <= 1e-9 * max(ref["inertia_last"][lv], 1.0)
