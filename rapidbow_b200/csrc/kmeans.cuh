@@ -126,9 +126,22 @@ void launchAssignF(const KMeansLevelF& lv, const NodeTile* tiles, const uint32_t
 void launchUpdateF(const KMeansLevelF& lv, cudaStream_t s);
 // out[0] = sum of inertiaNode[0, nbNodes) in a fixed order (deterministic).
 void launchInertiaSum(const double* inertiaNode, uint32_t nbNodes, double* out, cudaStream_t s);
-// Leaf of every member of the last level: leaf[members[i]] = node(i) * B + assign[i].
-void launchWriteLeaves(const KMeansLevel& lv, const NodeTile* tiles, const uint32_t* nTilesDev, uint32_t maxTiles,
-                       uint32_t* leaf, cudaStream_t s);
+// Lookup of few descriptors through a tree of centers in [0, 256) in one launch (tree: level 0).
+uint32_t launchLookupDirectF(const KMeansLevelF& tree, uint32_t L, uint64_t n, uint32_t* leaf, cudaStream_t s);
+// One level's groups of a lookup (device pointers).
+struct LookupLevel {
+    uint32_t* nodeCnt;   // [nodes]
+    uint32_t* nodeOff;   // [nodes]
+    uint32_t* counts;    // [nodes][16] members per child, added up by launchAssignF
+    NodeTile* tiles;
+    uint32_t* totals;    // [1] tiles
+};
+// Levels small enough for launchLookupNextLevel (larger trees regroup as builds do).
+bool lookupCountsChildren(uint32_t B, uint32_t L);
+void launchLookupInit(uint32_t n, const LookupLevel& level0, uint32_t* members, cudaStream_t s);
+// Members of `from` (assignments in lv.assign) moved to their children, the groups of `to`.
+void launchLookupNextLevel(const KMeansLevel& lv, const LookupLevel& from, const LookupLevel& to, uint32_t* cursor,
+                           uint32_t* tileOff, uint32_t* childMembers, cudaStream_t s);
 
 // Stable regroup of every node's members by assignment (Vocabulary.cpp:83-98):
 // children (g, b) are laid out in order g*B + b; childCnt/childOff have nbNodes*B entries.

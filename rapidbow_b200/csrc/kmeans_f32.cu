@@ -923,18 +923,183 @@ __global__ void __launch_bounds__(1024) inertiaSumKernel(const double* in, uint3
     if (threadIdx.x == 0) *out = part[0];
 }
 
-__global__ void writeLeavesKernel(KMeansLevel lv, const NodeTile* tiles, const uint32_t* nTilesDev, uint32_t* leaf)
+// ------------------------------------------------------------------ lookups
+// Few descriptors: a warp per descriptor takes it through every level.  Lane l holds dims 4 l .. + 3 and
+// sums (x - c)^2 over them in fp32 for every center; the 16 sums are reduced over the lanes together,
+// each step halving the centers a lane keeps.  All terms are positive, so a distance is off by less
+// than 2^-20 of itself, far inside the margin within which FP64 decides (as everywhere in this file).
+// Bound by the node reads (512 bytes per center, row and level).
+constexpr uint32_t kDirectFThreads = 128;
+__global__ void __launch_bounds__(kDirectFThreads) lookupDirectF(const float* __restrict__ centers,
+                                                                 const float2* __restrict__ bound, uint32_t B,
+                                                                 uint32_t L, const uint8_t* __restrict__ desc,
+                                                                 uint64_t n, uint32_t* __restrict__ leaf,
+                                                                 unsigned long long* refined)
 {
-    // warp per 128-member tile
-    const uint32_t T = *nTilesDev;
-    const uint32_t warpsTotal = gridDim.x * (blockDim.x / 32);
+    const uint64_t row = uint64_t(blockIdx.x) * (kDirectFThreads / 32) + threadIdx.x / 32;
+    if (row >= n) return;
     const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t t = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; t < T; t += warpsTotal) {
-        const NodeTile ti = tiles[t];
-        for (uint32_t r = lane; r < ti.count; r += 32) {
-            const uint64_t at = uint64_t(ti.start) + r;
-            leaf[lv.members[at]] = ti.node * lv.B + lv.assign[at];
+    const uint32_t xw = __ldg(reinterpret_cast<const uint32_t*>(desc + row * kDims) + lane);
+    const float x0 = float(xw & 0xFFu), x1 = float((xw >> 8) & 0xFFu);
+    const float x2 = float((xw >> 16) & 0xFFu), x3 = float(xw >> 24);
+    const float xLen = __fsqrt_ru(float(__reduce_add_sync(0xFFFFFFFFu, __dp4a(xw, xw, 0u))));
+    // the center whose distance this lane ends up with (two lanes hold each)
+    const uint32_t mine = ((lane >> 4) & 1u) * 8u + ((lane >> 3) & 1u) * 4u + ((lane >> 2) & 1u) * 2u + ((lane >> 1) & 1u);
+    uint64_t idx = 0, lb = 0;
+    uint32_t settled = 0;
+    for (uint32_t level = 0; level < L; level++) {
+        const float* c = centers + (lb + idx) * kMaxBranch * kDims + 4u * lane;
+        float acc[kMaxBranch];
+#pragma unroll
+        for (uint32_t b = 0; b < kMaxBranch; b++) {
+            acc[b] = 1e30f;
+            if (b < B) {
+                const float4 v = __ldg(reinterpret_cast<const float4*>(c + b * kDims));
+                const float e0 = x0 - v.x, e1 = x1 - v.y, e2 = x2 - v.z, e3 = x3 - v.w;
+                acc[b] = fmaf(e3, e3, fmaf(e2, e2, fmaf(e1, e1, e0 * e0)));
+            }
         }
+#pragma unroll
+        for (uint32_t half = 8; half >= 1; half >>= 1) {
+            const bool up = (lane & (2u * half)) != 0;
+#pragma unroll
+            for (uint32_t b = 0; b < half; b++) {
+                const float give = up ? acc[b] : acc[b + half];
+                acc[b] = (up ? acc[b + half] : acc[b]) + __shfl_xor_sync(0xFFFFFFFFu, give, 2u * half);
+            }
+        }
+        const float dist = acc[0] + __shfl_xor_sync(0xFFFFFFFFu, acc[0], 1);
+        // non-negative floats order like their bits
+        const uint32_t bits = __float_as_uint(dist);
+        const uint32_t least = __reduce_min_sync(0xFFFFFFFFu, bits);
+        uint32_t bi = __reduce_min_sync(0xFFFFFFFFu, bits == least ? mine : kMaxBranch);
+        const uint32_t next = __reduce_min_sync(0xFFFFFFFFu, mine == bi ? 0x7F800000u : bits);
+        const float best = __uint_as_float(least);
+        const float2 bnd = __ldg(bound + lb + idx);
+        const float thr = kMarginScale * __fmaf_rn(xLen, bnd.x, bnd.y);
+        if (!(__uint_as_float(next) - best > thr)) {
+            const uint32_t near = __reduce_or_sync(0xFFFFFFFFu, mine < B && !(dist - best > thr) ? 1u << mine : 0u);
+            bi = nearestFp64(c, near, double(x0), double(x1), double(x2), double(x3));
+            settled++;
+        }
+        idx = idx * B + bi;
+        lb = lb * B + 1;
+    }
+    if (lane == 0) {
+        leaf[row] = static_cast<uint32_t>(idx);
+        if (settled) atomicAdd(refined, (unsigned long long)settled);
+        atomicAdd(refined + 1, (unsigned long long)L);
+    }
+}
+
+// More descriptors: per level one assign launch (which also counts the children), one scan of the
+// counts, and one launch that moves the members to their children and lists the next level's tiles.
+// The order of a node's members does not matter to a lookup, so a warp takes its slots from the
+// children's cursors.
+__global__ void lookupInitKernel(uint32_t n, uint32_t* members, uint32_t* nodeCnt, uint32_t* nodeOff, NodeTile* tiles,
+                                 uint32_t* totals, uint32_t* counts)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) members[i] = i;
+    const uint32_t T = (n + 127) / 128;
+    if (i < T) tiles[i] = NodeTile{0u, i * 128u, min(128u, n - i * 128u), 0u};
+    if (i < kMaxBranch) counts[i] = 0;
+    if (i == 0) {
+        nodeCnt[0] = n;
+        nodeOff[0] = 0;
+        totals[0] = T;
+    }
+}
+
+constexpr uint32_t kLookupScanChildren = 32768; // one CTA scans this many
+__global__ void __launch_bounds__(1024) lookupScanKernel(const uint32_t* counts, uint32_t nbNodes, uint32_t B,
+                                                         uint32_t* childCnt, uint32_t* childOff, uint32_t* cursor,
+                                                         uint32_t* tileOff, uint32_t* totals)
+{
+    __shared__ uint32_t wa[32], wb[32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+    const uint32_t nc = nbNodes * B, per = (nc + 1023) / 1024;
+    const uint32_t c0 = min(nc, tid * per), c1 = min(nc, c0 + per);
+    uint32_t a = 0, t = 0;
+    for (uint32_t c = c0; c < c1; c++) {
+        const uint32_t v = counts[(c / B) * kMaxBranch + c % B];
+        a += v;
+        t += (v + 127) / 128;
+    }
+    uint32_t ia = a, it = t;
+#pragma unroll
+    for (uint32_t off = 1; off < 32; off <<= 1) {
+        const uint32_t xa = __shfl_up_sync(0xFFFFFFFFu, ia, off), xt = __shfl_up_sync(0xFFFFFFFFu, it, off);
+        if (lane >= off) {
+            ia += xa;
+            it += xt;
+        }
+    }
+    if (lane == 31) {
+        wa[w] = ia;
+        wb[w] = it;
+    }
+    __syncthreads();
+    if (w == 0) {
+        uint32_t va = wa[lane], vb = wb[lane];
+#pragma unroll
+        for (uint32_t off = 1; off < 32; off <<= 1) {
+            const uint32_t xa = __shfl_up_sync(0xFFFFFFFFu, va, off), xb = __shfl_up_sync(0xFFFFFFFFu, vb, off);
+            if (lane >= off) {
+                va += xa;
+                vb += xb;
+            }
+        }
+        wa[lane] = va;
+        wb[lane] = vb;
+    }
+    __syncthreads();
+    uint32_t ra = (w ? wa[w - 1] : 0u) + ia - a, rt = (w ? wb[w - 1] : 0u) + it - t;
+    for (uint32_t c = c0; c < c1; c++) {
+        const uint32_t v = counts[(c / B) * kMaxBranch + c % B];
+        childCnt[c] = v;
+        childOff[c] = ra;
+        cursor[c] = ra;
+        tileOff[c] = rt;
+        ra += v;
+        rt += (v + 127) / 128;
+    }
+    if (tid == 1023) totals[0] = wb[31];
+}
+
+__global__ void __launch_bounds__(256) lookupMoveKernel(KMeansLevel lv, const NodeTile* tiles, const uint32_t* nTiles,
+                                                        uint32_t* cursor, uint32_t* childMembers,
+                                                        const uint32_t* childCnt, const uint32_t* childOff,
+                                                        const uint32_t* tileOff, const uint32_t* nextTotals,
+                                                        NodeTile* nextTiles, uint32_t* nextCounts)
+{
+    const uint32_t lane = threadIdx.x & 31u, threads = gridDim.x * blockDim.x;
+    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x, nc = lv.nbNodes * lv.B;
+    for (uint32_t i = gid; i < nc * kMaxBranch; i += threads) nextCounts[i] = 0;
+    const uint32_t nt = *nextTotals;
+    for (uint32_t t = gid; t < nt; t += threads) {
+        uint32_t lo = 0, hi = nc; // the last child whose first tile is at most t
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) / 2;
+            if (tileOff[mid] <= t) lo = mid + 1;
+            else hi = mid;
+        }
+        const uint32_t g = lo - 1, k = t - tileOff[g];
+        nextTiles[t] = NodeTile{g, childOff[g] + k * 128u, min(128u, childCnt[g] - k * 128u), tileOff[g]};
+    }
+    // a warp per quarter of a tile
+    const uint32_t T4 = *nTiles * 4;
+    for (uint32_t q = gid / 32; q < T4; q += threads / 32) {
+        const NodeTile ti = tiles[q / 4];
+        const uint32_t r = 32 * (q % 4) + lane;
+        const bool valid = r < ti.count;
+        const uint32_t b = valid ? lv.assign[uint64_t(ti.start) + r] : 0xFFu;
+        const uint32_t same = __match_any_sync(0xFFFFFFFFu, b);
+        const uint32_t leader = __ffs(same) - 1;
+        uint32_t base = 0;
+        if (valid && lane == leader) base = atomicAdd(cursor + ti.node * lv.B + b, uint32_t(__popc(same)));
+        base = __shfl_sync(0xFFFFFFFFu, base, leader);
+        if (valid) childMembers[base + __popc(same & ((1u << lane) - 1u))] = lv.members[uint64_t(ti.start) + r];
     }
 }
 
@@ -997,11 +1162,33 @@ void launchInertiaSum(const double* inertiaNode, uint32_t nbNodes, double* out, 
     RBW_CUDA(cudaGetLastError());
 }
 
-void launchWriteLeaves(const KMeansLevel& lv, const NodeTile* tiles, const uint32_t* nTilesDev, uint32_t maxTiles,
-                       uint32_t* leaf, cudaStream_t s)
+uint32_t launchLookupDirectF(const KMeansLevelF& tree, uint32_t L, uint64_t n, uint32_t* leaf, cudaStream_t s)
 {
-    const uint32_t blocks = std::max(1u, std::min<uint32_t>((maxTiles + 7) / 8, 16384));
-    writeLeavesKernel<<<blocks, 256, 0, s>>>(lv, tiles, nTilesDev, leaf);
+    const uint64_t perBlock = kDirectFThreads / 32;
+    ScopedKernelTimer timer(kTimedAssign, s);
+    lookupDirectF<<<static_cast<uint32_t>((n + perBlock - 1) / perBlock), kDirectFThreads, 0, s>>>(
+        tree.centers, tree.bound, tree.base.B, L, tree.base.desc, n, leaf, tree.refined);
+    RBW_CUDA(cudaGetLastError());
+    return 1;
+}
+
+bool lookupCountsChildren(uint32_t B, uint32_t L) { return ipow(B, L - 1) <= kLookupScanChildren; }
+
+void launchLookupInit(uint32_t n, const LookupLevel& lvl, uint32_t* members, cudaStream_t s)
+{
+    lookupInitKernel<<<std::max(1u, (n + 255) / 256), 256, 0, s>>>(n, members, lvl.nodeCnt, lvl.nodeOff, lvl.tiles,
+                                                                  lvl.totals, lvl.counts);
+    RBW_CUDA(cudaGetLastError());
+}
+
+void launchLookupNextLevel(const KMeansLevel& lv, const LookupLevel& from, const LookupLevel& to, uint32_t* cursor,
+                           uint32_t* tileOff, uint32_t* childMembers, cudaStream_t s)
+{
+    lookupScanKernel<<<1, 1024, 0, s>>>(from.counts, lv.nbNodes, lv.B, to.nodeCnt, to.nodeOff, cursor, tileOff, to.totals);
+    const uint64_t warps = lv.nbMembers / 32 + lv.nbNodes + 1;
+    const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((warps + 7) / 8, uint64_t(currentSmCount()) * 8));
+    lookupMoveKernel<<<blocks, 256, 0, s>>>(lv, from.tiles, from.totals, cursor, childMembers, to.nodeCnt, to.nodeOff,
+                                            tileOff, to.totals, to.tiles, to.counts);
     RBW_CUDA(cudaGetLastError());
 }
 

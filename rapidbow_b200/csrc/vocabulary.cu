@@ -799,17 +799,85 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
     return voc;
 }
 
+// Where the one-launch descent of float trees ends: it takes 0.3 ns per row and level (512 bytes per
+// center), the level-by-level path some 20 us per level whatever the rows.  Measured, direct against
+// level by level, us per call: B=10 L=4: 731 rows 12 / 74, 48,000 64 / 86, 64,000 82 / 86, 80,000
+// 101 / 94; B=16 L=3: 48,000 57 / 62, 64,000 74 / 64; B=10 L=2: 32,000 29 / 35, 48,000 39 / 35.
+uint64_t directFloatRows(uint32_t L) { return 16000ull * L; }
+
 uint32_t Vocabulary::lookupFloat(const uint8_t* devDesc, uint64_t nTotal, uint32_t* devLeaf, cudaStream_t stream) const
 {
-    // Level by level: the descriptors grouped by node, one split-bf16 assign launch over all the
-    // level's nodes (FP64 re-score near ties), then the stable regroup into the children.
+    // Level by level: the descriptors grouped by node, one assign launch over all the level's nodes
+    // (FP64 re-score near ties), then the regroup into the children.
     const uint32_t B = mB, L = mL;
+    auto levelF = [&](uint32_t level, const uint8_t* desc, uint32_t n) {
+        const uint64_t lb = levelBeg(B, level);
+        KMeansLevelF lvf{};
+        lvf.base.B = B;
+        lvf.base.nbNodes = static_cast<uint32_t>(ipow(B, level));
+        lvf.base.nbMembers = n;
+        lvf.base.desc = desc;
+        lvf.base.err = mErrors.as<DeviceErrors>();
+        lvf.centers = mCentersF.as<float>() + lb * kMaxBranch * kDims;
+        lvf.split = mSplit.as<uint8_t>() + lb * kSplitBytes;
+        lvf.limbs = mLimbs ? 1u : 0u;
+        lvf.cn = mCnF.as<float>() + lb * kMaxBranch;
+        lvf.bound = mBound.as<float2>() + lb;
+        lvf.refined = mRefined.as<unsigned long long>();
+        lvf.lookupOnly = 1;
+        return lvf;
+    };
+    if (mLimbs && nTotal <= directFloatRows(L))
+        return launchLookupDirectF(levelF(0, devDesc, static_cast<uint32_t>(nTotal)), L, nTotal, devLeaf, stream);
     const uint64_t chunk = std::min<uint64_t>(nTotal, 1ull << 27);
     const uint64_t maxLevelNodes = ipow(B, L - 1);
     const uint32_t maxTiles128 = static_cast<uint32_t>(chunk / 128 + maxLevelNodes + 1);
     const uint32_t maxTiles32 = static_cast<uint32_t>(chunk / 32 + maxLevelNodes + 1);
     const cudaStream_t st = stream;
+    const bool counted = mLimbs && lookupCountsChildren(B, L);
     StreamBuffer members(chunk * 4, st), members2(chunk * 4, st), assign(chunk, st);
+    uint32_t kernels = 0;
+    if (counted) {
+        // two levels' groups: counts and offsets of the nodes, child counts, tiles, their number
+        const uint64_t words = maxLevelNodes * (2 + kMaxBranch) + uint64_t(maxTiles128) * 4 + 4;
+        StreamBuffer groups((2 * words + 2 * maxLevelNodes) * 4, st);
+        auto levelAt = [&](uint32_t k) {
+            uint32_t* p = groups.as<uint32_t>() + k * words;
+            LookupLevel g{};
+            g.tiles = reinterpret_cast<NodeTile*>(p); // 16-byte entries first
+            g.totals = p + uint64_t(maxTiles128) * 4;
+            g.nodeCnt = g.totals + 4;
+            g.nodeOff = g.nodeCnt + maxLevelNodes;
+            g.counts = g.nodeOff + maxLevelNodes;
+            return g;
+        };
+        uint32_t* cursor = groups.as<uint32_t>() + 2 * words;
+        uint32_t* tileOff = cursor + maxLevelNodes;
+        for (uint64_t off = 0; off < nTotal; off += chunk) {
+            const uint32_t n = static_cast<uint32_t>(std::min(chunk, nTotal - off));
+            LookupLevel from = levelAt(0), to = levelAt(1);
+            launchLookupInit(n, from, members.as<uint32_t>(), stream);
+            kernels++;
+            for (uint32_t level = 0; level < L; level++) {
+                KMeansLevelF lvf = levelF(level, devDesc + off * kDims, n);
+                lvf.base.members = members.as<uint32_t>();
+                lvf.base.nodeOff = from.nodeOff;
+                lvf.base.nodeCnt = from.nodeCnt;
+                lvf.base.assign = assign.as<uint8_t>();
+                lvf.base.counts = level + 1 < L ? from.counts : nullptr;
+                lvf.base.leaf = level + 1 < L ? nullptr : devLeaf + off;
+                launchAssignF(lvf, from.tiles, from.totals, maxTiles128, stream);
+                kernels++;
+                if (level + 1 < L) {
+                    launchLookupNextLevel(lvf.base, from, to, cursor, tileOff, members2.as<uint32_t>(), stream);
+                    kernels += 2;
+                    std::swap(members, members2);
+                    std::swap(from, to);
+                }
+            }
+        }
+        return kernels;
+    }
     StreamBuffer nodeCnt(maxLevelNodes * 4, st), nodeOff(maxLevelNodes * 4, st);
     StreamBuffer childCnt(maxLevelNodes * 4, st), childOff(maxLevelNodes * 4, st), small(64, st);
     StreamBuffer tiles128(uint64_t(maxTiles128) * sizeof(NodeTile), st);
@@ -817,7 +885,6 @@ uint32_t Vocabulary::lookupFloat(const uint8_t* devDesc, uint64_t nTotal, uint32
     StreamBuffer scanTmp(scanTempWords(std::max<uint64_t>(uint64_t(B) * maxTiles32, maxLevelNodes)) * 4, st);
     StreamBuffer tileHist(uint64_t(B) * maxTiles32 * 4, st), tileScan(uint64_t(B) * maxTiles32 * 4, st);
     uint32_t* totals = small.as<uint32_t>();
-    uint32_t kernels = 0;
     for (uint64_t off = 0; off < nTotal; off += chunk) {
         const uint32_t n = static_cast<uint32_t>(std::min(chunk, nTotal - off));
         iotaKernel<<<blocksFor(n, 256), 256, 0, stream>>>(members.as<uint32_t>(), n);
@@ -827,38 +894,20 @@ uint32_t Vocabulary::lookupFloat(const uint8_t* devDesc, uint64_t nTotal, uint32
         RBW_CUDA(cudaMemcpyAsync(nodeOff.get(), &zero, 4, cudaMemcpyHostToDevice, stream));
         kernels++;
         for (uint32_t level = 0; level < L; level++) {
-            const uint32_t nbLv = static_cast<uint32_t>(ipow(B, level));
-            const uint64_t lb = levelBeg(B, level);
-            KMeansLevel lv{};
-            lv.B = B;
-            lv.nbNodes = nbLv;
-            lv.nbMembers = n;
-            lv.desc = devDesc + off * kDims;
-            lv.members = members.as<uint32_t>();
-            lv.nodeOff = nodeOff.as<uint32_t>();
-            lv.nodeCnt = nodeCnt.as<uint32_t>();
-            lv.assign = assign.as<uint8_t>();
-            lv.err = mErrors.as<DeviceErrors>();
-            KMeansLevelF lvf{};
-            lvf.base = lv;
-            lvf.centers = mCentersF.as<float>() + lb * kMaxBranch * kDims;
-            lvf.split = mSplit.as<uint8_t>() + lb * kSplitBytes;
-            lvf.limbs = mLimbs ? 1u : 0u;
-            lvf.cn = mCnF.as<float>() + lb * kMaxBranch;
-            lvf.bound = mBound.as<float2>() + lb;
-            lvf.refined = mRefined.as<unsigned long long>();
-            lvf.lookupOnly = 1;
-            buildNodeTiles(lv.nodeCnt, lv.nodeOff, nbLv, 128, tileOff.as<uint32_t>(), scanTmp.as<uint32_t>(),
-                           tiles128.as<NodeTile>(), maxTiles128, totals, stream);
+            KMeansLevelF lvf = levelF(level, devDesc + off * kDims, n);
+            lvf.base.members = members.as<uint32_t>();
+            lvf.base.nodeOff = nodeOff.as<uint32_t>();
+            lvf.base.nodeCnt = nodeCnt.as<uint32_t>();
+            lvf.base.assign = assign.as<uint8_t>();
+            lvf.base.leaf = level + 1 < L ? nullptr : devLeaf + off;
+            buildNodeTiles(nodeCnt.as<uint32_t>(), nodeOff.as<uint32_t>(), lvf.base.nbNodes, 128, tileOff.as<uint32_t>(),
+                           scanTmp.as<uint32_t>(), tiles128.as<NodeTile>(), maxTiles128, totals, stream);
             launchAssignF(lvf, tiles128.as<NodeTile>(), totals, maxTiles128, stream);
             kernels += 7;
-            if (level + 1 == L) {
-                launchWriteLeaves(lv, tiles128.as<NodeTile>(), totals, maxTiles128, devLeaf + off, stream);
-                kernels++;
-            } else {
+            if (level + 1 < L) {
                 RegroupScratch rs{tileHist.as<uint32_t>(), tileScan.as<uint32_t>(), scanTmp.as<uint32_t>(),
                                   tiles32.as<NodeTile>(), tileOff.as<uint32_t>(), totals, maxTiles32};
-                launchRegroup(lv, rs, members2.as<uint32_t>(), childCnt.as<uint32_t>(), childOff.as<uint32_t>(),
+                launchRegroup(lvf.base, rs, members2.as<uint32_t>(), childCnt.as<uint32_t>(), childOff.as<uint32_t>(),
                               stream);
                 kernels += 11;
                 std::swap(members, members2);

@@ -171,7 +171,7 @@ def test_uint8_build_injected_init_matches_oracle(oracle):
 
 
 @pytest.mark.parametrize("scale,shift", [(1.0, 0.0), (255.99 / 255, 0.0), (3.0, -100.0), (1.0, -0.001), (1.01, 0.0)])
-@pytest.mark.parametrize("n", [1, 127, 128, 129, 30_011])
+@pytest.mark.parametrize("n", [1, 2, 127, 128, 129, 48_000, 48_001])
 def test_float_lookup_inside_and_outside_the_fixed_point_range(oracle, scale, shift, n):
     """Centers in [0, 256) take the fixed-point operand, any other value the bf16 one; both equal FP64,
     near ties (copies of rows among the centers) included."""
@@ -184,7 +184,7 @@ def test_float_lookup_inside_and_outside_the_fixed_point_range(oracle, scale, sh
     centers[0, 0, 0] = 255.0
     centers = (centers * np.float32(scale) + np.float32(shift)).astype(np.float32)
     voc = rbw.vocabulary_from_host_f32(B, L, centers, np.full(nodes, 1023, np.uint32), np.ones((nodes, B), np.float32))
-    desc = np.concatenate([data, edge_descriptors(np.clip(centers, 0, 255).astype(np.uint8), 30_011, 62)])[-n:]
+    desc = np.concatenate([data, edge_descriptors(np.clip(centers, 0, 255).astype(np.uint8), 48_001, 62)])[-n:]
     assert np.array_equal(_lookup(voc, np.ascontiguousarray(desc)), oracle.lookup_f32(centers, B, L, desc, threads=THREADS))
 
 
@@ -207,3 +207,15 @@ def test_float_build_of_duplicated_rows_matches_fp64_oracle(oracle, n_distinct, 
     st = voc.build_stats()
     for lv in range(L):
         assert abs(st["inertia_last"][lv] - ref["inertia_last"][lv]) <= 1e-9 * max(ref["inertia_last"][lv], 1.0)
+
+
+@pytest.mark.parametrize("B,L,n", [(16, 1, 16_001), (2, 8, 140_003), (16, 5, 90_001), (10, 4, 64_001), (3, 3, 250_000)])
+def test_float_lookup_by_levels_matches_fp64_oracle(oracle, B, L, n):
+    """Above the one-launch limit: children counted by the assign and scanned in one CTA, or (trees
+    with more than 32,768 last-level nodes) regrouped as builds do; empty nodes in most levels."""
+    centers, masks, weights = random_tree(B, L, seed=B + L, dup_rate=0.2)
+    centers = centers.astype(np.float32)
+    centers[:, 1::2] = np.minimum(centers[:, 1::2] + np.float32(0.25), 255)
+    voc = rbw.vocabulary_from_host_f32(B, L, centers, masks, weights)
+    desc = edge_descriptors(centers.astype(np.uint8), n, seed=n)
+    assert np.array_equal(_lookup(voc, desc), oracle.lookup_f32(centers, B, L, desc, threads=THREADS))
