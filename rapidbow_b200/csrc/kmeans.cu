@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(kAssignThreads, kAssignCtasPerSm) assignKernel
                                                                   const uint32_t* nTilesDev)
 {
     extern __shared__ uint8_t smemRaw[];
-    AssignSmem& S = *reinterpret_cast<AssignSmem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
+    AssignSmem& S = *reinterpret_cast<AssignSmem*>(smemAligned(smemRaw));
     const uint32_t tid = threadIdx.x, lane = tid % 32;
     const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid / 32, 0); // uniform
     const uint32_t T = *nTilesDev;

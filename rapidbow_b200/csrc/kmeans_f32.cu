@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kAfThreads, kAfCtasPerSm) assignKernelF(KMeans
                                                                          const uint32_t* nTilesDev)
 {
     extern __shared__ uint8_t smemRaw[];
-    AssignFSmem& S = *reinterpret_cast<AssignFSmem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
+    AssignFSmem& S = *reinterpret_cast<AssignFSmem*>(smemAligned(smemRaw));
     const KMeansLevel& L0 = lv.base;
     const uint32_t tid = threadIdx.x, lane = tid % 32;
     const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid / 32, 0); // uniform
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(kAxThreads, kAxCtasPerSm) assignKernelX(KMeans
                                                                          const uint32_t* nTilesDev)
 {
     extern __shared__ uint8_t smemRaw[];
-    AssignXSmem& S = *reinterpret_cast<AssignXSmem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
+    AssignXSmem& S = *reinterpret_cast<AssignXSmem*>(smemAligned(smemRaw));
     const KMeansLevel& L0 = lv.base;
     const uint32_t tid = threadIdx.x, lane = tid % 32;
     const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid / 32, 0); // uniform

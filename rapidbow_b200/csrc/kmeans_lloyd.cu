@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kRows * kGroups, kCtasPerSm)
 {
     using Smem = LloydSmem<kTiles, kGroups>;
     extern __shared__ uint8_t smemRaw[];
-    Smem& S = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
+    Smem& S = *reinterpret_cast<Smem*>(smemAligned(smemRaw));
     LloydThread th = lloydSetup(S);
     const uint32_t nList = *listCount;
     while (!th.failed) {
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kRows * kShareGroups, 1)
 {
     using Smem = LloydSmem<kShareTiles, kShareGroups>;
     extern __shared__ uint8_t smemRaw[];
-    Smem& S = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
+    Smem& S = *reinterpret_cast<Smem*>(smemAligned(smemRaw));
     LloydThread th = lloydSetup(S);
     const uint32_t m = cls.counters[kLloydClasses]; // at most one node per CTA
     if (m > 0) {

@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     lookupPassTc(const __grid_constant__ CUtensorMap tmapTile, const PassParams p)
 {
     extern __shared__ uint8_t smemRaw[];
-    TcSmem& S = *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
+    TcSmem& S = *reinterpret_cast<TcSmem*>(smemAligned(smemRaw));
     const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x / 32, 0); // uniform
     const uint32_t lane = threadIdx.x % 32;
     const uint32_t T = p.tiles == nullptr ? static_cast<uint32_t>((p.nRows + kTileRows - 1) / kTileRows)
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(kRingThreads, 1)
     lookupPassRing(const __grid_constant__ CUtensorMap tmapTile, const PassParams p)
 {
     extern __shared__ uint8_t smemRaw[];
-    TcSmem& S = *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
+    TcSmem& S = *reinterpret_cast<TcSmem*>(smemAligned(smemRaw));
     const uint32_t warp = threadIdx.x / 32;
     const uint32_t lane = threadIdx.x % 32;
     const uint32_t T = p.tiles == nullptr ? static_cast<uint32_t>((p.nRows + kTileRows - 1) / kTileRows)

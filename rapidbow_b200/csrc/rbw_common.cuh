@@ -176,6 +176,10 @@ __device__ __forceinline__ bool mbarWait(uint64_t* bar, uint32_t parity, volatil
     }
 }
 
+// First 1,024-byte boundary of a dynamic shared memory block.  An offset from the array and not a
+// rounded pointer: the compiler then knows the address space and emits shared loads and stores.
+__device__ __forceinline__ uint8_t* smemAligned(uint8_t* raw) { return raw + ((0u - smemAddr(raw)) & 1023u); }
+
 // 4-byte asynchronous global -> shared copy (no register dependency) and its group fences.
 __device__ __forceinline__ void cpAsync4(void* dst, const void* src)
 {
