@@ -34,7 +34,7 @@ B, L = 16, 4
 N_TRAIN = 2_000_000
 N_LOOKUP = 10_000_000
 BYTES_PER_DESC = 132  # 128 B read + 4 B leaf written (algorithmic, per descriptor per pass)
-# DRAM bytes per descriptor of one lookupPassTc launch: dram__bytes_read.sum + dram__bytes_write.sum
+# DRAM bytes per descriptor of one lookupPassSorted launch: dram__bytes_read.sum + dram__bytes_write.sum
 # of an ncu capture of a 2M-descriptor lookup (B=16, L=4; both pass launches averaged).  Traffic
 # grows in proportion to the descriptors, so it is scaled to the timed launch.
 LOOKUP_PASS_DRAM_BYTES_PER_DESC = 136.6
@@ -293,7 +293,7 @@ def run_ours(args, world, rank, local):
     value = world * n / (ms / 1e3)
     fp32_value = world * n / (ms_simt / 1e3)
     ring = args.algo == "tensor_u8_ring" or (args.algo == "auto" and tuned is not None and tuned["value"] == 2)
-    pass_kernel = "lookupPassRing" if ring else "lookupPassTc"
+    pass_kernel = "lookupPassRing" if ring else "lookupPassSorted"
     hbm_peak, peak_kind = peaks()
     k_avg_ms = k_ms / max(k_n, 1)
     achieved = n * BYTES_PER_DESC / (k_avg_ms / 1e3) / 1e9

@@ -4,15 +4,16 @@
 // Three implementations, launchLookupDirect() and two behind launchLookup():
 //   * lookupDirect  : a warp per descriptor, every level in one launch, dp4a dot products (exact);
 //                     for few descriptors, where launches and the regroup cost more than the work.
-//   * lookupPassTc  : tcgen05 kind::i8 (u8 x u8 -> s32, exact) over level pairs.  A pass takes
-//                     the descriptors grouped by their node at level 2p, stages 128-row tiles in
-//                     shared memory (a TMA tiled load in input order for the first pass, a 16-byte
-//                     cp.async gather through the permutation afterwards), runs one MMA against
-//                     the node's 16 centers (level 2p) and one against all of its children's
-//                     centers (level 2p+1, N = 16*B), and picks the argmin of |c|^2 - 2 x.c
-//                     from tensor memory.  Between passes a device
-//                     counting sort (histogram fused into the pass epilogue, scan, scatter)
-//                     groups the descriptors by their node at level 2p+2.
+//   * lookupPassSorted : tcgen05 kind::i8 (u8 x u8 -> s32, exact) over level pairs.  A pass takes
+//                     the descriptors grouped by their node at level 2p, stages them in shared
+//                     memory (TMA tile loads in input order for the first pass, a 16-byte cp.async
+//                     gather through the permutation afterwards), runs one MMA against the node's
+//                     16 centers (level 2p), sorts the rows by branch, runs one against the
+//                     children's centers that a tile's rows need (level 2p+1), and picks the argmin
+//                     of |c|^2 - 2 x.c from tensor memory.  Between passes a device counting sort
+//                     (histogram, scan, scatter) groups the descriptors by their node at level 2p+2.
+//                     Two schedules without the sort stay selectable (lookupPassRing,
+//                     lookupPassWarpNode).
 //   * lookupSimtF32 : plain FP32 SIMT kernel (one thread per descriptor, 16 fp32 accumulators),
 //                     the comparison baseline.  Exact for uint8 data (all sums < 2^24).
 #include "lookup.cuh"
@@ -43,9 +44,7 @@ constexpr uint32_t kTcThreads = 32 * (3 + 2 * kTeamWarps); // TMA, two MMA issue
 constexpr uint32_t kRingThreads = kTcThreads + 32;          // ring schedule: three MMA issuers
 constexpr uint32_t kSmemHistMax = 1024;
 constexpr uint32_t kRegroupCtas = 148;                // regroup kernels' CTAs (one per SM on 148 SMs)
-// Two accumulator buffers of 256 columns; tile t uses buffer t & 1.  Its level-2p MMA (16
-// columns) lands in the first columns of the buffer and is read by the buffer's epilogue team
-// before the children MMA of the same tile overwrites the buffer.
+// Warp-node schedule: two accumulator buffers of 256 columns; tile t uses buffer t & 1.
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemBuf = 256;
 constexpr uint32_t kTileCache = 1024;
@@ -70,11 +69,8 @@ struct TcSmem {
     uint64_t aEmpty[kStages];
     uint64_t bFull[2];
     uint64_t bEmpty[2];
-    uint64_t accA[2];     // level-2p MMA into buffer j complete (one phase per use of j)
-    uint64_t aRead[2];    // team j has read the level-2p accumulators of buffer j
     uint64_t accB[2];     // children MMA into buffer j complete
     uint64_t bufFree[2];  // the last reader of buffer j is done with it
-    uint64_t lowFree[2];  // team j has read columns [0, 128) of buffer j (two levels only)
     uint64_t mmaDone;
     // ring schedule (lookupPassRing)
     uint64_t nodeAcc[8];  // node-level MMA of tile t complete (entry t % kNodeEntries)
@@ -285,6 +281,16 @@ __device__ __forceinline__ void emitRow(TcSmem& S, const PassParams& p, bool sme
     }
 }
 
+__device__ __forceinline__ void emitNode(const PassParams& p, uint32_t orig, uint32_t node)
+{
+    if (p.isFinal) {
+        p.out[orig] = node;
+    } else {
+        p.nodeNext[orig] = node;
+        if (p.binCount != nullptr) atomicAdd(&p.binCount[node], 1u);
+    }
+}
+
 // ------------------------------------------------------------------ producer warp
 // Stages the CTA's tiles [t0, t0 + nT) into the kStages shared-memory slots (arrival on aFull[s],
 // waits on aEmpty[s]) and each centre group's block (node + children, bFull / bEmpty).
@@ -418,15 +424,12 @@ __device__ __forceinline__ void passProducer(TcSmem& S, const PassParams& p, con
     __syncwarp();
 }
 
-// kWarpNode = false: both levels on tcgen05, the node-level MMA and the children MMA of a tile in
-// the same TMEM buffer (the children MMA waits until the team has read the node level).
-// kWarpNode = true: the epilogue teams take the node level from the shared-memory tile with
-// warp-level MMAs (warpNodeArgmin) while the children MMA runs, which is then issued as soon as
-// the tile has landed and its buffer is free; a tile slot is released once both its children MMA
-// and the team's reads are done.
-template <bool kWarpNode>
+// Warp-node schedule: the epilogue teams take the node level from the shared-memory tile with
+// warp-level MMAs (warpNodeArgmin) while the children MMA runs, which is issued as soon as the tile
+// has landed and its buffer is free; a tile slot is released once both its children MMA and the
+// team's reads are done.
 __global__ void __launch_bounds__(kTcThreads, 1)
-    lookupPassTc(const __grid_constant__ CUtensorMap tmapTile, const PassParams p)
+    lookupPassWarpNode(const __grid_constant__ CUtensorMap tmapTile, const PassParams p)
 {
     extern __shared__ uint8_t smemRaw[];
     TcSmem& S = *reinterpret_cast<TcSmem*>(smemAligned(smemRaw));
@@ -445,17 +448,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kStages; s++) {
             mbarInit(&S.aFull[s], 1);
-            // kWarpNode: the children MMA's commit (two levels) and the four warps of the team
-            mbarInit(&S.aEmpty[s], kWarpNode ? (two ? 1u : 0u) + kTeamWarps : 1u);
+            // the children MMA's commit (two levels) and the four warps of the team
+            mbarInit(&S.aEmpty[s], (two ? 1u : 0u) + kTeamWarps);
         }
         for (uint32_t j = 0; j < 2; j++) {
             mbarInit(&S.bFull[j], 1);
             mbarInit(&S.bEmpty[j], 2 + 2 * kTeamWarps); // both MMA issuers + both epilogue teams
-            mbarInit(&S.accA[j], 1);
-            mbarInit(&S.aRead[j], kTeamWarps);
             mbarInit(&S.accB[j], 1);
             mbarInit(&S.bufFree[j], kTeamWarps);
-            mbarInit(&S.lowFree[j], kTeamWarps);
         }
         mbarInit(&S.mmaDone, 2);
         S.abortFlag = 0;
@@ -480,20 +480,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         passProducer(S, p, &tmapTile, t0, nT, lane, abortFlag);
     } else if (nT > 0 && (warp == 1 || warp == kIssuer1Warp)) {
         // ------------------------------------------------------------ MMA issuers (one thread each)
-        // Issuer j (warp 1 for j = 0, warp kIssuer1Warp for j = 1) issues the MMAs of the tiles
-        // t with t & 1 == j, which accumulate in TMEM buffer j (columns [256 j, 256 j + 256)):
-        // a(t) (level 2p, 16 columns) needs only the buffer's first 16 columns, which epilogue
-        // team j releases after the first 128-column load of tile t-2, so the level-2p MMA of
-        // tile t overlaps the rest of that read; b(t) (children, 16 B columns) waits for the
-        // whole buffer and for the team to have read a(t).  One level: a(t) only, released after
-        // the team's read.  Two issuers let one buffer's MMAs go while the other's thread
-        // waits; commits track only the committing thread's MMAs, so each buffer's barriers see
-        // exactly its own tiles.  Both issuers pass every tile and commit once per centre group
-        // on the producer's "centre block free" barrier.
+        // Issuer j (warp 1 for j = 0, warp kIssuer1Warp for j = 1) issues the children MMAs of the
+        // tiles t with t & 1 == j, which accumulate in TMEM buffer j (columns [256 j, 256 j + 256)).
+        // Two issuers let one buffer's MMAs go while the other's thread waits; commits track only
+        // the committing thread's MMAs, so each buffer's barriers see exactly its own tiles.  Both
+        // pass every tile and commit once per centre group on the producer's "centre block free"
+        // barrier.
         {
             const bool issuer = electOne();
             const uint32_t jm = warp == 1 ? 0u : 1u;
-            const uint32_t idescA = idescU8(16);
             const uint32_t idescB = idescU8(16 * p.B);
             uint32_t prevGroup = 0xFFFFFFFFu, slot = 1, uses0 = 0, uses1 = 0;
             bool ok = true;
@@ -505,42 +500,18 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     if (!mbarWait(&S.bFull[slot], u & 1u, abortFlag, p.err, 20)) break;
                     prevGroup = ti.group;
                 }
-                if constexpr (kWarpNode) {
-                    // children only: as soon as the tile has landed and team j has read the
-                    // buffer's previous tile
-                    if ((t & 1u) == jm && two) {
-                        const uint32_t s = t % kStages;
-                        if (!mbarWait(&S.aFull[s], (t / kStages) & 1u, abortFlag, p.err, 21)) break;
-                        if (t >= 2 && !mbarWait(&S.bufFree[jm], ((t >> 1) - 1u) & 1u, abortFlag, p.err, 25)) break;
-                        tcFenceAfter();
-                        mmaU8x4(issuer, tmem + kTmemBuf * jm, smemDescSw128(smemAddr(S.a[s])), 32u,
-                                smemDescSw128(smemAddr(S.b[slot]) + kNodeBytes), 32u, idescB, 0u);
-                        if (issuer) {
-                            mmaCommit(&S.accB[jm]);
-                            mmaCommit(&S.aEmpty[s]);
-                        }
-                    }
-                } else if ((t & 1u) == jm) {
-                    const uint32_t j = jm;
+                // as soon as the tile has landed and team j has read the buffer's previous tile
+                if ((t & 1u) == jm && two) {
                     const uint32_t s = t % kStages;
                     if (!mbarWait(&S.aFull[s], (t / kStages) & 1u, abortFlag, p.err, 21)) break;
-                    if (t >= 2 && !mbarWait(two ? &S.lowFree[j] : &S.bufFree[j], ((t >> 1) - 1u) & 1u, abortFlag,
-                                            p.err, 22))
-                        break;
+                    if (t >= 2 && !mbarWait(&S.bufFree[jm], ((t >> 1) - 1u) & 1u, abortFlag, p.err, 25)) break;
                     tcFenceAfter();
-                    const uint64_t aDesc = smemDescSw128(smemAddr(S.a[s]));
-                    mmaU8x4(issuer, tmem + kTmemBuf * j, aDesc, 32u, smemDescSw128(smemAddr(S.b[slot])), 32u, idescA,
-                            0u);
-                    if (issuer) mmaCommit(&S.accA[j]);
-                    if (two) {
-                        if (!mbarWait(&S.aRead[j], (t >> 1) & 1u, abortFlag, p.err, 23)) break;
-                        if (t >= 2 && !mbarWait(&S.bufFree[j], ((t >> 1) - 1u) & 1u, abortFlag, p.err, 25)) break;
-                        tcFenceAfter();
-                        mmaU8x4(issuer, tmem + kTmemBuf * j, aDesc, 32u,
-                                smemDescSw128(smemAddr(S.b[slot]) + kNodeBytes), 32u, idescB, 0u);
-                        if (issuer) mmaCommit(&S.accB[j]);
+                    mmaU8x4(issuer, tmem + kTmemBuf * jm, smemDescSw128(smemAddr(S.a[s])), 32u,
+                            smemDescSw128(smemAddr(S.b[slot]) + kNodeBytes), 32u, idescB, 0u);
+                    if (issuer) {
+                        mmaCommit(&S.accB[jm]);
+                        mmaCommit(&S.aEmpty[s]);
                     }
-                    if (issuer) mmaCommit(&S.aEmpty[s]);
                 }
                 if (lastOfGroupSmem(S, p, t0, nT, t, ti.group) && issuer) mmaCommit(&S.bEmpty[slot]);
             }
@@ -551,13 +522,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     } else if (nT > 0 && warp >= 2 && warp < 2 + 2 * kTeamWarps) {
         // ------------------------------------------------------------ epilogue teams
         // Team j (warps 2 + 4 j .. 5 + 4 j, one per TMEM lane quarter; each thread owns one tile
-        // row) serves buffer j: the tiles t with t & 1 == j.  Per tile it reads the level-2p
-        // accumulators and picks the branch (releasing them to the children MMA), then reads the
-        // row's 16 * B children columns in 64-column loads -- releasing the first 128
-        // columns, where the next level-2p MMA of the buffer lands, after the first load and the
-        // buffer after the second -- and keeps the 16 columns of the chosen child.  The branch
-        // stays in a register.  With one level the team releases the buffer after the level-2p
-        // read.  Each team passes every tile so that both arrive once per centre group on bEmpty.
+        // row) serves buffer j: the tiles t with t & 1 == j.  Per tile it picks the branch of each row
+        // from the tile itself, then reads the row's 16 * B children columns in 64-column loads and
+        // keeps the 16 columns of the chosen child.  The branch stays in a register.  Each team
+        // passes every tile so that both arrive once per centre group on bEmpty.
         const uint32_t team = (warp - 2u) / kTeamWarps;
         const uint32_t q = warp & 3u;
         const uint32_t row = q * 32u + lane;
@@ -579,28 +547,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             if (j == team) {
                 const uint32_t orig = row < ti.count ? (gather ? __ldg(p.perm + ti.start + row) : ti.start + row) : 0u;
                 const uint32_t base = tRow + kTmemBuf * j;
-                uint32_t b;
-                if constexpr (kWarpNode) {
-                    // node level from the shared-memory tile (warp-level MMAs), while the
-                    // children MMA of the same tile runs on the tensor core
-                    const uint32_t s = t % kStages;
-                    if (!mbarWait(&S.aFull[s], (t / kStages) & 1u, abortFlag, p.err, 34)) break;
-                    b = warpNodeArgmin(smemAddr(S.a[s]), smemAddr(S.b[slot]), q, lane, &S.cn[slot][0][0]);
-                    __syncwarp();
-                    if (lane == 0) mbarArrive(&S.aEmpty[s]); // this warp is done reading the tile
-                } else {
-                    if (!mbarWait(&S.accA[j], (t >> 1) & 1u, abortFlag, p.err, 30)) break;
-                    tcFenceAfter();
-                    {
-                        uint32_t r[16];
-                        tmemLoad16(base, r);
-                        tmemWaitTie(r);
-                        b = argminScores(r, &S.cn[slot][0][0]);
-                    }
-                    tcFenceBefore();
-                    __syncwarp();
-                    if (lane == 0) mbarArrive(two ? &S.aRead[j] : &S.bufFree[j]);
-                }
+                // node level from the shared-memory tile (warp-level MMAs), while the children MMA of
+                // the same tile runs on the tensor core
+                const uint32_t s = t % kStages;
+                if (!mbarWait(&S.aFull[s], (t / kStages) & 1u, abortFlag, p.err, 34)) break;
+                const uint32_t b = warpNodeArgmin(smemAddr(S.a[s]), smemAddr(S.b[slot]), q, lane, &S.cn[slot][0][0]);
+                __syncwarp();
+                if (lane == 0) mbarArrive(&S.aEmpty[s]); // this warp is done reading the tile
                 if (!two) {
                     if (row < ti.count) emitRow(S, p, smemHist, orig, ti.group * p.B + b);
                 } else {
@@ -621,12 +574,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     };
                     pick(0);
                     pick(1);
-                    if constexpr (!kWarpNode) {
-                        // columns [0, 128) have been read: the level-2p MMA of tile t + 2 may start
-                        tcFenceBefore();
-                        __syncwarp();
-                        if (lane == 0) mbarArrive(&S.lowFree[j]);
-                    }
                     if (p.B > 8) {
                         pick(2);
                         pick(3);
@@ -797,7 +744,7 @@ __global__ void __launch_bounds__(kRingThreads, 1)
         for (uint32_t t = 0; t < nT; t++) {
             const TileInfo ti = tileAtSmem(S, p, t0, t);
             if (ti.group != prevGroup) {
-                // every team waits for every group's block (see lookupPassTc)
+                // every team waits for every group's block (see lookupPassWarpNode)
                 slot ^= 1u;
                 const uint32_t u = slot ? uses1++ : uses0++;
                 if (!mbarWait(&S.bFull[slot], u & 1u, abortFlag, p.err, 50)) break;
@@ -879,11 +826,526 @@ __global__ void __launch_bounds__(kRingThreads, 1)
     }
 }
 
+// ------------------------------------------------------------------ sorted schedule
+// Super-tiles of two 128-row tiles of one node, their rows sorted by the branch taken at level 2p
+// before the children are scored: a tile of the sorted rows then meets the 8-9 children of its rows
+// instead of all 16, in the MMA (N = 16 per child), and a warp's 32 rows meet 2-3, so that a thread
+// reads 48 columns of tensor memory to keep 16 and not 256.  Warps:
+//   * two teams of eight workers (one thread per row; warp w reads TMEM lane quarter w % 4 of tile
+//     w / 4), team t takes super-tiles t, t + 2, ...; while one waits for its children the other sorts:
+//     P1 branch from the node level; P2 counting sort of the 256 rows by branch; P3 the rows, held in
+//     registers since P1, go back to the buffer in sorted order (eight lanes per row: no bank
+//     conflicts); P4 the thread of sorted row r takes its child's 16 columns; P5 argmin, and the leaf
+//     or the next level's node is written;
+//   * the MMA issuer: the children (M = 128, N = 16 per child) of super-tile s once it is sorted, then
+//     the node level (N = 16) of s + 2;
+//   * two producers: TMA tile loads in the first pass; afterwards each gathers one tile of a
+//     super-tile, 16 bytes per lane; the first also loads each group's centers;
+//   * the norms warp turns a group's |c|^2 into the keys of argminKeys.
+// The n-th group of a CTA uses center slot n & 1, for the (n >> 1)-th time.
+//
+// What bounds it: a team's chain from the node level to the leaf, ~4,900 cycles per 256 rows at 16
+// warps with IPC 0.42 per scheduler, two teams at once (memory: 2 x 700 per 128 rows; tensor pipe
+// ~470).  Its instruction footprint counts: each wait keeps only its loop inline and
+// no loop over super-tiles is unrolled (16-byte instructions, 74 -> 29 KB: 505 -> 349 us).  Three
+// teams would have 72 registers a thread; the rows held over the sort alone take 32.
+// 10,000,003 rows, B = 16, L = 4: first pass 505 -> 352 us, second 490 -> 452 us against two teams
+// that read all 16 B columns; whole lookups: 1,000,000 rows, B = 10, L = 6: 348 -> 322 us; 500,000
+// rows, B = 16, L = 4: 94 -> 81 us; 60,000 rows, B = 10, L = 6: 179 -> 179 us; 4,000,000 rows, B = 2,
+// L = 8: 836 -> 785 us.
+//
+// Tile j's child c lands in columns 16 (c + j) of the children area: the two tiles share at most one
+// child.  Up to B = 13 both teams' areas fit beside the node columns, above that they take turns.
+constexpr uint32_t kSubTiles = 2;
+constexpr uint32_t kSuperRows = kSubTiles * kTileRows;     // 256
+constexpr uint32_t kSuperBufs = 4;
+constexpr uint32_t kSortTeamWarps = kSuperRows / 32;       // 8
+constexpr uint32_t kSortIssuer = 2 * kSortTeamWarps;       // warp 16, then the producers
+constexpr uint32_t kSortThreads = 32 * (kSortIssuer + 4);
+constexpr uint32_t kSortNodeCols = 16 * kSubTiles;         // one super-tile's node level
+constexpr uint32_t kSortKidCol = 2 * kSortNodeCols;
+static_assert(kSortKidCol + 16 * (kMaxBranch + kSubTiles - 1) <= kTmemCols, "sorted schedule exceeds tensor memory");
+constexpr uint32_t kSortTileCache = 512;
+constexpr uint32_t kLastOfGroup = 1, kNextIsLast = 2, kFirstOfGroup = 4; // TileInfo::pad of a super-tile
+
+struct SortSmem {
+    uint8_t a[kSuperBufs][kSubTiles * kTileBytes];
+    uint8_t b[2][kBBlockBytes];
+    alignas(16) int32_t cn[2][17][16];   // keys of |c|^2 of each B slot: row 0 = node, rows 1.. = children
+    TileInfo tileCache[kSortTileCache];  // this CTA's super-tiles (passes after the first)
+    uint32_t orig[2][kSuperRows];        // by team and sorted position: row id
+    uint8_t child[2][kSuperRows];        // ... and branch
+    uint32_t cnt[2][2][16];              // rows per branch, by team and turn
+    uint32_t binBase[2][17];             // first sorted position of each branch; [16] = rows
+    uint64_t aFull[kSuperBufs], aFree[kSuperBufs];
+    uint64_t bFull[2], bEmpty[2], cnReady[2];
+    uint64_t nodeDone[2], counted[2], sorted[2], kidsDone[2], kidsRead[2]; // by team
+    uint64_t mmaDone;
+    uint32_t tmemBase, abortFlag, noAbort;
+};
+constexpr size_t kSortSmemBytes = sizeof(SortSmem) + 1024;
+static_assert(kSortSmemBytes <= 227 * 1024, "shared memory");
+
+// Super-tile i of this CTA, with its place in its group's run here.
+__device__ __forceinline__ TileInfo superTileGlobal(const TileInfo* tiles, uint32_t nT, uint32_t i)
+{
+    TileInfo ti = tiles[i];
+    auto sameGroup = [&](uint32_t k) { return k < nT && tiles[k].group == ti.group; };
+    ti.pad = !sameGroup(i + 1) ? kLastOfGroup : !sameGroup(i + 2) ? kNextIsLast : 0u;
+    if (i == 0 || !sameGroup(i - 1)) ti.pad |= kFirstOfGroup;
+    return ti;
+}
+template <bool kGather>
+__device__ __forceinline__ TileInfo superTile(const SortSmem& S, const PassParams& p, uint32_t t0, uint32_t nT, uint32_t i)
+{
+    if (kGather) return S.tileCache[i];
+    const uint32_t start = (t0 + i) * kSuperRows; // first pass: rows in order, at most 2^30
+    return TileInfo{0u, start, min(static_cast<uint32_t>(p.nRows) - start, kSuperRows),
+                    (i + 1 >= nT ? kLastOfGroup : i + 2 >= nT ? kNextIsLast : 0u) | (i == 0 ? kFirstOfGroup : 0u)};
+}
+
+// mbarWait by a whole warp, with one answer for all its lanes.
+// Whether a phase is complete, without waiting.
+__device__ __forceinline__ bool mbarTest(uint64_t* bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(smemAddr(bar)), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+__device__ __noinline__ void waitTimedOut(uint32_t abortFlag, DeviceErrors* err, uint32_t site, uint32_t parity)
+{
+    *static_cast<volatile uint32_t*>(__cvta_shared_to_generic(abortFlag)) = 1;
+    if (err != nullptr && atomicCAS(&err->code, 0u, 1u) == 0u) {
+        err->where = site;
+        err->block = blockIdx.x;
+        err->detail = parity;
+    }
+}
+__device__ __forceinline__ bool waitWarp(uint64_t* bar, uint32_t parity, volatile uint32_t* abortFlag, DeviceErrors* err,
+                                         uint32_t site)
+{
+    if (__all_sync(0xFFFFFFFFu, mbarTryWait(bar, parity))) return true;
+    const uint64_t t0 = globalTimerNs();
+    do {
+        const bool late = globalTimerNs() - t0 > kWaitLimitNs;
+        if (__any_sync(0xFFFFFFFFu, late || *abortFlag != 0)) {
+            waitTimedOut(smemAddr(const_cast<uint32_t*>(abortFlag)), err, site, parity);
+            return false;
+        }
+    } while (!__all_sync(0xFFFFFFFFu, mbarTryWait(bar, parity)));
+    return true;
+}
+
+// argmin_b (|c_b|^2 - 2 x.c_b), lowest b on ties (vocTreeLookUp.cu:108-125), as the minimum of
+// 16 (|c_b|^2 - 2 x.c_b) + b: a score lies in (-2^24, 2^23), so that fits 32 bits, and the low bits
+// are the lowest branch of the lowest score.  key: 16 |c_b|^2 + b.
+__device__ __forceinline__ int32_t normKey(int32_t cn, uint32_t b, uint32_t B)
+{
+    return b < B ? cn * 16 + static_cast<int32_t>(b) : 0x7FFFFFFF;
+}
+__device__ __forceinline__ uint32_t argminKeys(const uint32_t (&dot)[16], const int4 (&key)[4])
+{
+    int32_t best = 0x7FFFFFFF;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) {
+        const int32_t c[4] = {key[i].x, key[i].y, key[i].z, key[i].w};
+        int32_t q[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) q[k] = c[k] - 32 * static_cast<int32_t>(dot[4 * i + k]);
+        best = min(min(best, q[0]), q[1]);
+        best = min(min(best, q[2]), q[3]);
+    }
+    return static_cast<uint32_t>(best) & 15u;
+}
+__device__ __forceinline__ void loadKeys(const int32_t* node, int4 (&key)[4])
+{
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) key[i] = reinterpret_cast<const int4*>(node)[i];
+}
+
+template <bool kGather>
+__global__ void __launch_bounds__(kSortThreads, 1)
+    lookupPassSorted(const __grid_constant__ CUtensorMap tmapTile, const PassParams p)
+{
+    extern __shared__ uint8_t smemRaw[];
+    SortSmem& S = *reinterpret_cast<SortSmem*>(smemAligned(smemRaw));
+    const uint32_t tid = threadIdx.x, lane = tid % 32;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid / 32, 0); // uniform
+    const uint32_t T = !kGather ? static_cast<uint32_t>((p.nRows + kSuperRows - 1) / kSuperRows) : *p.nTilesDev;
+    const uint32_t t0 = static_cast<uint32_t>(uint64_t(T) * blockIdx.x / gridDim.x);
+    const uint32_t t1 = static_cast<uint32_t>(uint64_t(T) * (blockIdx.x + 1) / gridDim.x);
+    const uint32_t nT = t1 - t0;
+    if (nT == 0) return; // uniform
+    const bool two = p.twoLevels != 0;
+    const uint32_t kidCols = 16 * (p.B + kSubTiles - 1);
+    const bool ownKids = kSortKidCol + 2 * kidCols <= kTmemCols; // a children area for each team
+    volatile uint32_t* abortFlag = &S.abortFlag;
+    if (tid == 0) {
+        for (uint32_t i = 0; i < kSuperBufs; i++) {
+            mbarInit(&S.aFull[i], kGather ? 2 : 1);
+            mbarInit(&S.aFree[i], 1);
+        }
+        for (uint32_t j = 0; j < 2; j++) {
+            mbarInit(&S.bFull[j], 1);
+            mbarInit(&S.bEmpty[j], 1 + 2 * kSortTeamWarps); // the issuer's MMAs and both teams' norms
+            mbarInit(&S.cnReady[j], 1);
+            mbarInit(&S.nodeDone[j], 1);
+            mbarInit(&S.counted[j], kSortTeamWarps);
+            mbarInit(&S.sorted[j], kSortTeamWarps);
+            mbarInit(&S.kidsDone[j], 1);
+            mbarInit(&S.kidsRead[j], kSortTeamWarps);
+        }
+        mbarInit(&S.mmaDone, 1);
+        S.abortFlag = 0;
+        S.noAbort = 0;
+        fenceMbarInit();
+    }
+    if (tid < 64) (&S.cnt[0][0][0])[tid] = 0;
+    if (kGather) {
+#pragma unroll 1
+        for (uint32_t i = tid; i < nT; i += blockDim.x) S.tileCache[i] = superTileGlobal(p.tiles + t0, nT, i);
+    }
+    if (warp == 0) {
+        tmemAlloc(&S.tmemBase, kTmemCols);
+        tmemRelinquish();
+    }
+    tcFenceBefore();
+    __syncthreads();
+    tcFenceAfter();
+    const uint32_t tmem = S.tmemBase;
+    if (warp == kSortIssuer + 3) {
+        // ------------------------------------------------------------ norms
+        uint32_t n = 0;
+        #pragma unroll 1
+        for (uint32_t s = 0; s < nT; s++) {
+            if (!(superTile<kGather>(S, p, t0, nT, s).pad & kFirstOfGroup)) continue;
+            const uint32_t slot = n & 1u;
+            if (!waitWarp(&S.bFull[slot], (n >> 1) & 1u, abortFlag, p.err, 73)) break;
+            n++;
+            const uint32_t words = two ? 16 * (1 + p.B) : 16;
+            int32_t* cn = &S.cn[slot][0][0];
+#pragma unroll 1
+            for (uint32_t i = lane; i < words; i += 32) cn[i] = normKey(cn[i], i % 16, p.B);
+            __syncwarp();
+            if (lane == 0) mbarArrive(&S.cnReady[slot]);
+        }
+    } else if (warp > kSortIssuer) {
+        // ------------------------------------------------------------ producers
+        const uint32_t which = warp - kSortIssuer - 1; // the tile of each super-tile that this one gathers
+        uint32_t n = 0, issued = 0, published = 0; // n: groups loaded
+        auto publishUpTo = [&](uint32_t end) { // gathered rows: generic writes, read by the MMA
+            if (published >= end) return;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                for (uint32_t i = published; i < end; i++) mbarArrive(&S.aFull[i % kSuperBufs]);
+            published = end;
+        };
+        // lane l holds the ids of rows l, l + 32, .. of its tile (past the count: the first row)
+        uint32_t y[4] = {0, 0, 0, 0};
+        auto loadIds = [&](uint32_t s) {
+            const TileInfo ti = superTile<kGather>(S, p, t0, nT, s);
+#pragma unroll
+            for (uint32_t j = 0; j < 4; j++) {
+                const uint32_t r = kTileRows * which + 32 * j + lane;
+                y[j] = __ldg(p.perm + ti.start + (r < ti.count ? r : 0u));
+            }
+        };
+        if (kGather) loadIds(0);
+        #pragma unroll 1
+        for (uint32_t s = 0; s < nT && (kGather || which == 0); s++) {
+            const TileInfo ti = superTile<kGather>(S, p, t0, nT, s);
+            const uint32_t buf = s % kSuperBufs, tiles = (ti.count + kTileRows - 1) / kTileRows;
+            if (which == 0 && (ti.pad & kFirstOfGroup)) {
+                const uint32_t slot = n & 1u;
+                if (kGather) { // the slot is released behind super-tiles that must be published first
+                    cpAsyncWait<0>();
+                    publishUpTo(issued);
+                }
+                if (!waitWarp(&S.bEmpty[slot], ((n >> 1) & 1u) ^ 1u, abortFlag, p.err, 60)) break;
+                n++;
+                if (lane == 0) {
+                    const uint32_t nb = two ? p.B : 0u;
+                    mbarArriveExpectTx(&S.bFull[slot], (kNodeBytes + 64u) * (1u + nb));
+                    bulkLoad(S.b[slot], p.centersSw + (p.lbA + ti.group) * kNodeBytes, kNodeBytes, &S.bFull[slot]);
+                    bulkLoad(&S.cn[slot][0][0], p.cnorm + (p.lbA + ti.group) * kMaxBranch, 64u, &S.bFull[slot]);
+                    if (two) {
+                        const uint64_t c0 = p.lbB + uint64_t(ti.group) * p.B;
+                        bulkLoad(S.b[slot] + kNodeBytes, p.centersSw + c0 * kNodeBytes, kNodeBytes * p.B, &S.bFull[slot]);
+                        bulkLoad(&S.cn[slot][1][0], p.cnorm + c0 * kMaxBranch, 64u * p.B, &S.bFull[slot]);
+                    }
+                }
+                __syncwarp();
+            }
+            if (!waitWarp(&S.aFree[buf], ((s / kSuperBufs) & 1u) ^ 1u, abortFlag, p.err, 61)) break;
+            if (!kGather) {
+                if (lane == 0) {
+                    mbarArriveExpectTx(&S.aFull[buf], tiles * kTileBytes);
+#pragma unroll 1
+                    for (uint32_t j = 0; j < tiles; j++)
+                        tmaLoad2d(S.a[buf] + j * kTileBytes, &tmapTile, 0, static_cast<int32_t>(ti.start + j * kTileRows),
+                                  &S.aFull[buf]);
+                }
+                issued = s + 1;
+                __syncwarp();
+                continue;
+            }
+            if (which < tiles) {
+                // eight lanes copy the eight chunks of a row: four whole rows per instruction, rows
+                // 4 i + lane / 8 of the tile
+                const uint32_t ch = (lane & 7u) << 4;
+                const uint32_t dst = smemAddr(S.a[buf]) + which * kTileBytes + (lane / 8) * kDims + (ch ^ ((lane / 8) << 4));
+                const uint8_t* src = p.desc + ch;
+#pragma unroll
+                for (uint32_t i = 0; i < 32; i++) {
+                    const uint32_t id = __shfl_sync(0xFFFFFFFFu, y[i / 8], 4 * (i % 8) + lane / 8);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((dst ^ ((i & 1u) << 6)) + 4 * i * kDims),
+                                 "l"(src + uint64_t(id) * kDims)
+                                 : "memory");
+                }
+            }
+            cpAsyncCommit();
+            if (s + 1 < nT) loadIds(s + 1); // used behind the wait below
+            issued = s + 1;
+            cpAsyncWait<1>();
+            publishUpTo(s);
+        }
+        // Drain: every load this warp issued must land before the CTA can exit, aborted or not.
+        if (kGather) {
+            cpAsyncWait<0>();
+            publishUpTo(issued);
+        } else {
+            const uint32_t armed = min(issued, kSuperBufs);
+            for (uint32_t i = 0; i < armed; i++) {
+                const uint32_t last = ((issued - 1 - i) / kSuperBufs) * kSuperBufs + i; // last use of buffer i
+                waitWarp(&S.aFull[i], (last / kSuperBufs) & 1u, &S.noAbort, p.err, 62);
+            }
+        }
+        for (uint32_t i = n > 2 ? n - 2 : 0; i < n; i++) waitWarp(&S.bFull[i & 1u], (i >> 1) & 1u, &S.noAbort, p.err, 62);
+        __syncwarp();
+    } else if (warp == kSortIssuer) {
+        // ------------------------------------------------------------ MMA issuer
+        const bool issuer = electOne();
+        // Whichever step's inputs are ready first: with groups of few rows the node level of the next
+        // group waits for its centers, which wait for the children of an earlier one.
+        uint32_t node = 0, kid = 0, nodeN = 0, kidN = 0; // next super-tile of each step, groups before it
+        uint64_t idle = 0;
+        while (kid < nT) {
+            if (kid < node && __all_sync(0xFFFFFFFFu, mbarTest(&S.sorted[kid & 1u], (kid >> 1) & 1u)) &&
+                (!two || ownKids || kid == 0 || // own area: the team has read it before it sorted these rows
+                 __all_sync(0xFFFFFFFFu, mbarTest(&S.kidsRead[(kid & 1u) ^ 1u], ((kid - 1) >> 1) & 1u)))) {
+                // the children of super-tile `kid`, whose rows are sorted (one level: whose team has
+                // read the node level)
+                const uint32_t team = kid & 1u, buf = kid % kSuperBufs;
+                const TileInfo ti = superTile<kGather>(S, p, t0, nT, kid);
+                if (ti.pad & kFirstOfGroup) kidN++;
+                const uint32_t slot = (kidN - 1) & 1u;
+                tcFenceAfter();
+                if (two) {
+                    const uint32_t kids = tmem + kSortKidCol + (ownKids ? team * kidCols : 0u);
+                    const uint32_t base = lane < 16 ? S.binBase[team][lane] : 0u;
+                    const uint32_t end = lane < 16 ? S.binBase[team][lane + 1] : 0u;
+                    const uint32_t tiles = (ti.count + kTileRows - 1) / kTileRows;
+#pragma unroll 1
+                    for (uint32_t j = 0; j < tiles; j++) {
+                        // children with rows in sorted positions [128 j, 128 j + 128)
+                        const uint32_t here =
+                            __ballot_sync(0xFFFFFFFFu, end > base && base < kTileRows * (j + 1) && end > kTileRows * j);
+                        if (here == 0) continue;
+                        const uint32_t c0 = __ffs(here) - 1, c1 = 31u - __clz(here);
+                        mmaU8x4(issuer, kids + 16u * (c0 + j), smemDescSw128(smemAddr(S.a[buf]) + j * kTileBytes), 32u,
+                                smemDescSw128(smemAddr(S.b[slot]) + kNodeBytes * (1u + c0)), 32u,
+                                idescU8(16u * (c1 - c0 + 1u)), 0u);
+                    }
+                    if (issuer) mmaCommit(&S.kidsDone[team]);
+                }
+                if (issuer) {
+                    mmaCommit(&S.aFree[buf]); // after the last MMA that reads the buffer
+                    if (ti.pad & kLastOfGroup) mmaCommit(&S.bEmpty[slot]);
+                }
+                kid++;
+                idle = 0;
+                continue;
+            }
+            // the node level of super-tile `node`, into its team's columns: the team has read them
+            // before it sorted `node` - 2
+            const uint32_t buf = node % kSuperBufs;
+            if (node < nT && node < kid + 2 && __all_sync(0xFFFFFFFFu, mbarTest(&S.aFull[buf], (node / kSuperBufs) & 1u))) {
+                const TileInfo ti = superTile<kGather>(S, p, t0, nT, node);
+                const uint32_t n = nodeN + (ti.pad & kFirstOfGroup ? 1u : 0u);
+                if (__all_sync(0xFFFFFFFFu, mbarTest(&S.bFull[(n - 1) & 1u], ((n - 1) >> 1) & 1u))) {
+                    tcFenceAfter();
+                    const uint32_t tiles = (ti.count + kTileRows - 1) / kTileRows;
+#pragma unroll 1
+                    for (uint32_t j = 0; j < tiles; j++)
+                        mmaU8x4(issuer, tmem + kSortNodeCols * (node & 1u) + 16u * j,
+                                smemDescSw128(smemAddr(S.a[buf]) + j * kTileBytes), 32u,
+                                smemDescSw128(smemAddr(S.b[(n - 1) & 1u])), 32u, idescU8(16), 0u);
+                    if (issuer) mmaCommit(&S.nodeDone[node & 1u]);
+                    nodeN = n;
+                    node++;
+                    idle = 0;
+                    continue;
+                }
+            }
+            const uint64_t now = globalTimerNs();
+            if (idle == 0) idle = now;
+            if (__any_sync(0xFFFFFFFFu, now - idle > kWaitLimitNs || *abortFlag != 0)) {
+                waitTimedOut(smemAddr(&S.abortFlag), p.err, 63, kid & 1u);
+                break;
+            }
+        }
+        if (issuer) mmaCommit(&S.mmaDone);
+        waitWarp(&S.mmaDone, 0, abortFlag, p.err, 67);
+    } else {
+        // ------------------------------------------------------------ workers
+        const uint32_t team = warp / kSortTeamWarps, tw = warp % kSortTeamWarps, row = 32 * tw + lane;
+        const uint32_t quarter = ((warp % 4) * 32u) << 16, tile = tw / 4;
+        const uint32_t kids = tmem + kSortKidCol + (ownKids ? team * kidCols : 0u) + 16u * tile + quarter;
+        const uint32_t node = tmem + kSortNodeCols * team + 16u * tile + quarter;
+        // rows 32 tw + 4 i + lane / 8, chunk lane % 8 of each: 128-byte swizzle, i even and odd
+        const uint32_t ch = (lane & 7u) << 4;
+        const uint32_t from0 = (32 * tw + lane / 8) * kDims + (ch ^ ((lane / 8) << 4));
+        uint32_t n = 0xFFFFFFFFu, ready = 0xFFFFFFFFu; // group of super-tile s; the last one whose norms were awaited
+        #pragma unroll 1
+        for (uint32_t s = team; s < nT; s += 2) {
+            if (s > 0 && (superTile<kGather>(S, p, t0, nT, s - 1).pad & kFirstOfGroup)) n++;
+            const TileInfo ti = superTile<kGather>(S, p, t0, nT, s);
+            if (ti.pad & kFirstOfGroup) n++;
+            const uint32_t slot = n & 1u;
+            const uint32_t turn = s >> 1, par = turn & 1u, buf = s % kSuperBufs;
+            const bool valid = row < ti.count, some = 32 * tw < ti.count;
+            const uint32_t orig = valid ? (kGather ? __ldg(p.perm + ti.start + row) : ti.start + row) : 0u;
+            if (n != ready && !waitWarp(&S.cnReady[slot], (n >> 1) & 1u, abortFlag, p.err, 70)) break;
+            ready = n;
+            if (!waitWarp(&S.nodeDone[team], par, abortFlag, p.err, 72)) break;
+            if (!waitWarp(&S.aFull[buf], (s / kSuperBufs) & 1u, abortFlag, p.err, 71)) break;
+            // P1
+            uint32_t b = 0;
+            if (some) {
+                tcFenceAfter();
+                uint32_t r[16];
+                tmemLoad16(node, r);
+                int4 key[4];
+                loadKeys(&S.cn[slot][0][0], key);
+                tmemWaitTie(r);
+                tcFenceBefore();
+                b = argminKeys(r, key);
+            }
+            // bEmpty's arrivals, one per warp of both teams: with the team's last super-tile of the
+            // group, or for the other team too where the group has but one
+            const uint32_t release = ti.pad & kLastOfGroup ? (ti.pad & kFirstOfGroup ? 2u : 1u) : ti.pad & kNextIsLast ? 1u : 0u;
+            if (!two) {
+                if (valid) emitNode(p, orig, ti.group * p.B + b);
+                __syncwarp();
+                if (lane == 0) {
+                    for (uint32_t i = 0; i < release; i++) mbarArrive(&S.bEmpty[slot]);
+                    mbarArrive(&S.sorted[team]);
+                }
+                continue;
+            }
+            uint4 v[8]; // the warp's rows, held until they are moved
+            if (some) {
+#pragma unroll
+                for (uint32_t i = 0; i < 8; i++)
+                    v[i] = *reinterpret_cast<const uint4*>(S.a[buf] + ((from0 + 4 * i * kDims) ^ ((i & 1u) << 6)));
+            }
+            // P2: this row's place among the warp's rows of its branch, and theirs in the super-tile
+            uint32_t peers = __ballot_sync(0xFFFFFFFFu, valid);
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++) {
+                const uint32_t bit = __ballot_sync(0xFFFFFFFFu, (b >> i) & 1u);
+                peers &= (b >> i) & 1u ? bit : ~bit;
+            }
+            const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+            uint32_t* cnt = S.cnt[team][par];
+            uint32_t off = 0;
+            if (valid && rank == 0) off = atomicAdd(&cnt[b], __popc(peers));
+            __syncwarp();
+            if (lane == 0) mbarArrive(&S.counted[team]); // counted, rows read
+            off = __shfl_sync(0xFFFFFFFFu, off, valid ? __ffs(peers) - 1 : 0) + rank;
+            if (!waitWarp(&S.counted[team], par, abortFlag, p.err, 74)) break;
+            const uint32_t total = lane < 16 ? cnt[lane] : 0u;
+            uint32_t incl = total;
+#pragma unroll
+            for (uint32_t d = 1; d < 16; d <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                if (lane >= d) incl += x;
+            }
+            if (tw == 0 && lane < 16) {
+                S.binBase[team][lane] = incl - total;
+                if (lane == 15) S.binBase[team][16] = incl;
+                S.cnt[team][par ^ 1u][lane] = 0; // last read before this turn's counted
+            }
+            const uint32_t first = __shfl_sync(0xFFFFFFFFu, incl - total, b);
+            const uint32_t pos = valid ? first + off : row; // rows past the count stay
+            // P3
+            if (valid) {
+                S.orig[team][pos] = orig;
+                S.child[team][pos] = static_cast<uint8_t>(b);
+            }
+            if (some) {
+                const uint32_t at = pos * kDims + ((pos & 7u) << 4);
+#pragma unroll
+                for (uint32_t i = 0; i < 8; i++)
+                    *reinterpret_cast<uint4*>(S.a[buf] + (__shfl_sync(0xFFFFFFFFu, at, 4 * i + lane / 8) ^ ch)) = v[i];
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbarArrive(&S.sorted[team]);
+            // P4
+            if (!waitWarp(&S.sorted[team], par, abortFlag, p.err, 68)) break;
+            const uint32_t child = valid ? S.child[team][row] : 0u;
+            const uint32_t id = valid ? S.orig[team][row] : 0u;
+            int4 key[4];
+            loadKeys(&S.cn[slot][1 + child][0], key);
+            __syncwarp();
+            if (lane == 0)
+                for (uint32_t i = 0; i < release; i++) mbarArrive(&S.bEmpty[slot]);
+            if (!waitWarp(&S.kidsDone[team], par, abortFlag, p.err, 69)) break;
+            uint32_t sel[16];
+            if (some) {
+                tcFenceAfter();
+                const uint32_t live = min(ti.count - 32 * tw, 32u);
+                const uint32_t c0 = __shfl_sync(0xFFFFFFFFu, child, 0), c1 = __shfl_sync(0xFFFFFFFFu, child, live - 1);
+                uint32_t r[16];
+                tmemLoad16(kids + 16u * c0, sel);
+                tmemLoad16(kids + 16u * min(c0 + 1u, c1), r);
+                tmemWaitTie(sel);
+                tmemWaitTie(r);
+#pragma unroll
+                for (int i = 0; i < 16; i++) sel[i] = child == c0 ? sel[i] : r[i];
+                #pragma unroll 1
+                for (uint32_t c = c0 + 2; c <= c1; c++) {
+                    tmemLoad16(kids + 16u * c, r);
+                    tmemWaitTie(r);
+#pragma unroll
+                    for (int i = 0; i < 16; i++) sel[i] = child == c ? r[i] : sel[i];
+                }
+                tcFenceBefore();
+            }
+            __syncwarp();
+            if (lane == 0) mbarArrive(&S.kidsRead[team]);
+            // P5
+            if (valid) emitNode(p, id, (ti.group * p.B + child) * p.B + argminKeys(sel, key));
+        }
+    }
+    tcFenceBefore();
+    __syncthreads();
+    if (warp == 0) {
+        tcFenceAfter();
+        tmemDealloc(tmem, kTmemCols);
+    }
+}
+
 // ------------------------------------------------------------------ regroup kernels
 // Exclusive scans of the bin histogram: rowOff = scan(count), tileOff = scan(ceil(count/128));
 // totals[0] = number of tiles, totals[1] = number of rows.
 __global__ void __launch_bounds__(1024) scanBins(const uint32_t* count, uint32_t nb, uint32_t* rowOff,
-                                                 uint32_t* tileOff, uint32_t* totals)
+                                                 uint32_t* tileOff, uint32_t* totals, uint32_t tileRows)
 {
     __shared__ uint32_t wa[32], wb[32];
     __shared__ uint32_t carryA, carryB;
@@ -896,7 +1358,7 @@ __global__ void __launch_bounds__(1024) scanBins(const uint32_t* count, uint32_t
     for (uint32_t base = 0; base < nb; base += 1024) {
         const uint32_t i = base + tid;
         const uint32_t c = i < nb ? count[i] : 0u;
-        const uint32_t tc = (c + kTileRows - 1) / kTileRows;
+        const uint32_t tc = (c + tileRows - 1) / tileRows;
         uint32_t a = c, b = tc;
 #pragma unroll
         for (uint32_t off = 1; off < 32; off <<= 1) {
@@ -948,7 +1410,7 @@ __global__ void __launch_bounds__(1024) scanBins(const uint32_t* count, uint32_t
 
 // One thread per tile: find its bin (last bin with tileOff <= t) and describe its rows.
 __global__ void buildTiles(const uint32_t* count, const uint32_t* rowOff, const uint32_t* tileOff, uint32_t nb,
-                           const uint32_t* totals, uint32_t maxTiles, TileInfo* tiles)
+                           const uint32_t* totals, uint32_t maxTiles, TileInfo* tiles, uint32_t tileRows)
 {
     const uint32_t nTiles = totals[0];
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nTiles && t < maxTiles;
@@ -960,8 +1422,8 @@ __global__ void buildTiles(const uint32_t* count, const uint32_t* rowOff, const 
         }
         const uint32_t g = lo - 1;
         const uint32_t k = t - tileOff[g];
-        const uint32_t c = count[g] - k * kTileRows;
-        tiles[t] = TileInfo{g, rowOff[g] + k * kTileRows, c < kTileRows ? c : kTileRows, 0u};
+        const uint32_t c = count[g] - k * tileRows;
+        tiles[t] = TileInfo{g, rowOff[g] + k * tileRows, c < tileRows ? c : tileRows, 0u};
     }
 }
 
@@ -1069,7 +1531,8 @@ __global__ void __launch_bounds__(kRegroupThreads) regroupHist(const uint32_t* n
 
 // One CTA of 1024 threads: thread (k, b) owns bin b's CTAs [k * len, (k + 1) * len).
 __global__ void __launch_bounds__(1024) regroupScan(uint32_t* ctaHist, uint32_t nCta, uint32_t nb, uint32_t* count,
-                                                    uint32_t* rowOff, uint32_t* tileOff, uint32_t* totals)
+                                                    uint32_t* rowOff, uint32_t* tileOff, uint32_t* totals,
+                                                    uint32_t tileRows)
 {
     __shared__ uint32_t part[1024];
     __shared__ uint32_t wa[32], wb[32];
@@ -1102,7 +1565,7 @@ __global__ void __launch_bounds__(1024) regroupScan(uint32_t* ctaHist, uint32_t 
     }
     // exclusive scans over bins of total and ceil(total / 128) (threads k == 0 hold the bins)
     const bool owner = active && k == 0;
-    const uint32_t ca = owner ? total : 0u, cb = owner ? (total + kTileRows - 1) / kTileRows : 0u;
+    const uint32_t ca = owner ? total : 0u, cb = owner ? (total + tileRows - 1) / tileRows : 0u;
     uint32_t a = ca, t = cb;
 #pragma unroll
     for (uint32_t off = 1; off < 32; off <<= 1) {
@@ -1491,20 +1954,23 @@ uint32_t launchLookup(const DeviceTree& tree, const uint8_t* desc, uint64_t n, u
     }
     const bool warpNode = algo == kLookupTensorU8WarpNode;
     const bool ring = algo == kLookupTensorU8Ring;
-    static std::atomic<uint64_t> attrSet{0}, attrSetW{0}, attrSetR{0}, attrSetS{0};
+    static std::atomic<uint64_t> attrSetW{0}, attrSetR{0}, attrSetS{0}, attrSetO{0}, attrSetG{0};
     setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(regroupScatter), static_cast<int>(kScatterSmemBytes),
                                    attrSetS);
     if (ring) {
         setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(lookupPassRing),
                                        static_cast<int>(kTcSmemBytes), attrSetR);
     } else if (warpNode) {
-        setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(lookupPassTc<true>),
+        setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(lookupPassWarpNode),
                                        static_cast<int>(kTcSmemBytes), attrSetW);
     } else {
-        setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(lookupPassTc<false>),
-                                       static_cast<int>(kTcSmemBytes), attrSet);
+        setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(lookupPassSorted<false>),
+                                       static_cast<int>(kSortSmemBytes), attrSetO);
+        setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(lookupPassSorted<true>),
+                                       static_cast<int>(kSortSmemBytes), attrSetG);
     }
     const CUtensorMap tmapTile = makeRowMap(desc, n, kTileRows);
+    const uint32_t tileRows = ring || warpNode ? kTileRows : kSuperRows;
     const uint32_t B = tree.B, L = tree.L;
     const uint32_t passes = (L + 1) / 2;
     const uint32_t grid = static_cast<uint32_t>(currentSmCount());
@@ -1552,9 +2018,14 @@ uint32_t launchLookup(const DeviceTree& tree, const uint8_t* desc, uint64_t n, u
             if (ring) {
                 lookupPassRing<<<grid, kRingThreads, kTcSmemBytes, stream>>>(tmapTile, p);
             } else if (warpNode) {
-                lookupPassTc<true><<<grid, kTcThreads, kTcSmemBytes, stream>>>(tmapTile, p);
+                lookupPassWarpNode<<<grid, kTcThreads, kTcSmemBytes, stream>>>(tmapTile, p);
+            } else if (pass == 0) {
+                lookupPassSorted<false><<<grid, kSortThreads, kSortSmemBytes, stream>>>(tmapTile, p);
             } else {
-                lookupPassTc<false><<<grid, kTcThreads, kTcSmemBytes, stream>>>(tmapTile, p);
+                // a CTA holds its tile list: several rounds of CTAs where the lists would be longer
+                const uint64_t lists = (n / kSuperRows + bins) / kSortTileCache + 1;
+                const uint32_t rounds = static_cast<uint32_t>((lists + grid - 1) / grid);
+                lookupPassSorted<true><<<grid * rounds, kSortThreads, kSortSmemBytes, stream>>>(tmapTile, p);
             }
             RBW_CUDA(cudaGetLastError());
         }
@@ -1567,17 +2038,17 @@ uint32_t launchLookup(const DeviceTree& tree, const uint8_t* desc, uint64_t n, u
                 regroupHist<<<kRegroupCtas, kRegroupThreads, 0, stream>>>(scratch.nodeNext, n, per, nbBins,
                                                                          scratch.ctaHist);
                 regroupScan<<<1, 1024, 0, stream>>>(scratch.ctaHist, kRegroupCtas, nbBins, count, rowOff, tileOff,
-                                                    totals);
-                buildTiles<<<tileBlocks, 256, 0, stream>>>(count, rowOff, tileOff, nbBins, totals, maxTiles, tiles);
+                                                    totals, tileRows);
+                buildTiles<<<tileBlocks, 256, 0, stream>>>(count, rowOff, tileOff, nbBins, totals, maxTiles, tiles, tileRows);
                 regroupScatter<<<kRegroupCtas, kRegroupThreads, kScatterSmemBytes, stream>>>(
                     scratch.nodeNext, n, per, nbBins, scratch.ctaHist, scratch.perm);
                 RBW_CUDA(cudaGetLastError());
                 kernels += 4;
                 continue;
             }
-            scanBins<<<1, 1024, 0, stream>>>(count, nbBins, rowOff, tileOff, totals);
+            scanBins<<<1, 1024, 0, stream>>>(count, nbBins, rowOff, tileOff, totals, tileRows);
             RBW_CUDA(cudaGetLastError());
-            buildTiles<<<tileBlocks, 256, 0, stream>>>(count, rowOff, tileOff, nbBins, totals, maxTiles, tiles);
+            buildTiles<<<tileBlocks, 256, 0, stream>>>(count, rowOff, tileOff, nbBins, totals, maxTiles, tiles, tileRows);
             RBW_CUDA(cudaGetLastError());
             RBW_CUDA(cudaMemsetAsync(cursor, 0, sizeof(uint32_t) * nbBins, stream));
             const uint32_t rows = tunedValue(kTuneScatterRows, B, L, n);

@@ -8,7 +8,7 @@
 namespace rbw {
 
 enum TimedKernel : uint32_t {
-    kTimedLookupPass = 0,   // tensor-core lookup pass (lookupPassTc)
+    kTimedLookupPass = 0,   // tensor-core lookup pass (lookupPassSorted, -Ring or -WarpNode)
     kTimedLookupSimt = 1,   // FP32 SIMT lookup
     kTimedRegroup = 2,      // scan + tile list + scatter between lookup passes
     kTimedAssign = 3,       // k-means assign

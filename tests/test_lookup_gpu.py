@@ -157,6 +157,32 @@ def test_auto_lookup_matches_oracle_on_both_sides_of_the_direct_limit(oracle, B,
         assert np.array_equal(got, want), f"n={n}: {np.count_nonzero(got != want)} mismatches"
 
 
+@pytest.mark.parametrize("B,L", [(2, 4), (5, 3), (13, 2), (14, 2), (16, 1), (16, 2), (16, 3), (16, 4)])
+def test_sorted_passes_match_oracle(oracle, B, L):
+    """Tensor-core passes around the 128-row tiles and 256-row super-tiles, with all rows on one branch
+    and with rows on every branch, with children areas for both teams (B <= 13) and one shared."""
+    centers, masks, weights = random_tree(B, L, seed=B * L, dup_rate=0.3)
+    voc = rbw.vocabulary_from_host(B, L, centers, masks, weights)
+    for n in (1, 31, 128, 129, 256, 257, 385, 148 * 256, 148 * 512 + 1):
+        desc = edge_descriptors(centers, n, seed=n)
+        same = np.repeat(desc[:1], n, axis=0)
+        for d in (desc, same):
+            got = _lookup(voc, d, "tensor_u8")
+            want = oracle.lookup(centers, B, L, d, threads=8)
+            assert np.array_equal(got, want), f"n={n}: {np.count_nonzero(got != want)} mismatches"
+    assert voc.device_errors() == (0, 0)
+
+
+def test_sorted_pass_with_more_tiles_than_one_round_of_ctas_holds():
+    """65,536 groups and 2.8M rows: tile lists longer than one CTA per SM can hold."""
+    centers, masks, weights = random_tree(16, 5, seed=5)
+    voc = rbw.vocabulary_from_host(16, 5, centers, masks, weights)
+    desc = torch.randint(0, 256, (2_800_003, 128), dtype=torch.uint8, device="cuda",
+                         generator=torch.Generator("cuda").manual_seed(1))
+    assert torch.equal(voc.lookup(desc, algo="tensor_u8"), voc.lookup(desc, algo="simt_f32"))
+    assert voc.device_errors() == (0, 0)
+
+
 @pytest.mark.parametrize("B,L,float_centers", [(16, 3, False), (10, 6, False), (3, 7, False), (16, 2, True), (9, 4, True)])
 def test_centers_come_back_as_they_went_in(B, L, float_centers):
     """Trees above and below one 32 MiB piece of the packed copy, with and without padded slots, and
