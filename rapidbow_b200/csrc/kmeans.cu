@@ -74,10 +74,16 @@ __global__ void __launch_bounds__(kScanBlock) scanSingle(uint32_t* data, uint32_
     }
 }
 
+// kOwnSums: blockOff holds the blocks' sums (at most kScanBlock of them), each block adds up those
+// before it; else their scan.
+template <bool kOwnSums>
 __global__ void __launch_bounds__(kScanBlock) scanApply(const uint32_t* in, uint64_t n, const uint32_t* blockOff,
                                                         uint32_t* out)
 {
     __shared__ uint32_t ws[32];
+    uint32_t before = 0;
+    if (kOwnSums) blockExclusiveScan(threadIdx.x < blockIdx.x ? blockOff[threadIdx.x] : 0u, ws, before);
+    else before = blockOff[blockIdx.x];
     const uint64_t base = uint64_t(blockIdx.x) * kScanTile + threadIdx.x * kScanPerThread;
     uint32_t v[kScanPerThread];
     uint32_t s = 0;
@@ -87,7 +93,7 @@ __global__ void __launch_bounds__(kScanBlock) scanApply(const uint32_t* in, uint
         s += v[k];
     }
     uint32_t total;
-    uint32_t e = blockExclusiveScan(s, ws, total) + blockOff[blockIdx.x];
+    uint32_t e = blockExclusiveScan(s, ws, total) + before;
 #pragma unroll
     for (uint32_t k = 0; k < kScanPerThread; k++) {
         if (base + k < n) out[base + k] = e;
@@ -125,6 +131,44 @@ __global__ void fillNodeTiles(const uint32_t* cnt, const uint32_t* off, const ui
         const uint32_t k = t - tileOff[g];
         const uint32_t c = cnt[g] - k * d;
         tiles[t] = NodeTile{g, off[g] + k * d, c < d ? c : d, tileOff[g]};
+    }
+}
+
+// The whole tile list in one launch where a CTA can scan the nodes' tile counts by itself: each does,
+// then fills its share of the list; the first also writes the offsets and the total.
+constexpr uint32_t kTileListNodes = kScanTile;
+__global__ void __launch_bounds__(kScanBlock) nodeTilesKernel(const uint32_t* cnt, const uint32_t* off, uint32_t nbNodes,
+                                                              uint32_t d, uint32_t maxTiles, uint32_t* tileOff,
+                                                              uint32_t* totals, NodeTile* tiles)
+{
+    __shared__ uint32_t ws[32];
+    __shared__ uint32_t first[kTileListNodes];
+    uint32_t v[kScanPerThread], sum = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kScanPerThread; k++) {
+        const uint32_t g = threadIdx.x * kScanPerThread + k;
+        v[k] = g < nbNodes ? (cnt[g] + d - 1) / d : 0u;
+        sum += v[k];
+    }
+    uint32_t total;
+    uint32_t e = blockExclusiveScan(sum, ws, total);
+#pragma unroll
+    for (uint32_t k = 0; k < kScanPerThread; k++) {
+        const uint32_t g = threadIdx.x * kScanPerThread + k;
+        first[g] = e;
+        if (blockIdx.x == 0 && g < nbNodes) tileOff[g] = e;
+        e += v[k];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) totals[0] = total;
+    __syncthreads();
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total && t < maxTiles; t += gridDim.x * blockDim.x) {
+        uint32_t lo = 0, hi = nbNodes;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) / 2;
+            if (first[mid] <= t) lo = mid + 1; else hi = mid;
+        }
+        const uint32_t g = lo - 1, k = t - first[g], c = cnt[g] - k * d;
+        tiles[t] = NodeTile{g, off[g] + k * d, c < d ? c : d, first[g]};
     }
 }
 
@@ -666,33 +710,13 @@ __global__ void regroupHistKernel(KMeansLevel lv, const NodeTile* tiles, const u
     }
 }
 
-__global__ void regroupChildKernel(KMeansLevel lv, const uint32_t* tileOffNode, uint32_t maxTiles,
-                                   const uint32_t* tileHist, const uint32_t* tileScan, uint32_t* childCnt,
-                                   uint32_t* childOff)
-{
-    // thread per node: child sizes from the per-center scans over the node's tiles, children
-    // laid out in center order (Vocabulary.cpp:83-98)
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= lv.nbNodes) return;
-    const uint32_t first = tileOffNode[g];
-    const uint32_t nt = (lv.nodeCnt[g] + kRegroupRows - 1) / kRegroupRows;
-    uint32_t off = lv.nodeOff[g];
-    for (uint32_t b = 0; b < lv.B; b++) {
-        uint32_t c = 0;
-        if (nt) {
-            const uint64_t row = uint64_t(b) * maxTiles;
-            const uint32_t lastT = first + nt - 1;
-            c = tileScan[row + lastT] - tileScan[row + first] + tileHist[row + lastT];
-        }
-        childCnt[uint64_t(g) * lv.B + b] = c;
-        childOff[uint64_t(g) * lv.B + b] = off;
-        off += c;
-    }
-}
-
+// Warp per 32-member tile.  A node's children lie in center order from its own offset
+// (Vocabulary.cpp:83-98): lane q takes the size of child q from the scan over the node's tiles (of
+// which only differences within a row are used), a scan over the lanes gives their offsets, and the
+// warp of a node's first tile writes both.
 __global__ void regroupScatterKernel(KMeansLevel lv, const NodeTile* tiles, const uint32_t* nTilesDev,
-                                     uint32_t maxTiles, const uint32_t* tileScan, const uint32_t* childOff,
-                                     uint32_t* childMembers)
+                                     uint32_t maxTiles, const uint32_t* tileHist, const uint32_t* tileScan,
+                                     uint32_t* childCnt, uint32_t* childOff, uint32_t* childMembers)
 {
     const uint32_t T = *nTilesDev;
     const uint32_t warpsTotal = gridDim.x * (blockDim.x / 32);
@@ -701,13 +725,37 @@ __global__ void regroupScatterKernel(KMeansLevel lv, const NodeTile* tiles, cons
         const NodeTile ti = tiles[t];
         const bool valid = lane < ti.count;
         const uint32_t b = valid ? lv.assign[ti.start + lane] : 0xFFu;
+        const uint32_t member = valid ? lv.members[ti.start + lane] : 0u;
         const uint32_t same = __match_any_sync(0xFFFFFFFFu, b);
         const uint32_t rank = __popc(same & ((1u << lane) - 1u));
-        if (valid) {
-            const uint64_t row = uint64_t(b) * maxTiles;
-            const uint32_t within = tileScan[row + t] - tileScan[row + ti.first];
-            const uint32_t dst = childOff[uint64_t(ti.node) * lv.B + b] + within + rank;
-            childMembers[dst] = lv.members[ti.start + lane];
+        uint32_t size = 0, within = 0; // of child `lane`: its members, and those before this tile
+        if (lane < lv.B) {
+            const uint32_t lastT = ti.first + (lv.nodeCnt[ti.node] + kRegroupRows - 1) / kRegroupRows - 1;
+            const uint64_t row = uint64_t(lane) * maxTiles;
+            const uint32_t base = tileScan[row + ti.first];
+            size = tileScan[row + lastT] - base + tileHist[row + lastT];
+            within = tileScan[row + t] - base;
+        }
+        uint32_t off = size;
+#pragma unroll
+        for (uint32_t k = 1; k < kMaxBranch; k <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, off, k);
+            if (lane >= k) off += x;
+        }
+        off += lv.nodeOff[ti.node] - size;
+        if (t == ti.first && lane < lv.B) {
+            childCnt[uint64_t(ti.node) * lv.B + lane] = size;
+            childOff[uint64_t(ti.node) * lv.B + lane] = off;
+        }
+        const uint32_t at = __shfl_sync(0xFFFFFFFFu, off + within, b & 31u);
+        if (valid) childMembers[at + rank] = member;
+    }
+    // nodes without members have no tile
+    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < lv.nbNodes; g += gridDim.x * blockDim.x) {
+        if (lv.nodeCnt[g] != 0) continue;
+        for (uint32_t b = 0; b < lv.B; b++) {
+            childCnt[uint64_t(g) * lv.B + b] = 0;
+            childOff[uint64_t(g) * lv.B + b] = lv.nodeOff[g];
         }
     }
 }
@@ -725,8 +773,12 @@ void exclusiveScanU32(const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* t
     if (n == 0) return;
     const uint32_t blocks = static_cast<uint32_t>((n + kScanTile - 1) / kScanTile);
     scanBlockSums<<<blocks, kScanBlock, 0, s>>>(in, n, tmp);
-    scanSingle<<<1, kScanBlock, 0, s>>>(tmp, blocks);
-    scanApply<<<blocks, kScanBlock, 0, s>>>(in, n, tmp, out);
+    if (blocks <= kScanBlock) {
+        scanApply<true><<<blocks, kScanBlock, 0, s>>>(in, n, tmp, out);
+    } else {
+        scanSingle<<<1, kScanBlock, 0, s>>>(tmp, blocks);
+        scanApply<false><<<blocks, kScanBlock, 0, s>>>(in, n, tmp, out);
+    }
     RBW_CUDA(cudaGetLastError());
 }
 
@@ -734,6 +786,14 @@ void buildNodeTiles(const uint32_t* nodeCnt, const uint32_t* nodeOff, uint32_t n
                     uint32_t* tileOff, uint32_t* tmp, NodeTile* tiles, uint32_t maxTiles, uint32_t* totals,
                     cudaStream_t s)
 {
+    // Six launches of ~4 us each with their gaps against one of ~4 us (with a level's other launches
+    // halved as well, a build of 200,000 rows takes 745 us and not 826).
+    if (nbNodes <= kTileListNodes) {
+        const uint32_t blocks = std::max(1u, std::min<uint32_t>((maxTiles + kScanBlock - 1) / kScanBlock, 296));
+        nodeTilesKernel<<<blocks, kScanBlock, 0, s>>>(nodeCnt, nodeOff, nbNodes, tileRows, maxTiles, tileOff, totals, tiles);
+        RBW_CUDA(cudaGetLastError());
+        return;
+    }
     ceilDivKernel<<<(nbNodes + 255) / 256, 256, 0, s>>>(nodeCnt, nbNodes, tileRows, tileOff);
     exclusiveScanU32(tileOff, tileOff, nbNodes, tmp, s);
     tilesTotal<<<1, 1, 0, s>>>(nodeCnt, tileOff, nbNodes, tileRows, totals);
@@ -794,15 +854,14 @@ void launchRegroup(const KMeansLevel& lv, const RegroupScratch& rs, uint32_t* ch
 {
     buildNodeTiles(lv.nodeCnt, lv.nodeOff, lv.nbNodes, kRegroupRows, rs.tileOff, rs.scanTmp, rs.tiles, rs.maxTiles,
                    rs.totals, s);
-    RBW_CUDA(cudaMemsetAsync(rs.tileHist, 0, sizeof(uint32_t) * uint64_t(lv.B) * rs.maxTiles, s));
+    // Entries past the last tile of each row are not written: they add the same to every scan value
+    // of the later rows.
     const uint32_t warpsPerBlock = 8;
     const uint32_t blocks = std::max(1u, std::min<uint32_t>((rs.maxTiles + warpsPerBlock - 1) / warpsPerBlock, 16384));
     regroupHistKernel<<<blocks, 32 * warpsPerBlock, 0, s>>>(lv, rs.tiles, rs.totals, rs.maxTiles, rs.tileHist);
     exclusiveScanU32(rs.tileHist, rs.tileScan, uint64_t(lv.B) * rs.maxTiles, rs.scanTmp, s);
-    regroupChildKernel<<<(lv.nbNodes + 255) / 256, 256, 0, s>>>(lv, rs.tileOff, rs.maxTiles, rs.tileHist,
-                                                                rs.tileScan, childCnt, childOff);
-    regroupScatterKernel<<<blocks, 32 * warpsPerBlock, 0, s>>>(lv, rs.tiles, rs.totals, rs.maxTiles, rs.tileScan,
-                                                                childOff, childMembers);
+    regroupScatterKernel<<<blocks, 32 * warpsPerBlock, 0, s>>>(lv, rs.tiles, rs.totals, rs.maxTiles, rs.tileHist,
+                                                               rs.tileScan, childCnt, childOff, childMembers);
     RBW_CUDA(cudaGetLastError());
 }
 

@@ -138,6 +138,17 @@ def test_build_resident_node_sizes_match_oracle(oracle, n, B, iters, check):
     assert voc.build_stats()["iterations"] == want
 
 
+@pytest.mark.parametrize("B,L,n", [(16, 4, 20_011), (8, 5, 9_000), (9, 5, 9_000), (2, 8, 70_001), (16, 2, 33)])
+def test_build_tile_lists_and_children_match_oracle(oracle, B, L, n):
+    """Levels of up to 4,096 nodes, whose tile list is one launch, and of more; many nodes without
+    members."""
+    desc = sift_like(n, seed=n + B).numpy()
+    voc = rbw.build_vocabulary(torch.from_numpy(desc).cuda(), B, nb_doc=40, nb_levels=L, init="kmeans++", seed=5,
+                               max_iterations=4, ieee_division=True)
+    ref = oracle.build_vocabulary(desc, 40, B, L, max_iter=4, init=INIT_KMEANSPP, seed=5)
+    _tree_equal(voc, ref)
+
+
 @pytest.mark.parametrize("rows_per_sm,extra,L", [(12, -1, 2), (1536, 0, 1), (1536, 1, 1), (400, 77, 2)])
 def test_build_shared_level_edges_match_oracle(oracle, rows_per_sm, extra, L):
     """Levels whose streamed rows fit the SMs together run in one cooperative launch, nodes spread
