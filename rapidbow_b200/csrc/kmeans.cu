@@ -256,20 +256,36 @@ constexpr uint32_t kPPCtasPerSm = 6; // by shared memory: 32 KB of candidate row
 // i holds candidate i's D^2 weight; each pick's prefix sums are warp scans plus one pass over the
 // eight warp totals, and every thread draws the same random numbers, so a pick costs two
 // barriers.  Registers stay low enough for six CTAs per SM (deep levels have 10^5 nodes).
-__global__ void __launch_bounds__(kPPSample, kPPCtasPerSm) kmeansPPKernel(KMeansLevel lv, uint64_t seed,
-                                                                          uint32_t level, uint32_t* nValidOut)
-{
+//
+// Distances are |x|^2 + |p|^2 - 2 x.p by dp4a (exact), each row's norm taken once.
+struct PPSmem {
     // candidate rows, chunk c of row i at [i][c ^ (i & 7)] (a quarter-warp reading its own rows
     // hits 32 different banks)
-    __shared__ uint4 rowS[kPPSample][kDims / 16];
-    __shared__ uint32_t pos[kPPSample];
-    __shared__ uint32_t cand[kPPSample];
-    __shared__ uint32_t draw[kPPSample];
-    __shared__ uint32_t link[kPPSample];
-    __shared__ uint8_t found[kPPSample];
-    __shared__ unsigned long long warpSum[kPPWarps];
-    __shared__ uint32_t chosen[kMaxBranch];
-    const uint32_t g = blockIdx.x;
+    uint4 rowS[kPPSample][kDims / 16];
+    uint32_t pos[kPPSample];
+    uint32_t cand[kPPSample];
+    uint32_t draw[kPPSample]; // later the rows' |x|^2
+    uint32_t link[kPPSample];
+    uint8_t found[kPPSample];
+    uint32_t warpSum[kPPWarps];
+    uint32_t chosen[kMaxBranch];
+};
+__device__ __forceinline__ uint32_t dot16(const uint4& x, const uint4& y, uint32_t acc)
+{
+    return __dp4a(x.w, y.w, __dp4a(x.z, y.z, __dp4a(x.y, y.y, __dp4a(x.x, y.x, acc))));
+}
+
+__device__ __forceinline__ void kmeansPPNode(const KMeansLevel& lv, uint64_t seed, uint32_t level, uint32_t g,
+                                             uint32_t* nValidOut, PPSmem& sm)
+{
+    auto& rowS = sm.rowS;
+    auto& pos = sm.pos;
+    auto& cand = sm.cand;
+    auto& draw = sm.draw;
+    auto& link = sm.link;
+    auto& found = sm.found;
+    auto& warpSum = sm.warpSum;
+    auto& chosen = sm.chosen;
     const uint32_t n = lv.nodeCnt[g];
     const uint32_t tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
     const uint32_t S = n < kPPSample ? n : kPPSample;
@@ -321,7 +337,11 @@ __global__ void __launch_bounds__(kPPSample, kPPCtasPerSm) kmeansPPKernel(KMeans
         // ascending order: the positions are distinct, so each one's rank is its slot
         const uint32_t v = pos[tid];
         uint32_t rk = 0;
-        for (uint32_t q = 0; q < kPPSample; q++) rk += pos[q] < v ? 1u : 0u;
+#pragma unroll 4
+        for (uint32_t q = 0; q < kPPSample / 4; q++) {
+            const uint4 x = reinterpret_cast<const uint4*>(pos)[q];
+            rk += (x.x < v ? 1u : 0u) + (x.y < v ? 1u : 0u) + (x.z < v ? 1u : 0u) + (x.w < v ? 1u : 0u);
+        }
         cand[rk] = lv.members[lv.nodeOff[g] + v];
     } else if (tid < S) {
         cand[tid] = lv.members[lv.nodeOff[g] + tid];
@@ -334,54 +354,52 @@ __global__ void __launch_bounds__(kPPSample, kPPCtasPerSm) kmeansPPKernel(KMeans
         const uint32_t r = 32u * k + tid / 8, c = tid % 8;
         if (r < S) rowS[r][c ^ (r & 7u)] = reinterpret_cast<const uint4*>(lv.desc + uint64_t(cand[r]) * kDims)[c];
     }
-    // the squared distance of this thread's row to row p
-    auto distTo = [&](uint32_t p) -> unsigned long long {
-        uint32_t acc = 0;
-#pragma unroll
-        for (uint32_t c = 0; c < kDims / 16; c++) {
-            const uint4 x = rowS[tid][c ^ (tid & 7u)], y = rowS[p][c ^ (p & 7u)];
-            const uint32_t d0 = __vabsdiffu4(x.x, y.x), d1 = __vabsdiffu4(x.y, y.y);
-            const uint32_t d2v = __vabsdiffu4(x.z, y.z), d3 = __vabsdiffu4(x.w, y.w);
-            acc = __dp4a(d0, d0, acc);
-            acc = __dp4a(d1, d1, acc);
-            acc = __dp4a(d2v, d2v, acc);
-            acc = __dp4a(d3, d3, acc);
-        }
-        return acc;
-    };
     const uint32_t pick = static_cast<uint32_t>(splitmix64(s) % S);
     if (tid == 0) chosen[0] = pick;
     __syncthreads();
-    unsigned long long d2 = mine ? distTo(pick) : 0ull;
+    uint32_t norm = 0;
+    if (mine) {
+#pragma unroll
+        for (uint32_t c = 0; c < kDims / 16; c++) norm = dot16(rowS[tid][c ^ (tid & 7u)], rowS[tid][c ^ (tid & 7u)], norm);
+    }
+    draw[tid] = norm;
+    __syncthreads();
+    // the squared distance of this thread's row to row p
+    auto distTo = [&](uint32_t p) -> uint32_t {
+        uint32_t dot = 0;
+#pragma unroll
+        for (uint32_t c = 0; c < kDims / 16; c++) dot = dot16(rowS[tid][c ^ (tid & 7u)], rowS[p][c ^ (p & 7u)], dot);
+        return norm + draw[p] - 2 * dot;
+    };
+    uint32_t d2 = mine ? distTo(pick) : 0u;
     uint32_t nv = 1;
     for (uint32_t k = 1; k < lv.B; k++) {
         // inclusive prefix of d2 over the candidates: warp scan, then the earlier warps' totals
-        unsigned long long incl = d2;
+        uint32_t incl = d2;
 #pragma unroll
         for (uint32_t off = 1; off < 32; off <<= 1) {
-            const unsigned long long v = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, off);
             if (lane >= off) incl += v;
         }
         if (lane == 31) warpSum[warp] = incl;
         __syncthreads();
-        unsigned long long before = 0, total = 0;
+        uint32_t before = 0, total = 0;
 #pragma unroll
         for (uint32_t w = 0; w < kPPWarps; w++) {
-            const unsigned long long v = warpSum[w];
-            before += w < warp ? v : 0ull;
+            const uint32_t v = warpSum[w];
+            before += w < warp ? v : 0u;
             total += v;
         }
         if (total == 0) break; // uniform across the CTA
         incl += before;
-        const unsigned long long t = splitmix64(s) % total;
+        const uint32_t t = static_cast<uint32_t>(splitmix64(s) % total);
         // smallest i with prefix[i] > t: exactly one candidate has prefix > t >= prefix - d2
         const bool hit = mine && incl > t && incl - d2 <= t;
         if (hit) chosen[k] = tid;
         nv = k + 1;
         __syncthreads();
         if (mine) {
-            const unsigned long long d = distTo(chosen[k]);
-            if (d < d2) d2 = d;
+            d2 = min(d2, distTo(chosen[k]));
         }
         __syncthreads(); // warpSum is rewritten by the next pick
     }
@@ -394,6 +412,134 @@ __global__ void __launch_bounds__(kPPSample, kPPCtasPerSm) kmeansPPKernel(KMeans
             v = reinterpret_cast<const uint4*>(lv.desc + uint64_t(c) * kDims)[chunk];
         }
         reinterpret_cast<uint4*>(lv.centers + (uint64_t(g) * kMaxBranch + b) * kDims)[chunk] = v;
+    }
+}
+
+// list: nullptr (every node), or a count and the nodes to take.
+__global__ void __launch_bounds__(kPPSample, kPPCtasPerSm) kmeansPPKernel(KMeansLevel lv, uint64_t seed, uint32_t level,
+                                                                          const uint32_t* list, uint32_t* nValidOut)
+{
+    __shared__ PPSmem sm;
+    if (list == nullptr) {
+        kmeansPPNode(lv, seed, level, blockIdx.x, nValidOut, sm);
+        return;
+    }
+    const uint32_t count = list[0];
+    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+        kmeansPPNode(lv, seed, level, list[1 + i], nValidOut, sm);
+        __syncthreads();
+    }
+}
+
+// A warp per node for nodes of at most kPPSmall members, the larger ones listed for kmeansPPKernel.
+// The same specification; lane l holds candidates l, l + 32, ..  Bound by instructions, like the kernel
+// above, whose eight warps all run the picks' scans, divisions and barriers for a hundred rows.  100,000
+// nodes of 100 members on average, B = 10: 2,400 us there, 540 us here and 850 us there for the quarter
+// with more than 128 (a warp per node of 256 candidates has too little shared memory to share an SM: no
+// faster).
+constexpr uint32_t kPPSmall = 128;
+constexpr uint32_t kPPSmallNodes = 1024;
+constexpr uint32_t kPer = kPPSmall / 32; // candidates of a lane
+static_assert(uint64_t(kPPSample) * kDims * 255 * 255 < (uint64_t(1) << 32), "sums of the weights fit 32 bits");
+__global__ void __launch_bounds__(32) kmeansPPSmallKernel(KMeansLevel lv, uint64_t seed, uint32_t level, uint32_t* list,
+                                                          uint32_t* nValidOut)
+{
+    __shared__ uint4 rowS[kPPSmall][kDims / 16]; // as in PPSmem
+    const uint32_t g = blockIdx.x, lane = threadIdx.x;
+    const uint32_t n = lv.nodeCnt[g];
+    uint4* centers = reinterpret_cast<uint4*>(lv.centers + uint64_t(g) * kMaxBranch * kDims);
+    if (n > kPPSmall) {
+        if (lane == 0) list[1 + atomicAdd(list, 1u)] = g;
+        return;
+    }
+    if (n == 0) {
+        if (lane == 0) nValidOut[g] = 0;
+        for (uint32_t i = lane; i < kMaxBranch * 8; i += 32)
+            centers[i] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+        return;
+    }
+    uint32_t m[kPer];
+#pragma unroll
+    for (uint32_t j = 0; j < kPer; j++) {
+        const uint32_t r = 32 * j + lane;
+        m[j] = r < n ? lv.members[lv.nodeOff[g] + r] : 0u;
+    }
+    // eight lanes per row
+#pragma unroll
+    for (uint32_t j = 0; j < kPer; j++) {
+        if (32 * j >= n) break; // uniform
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++) {
+            const uint32_t r = 32 * j + 4 * k + lane / 8, c = lane % 8;
+            const uint32_t id = __shfl_sync(0xFFFFFFFFu, m[j], 4 * k + lane / 8);
+            if (r < n) cpAsync16(&rowS[r][c ^ (r & 7u)], lv.desc + uint64_t(id) * kDims + (c << 4));
+        }
+    }
+    cpAsyncCommit();
+    uint64_t s = seed ^ (uint64_t(level) * 0x9E3779B97F4A7C15ull) ^ (uint64_t(g) * 0xD1B54A32D192ED03ull);
+    uint32_t pick = static_cast<uint32_t>(splitmix64(s) % n);
+    cpAsyncWait<0>();
+    __syncwarp();
+    uint32_t norm[kPer], d2[kPer];
+#pragma unroll
+    for (uint32_t j = 0; j < kPer; j++) {
+        const uint32_t r = 32 * j + lane;
+        norm[j] = 0;
+        if (r < n) {
+#pragma unroll
+            for (uint32_t c = 0; c < kDims / 16; c++) norm[j] = dot16(rowS[r][c ^ (r & 7u)], rowS[r][c ^ (r & 7u)], norm[j]);
+        }
+        d2[j] = r < n ? 0xFFFFFFFFu : 0u;
+    }
+    uint32_t mine = 0, nv = 0; // lane k: the k-th pick
+    for (uint32_t k = 0;; k++) {
+        if (lane == k) mine = pick;
+        nv = k + 1;
+        if (nv == lv.B) break;
+        // weights against the pick, their sums per 32 candidates
+        uint32_t pn = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < kPer; j++) pn = pick / 32 == j ? norm[j] : pn;
+        pn = __shfl_sync(0xFFFFFFFFu, pn, pick % 32);
+        uint4 p[kDims / 16];
+#pragma unroll
+        for (uint32_t c = 0; c < kDims / 16; c++) p[c] = rowS[pick][c ^ (pick & 7u)];
+        uint32_t incl[kPer], total = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < kPer; j++) {
+            const uint32_t r = 32 * j + lane;
+            if (r < n) {
+                uint32_t dot = 0;
+#pragma unroll
+                for (uint32_t c = 0; c < kDims / 16; c++) dot = dot16(rowS[r][c ^ (r & 7u)], p[c], dot);
+                d2[j] = min(d2[j], norm[j] + pn - 2 * dot);
+            }
+            incl[j] = d2[j];
+            if (32 * j < n) { // uniform
+#pragma unroll
+                for (uint32_t off = 1; off < 32; off <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl[j], off);
+                    if (lane >= off) incl[j] += v;
+                }
+            }
+            incl[j] += total;
+            total = __shfl_sync(0xFFFFFFFFu, incl[j], 31);
+        }
+        if (total == 0) break; // uniform
+        const uint32_t t = static_cast<uint32_t>(splitmix64(s) % total);
+        // smallest candidate with prefix > t: exactly one has prefix > t >= prefix - d2
+#pragma unroll
+        for (uint32_t j = 0; j < kPer; j++) {
+            const uint32_t hit = __ballot_sync(0xFFFFFFFFu, incl[j] > t && incl[j] - d2[j] <= t);
+            if (hit) pick = 32 * j + __ffs(hit) - 1;
+        }
+    }
+    if (lane == 0) nValidOut[g] = nv;
+#pragma unroll
+    for (uint32_t i = 0; i < kMaxBranch * 8 / 32; i++) {
+        const uint32_t b = 4 * i + lane / 8, chunk = lane % 8;
+        const uint32_t c = __shfl_sync(0xFFFFFFFFu, mine, b < nv ? b : nv - 1);
+        centers[32 * i + lane] = b < lv.B ? rowS[c][chunk ^ (c & 7u)] : make_uint4(0, 0, 0, 0);
     }
 }
 
@@ -824,9 +970,18 @@ void launchCenterNorms(const KMeansLevel& lv, cudaStream_t s)
     RBW_CUDA(cudaGetLastError());
 }
 
-void launchKMeansPPInit(const KMeansLevel& lv, uint64_t seed, uint32_t level, uint32_t* nValid, cudaStream_t s)
+void launchKMeansPPInit(const KMeansLevel& lv, uint64_t seed, uint32_t level, uint32_t* nValid, uint32_t* list,
+                        cudaStream_t s)
 {
-    kmeansPPKernel<<<lv.nbNodes, kPPSample, 0, s>>>(lv, seed, level, nValid);
+    // A CTA per node, or, where the nodes have at most kPPSmall members on average and are many, a warp
+    // per node and a CTA for each larger one.
+    if (lv.nbNodes >= kPPSmallNodes && lv.nbMembers <= uint64_t(kPPSmall) * lv.nbNodes) {
+        RBW_CUDA(cudaMemsetAsync(list, 0, 4, s));
+        kmeansPPSmallKernel<<<lv.nbNodes, 32, 0, s>>>(lv, seed, level, list, nValid);
+        kmeansPPKernel<<<currentSmCount() * kPPCtasPerSm, kPPSample, 0, s>>>(lv, seed, level, list, nValid);
+    } else {
+        kmeansPPKernel<<<lv.nbNodes, kPPSample, 0, s>>>(lv, seed, level, nullptr, nValid);
+    }
     RBW_CUDA(cudaGetLastError());
 }
 

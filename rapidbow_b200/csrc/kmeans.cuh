@@ -50,8 +50,10 @@ void buildNodeTiles(const uint32_t* nodeCnt, const uint32_t* nodeOff, uint32_t n
 void launchInitCenters(const KMeansLevel& lv, const uint32_t* pos, uint64_t nbDescTotal, cudaStream_t s);
 // Initial centers from descriptor indices (kInvalidIdx -> 0xFF bytes): injected initialisation.
 void launchInitCentersFromDesc(const KMeansLevel& lv, const uint32_t* descIdx, uint64_t nbDescTotal, cudaStream_t s);
-// Seeded k-means++ over <= 256 sampled members per node; writes centers, cnorm and nValid[g].
-void launchKMeansPPInit(const KMeansLevel& lv, uint64_t seed, uint32_t level, uint32_t* nValid, cudaStream_t s);
+// Seeded k-means++ over <= 256 sampled members per node; writes centers and nValid[g].  list: scratch,
+// nbNodes + 1 words.
+void launchKMeansPPInit(const KMeansLevel& lv, uint64_t seed, uint32_t level, uint32_t* nValid, uint32_t* list,
+                        cudaStream_t s);
 // |c|^2 for every slot of this level's nodes (padding slots b >= B get kPadNorm).
 void launchCenterNorms(const KMeansLevel& lv, cudaStream_t s);
 

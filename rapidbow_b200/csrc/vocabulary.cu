@@ -651,7 +651,7 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
             launchInitCenters(lv, picks.as<uint32_t>(), n, stream);
             RBW_CUDA(cudaStreamSynchronize(stream)); // hostPicks is reused next level
         } else if (opts.initMode == kInitKMeansPP) {
-            launchKMeansPPInit(lv, opts.seed, level, nValid.as<uint32_t>(), stream);
+            launchKMeansPPInit(lv, opts.seed, level, nValid.as<uint32_t>(), picks.as<uint32_t>(), stream);
             hostNValid.resize(nbLv);
             RBW_CUDA(cudaMemcpyAsync(hostNValid.data(), nValid.get(), nbLv * 4, cudaMemcpyDeviceToHost, stream));
             RBW_CUDA(cudaStreamSynchronize(stream));

@@ -149,6 +149,19 @@ def test_build_tile_lists_and_children_match_oracle(oracle, B, L, n):
     _tree_equal(voc, ref)
 
 
+@pytest.mark.parametrize("B,L,n,distinct", [(4, 6, 60_000, 0), (11, 4, 100_003, 0), (16, 4, 200_001, 900)])
+def test_build_kmeanspp_small_nodes_match_oracle(oracle, B, L, n, distinct):
+    """Levels of 1,000 and more small nodes, where a warp seeds a node of at most 128 members and a CTA
+    each larger one; repeated rows (weights that reach zero)."""
+    desc = sift_like(distinct or n, seed=n + B).numpy()
+    if distinct:
+        desc = np.ascontiguousarray(desc[np.random.default_rng(n).integers(0, distinct, n) ** 2 % distinct])
+    voc = rbw.build_vocabulary(torch.from_numpy(desc).cuda(), B, nb_doc=40, nb_levels=L, init="kmeans++", seed=6,
+                               max_iterations=3, ieee_division=True)
+    ref = oracle.build_vocabulary(desc, 40, B, L, max_iter=3, init=INIT_KMEANSPP, seed=6)
+    _tree_equal(voc, ref)
+
+
 @pytest.mark.parametrize("rows_per_sm,extra,L", [(12, -1, 2), (1536, 0, 1), (1536, 1, 1), (400, 77, 2)])
 def test_build_shared_level_edges_match_oracle(oracle, rows_per_sm, extra, L):
     """Levels whose streamed rows fit the SMs together run in one cooperative launch, nodes spread
