@@ -1402,16 +1402,19 @@ public:
         const uint32_t nDocs = mIndexed;
         const int sms = currentSmCount();
         // Document range per scoring CTA.  With grouped inverted files it is csrPerCta shards of
-        // kShardDocs documents: the most (up to kGroupedShards) that still gives two CTAs per SM, so
-        // a small batch spreads over the GPU; with one inverted file per segment, kSmemDocs
-        // documents (every CTA of a query walks the whole list).
+        // kShardDocs documents, as many as leave enough CTAs for the SMs to end together: four from
+        // eight CTAs per SM, two from four, of which two run at a time (20,000 images: 256 queries
+        // on 1,024 CTAs 1,118 us, on 512 1,190; 150 queries on 1,200 CTAs 887 us, on 300 1,155;
+        // 45,000 images, 100 queries on 900 CTAs 1,247 us, on 500 1,521); with one inverted file
+        // per segment, kSmemDocs documents
+        // (every CTA of a query walks the whole list).
         uint32_t csrPerCta = 1, shardDocs = std::min(std::max(nDocs, 1u), kSmemDocs);
         const bool grouped = groupedIndex();
         const uint64_t wanted = 2 * uint64_t(sms);
         if (grouped) {
             csrPerCta = kGroupedShards;
-            while (csrPerCta > 1 &&
-                   uint64_t(nq) * ((nDocs + csrPerCta * kShardDocs - 1) / (csrPerCta * kShardDocs)) < wanted)
+            while (csrPerCta > 1 && uint64_t(nq) * ((nDocs + csrPerCta * kShardDocs - 1) / (csrPerCta * kShardDocs)) <
+                                        (csrPerCta > 2 ? 4 * wanted : 2 * wanted))
                 csrPerCta /= 2;
             shardDocs = std::min(std::max(nDocs, 1u), csrPerCta * kShardDocs);
         }
