@@ -840,22 +840,21 @@ __global__ void __launch_bounds__(kRingThreads, 1)
 //   * the MMA issuer: the children (M = 128, N = 16 per child) of super-tile s once it is sorted, then
 //     the node level (N = 16) of s + 2;
 //   * two producers: TMA tile loads in the first pass; afterwards each gathers one tile of a
-//     super-tile, 16 bytes per lane; the first also loads each group's centers;
-//   * the norms warp turns a group's |c|^2 into the keys of argminKeys.
-// The n-th group of a CTA uses center slot n & 1, for the (n >> 1)-th time.
+//     super-tile, 16 bytes per lane;
+//   * the centers warp loads each group's block and turns its |c|^2 into the keys of argminKeys.
+// A CTA's groups use the center slots in turn: as many as fit two blocks of B = 16, since with few rows
+// per group the time from a slot's release to its next block's arrival is what a team waits for
+// (100 rows per group, B = 10: 140 us with two slots, 108 us with three).
 //
 // What bounds it: a team's chain from the node level to the leaf, ~4,900 cycles per 256 rows at 16
 // warps with IPC 0.42 per scheduler, two teams at once (memory: 2 x 700 per 128 rows; tensor pipe
 // ~470).  Its instruction footprint counts: each wait keeps only its loop inline and
 // no loop over super-tiles is unrolled (16-byte instructions, 74 -> 29 KB: 505 -> 349 us).  Three
 // teams would have 72 registers a thread; the rows held over the sort alone take 32.
-// 10,000,003 rows, B = 16, L = 4: first pass 505 -> 352 us, second 490 -> 452 us against two teams
-// that read all 16 B columns; whole lookups: 1,000,000 rows, B = 10, L = 6: 348 -> 322 us; 500,000
-// rows, B = 16, L = 4: 94 -> 81 us; 60,000 rows, B = 10, L = 6: 179 -> 179 us; 4,000,000 rows, B = 2,
-// L = 8: 836 -> 785 us.
-//
-// Tile j's child c lands in columns 16 (c + j) of the children area: the two tiles share at most one
-// child.  Up to B = 13 both teams' areas fit beside the node columns, above that they take turns.
+// 10,000,003 rows, B = 16, L = 4: first pass 505 -> 350 us, second 490 -> 455 us against two teams
+// that read all 16 B columns; whole lookups: 1,000,000 rows, B = 10, L = 6: 348 -> 293 us; 500,000
+// rows, B = 16, L = 4: 94 -> 83 us; 150,000 rows, B = 16, L = 5: 446 -> 326 us; 60,000 rows, B = 10,
+// L = 6: 179 -> 159 us; 4,000,000 rows, B = 2, L = 8: 836 -> 804 us.
 constexpr uint32_t kSubTiles = 2;
 constexpr uint32_t kSuperRows = kSubTiles * kTileRows;     // 256
 constexpr uint32_t kSuperBufs = 4;
@@ -866,25 +865,39 @@ constexpr uint32_t kSortNodeCols = 16 * kSubTiles;         // one super-tile's n
 constexpr uint32_t kSortKidCol = 2 * kSortNodeCols;
 static_assert(kSortKidCol + 16 * (kMaxBranch + kSubTiles - 1) <= kTmemCols, "sorted schedule exceeds tensor memory");
 constexpr uint32_t kSortTileCache = 512;
+constexpr uint32_t kMaxSlots = 4; // center blocks
 constexpr uint32_t kLastOfGroup = 1, kNextIsLast = 2, kFirstOfGroup = 4; // TileInfo::pad of a super-tile
 
 struct SortSmem {
     uint8_t a[kSuperBufs][kSubTiles * kTileBytes];
-    uint8_t b[2][kBBlockBytes];
-    alignas(16) int32_t cn[2][17][16];   // keys of |c|^2 of each B slot: row 0 = node, rows 1.. = children
+    uint8_t b[2 * kBBlockBytes];
+    alignas(16) int32_t cn[kMaxSlots][17][16];   // keys of |c|^2 of each B slot: row 0 = node, rows 1.. = children
     TileInfo tileCache[kSortTileCache];  // this CTA's super-tiles (passes after the first)
     uint32_t orig[2][kSuperRows];        // by team and sorted position: row id
     uint8_t child[2][kSuperRows];        // ... and branch
     uint32_t cnt[2][2][16];              // rows per branch, by team and turn
     uint32_t binBase[2][17];             // first sorted position of each branch; [16] = rows
     uint64_t aFull[kSuperBufs], aFree[kSuperBufs];
-    uint64_t bFull[2], bEmpty[2], cnReady[2];
+    uint64_t bFull[kMaxSlots], bEmpty[kMaxSlots], cnReady[kMaxSlots];
     uint64_t nodeDone[2], counted[2], sorted[2], kidsDone[2], kidsRead[2]; // by team
     uint64_t mmaDone;
     uint32_t tmemBase, abortFlag, noAbort;
 };
 constexpr size_t kSortSmemBytes = sizeof(SortSmem) + 1024;
 static_assert(kSortSmemBytes <= 227 * 1024, "shared memory");
+
+// The center slot of a group and the parity of its use, before the first group; next() per group.
+struct CenterSlot {
+    uint32_t i, parity;
+    __device__ __forceinline__ explicit CenterSlot(uint32_t slots) : i{slots - 1u}, parity{1u} {}
+    __device__ __forceinline__ void next(uint32_t slots)
+    {
+        if (++i == slots) {
+            i = 0;
+            parity ^= 1u;
+        }
+    }
+};
 
 // Super-tile i of this CTA, with its place in its group's run here.
 __device__ __forceinline__ TileInfo superTileGlobal(const TileInfo* tiles, uint32_t nT, uint32_t i)
@@ -939,6 +952,17 @@ __device__ __forceinline__ bool waitWarp(uint64_t* bar, uint32_t parity, volatil
     return true;
 }
 
+// For a warp that polls several barriers: whether nothing has been ready since `since` (0: just now)
+// for too long, or another warp gave up.
+__device__ __forceinline__ bool idleTooLong(uint64_t& since, volatile uint32_t* abortFlag, DeviceErrors* err, uint32_t site)
+{
+    const uint64_t now = globalTimerNs();
+    if (since == 0) since = now;
+    if (!__any_sync(0xFFFFFFFFu, now - since > kWaitLimitNs || *abortFlag != 0)) return false;
+    waitTimedOut(smemAddr(const_cast<uint32_t*>(abortFlag)), err, site, 0);
+    return true;
+}
+
 // argmin_b (|c_b|^2 - 2 x.c_b), lowest b on ties (vocTreeLookUp.cu:108-125), as the minimum of
 // 16 (|c_b|^2 - 2 x.c_b) + b: a score lies in (-2^24, 2^23), so that fits 32 bits, and the low bits
 // are the lowest branch of the lowest score.  key: 16 |c_b|^2 + b.
@@ -981,6 +1005,8 @@ __global__ void __launch_bounds__(kSortThreads, 1)
     if (nT == 0) return; // uniform
     const bool two = p.twoLevels != 0;
     const uint32_t kidCols = 16 * (p.B + kSubTiles - 1);
+    const uint32_t blockBytes = kNodeBytes * (two ? 1u + p.B : 1u);
+    const uint32_t slots = min(2 * kBBlockBytes / blockBytes, kMaxSlots);
     const bool ownKids = kSortKidCol + 2 * kidCols <= kTmemCols; // a children area for each team
     volatile uint32_t* abortFlag = &S.abortFlag;
     if (tid == 0) {
@@ -988,10 +1014,12 @@ __global__ void __launch_bounds__(kSortThreads, 1)
             mbarInit(&S.aFull[i], kGather ? 2 : 1);
             mbarInit(&S.aFree[i], 1);
         }
-        for (uint32_t j = 0; j < 2; j++) {
+        for (uint32_t j = 0; j < kMaxSlots; j++) {
             mbarInit(&S.bFull[j], 1);
             mbarInit(&S.bEmpty[j], 1 + 2 * kSortTeamWarps); // the issuer's MMAs and both teams' norms
             mbarInit(&S.cnReady[j], 1);
+        }
+        for (uint32_t j = 0; j < 2; j++) {
             mbarInit(&S.nodeDone[j], 1);
             mbarInit(&S.counted[j], kSortTeamWarps);
             mbarInit(&S.sorted[j], kSortTeamWarps);
@@ -1017,25 +1045,61 @@ __global__ void __launch_bounds__(kSortThreads, 1)
     tcFenceAfter();
     const uint32_t tmem = S.tmemBase;
     if (warp == kSortIssuer + 3) {
-        // ------------------------------------------------------------ norms
-        uint32_t n = 0;
-        #pragma unroll 1
-        for (uint32_t s = 0; s < nT; s++) {
-            if (!(superTile<kGather>(S, p, t0, nT, s).pad & kFirstOfGroup)) continue;
-            const uint32_t slot = n & 1u;
-            if (!waitWarp(&S.bFull[slot], (n >> 1) & 1u, abortFlag, p.err, 73)) break;
-            n++;
-            const uint32_t words = two ? 16 * (1 + p.B) : 16;
-            int32_t* cn = &S.cn[slot][0][0];
+        // ------------------------------------------------------------ centers
+        // two cursors over the groups: the next to load and the next whose norms become keys,
+        // whichever can go on
+        CenterSlot loadAt(slots), keyAt(slots);
+        uint32_t load = 0, key = 0; // super-tiles passed by each
+        uint64_t idle = 0;
+        while (key < nT) {
+            while (key < nT && !(superTile<kGather>(S, p, t0, nT, key).pad & kFirstOfGroup)) key++;
+            while (load < nT && !(superTile<kGather>(S, p, t0, nT, load).pad & kFirstOfGroup)) load++;
+            CenterSlot at = keyAt;
+            at.next(slots);
+            if (key < load && __all_sync(0xFFFFFFFFu, mbarTest(&S.bFull[at.i], at.parity))) {
+                const uint32_t words = two ? 16 * (1 + p.B) : 16;
+                int32_t* cn = &S.cn[at.i][0][0];
 #pragma unroll 1
-            for (uint32_t i = lane; i < words; i += 32) cn[i] = normKey(cn[i], i % 16, p.B);
-            __syncwarp();
-            if (lane == 0) mbarArrive(&S.cnReady[slot]);
+                for (uint32_t i = lane; i < words; i += 32) cn[i] = normKey(cn[i], i % 16, p.B);
+                __syncwarp();
+                if (lane == 0) mbarArrive(&S.cnReady[at.i]);
+                keyAt = at;
+                key++;
+                idle = 0;
+                continue;
+            }
+            at = loadAt;
+            at.next(slots);
+            if (load < nT && __all_sync(0xFFFFFFFFu, mbarTest(&S.bEmpty[at.i], at.parity ^ 1u))) {
+                if (lane == 0) {
+                    const uint32_t group = superTile<kGather>(S, p, t0, nT, load).group, nb = two ? p.B : 0u;
+                    uint8_t* b = S.b + at.i * blockBytes;
+                    mbarArriveExpectTx(&S.bFull[at.i], (kNodeBytes + 64u) * (1u + nb));
+                    bulkLoad(b, p.centersSw + (p.lbA + group) * kNodeBytes, kNodeBytes, &S.bFull[at.i]);
+                    bulkLoad(&S.cn[at.i][0][0], p.cnorm + (p.lbA + group) * kMaxBranch, 64u, &S.bFull[at.i]);
+                    if (two) {
+                        const uint64_t c0 = p.lbB + uint64_t(group) * p.B;
+                        bulkLoad(b + kNodeBytes, p.centersSw + c0 * kNodeBytes, kNodeBytes * p.B, &S.bFull[at.i]);
+                        bulkLoad(&S.cn[at.i][1][0], p.cnorm + c0 * kMaxBranch, 64u * p.B, &S.bFull[at.i]);
+                    }
+                }
+                __syncwarp();
+                loadAt = at;
+                load++;
+                idle = 0;
+                continue;
+            }
+            if (idleTooLong(idle, abortFlag, p.err, 60)) break;
+        }
+        // the loads that no one waited for (aborted) must land before the CTA can exit
+        while (keyAt.i != loadAt.i || keyAt.parity != loadAt.parity) {
+            keyAt.next(slots);
+            waitWarp(&S.bFull[keyAt.i], keyAt.parity, &S.noAbort, p.err, 62);
         }
     } else if (warp > kSortIssuer) {
         // ------------------------------------------------------------ producers
         const uint32_t which = warp - kSortIssuer - 1; // the tile of each super-tile that this one gathers
-        uint32_t n = 0, issued = 0, published = 0; // n: groups loaded
+        uint32_t issued = 0, published = 0;
         auto publishUpTo = [&](uint32_t end) { // gathered rows: generic writes, read by the MMA
             if (published >= end) return;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1055,31 +1119,10 @@ __global__ void __launch_bounds__(kSortThreads, 1)
             }
         };
         if (kGather) loadIds(0);
-        #pragma unroll 1
+#pragma unroll 1
         for (uint32_t s = 0; s < nT && (kGather || which == 0); s++) {
             const TileInfo ti = superTile<kGather>(S, p, t0, nT, s);
             const uint32_t buf = s % kSuperBufs, tiles = (ti.count + kTileRows - 1) / kTileRows;
-            if (which == 0 && (ti.pad & kFirstOfGroup)) {
-                const uint32_t slot = n & 1u;
-                if (kGather) { // the slot is released behind super-tiles that must be published first
-                    cpAsyncWait<0>();
-                    publishUpTo(issued);
-                }
-                if (!waitWarp(&S.bEmpty[slot], ((n >> 1) & 1u) ^ 1u, abortFlag, p.err, 60)) break;
-                n++;
-                if (lane == 0) {
-                    const uint32_t nb = two ? p.B : 0u;
-                    mbarArriveExpectTx(&S.bFull[slot], (kNodeBytes + 64u) * (1u + nb));
-                    bulkLoad(S.b[slot], p.centersSw + (p.lbA + ti.group) * kNodeBytes, kNodeBytes, &S.bFull[slot]);
-                    bulkLoad(&S.cn[slot][0][0], p.cnorm + (p.lbA + ti.group) * kMaxBranch, 64u, &S.bFull[slot]);
-                    if (two) {
-                        const uint64_t c0 = p.lbB + uint64_t(ti.group) * p.B;
-                        bulkLoad(S.b[slot] + kNodeBytes, p.centersSw + c0 * kNodeBytes, kNodeBytes * p.B, &S.bFull[slot]);
-                        bulkLoad(&S.cn[slot][1][0], p.cnorm + c0 * kMaxBranch, 64u * p.B, &S.bFull[slot]);
-                    }
-                }
-                __syncwarp();
-            }
             if (!waitWarp(&S.aFree[buf], ((s / kSuperBufs) & 1u) ^ 1u, abortFlag, p.err, 61)) break;
             if (!kGather) {
                 if (lane == 0) {
@@ -1124,14 +1167,14 @@ __global__ void __launch_bounds__(kSortThreads, 1)
                 waitWarp(&S.aFull[i], (last / kSuperBufs) & 1u, &S.noAbort, p.err, 62);
             }
         }
-        for (uint32_t i = n > 2 ? n - 2 : 0; i < n; i++) waitWarp(&S.bFull[i & 1u], (i >> 1) & 1u, &S.noAbort, p.err, 62);
         __syncwarp();
     } else if (warp == kSortIssuer) {
         // ------------------------------------------------------------ MMA issuer
         const bool issuer = electOne();
         // Whichever step's inputs are ready first: with groups of few rows the node level of the next
         // group waits for its centers, which wait for the children of an earlier one.
-        uint32_t node = 0, kid = 0, nodeN = 0, kidN = 0; // next super-tile of each step, groups before it
+        uint32_t node = 0, kid = 0; // next super-tile of each step
+        CenterSlot nodeAt(slots), kidAt(slots);
         uint64_t idle = 0;
         while (kid < nT) {
             if (kid < node && __all_sync(0xFFFFFFFFu, mbarTest(&S.sorted[kid & 1u], (kid >> 1) & 1u)) &&
@@ -1141,8 +1184,7 @@ __global__ void __launch_bounds__(kSortThreads, 1)
                 // read the node level)
                 const uint32_t team = kid & 1u, buf = kid % kSuperBufs;
                 const TileInfo ti = superTile<kGather>(S, p, t0, nT, kid);
-                if (ti.pad & kFirstOfGroup) kidN++;
-                const uint32_t slot = (kidN - 1) & 1u;
+                if (ti.pad & kFirstOfGroup) kidAt.next(slots);
                 tcFenceAfter();
                 if (two) {
                     const uint32_t kids = tmem + kSortKidCol + (ownKids ? team * kidCols : 0u);
@@ -1157,14 +1199,14 @@ __global__ void __launch_bounds__(kSortThreads, 1)
                         if (here == 0) continue;
                         const uint32_t c0 = __ffs(here) - 1, c1 = 31u - __clz(here);
                         mmaU8x4(issuer, kids + 16u * (c0 + j), smemDescSw128(smemAddr(S.a[buf]) + j * kTileBytes), 32u,
-                                smemDescSw128(smemAddr(S.b[slot]) + kNodeBytes * (1u + c0)), 32u,
+                                smemDescSw128(smemAddr(S.b) + kidAt.i * blockBytes + kNodeBytes * (1u + c0)), 32u,
                                 idescU8(16u * (c1 - c0 + 1u)), 0u);
                     }
                     if (issuer) mmaCommit(&S.kidsDone[team]);
                 }
                 if (issuer) {
                     mmaCommit(&S.aFree[buf]); // after the last MMA that reads the buffer
-                    if (ti.pad & kLastOfGroup) mmaCommit(&S.bEmpty[slot]);
+                    if (ti.pad & kLastOfGroup) mmaCommit(&S.bEmpty[kidAt.i]);
                 }
                 kid++;
                 idle = 0;
@@ -1175,28 +1217,24 @@ __global__ void __launch_bounds__(kSortThreads, 1)
             const uint32_t buf = node % kSuperBufs;
             if (node < nT && node < kid + 2 && __all_sync(0xFFFFFFFFu, mbarTest(&S.aFull[buf], (node / kSuperBufs) & 1u))) {
                 const TileInfo ti = superTile<kGather>(S, p, t0, nT, node);
-                const uint32_t n = nodeN + (ti.pad & kFirstOfGroup ? 1u : 0u);
-                if (__all_sync(0xFFFFFFFFu, mbarTest(&S.bFull[(n - 1) & 1u], ((n - 1) >> 1) & 1u))) {
+                CenterSlot at = nodeAt;
+                if (ti.pad & kFirstOfGroup) at.next(slots);
+                if (__all_sync(0xFFFFFFFFu, mbarTest(&S.bFull[at.i], at.parity))) {
                     tcFenceAfter();
                     const uint32_t tiles = (ti.count + kTileRows - 1) / kTileRows;
 #pragma unroll 1
                     for (uint32_t j = 0; j < tiles; j++)
                         mmaU8x4(issuer, tmem + kSortNodeCols * (node & 1u) + 16u * j,
                                 smemDescSw128(smemAddr(S.a[buf]) + j * kTileBytes), 32u,
-                                smemDescSw128(smemAddr(S.b[(n - 1) & 1u])), 32u, idescU8(16), 0u);
+                                smemDescSw128(smemAddr(S.b) + at.i * blockBytes), 32u, idescU8(16), 0u);
                     if (issuer) mmaCommit(&S.nodeDone[node & 1u]);
-                    nodeN = n;
+                    nodeAt = at;
                     node++;
                     idle = 0;
                     continue;
                 }
             }
-            const uint64_t now = globalTimerNs();
-            if (idle == 0) idle = now;
-            if (__any_sync(0xFFFFFFFFu, now - idle > kWaitLimitNs || *abortFlag != 0)) {
-                waitTimedOut(smemAddr(&S.abortFlag), p.err, 63, kid & 1u);
-                break;
-            }
+            if (idleTooLong(idle, abortFlag, p.err, 63)) break;
         }
         if (issuer) mmaCommit(&S.mmaDone);
         waitWarp(&S.mmaDone, 0, abortFlag, p.err, 67);
@@ -1209,18 +1247,25 @@ __global__ void __launch_bounds__(kSortThreads, 1)
         // rows 32 tw + 4 i + lane / 8, chunk lane % 8 of each: 128-byte swizzle, i even and odd
         const uint32_t ch = (lane & 7u) << 4;
         const uint32_t from0 = (32 * tw + lane / 8) * kDims + (ch ^ ((lane / 8) << 4));
-        uint32_t n = 0xFFFFFFFFu, ready = 0xFFFFFFFFu; // group of super-tile s; the last one whose norms were awaited
-        #pragma unroll 1
+        CenterSlot at(slots);
+        bool fresh = false; // a group whose norms were not awaited yet
+#pragma unroll 1
         for (uint32_t s = team; s < nT; s += 2) {
-            if (s > 0 && (superTile<kGather>(S, p, t0, nT, s - 1).pad & kFirstOfGroup)) n++;
             const TileInfo ti = superTile<kGather>(S, p, t0, nT, s);
-            if (ti.pad & kFirstOfGroup) n++;
-            const uint32_t slot = n & 1u;
+            if (s > 0 && (superTile<kGather>(S, p, t0, nT, s - 1).pad & kFirstOfGroup)) {
+                at.next(slots);
+                fresh = true;
+            }
+            if (ti.pad & kFirstOfGroup) {
+                at.next(slots);
+                fresh = true;
+            }
+            const uint32_t slot = at.i;
             const uint32_t turn = s >> 1, par = turn & 1u, buf = s % kSuperBufs;
             const bool valid = row < ti.count, some = 32 * tw < ti.count;
             const uint32_t orig = valid ? (kGather ? __ldg(p.perm + ti.start + row) : ti.start + row) : 0u;
-            if (n != ready && !waitWarp(&S.cnReady[slot], (n >> 1) & 1u, abortFlag, p.err, 70)) break;
-            ready = n;
+            if (fresh && !waitWarp(&S.cnReady[slot], at.parity, abortFlag, p.err, 70)) break;
+            fresh = false;
             if (!waitWarp(&S.nodeDone[team], par, abortFlag, p.err, 72)) break;
             if (!waitWarp(&S.aFull[buf], (s / kSuperBufs) & 1u, abortFlag, p.err, 71)) break;
             // P1
@@ -1318,7 +1363,7 @@ __global__ void __launch_bounds__(kSortThreads, 1)
                 tmemWaitTie(r);
 #pragma unroll
                 for (int i = 0; i < 16; i++) sel[i] = child == c0 ? sel[i] : r[i];
-                #pragma unroll 1
+        #pragma unroll 1
                 for (uint32_t c = c0 + 2; c <= c1; c++) {
                     tmemLoad16(kids + 16u * c, r);
                     tmemWaitTie(r);
