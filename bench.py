@@ -280,7 +280,7 @@ def run_ours(args, world, rank, local):
         e = Autotuner.for_current_device().tune_lookup(voc, desc)
         tuned = {"param": "lookup_schedule", "value": e["value"], "default": 1, "tuned_ms": e["ms"],
                  "default_ms": e["default_ms"], "candidates_ms": e["candidates"],
-                 "kernel": "tensor-core pass (1 = level pairs in two buffers, 2 = three-slot ring), per launch"}
+                 "kernel": "tensor-core pass (1 = rows sorted by branch, 2 = three-slot ring), per launch"}
     with ClockSampler(local) as clocks:
         ms, launches, (k_ms, k_n) = timed(args.algo, args.steps, args.warmup, "lookup_pass_tc")
     regroup_ms, regroup_n = timed.regroup
@@ -610,9 +610,9 @@ def build_bench(args, dev, rank):
                     "default_assign_ms": e["default_ms"]}
             if "sums" in e:
                 tune["sums"] = {"value": e["sums"]["value"], "candidates_ms": e["sums"]["candidates"],
-                                "note": "1 = shared-memory atomics, 2 = a second MMA per tile"}
+                                "note": "1 and 2 give the same sums, by a second MMA per tile"}
         voc2, s2, a_ms, u_ms = timed_build(c2, 10, 6, 3, float_centers=fl)
-        res = {"workload": ("build (float centers: split-bf16 distances, FP64 re-score, FP64 inertia): " if fl
+        res = {"workload": ("build (float centers: fixed-point distances, FP64 re-score, FP64 inertia): " if fl
                             else "build (uint8 centers): ") + wl2,
                "value": s2, "unit": "s", "higher_is_better": False,
                "assign_kernel_ms_per_build": a_ms, "update_kernel_ms_per_build": u_ms,

@@ -9,8 +9,8 @@ tree levels, descriptor-count bucket = floor(log2(n))):
     assign_f32_ctas_per_sm  float-center assign, CTAs per SM: 1..3          (default 3)
     scatter_rows            lookup regroup scatter of more than 1,024 bins, rows per thread:
                             8|16|32 (default 16)
-    lookup_schedule         tensor-core lookup schedule of algo "auto": 1 level pairs in two
-                            accumulator buffers, 2 the three-slot ring (default 1)
+    lookup_schedule         tensor-core lookup schedule of algo "auto": 1 rows sorted by
+                            branch, 2 the three-slot ring (default 1)
     assign_sums             1 or 2, kept for saved files: the uint8 k-means center sums have one
                             form (a second MMA per tile) whatever the value
     db_shard_tables         DataBase inverted file: 1 one CSR per 2,560-document shard while
@@ -156,9 +156,8 @@ class Autotuner:
 
     def tune_build(self, desc, B: int, L: int, float_centers: bool = False, repeats: int = 2, **build_kw) -> dict:
         """Tunes the assign kernel on a build of `desc` (CUDA uint8 [n, 128]); the build itself is
-        the workload, timed by the library's assign-kernel events.  uint8 centers: the center sums
-        (shared atomics or the tensor core) first, then the CTAs per SM for the chosen sums;
-        returns the second entry, with the first under "sums"."""
+        the workload, timed by the library's assign-kernel events.  uint8 centers: the entry of
+        the CTAs per SM, with that of the center sums (which have one form) under "sums"."""
         from . import build_vocabulary, timing_enable, timing_read, timing_reset
 
         n = desc.shape[0]
@@ -175,8 +174,7 @@ class Autotuner:
         if float_centers:
             return self.tune("assign_f32_ctas_per_sm", B, 0, n, measure)
         sums = self.tune("assign_sums", B, 0, n, measure)
-        e = self.tune("assign_ctas_per_sm", B, 0, n, measure,
-                      candidates=[v for v in CANDIDATES["assign_ctas_per_sm"] if sums["value"] == 1 or v <= 4])
+        e = self.tune("assign_ctas_per_sm", B, 0, n, measure)
         return dict(e, sums=sums)
 
     def tune_lookup(self, voc, desc, repeats: int = 3) -> dict:
