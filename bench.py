@@ -37,11 +37,11 @@ BYTES_PER_DESC = 132  # 128 B read + 4 B leaf written (algorithmic, per descript
 # DRAM bytes per descriptor of one lookupPassSorted launch: dram__bytes_read.sum + dram__bytes_write.sum
 # of an ncu capture of a 2M-descriptor lookup (B=16, L=4; both pass launches averaged).  Traffic
 # grows in proportion to the descriptors, so it is scaled to the timed launch.
-LOOKUP_PASS_DRAM_BYTES_PER_DESC = 136.6
-# DRAM bytes of one scoring launch (queryPrepKernel + scoreKernel: 2.6 MB + 1.388 GB read,
-# 3.9 MB written) on the seeded 20,000-image database with 256 queries, top-50, from an ncu
-# capture of that workload.
-SCORE_DRAM_BYTES_20K_IMAGES = 1_394_930_000
+LOOKUP_PASS_DRAM_BYTES_PER_DESC = 135.1
+# DRAM bytes of one scoring launch (queryPrepKernel + scoreKernel: 2.5 MB + 515.2 MB read, 0.2 MB
+# written) on the seeded 20,000-image database with 256 queries, top-50, from an ncu capture of
+# that workload.
+SCORE_DRAM_BYTES_20K_IMAGES = 517_930_000
 WORKLOAD = ("lookup of 10M fresh SIFT-like descriptors per GPU through a 65,536-word tree "
             "(B=16, L=4) trained on 2M descriptors (k-means++ init, 10 Lloyd iterations)")
 

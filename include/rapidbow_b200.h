@@ -56,8 +56,8 @@ enum {
  * (kmeans.cu:367); RBW_BUILD_IEEE_DIVISION uses the correctly rounded quotient instead.
  * RBW_BUILD_FLOAT_CENTERS (no counterpart in the reference, whose centers are uint8) keeps fp32
  * centers, c = float(double(sum) / double(count)) of the exact integer sums; distances come from
- * the tensor cores with each center split into hi + lo bf16 parts and fp32 accumulation, and
- * every descriptor whose best-versus-second margin is within the stated error bound is re-scored
+ * the tensor cores with each center as 24-bit fixed point in three bytes (hi + lo bf16 parts for uploaded
+ * centers outside [0, 256)), and every descriptor whose best-versus-second margin is within the stated error bound is re-scored
  * in FP64 on the GPU, so assignments equal those of an FP64 evaluation (lowest index on ties).
  * Lookups through such a vocabulary use the same arithmetic. */
 enum { RBW_BUILD_IEEE_DIVISION = 1, RBW_BUILD_FLOAT_CENTERS = 2 };
@@ -89,12 +89,14 @@ typedef struct rbw_vocabulary rbw_vocabulary;
 
 /* Lookup algorithms. */
 enum {
-    RBW_LOOKUP_AUTO = 0,       /* fastest exact path */
-    RBW_LOOKUP_TENSOR_U8 = 1,  /* tcgen05 uint8 tensor-core descent with device regroup */
+    RBW_LOOKUP_AUTO = 0,       /* fastest exact path: one launch, a warp per descriptor, for few descriptors
+                                  (up to 32,768 for two levels, 100,000 for four, 200,000 above), else tensor cores */
+    RBW_LOOKUP_TENSOR_U8 = 1,  /* tcgen05 uint8 tensor-core descent with device regroup, rows sorted by branch
+                                  within each level pair */
     RBW_LOOKUP_SIMT_F32 = 2,   /* plain FP32 SIMT descent (comparison baseline) */
-    RBW_LOOKUP_TENSOR_U8_WARPNODE = 3, /* as TENSOR_U8, the node level of each level pair by warp-level MMAs
+    RBW_LOOKUP_TENSOR_U8_WARPNODE = 3, /* without the sort, the node level of each level pair by warp-level MMAs
                                           in the epilogue warps, so the children MMA need not wait for it */
-    RBW_LOOKUP_TENSOR_U8_RING = 4      /* as TENSOR_U8, the node level and the children (in halves) in
+    RBW_LOOKUP_TENSOR_U8_RING = 4      /* without the sort, the node level and the children (in halves) in
                                           separate tensor-memory columns: one issuer, a three-slot ring */
 };
 
@@ -373,14 +375,14 @@ RBW_API int rbw_idf_weights(uint32_t nb_doc, const uint32_t* occ, uint64_t n, fl
  * (parameter, branch factor, tree levels, descriptor-count bucket = floor(log2(n))); levels 0
  * matches any depth.  Unset entries use the defaults. */
 enum {
-    RBW_TUNE_ASSIGN_CTAS_PER_SM = 0,     /* uint8 k-means assign: CTAs per SM, 1..8 (default 6) */
+    RBW_TUNE_ASSIGN_CTAS_PER_SM = 0,     /* uint8 k-means assign: CTAs per SM, 1..8, of which at most five run */
     RBW_TUNE_ASSIGN_F32_CTAS_PER_SM = 1, /* float-center assign: CTAs per SM, 1..3 (default 3) */
     RBW_TUNE_SCATTER_ROWS = 2,           /* lookup regroup: rows per thread, 8, 16 or 32 (default 16) */
     RBW_TUNE_DB_SHARD_TABLES = 3,        /* DataBase inverted file, keyed by documents instead of
                                             descriptors: 1 grouped tables per 2,560-document shard
                                             while those tables stay small (default), 2 one CSR */
-    RBW_TUNE_LOOKUP_SCHEDULE = 4,        /* the tensor-core schedule RBW_LOOKUP_AUTO runs: 1 level
-                                            pairs in two buffers (default), 2 the three-slot ring */
+    RBW_TUNE_LOOKUP_SCHEDULE = 4,        /* the tensor-core schedule RBW_LOOKUP_AUTO runs: 1 sorted
+                                            rows (default), 2 the three-slot ring */
     RBW_TUNE_ASSIGN_SUMS = 5             /* 1 or 2, accepted for saved tuning files: the uint8 k-means
                                             center sums always come from a second MMA per tile */
 };

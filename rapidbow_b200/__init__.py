@@ -358,7 +358,7 @@ def build_vocabulary(descriptors, branch_factor: int = 16, nb_doc: int = 1, nb_l
                      ieee_division: bool = False, float_centers: bool = False) -> Vocabulary:
     """rbow::buildVocabulary (RapidBoW.h:82-88); descriptors is a CUDA uint8 tensor [n, 128].
     ieee_division=True rounds centers with the correctly rounded quotient instead of the
-    reference's fast-math division; float_centers=True keeps fp32 centers (split-bf16 distances
+    reference's fast-math division; float_centers=True keeps fp32 centers (fixed-point distances
     with an FP64 re-score near ties, see RBW_BUILD_FLOAT_CENTERS)."""
     lib = load_library()
     o = BuildOptions()

@@ -1,7 +1,7 @@
 // Hierarchical k-means kernels.  Distances are exact integers: score_b = |c_b|^2 - 2 x.c_b with
 // x.c_b from the tensor core (tcgen05.mma.kind::i8, u8 x u8 -> s32) in the assign step and from
 // dp4a in k-means++, argmin with the lowest index on ties (kmeans.cu:131-135).
-// Center sums are exact (u32 in shared memory, u64 in global memory).
+// Center sums are exact (s32 in tensor memory, u64 in global memory).
 #include "kmeans.cuh"
 #include "timing.h"
 #include "tuning.h"
@@ -562,10 +562,11 @@ __global__ void __launch_bounds__(32) kmeansPPSmallKernel(KMeansLevel lv, uint64
 //
 // A tile costs the SM 8 x 45 cycles of tensor pipe and its 16 KB of gathered rows, which is more
 // (0.37 us per tile at HBM speed); the wait -> MMA -> read -> MMA chain of a tile (~1 us) is hidden
-// by five CTAs per SM, each gathering its next tile while one is scored.  The 60 steps of a
-// 10M-member build (B = 10, L = 6): 18.2 ms, 0.30 ms per step against 0.20 ms to read the rows;
-// 39.6 ms with the sums by shared atomics (128 per member), 35.3 ms by MMAs over a tile
-// transposed in shared memory.
+// by five CTAs per SM, each gathering its next tile while one is scored.  10M members, B = 10: 0.22 ms
+// per step against 0.20 ms to read the rows (0.30 ms where the nodes are small and their sums as many
+// bytes as the rows: those stay on chip, see kmeans_lloyd.cu).  The 60 steps of a build took 39.6 ms with
+// the sums by shared atomics (128 per member), 35.3 ms by MMAs over a tile transposed in shared
+// memory, 18.2 ms with these.
 constexpr uint32_t kAssignThreads = 128;
 constexpr uint32_t kAssignRows = 128;
 constexpr uint32_t kAssignTmemCols = 32; // the smallest allocation: distances | sums

@@ -855,6 +855,9 @@ __global__ void __launch_bounds__(kRingThreads, 1)
 // that read all 16 B columns; whole lookups: 1,000,000 rows, B = 10, L = 6: 348 -> 293 us; 500,000
 // rows, B = 16, L = 4: 94 -> 83 us; 150,000 rows, B = 16, L = 5: 446 -> 326 us; 60,000 rows, B = 10,
 // L = 6: 179 -> 159 us; 4,000,000 rows, B = 2, L = 8: 836 -> 804 us.
+//
+// Tile j's child c lands in columns 16 (c + j) of the children area: the two tiles share at most one
+// child.  Up to B = 13 both teams' areas fit beside the node columns, above that they take turns.
 constexpr uint32_t kSubTiles = 2;
 constexpr uint32_t kSuperRows = kSubTiles * kTileRows;     // 256
 constexpr uint32_t kSuperBufs = 4;
@@ -1966,11 +1969,11 @@ LookupScratch carveLookupScratch(void* base, uint32_t B, uint32_t L, uint64_t n)
 
 // Where lookupDirect ends.  It is bound by the L1's load path (a node is 2 KB per row and level,
 // 0.11 ns per row and level whatever the tree) above the ~11 us a call takes on the host; the
-// tensor-core path starts at one pass (12 us) up to L = 2, two passes and a regroup (41-43 us) up
+// tensor-core path starts at one pass (13 us) up to L = 2, two passes and a regroup (38-42 us) up
 // to L = 4, and three of more bins above.  Measured, direct against tensor, us per call: B=16 L=4:
-// 731 rows 11 / 43, 64,000 29 / 49, 100,000 43 / 54, 150,000 64 / 60; B=16 L=2: 32,000 11 / 13,
-// 48,000 14 / 13; B=10 L=6: 16,000 14 / 155, 200,000 123 / 213, 400,000 240 / 239; B=2 L=8:
-// 200,000 142 / 135.
+// 731 rows 11 / 42, 64,000 29 / 47, 100,000 43 / 51, 150,000 64 / 55; B=16 L=3: 100,000 33 / 47;
+// B=16 L=2: 32,000 11 / 13, 48,000 14 / 13; B=10 L=6: 16,000 14 / 133, 200,000 122 / 176; B=16 L=5:
+// 200,000 105 / 321; B=2 L=8: 200,000 143 / 131.
 uint64_t directLookupRows(uint32_t, uint32_t L) { return L <= 2 ? 32768 : L <= 4 ? 100000 : 200000; }
 
 uint32_t launchLookupDirect(const DeviceTree& tree, const uint8_t* desc, uint64_t n, uint32_t* leaf,

@@ -88,7 +88,7 @@ struct BuildOptions {
     uint64_t seed = 0;
     const uint32_t* injected = nullptr; // host [levelBeg(L)][B] descriptor indices
     bool ieeeDivision = false;          // center update rounding: false = reference (fast-math)
-    bool floatCenters = false;          // fp32 centers, split-bf16 distances with FP64 re-score
+    bool floatCenters = false;          // fp32 centers, fixed-point distances with FP64 re-score
 };
 
 struct BuildStats {
@@ -108,8 +108,8 @@ public:
     // masks [levelBeg(L)] (bit b = valid center), weights [levelBeg(L)][B].
     static std::unique_ptr<Vocabulary> fromHost(uint32_t B, uint32_t L, const uint8_t* centers, const uint32_t* masks,
                                                 const float* weights);
-    // The same with fp32 centers [levelBeg(L)][B][128]: lookups descend with split-bf16
-    // distances and an FP64 re-score near ties.
+    // The same with fp32 centers [levelBeg(L)][B][128]: lookups descend with fixed-point
+    // distances (split-bf16 ones for centers outside [0, 256)) and an FP64 re-score near ties.
     static std::unique_ptr<Vocabulary> fromHostF32(uint32_t B, uint32_t L, const float* centers,
                                                    const uint32_t* masks, const float* weights);
     // Hierarchical k-means build on the GPU (Vocabulary.cpp:32-121).  Synchronous.
