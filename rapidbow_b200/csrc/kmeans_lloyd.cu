@@ -450,8 +450,9 @@ __global__ void __launch_bounds__(kRows * kGroups, kCtasPerSm)
 }
 
 // One cooperative launch, a CTA per SM: the larger nodes are spread over the CTAs (every node's
-// tiles in parts of at most t tiles, with the smallest t whose parts fit the grid), and CTAs that
-// are done, or had no part, take resident nodes (`tail`), the largest class first.  For levels
+// tiles in parts of at most t tiles, with the smallest t whose parts fit the grid and leave CTAs for
+// the resident nodes), and CTAs that are done, or had no part, take those (`tail`), the largest class
+// first.  For levels
 // whose streamed rows fit the SMs' shared memory together (220,000 rows): a step is two MMA chains,
 // 2,048 atomic adds per CTA and one meeting of the node's CTAs, where the streaming path takes two
 // launches, a cleared counter and, every few steps, a read-back of it.
@@ -479,8 +480,15 @@ __global__ void __launch_bounds__(kRows * kShareGroups, 1)
             if (th.lane == 0) total[th.warp] = sum;
         }
         __syncthreads();
+        // The most CTAs (fewest tiles each) that leave enough for the small nodes: a small node's step
+        // takes about half the time of a shared one, so as many CTAs as half those nodes finish them
+        // meanwhile.  (200,000 rows, 256 nodes: 103 us with all CTAs on the few large ones first, 75 us
+        // with a third of them; with no small nodes fewer CTAs are slower, 276 -> 383 us.)
+        uint32_t small = 0;
+        for (uint32_t c = 0; tail && c < kLloydClasses; c++) small += cls.counters[c];
+        const uint32_t most = gridDim.x - min(small / 2, gridDim.x);
         uint32_t t = 1;
-        while (t < kShareTiles && total[t - 1] > gridDim.x) t++;
+        while (t < kShareTiles && total[t - 1] > most) t++;
         for (uint32_t i = th.tid; i < m; i += blockDim.x) {
             uint32_t first = 0;
             for (uint32_t j = 0; j < i; j++) first += (tiles[j] + t - 1u) / t;
