@@ -2070,8 +2070,9 @@ uint32_t launchLookup(const DeviceTree& tree, const uint8_t* desc, uint64_t n, u
             } else if (pass == 0) {
                 lookupPassSorted<false><<<grid, kSortThreads, kSortSmemBytes, stream>>>(tmapTile, p);
             } else {
-                // a CTA holds its tile list: several rounds of CTAs where the lists would be longer
-                const uint64_t lists = (n / kSuperRows + bins) / kSortTileCache + 1;
+                // a CTA holds its tile list: several rounds of CTAs where the lists would be longer (a
+                // group with rows has at most one super-tile that is not full)
+                const uint64_t lists = (n / kSuperRows + std::min<uint64_t>(bins, n)) / kSortTileCache + 1;
                 const uint32_t rounds = static_cast<uint32_t>((lists + grid - 1) / grid);
                 lookupPassSorted<true><<<grid * rounds, kSortThreads, kSortSmemBytes, stream>>>(tmapTile, p);
             }
