@@ -927,7 +927,11 @@ __global__ void __launch_bounds__(1024) inertiaSumKernel(const double* in, uint3
 // Few descriptors: a warp per descriptor takes it through every level.  Lane l holds dims 4 l .. + 3 and
 // sums (x - c)^2 over them in fp32 for every center; the 16 sums are reduced over the lanes together,
 // each step halving the centers a lane keeps.  All terms are positive, so a distance is off by less
-// than 2^-20 of itself, far inside the margin within which FP64 decides (as everywhere in this file).
+// than 2^-20 of itself (eleven roundings: the difference counts twice, then four products and five sums
+// over the lanes), whatever the centers' length: unlike |c|^2 - 2 x.c it holds |x|^2, which for centers
+// much shorter than the row is far more than kMarginScale's part.  Two distances within 2^-18 of the
+// smaller one are therefore left to FP64 too, and what the squares of tiny differences lose by
+// underflow (2^-142 over all dims) by the constant.
 // Bound by the node reads (512 bytes per center, row and level).
 constexpr uint32_t kDirectFThreads = 128;
 __global__ void __launch_bounds__(kDirectFThreads) lookupDirectF(const float* __restrict__ centers,
@@ -976,7 +980,7 @@ __global__ void __launch_bounds__(kDirectFThreads) lookupDirectF(const float* __
         const uint32_t next = __reduce_min_sync(0xFFFFFFFFu, mine == bi ? 0x7F800000u : bits);
         const float best = __uint_as_float(least);
         const float2 bnd = __ldg(bound + lb + idx);
-        const float thr = kMarginScale * __fmaf_rn(xLen, bnd.x, bnd.y);
+        const float thr = __fmaf_rn(kMarginScale, __fmaf_rn(xLen, bnd.x, bnd.y), __fmaf_rn(best, 0x1p-18f, 0x1p-100f));
         if (!(__uint_as_float(next) - best > thr)) {
             const uint32_t near = __reduce_or_sync(0xFFFFFFFFu, mine < B && !(dist - best > thr) ? 1u << mine : 0u);
             bi = nearestFp64(c, near, double(x0), double(x1), double(x2), double(x3));

@@ -219,3 +219,22 @@ def test_float_lookup_by_levels_matches_fp64_oracle(oracle, B, L, n):
     voc = rbw.vocabulary_from_host_f32(B, L, centers, masks, weights)
     desc = edge_descriptors(centers.astype(np.uint8), n, seed=n)
     assert np.array_equal(_lookup(voc, desc), oracle.lookup_f32(centers, B, L, desc, threads=THREADS))
+
+
+@pytest.mark.parametrize("scale", [1e-20, 0.001, 0.003, 0.03, 0.3])
+@pytest.mark.parametrize("bright", [False, True])
+def test_float_lookup_of_centers_much_shorter_than_the_rows(oracle, scale, bright):
+    """Centers in [0, scale) and rows of |x| near 500 or near 2,300 (a few of them zero): distances that
+    agree in their leading bits.  The words are FP64's in the one-launch descent and level by level, on
+    both sides of the limit between them (16,000 rows per level)."""
+    rng = np.random.default_rng(int(bright))
+    B, n = 10, 16_001
+    centers = (rng.random((1, B, 128)) * scale).astype(np.float32)
+    desc = rng.integers(150, 256, (n, 128), dtype=np.uint8) if bright else sift_like(n, seed=63).numpy()
+    desc[:3] = 0
+    voc = rbw.vocabulary_from_host_f32(B, 1, centers, np.full(1, 1023, np.uint32), np.ones((1, B), np.float32))
+    want = oracle.lookup_f32(centers, B, 1, desc, threads=THREADS)
+    for m in (700, n - 1, n):
+        got = _lookup(voc, desc[:m])
+        assert voc.last_kernels == 1 if m < n else voc.last_kernels > 1
+        assert np.array_equal(got, want[:m]), f"{m} rows: {np.count_nonzero(got != want[:m])} differ"
