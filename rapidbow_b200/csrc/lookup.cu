@@ -1064,6 +1064,8 @@ __global__ void __launch_bounds__(kSortThreads, 1)
                 int32_t* cn = &S.cn[at.i][0][0];
 #pragma unroll 1
                 for (uint32_t i = lane; i < words; i += 32) cn[i] = normKey(cn[i], i % 16, p.B);
+                // the slot's next block is written over these generic writes by bulk copies
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbarArrive(&S.cnReady[at.i]);
                 keyAt = at;

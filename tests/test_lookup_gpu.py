@@ -183,6 +183,20 @@ def test_sorted_pass_with_more_tiles_than_one_round_of_ctas_holds():
     assert voc.device_errors() == (0, 0)
 
 
+@pytest.mark.parametrize("B,L", [(3, 8), (10, 4), (12, 4)])
+def test_center_slots_used_again_and_again_hold_their_own_norms(B, L):
+    """Groups of few rows: every CTA loads many center blocks into its two to four slots, over the norm
+    keys of the blocks before.  Each of several lookups equals the FP32 kernel."""
+    centers, masks, weights = random_tree(B, L, seed=B * L + 1, dup_rate=0.2)
+    voc = rbw.vocabulary_from_host(B, L, centers, masks, weights)
+    desc = torch.randint(0, 256, (250_007, 128), dtype=torch.uint8, device="cuda",
+                         generator=torch.Generator("cuda").manual_seed(B))
+    want = voc.lookup(desc, algo="simt_f32")
+    for _ in range(6):
+        assert torch.equal(voc.lookup(desc, algo="tensor_u8"), want)
+    assert voc.device_errors() == (0, 0)
+
+
 @pytest.mark.parametrize("B,L,float_centers", [(16, 3, False), (10, 6, False), (3, 7, False), (16, 2, True), (9, 4, True)])
 def test_centers_come_back_as_they_went_in(B, L, float_centers):
     """Trees above and below one 32 MiB piece of the packed copy, with and without padded slots, and
