@@ -301,11 +301,14 @@ __device__ bool l1NormBlockExact(const uint32_t* sorted, uint32_t n, const float
     __shared__ uint64_t sBase[kMaxLevels]; // first weight of the level it above the leaves
     if (threadIdx.x < L) sBase[threadIdx.x] = levelBegDev(B, L - 1 - threadIdx.x) * B;
     __shared__ int32_t sLsb;
-    __shared__ uint32_t sBad, sMinBig, sMaxTiny, sTiny;
+    // sBad and sOver: the first and second pass; no barrier lies between the reads of sBad below and the
+    // second pass of a faster warp
+    __shared__ uint32_t sBad, sOver, sMinBig, sMaxTiny, sTiny;
     __shared__ unsigned long long sTotal;
     if (threadIdx.x == 0) {
         sLsb = 0x7FFFFFFF;
         sBad = 0;
+        sOver = 0;
         sMinBig = 0xFFFFFFFFu;
         sMaxTiny = 0;
         sTiny = 0;
@@ -406,11 +409,11 @@ __device__ bool l1NormBlockExact(const uint32_t* sorted, uint32_t n, const float
     for (uint32_t off = 16; off > 0; off >>= 1) total += __shfl_xor_sync(0xFFFFFFFFu, total, off);
     const bool nowBad = __any_sync(0xFFFFFFFFu, bad);
     if ((threadIdx.x & 31u) == 0) {
-        if (nowBad) atomicOr(&sBad, 1u);
+        if (nowBad) atomicOr(&sOver, 1u);
         atomicAdd(&sTotal, total);
     }
     __syncthreads();
-    if (sBad || sTotal >= kLimit) return false;
+    if (sOver || sTotal >= kLimit) return false;
     *norm = ldexp(static_cast<double>(sTotal), e);
     return true;
 }

@@ -141,6 +141,32 @@ def test_norms_bit_exact_for_every_weight_spread(oracle, kind):
         check_query(db, odb, q, 25)
 
 
+def test_documents_beyond_the_exact_norm_keep_every_pair(oracle):
+    """Thousands of documents whose norm is found not to be exact only in the block's second pass: their
+    norms, postings and queries are the oracle's (every warp's pairs are counted, whichever warp notices
+    first)."""
+    B, L, n_docs = 16, 2, 3000
+    rng = np.random.default_rng(65)
+    centers, masks, weights = random_tree(B, L, 66, dup_rate=0.0)
+    weights = rng.uniform(0.5, 12.0, weights.shape).astype(np.float32)
+    weights[rng.random(weights.shape) < 0.3] = np.float32(3e-9)
+    voc = rbw.vocabulary_from_host(B, L, centers, masks, weights)
+    docs = [rng.integers(0, B ** L, rng.integers(500, 1100), dtype=np.uint32) for _ in range(n_docs)]
+    off = np.concatenate([[0], np.cumsum([d.size for d in docs])]).astype(np.uint64)
+    odb = oracle.db(B, L, weights)
+    for i, d in enumerate(docs):
+        odb.add(i, d)
+    for _ in range(3):
+        db = rbw.DataBase(voc)
+        db.add_docs(np.arange(n_docs, dtype=np.uint32), np.concatenate(docs), off)
+        for leaf in range(0, B ** L, 17):
+            assert np.array_equal(db.postings(leaf), odb.postings(leaf))
+        for i in range(0, n_docs, 29):
+            assert np.float32(db.doc_rcp(i)) == np.float32(odb.doc_rcp(i)), i
+        for i in range(4):
+            check_query(db, odb, docs[i], 25)
+
+
 def test_documents_touched_only_through_clamped_words_are_results(oracle):
     """A document that shares with the query only words whose idf is clamped to FLT_MIN gets
     terms that round to zero in the fixed-point sum; it is still a result (score 2), as in the
