@@ -88,9 +88,10 @@ void launchLloydResident(const KMeansLevel& lv, const LloydClasses& cls, const u
 
 // The Lloyd loops of the nbShared streamed nodes of a level whose rows fit the SMs' shared memory
 // together (counters[kLloydShareCtas] <= SMs), each node spread over several CTAs, and with `tail`
-// those of the resident nodes too.  shareMem: lloydShareBytes(nbShared).
+// those of the resident nodes too.  shareMem: lloydShareBytes(nbShared).  False, with nothing launched,
+// where the stream's context owns too few SMs for the CTAs to meet (a green context).
 size_t lloydShareBytes(uint32_t nbShared);
-void launchLloydShared(const KMeansLevel& lv, const LloydClasses& cls, uint32_t nbShared, void* shareMem, bool tail,
+bool launchLloydShared(const KMeansLevel& lv, const LloydClasses& cls, uint32_t nbShared, void* shareMem, bool tail,
                        uint32_t maxIterations, cudaStream_t s);
 
 // ------------------------------------------------------------------ float-center mode

@@ -567,7 +567,7 @@ void launchLloydResident(const KMeansLevel& lv, const LloydClasses& cls, const u
 
 size_t lloydShareBytes(uint32_t nbShared) { return (uint64_t(nbShared) * kShareNodeWords + 32) * 4; }
 
-void launchLloydShared(const KMeansLevel& lv, const LloydClasses& cls, uint32_t nbShared, void* shareMem, bool tail,
+bool launchLloydShared(const KMeansLevel& lv, const LloydClasses& cls, uint32_t nbShared, void* shareMem, bool tail,
                        uint32_t maxIterations, cudaStream_t s)
 {
     ScopedKernelTimer timer(kTimedAssign, s);
@@ -580,8 +580,14 @@ void launchLloydShared(const KMeansLevel& lv, const LloydClasses& cls, uint32_t 
     uint32_t* mem = static_cast<uint32_t*>(shareMem);
     uint32_t tailArg = tail ? 1u : 0u;
     void* args[] = {&lvArg, &clsArg, &mem, &maxIterations, &tailArg};
-    RBW_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(lloydSharedKernel), dim3(currentSmCount()),
-                                         dim3(kRows * kShareGroups), args, smem, s));
+    const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(lloydSharedKernel),
+                                                      dim3(currentSmCount()), dim3(kRows * kShareGroups), args, smem, s);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError(); // answered here
+        return false;
+    }
+    RBW_CUDA(e);
+    return true;
 }
 
 } // namespace rbw

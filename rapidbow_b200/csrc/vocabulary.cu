@@ -688,7 +688,11 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
         for (uint32_t c = 0; c < kLloydClasses; c++) resident += hostLloyd[c];
         const uint32_t sms = static_cast<uint32_t>(currentSmCount()), nbShared = hostLloyd[kLloydClasses];
         const bool tail = resident <= 2 * sms;
-        const bool shared = !fl && hostLloyd[kLloydShareCtas] <= sms && (nbShared != 0 || tail);
+        bool shared = !fl && hostLloyd[kLloydShareCtas] <= sms && (nbShared != 0 || tail);
+        if (shared) {
+            StreamBuffer shareMem(lloydShareBytes(nbShared), st);
+            shared = launchLloydShared(lv, cls, nbShared, shareMem.get(), tail, opts.maxIterations, stream);
+        }
         const bool streamed = fl || (nbShared != 0 && !shared);
         if (streamed) {
             buildNodeTiles(fl ? lv.nodeCnt : cls.streamCnt, lv.nodeOff, nbLv, 128, tileOff.as<uint32_t>(),
@@ -697,10 +701,6 @@ std::unique_ptr<Vocabulary> Vocabulary::build(uint32_t B, uint32_t L, const uint
         }
         if (fl) RBW_CUDA(cudaMemsetAsync(lastChanged.get(), 0xFF, uint64_t(nbLv) * 4, stream));
         else if (!shared || !tail) launchLloydResident(lv, cls, hostLloyd, opts.maxIterations, stream);
-        if (shared) {
-            StreamBuffer shareMem(lloydShareBytes(nbShared), st);
-            launchLloydShared(lv, cls, nbShared, shareMem.get(), tail, opts.maxIterations, stream);
-        }
         uint32_t iters = 0;
         for (uint32_t it = 0; streamed && it < opts.maxIterations; it++) {
             const bool poll = (it + 1) % check == 0 || it + 1 == opts.maxIterations;

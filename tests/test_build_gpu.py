@@ -174,3 +174,37 @@ def test_build_shared_level_edges_match_oracle(oracle, rows_per_sm, extra, L):
     ref = oracle.build_vocabulary(desc, 30, B, L, max_iter=9, init=INIT_REFERENCE)
     _tree_equal(voc, ref)
     assert voc.build_stats()["iterations"][0] == min(9, -(-int(ref["iters"][0]) // 4) * 4)
+
+
+@pytest.mark.parametrize("n,L", [(1_000, 2), (20_000, 2), (150_000, 3)])
+def test_build_in_a_context_of_some_of_the_sms_matches_oracle(oracle, n, L):
+    """A stream whose context owns part of the SMs cannot run one cooperative launch over all of them:
+    levels whose nodes would be spread over the CTAs are streamed, small nodes run in their classes."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+
+    def ok(r):
+        assert int(r[0]) == 0, r[0]
+        return r[1] if len(r) == 2 else r[1:]
+
+    torch.zeros(1, device="cuda")
+    dev = ok(driver.cuDeviceGet(torch.cuda.current_device()))
+    sms = ok(driver.cuDeviceGetDevResource(dev, driver.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    part = ok(driver.cuDevSmResourceSplitByCount(1, sms, 0, sms.sm.smCount // 2))[0][0]
+    context = ok(driver.cuGreenCtxCreate(ok(driver.cuDevResourceGenerateDesc([part], 1)), dev,
+                                         driver.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+    stream = ok(driver.cuGreenCtxStreamCreate(context, driver.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    desc = sift_like(n, seed=n).numpy()
+    rows = torch.from_numpy(desc).cuda()
+    torch.cuda.synchronize()
+    B = 8
+    voc = rbw.build_vocabulary(rows, B, nb_doc=30, nb_levels=L, max_iterations=9, ieee_division=True, stream=int(stream))
+    ref = oracle.build_vocabulary(desc, 30, B, L, max_iter=9, init=INIT_REFERENCE)
+    _tree_equal(voc, ref)
+    beg = [sum(B ** i for i in range(level)) for level in range(L + 1)]
+    assert voc.build_stats()["iterations"] == [min(9, -(-int(max(ref["iters"][a:b])) // 4) * 4)
+                                               for a, b in zip(beg, beg[1:])]
+    del voc
+    ok((driver.cuStreamDestroy(stream)[0], None))
+    ok((driver.cuGreenCtxDestroy(context)[0], None))
+    other = rbw.build_vocabulary(rows, B, nb_doc=30, nb_levels=L, max_iterations=9, ieee_division=True)
+    _tree_equal(other, ref)  # no error is left behind
