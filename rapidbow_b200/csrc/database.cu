@@ -1188,6 +1188,27 @@ private:
     size_t mCap = 0;
 };
 
+// While it lives, this thread's calls are none of those that would end a stream capture going on in the
+// process (on streams of others): adding documents is host work to its callers, who may be capturing.
+class OutsideCaptures
+{
+public:
+    OutsideCaptures()
+    {
+        mSet = cudaThreadExchangeStreamCaptureMode(&mMode) == cudaSuccess;
+    }
+    ~OutsideCaptures()
+    {
+        if (mSet) cudaThreadExchangeStreamCaptureMode(&mMode);
+    }
+    OutsideCaptures(const OutsideCaptures&) = delete;
+    OutsideCaptures& operator=(const OutsideCaptures&) = delete;
+
+private:
+    cudaStreamCaptureMode mMode = cudaStreamCaptureModeRelaxed; // then the mode before
+    bool mSet = false;
+};
+
 struct Segment {
     PoolBuffer leafOff;   // u32 offset table (segIndex) + 1 tail entry
     PoolBuffer pairs;     // u64 slot << 32 | float bits of the leaf-level document entry
@@ -1302,6 +1323,7 @@ public:
         // validate the whole batch first: a failed call adds nothing
         std::unordered_map<uint32_t, uint32_t> seen;
         seen.reserve(nDocs);
+        const OutsideCaptures outside;
         const bool direct = nDocs && uploadsDirectly(leaves, off[0], off[nDocs]);
         for (uint32_t d = 0; d < nDocs; d++) {
             if (off[d + 1] < off[d] || off[d + 1] - off[d] > 0xFFFFFFFFull)

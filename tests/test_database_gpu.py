@@ -617,3 +617,44 @@ def test_large_batches_added_between_small_ones_match_oracle(oracle, pinned):
         assert np.array_equal(db.postings(int(leaf)), odb.postings(int(leaf)))
     for q in make_queries(docs, n_leaves, 6, seed=4):
         check_query(db, odb, q, 30)
+
+
+@pytest.mark.parametrize("other_thread", [False, True])
+def test_large_batches_can_be_added_during_a_stream_capture(oracle, other_thread):
+    """Adding documents leaves a capture that is going on in the process alone, in the same thread or
+    another, whatever the batch's size."""
+    import threading
+
+    import torch
+
+    B, L, n_docs = 16, 2, 200
+    rng = np.random.default_rng(21)
+    centers, masks, weights = random_tree(B, L, 22, dup_rate=0.0)
+    voc = rbw.vocabulary_from_host(B, L, centers, masks, weights)
+    db, odb = rbw.DataBase(voc), oracle.db(B, L, weights)
+    docs = [rng.integers(0, B ** L, 500, dtype=np.uint32) for _ in range(n_docs)]
+    for i, d in enumerate(docs):
+        odb.add(i, d)
+    desc = torch.from_numpy(rng.integers(0, 256, (500, 128), dtype=np.uint8)).cuda()
+    out = torch.zeros(500, dtype=torch.int32, device="cuda")
+    want = voc.lookup(desc).clone()
+    torch.cuda.synchronize()
+
+    def add():
+        db.add_docs(np.arange(n_docs, dtype=np.uint32), np.concatenate(docs), np.arange(0, 500 * n_docs + 1, 500))
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        voc.lookup(desc, out)
+        if other_thread:
+            t = threading.Thread(target=add)
+            t.start()
+            t.join()
+        else:
+            add()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    assert db.info() == (n_docs, 500 * n_docs)
+    for i in range(4):
+        check_query(db, odb, docs[i], 20)
