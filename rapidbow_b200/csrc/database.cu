@@ -1325,13 +1325,23 @@ public:
         seen.reserve(nDocs);
         const OutsideCaptures outside;
         const bool direct = nDocs && uploadsDirectly(leaves, off[0], off[nDocs]);
+        // the first fault is the one reported: leaves that a direct upload has yet to check come before
+        auto firstChecked = [&](uint32_t docs) {
+            if (direct) checkLeaves(leaves + off[0], off[docs] - off[0]);
+        };
         for (uint32_t d = 0; d < nDocs; d++) {
-            if (off[d + 1] < off[d] || off[d + 1] - off[d] > 0xFFFFFFFFull)
+            if (off[d + 1] < off[d] || off[d + 1] - off[d] > 0xFFFFFFFFull) {
+                firstChecked(d);
                 throw Error(kInvalidArg, "bad document offsets");
+            }
             const uint32_t n = static_cast<uint32_t>(off[d + 1] - off[d]);
+            if (mSlotOf.count(ids[d])) firstChecked(d);
             checkDoc(ids[d], leaves + off[d], n);
             if (!direct) checkLeaves(leaves + off[d], n);
-            if (!seen.emplace(ids[d], d).second) throw Error(kDuplicate, "Duplicate document index");
+            if (!seen.emplace(ids[d], d).second) {
+                firstChecked(d + 1);
+                throw Error(kDuplicate, "Duplicate document index");
+            }
         }
         const bool uploaded = direct && uploadChecked(leaves + off[0], off[nDocs] - off[0]);
         for (uint32_t d = 0; d < nDocs; d++)

@@ -658,3 +658,39 @@ def test_large_batches_can_be_added_during_a_stream_capture(oracle, other_thread
     assert db.info() == (n_docs, 500 * n_docs)
     for i in range(4):
         check_query(db, odb, docs[i], 20)
+
+
+@pytest.mark.parametrize("per_doc", [10, 1000])  # batches that are staged on the host, and copied directly
+def test_first_fault_of_a_batch_is_the_one_reported(oracle, per_doc):
+    """A batch with several faults is refused for the first in document order, whatever its size: a bad
+    leaf before or in a document whose index repeats, or an index already present before a bad leaf."""
+    B, L, n_docs = 16, 2, 100
+    centers, masks, weights = random_tree(B, L, 23, dup_rate=0.0)
+    db = rbw.DataBase(rbw.vocabulary_from_host(B, L, centers, masks, weights))
+    db.add_doc(500, np.array([1], np.uint32))
+    ids0, off0 = np.arange(n_docs, dtype=np.uint32), np.arange(0, n_docs * per_doc + 1, per_doc).astype(np.uint64)
+
+    def status(repeat_at=None, present_at=None, bad_leaf_in=None, bad_offset_at=None):
+        ids, off, leaves = ids0.copy(), off0.copy(), np.zeros(n_docs * per_doc, np.uint32)
+        if repeat_at is not None:
+            ids[repeat_at] = 3
+        if present_at is not None:
+            ids[present_at] = 500
+        if bad_leaf_in is not None:
+            leaves[(bad_leaf_in + 1) * per_doc - 1] = B ** L
+        if bad_offset_at is not None:
+            off[bad_offset_at + 1] = off[bad_offset_at] - 1
+        with pytest.raises(rbw.RbwError) as e:
+            db.add_docs(ids, leaves, off)
+        assert db.info() == (1, 1)
+        return e.value.status, str(e.value)
+
+    bad, dup = rbw.RBW_ERR_INVALID_ARG, rbw.RBW_ERR_DUPLICATE
+    assert status(repeat_at=40, bad_leaf_in=39)[0] == bad
+    assert status(repeat_at=40, bad_leaf_in=40)[0] == bad
+    assert status(repeat_at=40, bad_leaf_in=41)[0] == dup
+    assert status(present_at=40, bad_leaf_in=39)[0] == bad
+    assert status(present_at=40, bad_leaf_in=40)[0] == dup
+    assert "leaf" in status(bad_offset_at=40, bad_leaf_in=39)[1]
+    assert "offsets" in status(bad_offset_at=40, bad_leaf_in=60)[1]
+    assert status(repeat_at=40)[0] == dup and status(present_at=0)[0] == dup and status(bad_leaf_in=0)[0] == bad
