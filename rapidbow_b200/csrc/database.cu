@@ -672,10 +672,13 @@ struct ScoreParams {
     uint32_t B;
     uint32_t L;
     uint32_t k;
-    unsigned long long* cand;  // [nq][shards][k] candidate keys when there are several shards
-    unsigned long long* selGlobal; // k > kMaxK: [nq][shards][selStride] selection buffers
+    uint32_t candStride;       // most results of one shard: min(k, shardDocs)
+    unsigned long long* cand;  // [nq][shards][candStride] candidate keys when there are several shards
+    unsigned long long* selGlobal; // [nq][shards][selStride] selection buffers for more than kMaxK results
+    unsigned long long* mergeGlobal; // ... of the merge, [nq][mergeStride] (may be the same memory)
     const uint32_t* order;     // launch order of the queries (nullptr: in index order)
-    uint32_t selStride;        // power of two >= k
+    uint32_t selStride;        // power of two >= candStride
+    uint32_t mergeStride;      // power of two >= min(k, shards * candStride)
     uint32_t* outDocs;         // [nq][k]
     float* outScores;          // [nq][k]
     uint32_t* outCount;        // [nq]
@@ -1128,8 +1131,8 @@ __global__ void __launch_bounds__(kThreads, kThreads >= 1024 ? 1 : 1024 / kThrea
     if (P.cand == nullptr) {
         writeResults(P, q, selp, want);
     } else {
-        unsigned long long* c = P.cand + (uint64_t(q) * gridDim.y + shard) * P.k;
-        for (uint32_t i = threadIdx.x; i < P.k; i += blockDim.x) c[i] = i < want ? selp[i] : ~0ull;
+        unsigned long long* c = P.cand + (uint64_t(q) * gridDim.y + shard) * P.candStride;
+        for (uint32_t i = threadIdx.x; i < P.candStride; i += blockDim.x) c[i] = i < want ? selp[i] : ~0ull;
     }
 }
 
@@ -1139,8 +1142,8 @@ __global__ void __launch_bounds__(kScoreThreads) mergeKernel(ScoreParams P, uint
     __shared__ uint32_t nValid;
     __shared__ unsigned long long sel[kMaxK];
     const uint32_t q = blockIdx.x;
-    const unsigned long long* c = P.cand + uint64_t(q) * shards * P.k;
-    const uint32_t n = shards * P.k;
+    const unsigned long long* c = P.cand + uint64_t(q) * shards * P.candStride;
+    const uint32_t n = shards * P.candStride;
     if (threadIdx.x == 0) nValid = 0;
     __syncthreads();
     uint32_t mine = 0;
@@ -1149,8 +1152,8 @@ __global__ void __launch_bounds__(kScoreThreads) mergeKernel(ScoreParams P, uint
     if ((threadIdx.x & 31u) == 0 && mine) atomicAdd(&nValid, mine);
     __syncthreads();
     const uint32_t want = P.k < nValid ? P.k : nValid;
-    unsigned long long* selp = P.selGlobal ? P.selGlobal + uint64_t(q) * shards * P.selStride : sel;
-    selectSmallest(c, n, want, selp, P.selGlobal ? P.selStride : kMaxK);
+    unsigned long long* selp = P.mergeGlobal ? P.mergeGlobal + uint64_t(q) * P.mergeStride : sel;
+    selectSmallest(c, n, want, selp, P.mergeGlobal ? P.mergeStride : kMaxK);
     writeResults(P, q, selp, want);
 }
 
@@ -1458,9 +1461,14 @@ public:
         uint32_t parts = 1;
         while (parts < kMaxParts && uint64_t(nq) * shards * parts * 2 <= wanted) parts *= 2;
         const size_t entBytes = std::max<uint64_t>(totalLeaves, 1) * mL * sizeof(Entry);
-        const size_t candBytes = shards > 1 ? size_t(nq) * shards * k * 8 : 16;
-        const uint32_t selStride = k > kMaxK ? nextPow2(k) : 0u;
-        const size_t selBytes = k > kMaxK ? size_t(nq) * shards * selStride * 8 : 16;
+        // a shard has no more results than documents, however large k is; the merge's buffers lie in the
+        // shards', which are read no more by then
+        const uint32_t candStride = std::min(k, shardDocs);
+        const size_t candBytes = shards > 1 ? size_t(nq) * shards * candStride * 8 : 16;
+        const uint32_t selStride = candStride > kMaxK ? nextPow2(candStride) : 0u;
+        const uint32_t mergeMax = static_cast<uint32_t>(std::min<uint64_t>(k, uint64_t(shards) * candStride));
+        const uint32_t mergeStride = shards > 1 && mergeMax > kMaxK ? nextPow2(mergeMax) : 0u;
+        const size_t selBytes = std::max<size_t>(size_t(nq) * std::max<size_t>(size_t(shards) * selStride, mergeStride) * 8, 16);
         const uint32_t bigStride = maxBig ? sortRoom(maxBig) : 0u;
         const size_t bigBytes = bigQ.empty() ? 16 : bigQ.size() * (size_t(bigStride) + 1) * 4;
         // one block of working memory, its parts 256 bytes apart
@@ -1516,8 +1524,11 @@ public:
             P.L = mL;
             P.k = k;
             P.cand = shards > 1 ? static_cast<unsigned long long*>(cand) : nullptr;
-            P.selGlobal = k > kMaxK ? static_cast<unsigned long long*>(selG) : nullptr;
+            P.candStride = candStride;
+            P.selGlobal = selStride ? static_cast<unsigned long long*>(selG) : nullptr;
             P.selStride = selStride;
+            P.mergeGlobal = mergeStride ? static_cast<unsigned long long*>(selG) : nullptr;
+            P.mergeStride = mergeStride;
             // more queries than one wave of scoring CTAs: start the longest ones first
             if (nq > uint32_t(sms) && nq <= kOrderMax) {
                 workOrderKernel<<<1, 1024, 0, stream>>>(work, nq, order);

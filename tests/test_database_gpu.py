@@ -694,3 +694,73 @@ def test_first_fault_of_a_batch_is_the_one_reported(oracle, per_doc):
     assert "leaf" in status(bad_offset_at=40, bad_leaf_in=39)[1]
     assert "offsets" in status(bad_offset_at=40, bad_leaf_in=60)[1]
     assert status(repeat_at=40)[0] == dup and status(present_at=0)[0] == dup and status(bad_leaf_in=0)[0] == bad
+
+
+_QUERY_MEMORY = """
+import numpy as np, torch
+import rapidbow_b200 as rbw
+from tests.helpers import random_tree
+
+n, nq, k = 100_000, 64, 100_000
+rng = np.random.default_rng(1)
+db = rbw.DataBase(rbw.vocabulary_from_host(16, 2, *random_tree(16, 2, 1)))
+db.add_docs(np.arange(n, dtype=np.uint32), rng.integers(0, 256, 4 * n).astype(np.uint32), np.arange(0, 4 * n + 1, 4))
+q = torch.randint(0, 256, (nq * 8,), dtype=torch.int32, device="cuda")
+off = torch.arange(0, nq * 8 + 1, 8, device="cuda")
+
+def free():
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+db.query_batched(q, off, 10)
+before = free()
+db.query_batched(q, off, k)
+print(before - free())
+"""
+
+
+def test_working_memory_of_queries_for_very_many_results(oracle):
+    """What 64 queries for 100,000 results each take from the pool (its memory stays reserved, so the
+    process is a new one): at most twice the keys of the results, a power of two of them per query, and
+    as much again for the shards' candidates."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _QUERY_MEMORY], capture_output=True, text=True, cwd=root, timeout=300)
+    assert r.returncode == 0, r.stderr
+    assert int(r.stdout.split()[-1]) <= 4 * 64 * 131_072 * 8
+
+
+@pytest.mark.parametrize("layout", [1, 2])
+@pytest.mark.parametrize("k", [1000, 1500, 2600, 6000, 30_000])
+def test_results_of_many_shards_match_oracle(oracle, k, layout):
+    """Shards of fewer documents than results are asked for, and selections in shared and in global
+    memory: single queries and batches over several shards."""
+    import torch
+
+    from rapidbow_b200 import autotune as at
+
+    B, L, n_docs = 16, 2, 24_000
+    rng = np.random.default_rng(29)
+    at.set_value("db_shard_tables", B, L, at.bucket(n_docs), layout)
+    try:
+        centers, masks, weights = random_tree(B, L, 30, dup_rate=0.0)
+        db, odb = rbw.DataBase(rbw.vocabulary_from_host(B, L, centers, masks, weights)), oracle.db(B, L, weights)
+        docs = rng.integers(0, B ** L, (n_docs, 3), dtype=np.uint32)
+        db.add_docs(np.arange(n_docs, dtype=np.uint32), docs.ravel(), np.arange(0, 3 * n_docs + 1, 3))
+        for i in range(n_docs):
+            odb.add(i, docs[i])
+        q = rng.integers(0, B ** L, 90, dtype=np.uint32)
+        got, scores = check_query(db, odb, q, k)
+        nq = 40
+        leaves = torch.from_numpy(np.tile(q.astype(np.int32), nq)).cuda()
+        d, s, c = db.query_batched(leaves, torch.arange(0, 90 * nq + 1, 90, device="cuda"), k)
+        for i in (0, nq // 2, nq - 1):
+            assert int(c[i]) == got.size
+            assert np.array_equal(d[i, : got.size].cpu().numpy().view(np.uint32), got)
+            assert np.array_equal(s[i, : got.size].cpu().numpy(), scores)
+    finally:
+        at.clear()
