@@ -256,7 +256,9 @@ std::unique_ptr<Vocabulary> Vocabulary::fromHostF32(uint32_t B, uint32_t L, cons
     std::unique_ptr<Vocabulary> v{new Vocabulary};
     v->allocate(B, L, true, nullptr);
     const uint64_t nodes = v->mNbNodes;
-    DeviceBuffer canon(nodes * B * kDims * sizeof(float));
+    VocabularyMemory canonMemory; // from the pool, like the tree: a cudaMalloc / cudaFree pair costs up to 0.6 ms
+    canonMemory.allocate(nodes * B * kDims * sizeof(float), nullptr);
+    const DeviceArray canon(canonMemory.get(), nodes * B * kDims * sizeof(float));
     RBW_CUDA(cudaMemcpy(canon.get(), centers, canon.bytes(), cudaMemcpyHostToDevice));
     unsigned long long* outside = v->mRefined.as<unsigned long long>(); // zero, and again below
     padFloatKernel<<<blocksFor(nodes * kMaxBranch * kDims, 256), 256>>>(canon.as<float>(), v->mCentersF.as<float>(),
@@ -343,8 +345,10 @@ std::unique_ptr<Vocabulary> Vocabulary::fromHost(uint32_t B, uint32_t L, const u
     std::unique_ptr<Vocabulary> v{new Vocabulary};
     v->allocate(B, L, false, nullptr);
     const uint64_t nodes = v->mNbNodes;
-    DeviceBuffer canon(nodes * B * kDims);
-    RBW_CUDA(cudaMemcpy(canon.get(), centers, nodes * B * kDims, cudaMemcpyHostToDevice));
+    VocabularyMemory canonMemory; // as in fromHostF32
+    canonMemory.allocate(nodes * B * kDims, nullptr);
+    const DeviceArray canon(canonMemory.get(), nodes * B * kDims);
+    RBW_CUDA(cudaMemcpy(canon.get(), centers, canon.bytes(), cudaMemcpyHostToDevice));
     padKernel<<<blocksFor(nodes * kMaxBranch * 8, 256), 256>>>(canon.as<uint8_t>(), v->mCenters.as<uint8_t>(), nodes, B);
     RBW_CUDA(cudaGetLastError());
     v->mMasks.assign(masks, masks + nodes);
