@@ -1279,12 +1279,32 @@ public:
         mNbLeaves = ipowDev(mB, mL);
         mNbWords = levelBeg(mB, mL) * mB;
         if (mNbLeaves >= 0xFFFFFFFFull) throw Error(kUnsupported, "tree too large for a DataBase");
-        mWeights.reset(mNbWords * 4);
-        RBW_CUDA(cudaMemcpy(mWeights.get(), v.weights().data(), mNbWords * 4, cudaMemcpyHostToDevice));
         mHostDocOff.push_back(0);
         mDevice = currentDevice();
+        try {
+            createDevice(v);
+        } catch (...) {
+            freeDevice();
+            throw;
+        }
+    }
+    ~DataBase()
+    {
+        waitQueriesOnStream();
+        freeDevice();
+    }
+
+private:
+    void createDevice(const Vocabulary& v)
+    {
         RBW_CUDA(cudaStreamCreateWithFlags(&mStream, cudaStreamNonBlocking));
         RBW_CUDA(cudaEventCreateWithFlags(&mIndexReady, cudaEventDisableTiming));
+        // all arrays come from the pool: one cudaMalloc / cudaFree pair alone, which maps and unmaps device
+        // memory when the process holds no other small block, takes 0.6 ms; and the copy is not the new
+        // stream's, whose first one from pageable memory takes 40 us more
+        mWeights.reserve(mNbWords * 4, 0, mStream);
+        RBW_CUDA(cudaStreamSynchronize(mStream));
+        RBW_CUDA(cudaMemcpy(mWeights.get(), v.weights().data(), mNbWords * 4, cudaMemcpyHostToDevice));
         // empty index: zero offsets in both segments, zero word counts
         for (Segment* sg : {&mMain, &mDelta}) {
             sg->leafOff.reserve((mNbLeaves + 1) * 4, 0, mStream);
@@ -1301,18 +1321,20 @@ public:
         RBW_CUDA(cudaEventRecord(mIndexReady, mStream));
         RBW_CUDA(cudaStreamSynchronize(mStream));
     }
-    ~DataBase()
+    void freeDevice()
     {
-        waitQueriesOnStream();
-        for (PoolBuffer* b : {&mNewLeaves, &mDocOff, &mDocPairs, &mPairCount, &mRcpF, &mSlotDoc, &mMainLeafPost, &mWordPost,
-                              &mMain.leafOff, &mMain.pairs, &mMain.tf, &mDelta.leafOff, &mDelta.pairs, &mDelta.tf})
+        if (mStream == nullptr) return; // nothing was made
+        for (PoolBuffer* b : {&mWeights, &mSkipCounts, &mNewLeaves, &mDocOff, &mDocPairs, &mPairCount, &mRcpF, &mSlotDoc,
+                              &mMainLeafPost, &mWordPost, &mMain.leafOff, &mMain.pairs, &mMain.tf, &mDelta.leafOff,
+                              &mDelta.pairs, &mDelta.tf})
             b->release(mStream);
         cudaStreamSynchronize(mStream);
         for (auto& kv : mQueryEvents) cudaEventDestroy(kv.second);
-        cudaEventDestroy(mIndexReady);
+        if (mIndexReady) cudaEventDestroy(mIndexReady);
         cudaStreamDestroy(mStream);
     }
 
+public:
     void addDoc(uint32_t id, const uint32_t* leaves, uint32_t n)
     {
         std::unique_lock<std::shared_mutex> lk(mMu);
@@ -1574,7 +1596,7 @@ public:
             return;
         }
         waitQueriesOnStream();
-        if (mSkipCounts.get() == nullptr) mSkipCounts.reset(mNbWords * 8);
+        mSkipCounts.reserve(mNbWords * 8, 0, mStream);
         RBW_CUDA(cudaMemcpyAsync(mSkipCounts.get(), host, mNbWords * 8, cudaMemcpyHostToDevice, mStream));
         RBW_CUDA(cudaEventRecord(mIndexReady, mStream));
         RBW_CUDA(cudaStreamSynchronize(mStream));
@@ -1924,8 +1946,6 @@ private:
 
     uint32_t mB, mL;
     uint64_t mNbLeaves = 0, mNbWords = 0;
-    DeviceBuffer mWeights;
-    DeviceBuffer mSkipCounts;      // counts set by setWordPostings
     bool mSkipExternal = false;
     // host state
     std::vector<uint32_t> mHostIds;        // slot -> document id
@@ -1935,6 +1955,8 @@ private:
     uint32_t mStageMaxN = 0;
     uint32_t mIndexed = 0;                 // documents in the device index
     // device state (library pool, ordered on mStream)
+    PoolBuffer mWeights;
+    PoolBuffer mSkipCounts;                // counts set by setWordPostings
     PoolBuffer mDocOff, mDocPairs, mPairCount, mRcpF, mSlotDoc;
     PoolBuffer mNewLeaves;                 // the first mUploaded leaves of documents [mIndexed, nSlots)
     uint64_t mUploaded = 0;
