@@ -1381,9 +1381,10 @@ public:
         if (k == 0) return 0;
         const uint64_t off[2] = {0, n};
         cudaStream_t s = mStream;
-        // offsets and leaves go in one copy; documents, scores and their count come back in one
-        // unless the room for them is large (the count first, then what there is)
-        constexpr uint32_t kOneCopy = 65536;
+        // offsets and leaves go in one copy; documents, scores and their count come back in one unless
+        // the room for them is large (the count first, then what there is).  30 documents, k = 1,000: 54
+        // us with one copy, 73 with three; 8,000: 64, 68; 16,000: 74, 68; 65,536: 155, 68
+        constexpr uint32_t kOneCopy = 8192;
         const size_t outWords = 2 * size_t(k) + 1;
         std::vector<uint32_t> in(4 + size_t(n)), out(k <= kOneCopy ? outWords : 0);
         std::memcpy(in.data(), off, sizeof(off));
