@@ -90,7 +90,8 @@ typedef struct rbw_vocabulary rbw_vocabulary;
 /* Lookup algorithms. */
 enum {
     RBW_LOOKUP_AUTO = 0,       /* fastest exact path: one launch, a warp per descriptor, for few descriptors
-                                  (up to 32,768 for two levels, 100,000 for four, 200,000 above), else tensor cores */
+                                  (up to 32,768 for two levels, 100,000 for four, 200,000 above, 150,000 for
+                                  six with B <= 4), else tensor cores */
     RBW_LOOKUP_TENSOR_U8 = 1,  /* tcgen05 uint8 tensor-core descent with device regroup, rows sorted by branch
                                   within each level pair */
     RBW_LOOKUP_SIMT_F32 = 2,   /* plain FP32 SIMT descent (comparison baseline) */

@@ -1970,13 +1970,21 @@ LookupScratch carveLookupScratch(void* base, uint32_t B, uint32_t L, uint64_t n)
 }
 
 // Where lookupDirect ends.  It is bound by the L1's load path (a node is 2 KB per row and level,
-// 0.11 ns per row and level whatever the tree) above the ~11 us a call takes on the host; the
-// tensor-core path starts at one pass (13 us) up to L = 2, two passes and a regroup (38-42 us) up
-// to L = 4, and three of more bins above.  Measured, direct against tensor, us per call: B=16 L=4:
+// 0.09-0.11 ns per row and level whatever the tree) above the ~9 us a call takes on the host; the
+// tensor-core path starts at one pass (10 us) up to L = 2, two passes and a regroup (38-42 us) up
+// to L = 4, and three and more above, where the size of the regroups tells: up to kSmemHistMax bins
+// each is counted and scanned per CTA.  Measured, direct against tensor, us per call: B=16 L=4:
 // 731 rows 11 / 42, 64,000 29 / 47, 100,000 43 / 51, 150,000 64 / 55; B=16 L=3: 100,000 33 / 47;
 // B=16 L=2: 32,000 11 / 13, 48,000 14 / 13; B=10 L=6: 16,000 14 / 133, 200,000 122 / 176; B=16 L=5:
-// 200,000 105 / 321; B=2 L=8: 200,000 143 / 131.
-uint64_t directLookupRows(uint32_t, uint32_t L) { return L <= 2 ? 32768 : L <= 4 ? 100000 : 200000; }
+// 200,000 105 / 321; B=2 L=8: 180,000 130 / 126, 200,000 143 / 130; small regroups only: B=2 L=6:
+// 140,000 78 / 83, 160,000 89 / 89, 200,000 111 / 95; B=4 L=6: 140,000 80 / 84, 200,000 111 / 96; B=5
+// L=6: 200,000 113 / 113; B=4 L=5: 180,000 85 / 84, 200,000 93 / 90.
+uint64_t directLookupRows(uint32_t B, uint32_t L)
+{
+    if (L <= 2) return 32768;
+    if (L <= 4) return 100000;
+    return L == 6 && B <= 4 ? 150000 : 200000;
+}
 
 uint32_t launchLookupDirect(const DeviceTree& tree, const uint8_t* desc, uint64_t n, uint32_t* leaf,
                             cudaStream_t stream)

@@ -157,6 +157,18 @@ def test_auto_lookup_matches_oracle_on_both_sides_of_the_direct_limit(oracle, B,
         assert np.array_equal(got, want), f"n={n}: {np.count_nonzero(got != want)} mismatches"
 
 
+@pytest.mark.parametrize("B,limit", [(2, 150_000), (4, 150_000), (5, 200_000)])
+def test_auto_lookup_limit_of_six_levels(oracle, B, limit):
+    """Six levels whose regroups are all small (B <= 4) go to the tensor cores from fewer rows on."""
+    centers, masks, weights = random_tree(B, 6, seed=B, dup_rate=0.3)
+    voc = rbw.vocabulary_from_host(B, 6, centers, masks, weights)
+    for n in (limit, limit + 1):
+        desc = edge_descriptors(centers, n, seed=n)
+        got = _lookup(voc, desc, "auto")
+        assert (voc.last_kernels == 1) == (n == limit)
+        assert np.array_equal(got, oracle.lookup(centers, B, 6, desc, threads=8))
+
+
 @pytest.mark.parametrize("B,L", [(2, 4), (5, 3), (13, 2), (14, 2), (16, 1), (16, 2), (16, 3), (16, 4)])
 def test_sorted_passes_match_oracle(oracle, B, L):
     """Tensor-core passes around the 128-row tiles and 256-row super-tiles, with all rows on one branch
