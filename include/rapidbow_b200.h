@@ -377,7 +377,8 @@ RBW_API int rbw_idf_weights(uint32_t nb_doc, const uint32_t* occ, uint64_t n, fl
  * matches any depth.  Unset entries use the defaults. */
 enum {
     RBW_TUNE_ASSIGN_CTAS_PER_SM = 0,     /* uint8 k-means assign: CTAs per SM, 1..8, of which at most five run */
-    RBW_TUNE_ASSIGN_F32_CTAS_PER_SM = 1, /* float-center assign: CTAs per SM, 1..3 (default 3) */
+    RBW_TUNE_ASSIGN_F32_CTAS_PER_SM = 1, /* float-center assign: CTAs per SM, 1..4 (default 4; centers
+                                            outside [0, 256): at most three run) */
     RBW_TUNE_SCATTER_ROWS = 2,           /* lookup regroup: rows per thread, 8, 16 or 32 (default 16) */
     RBW_TUNE_DB_SHARD_TABLES = 3,        /* DataBase inverted file, keyed by documents instead of
                                             descriptors: 1 grouped tables per 2,560-document shard

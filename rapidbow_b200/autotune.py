@@ -6,7 +6,8 @@ the library's kernels, rbw_timing_*) and the fastest is kept, per (parameter, br
 tree levels, descriptor-count bucket = floor(log2(n))):
 
     assign_ctas_per_sm      uint8 k-means assign, CTAs per SM: 2..8 (default 6; 5 fit)
-    assign_f32_ctas_per_sm  float-center assign, CTAs per SM: 1..3          (default 3)
+    assign_f32_ctas_per_sm  float-center assign, CTAs per SM: 1..4          (default 4; 3 fit for
+                            centers outside [0, 256))
     scatter_rows            lookup regroup scatter of more than 1,024 bins, rows per thread:
                             8|16|32 (default 16)
     lookup_schedule         tensor-core lookup schedule of algo "auto": 1 rows sorted by
@@ -36,9 +37,10 @@ from . import _check, load_library
 
 PARAMS = {"assign_ctas_per_sm": 0, "assign_f32_ctas_per_sm": 1, "scatter_rows": 2, "db_shard_tables": 3,
           "lookup_schedule": 4, "assign_sums": 5}
-DEFAULTS = {"assign_ctas_per_sm": 6, "assign_f32_ctas_per_sm": 3, "scatter_rows": 16, "db_shard_tables": 1,
+DEFAULTS = {"assign_ctas_per_sm": 6, "assign_f32_ctas_per_sm": 4, "scatter_rows": 16, "db_shard_tables": 1,
             "lookup_schedule": 1, "assign_sums": 1}
-CANDIDATES = {"assign_ctas_per_sm": (2, 3, 4, 5, 6, 7, 8), "assign_f32_ctas_per_sm": (1, 2, 3), "scatter_rows": (8, 16, 32),
+CANDIDATES = {"assign_ctas_per_sm": (2, 3, 4, 5, 6, 7, 8), "assign_f32_ctas_per_sm": (1, 2, 3, 4),
+              "scatter_rows": (8, 16, 32),
               "db_shard_tables": (1, 2), "lookup_schedule": (1, 2), "assign_sums": (1, 2)}
 FORMAT = "rapidbow_b200 tuning cache"
 VERSION = 1

@@ -1166,8 +1166,7 @@ void launchAssignF(const KMeansLevelF& lv, const NodeTile* tiles, const uint32_t
     const uint32_t sms = static_cast<uint32_t>(currentSmCount());
     ScopedKernelTimer timer(kTimedAssign, s);
     if (lv.limbs) {
-        // the tunable's largest value, also its default, stands for all that fit
-        const uint32_t perSm = tuned >= kAfCtasPerSm ? kAxCtasPerSm : tuned;
+        const uint32_t perSm = std::min(kAxCtasPerSm, tuned);
         setMaxDynamicSmemOncePerDevice(reinterpret_cast<const void*>(assignKernelX), int(kAxSmemBytes), attrX);
         assignKernelX<<<std::max(1u, std::min(maxTiles, sms * perSm)), kAxThreads, kAxSmemBytes, s>>>(lv, tiles, nTilesDev);
     } else {

@@ -16,7 +16,7 @@ bool valid(TuneParam p, uint32_t v)
 {
     switch (p) {
     case kTuneAssignCtasPerSm: return v >= 1 && v <= 8;
-    case kTuneAssignFCtasPerSm: return v >= 1 && v <= 3;
+    case kTuneAssignFCtasPerSm: return v >= 1 && v <= 4;
     case kTuneScatterRows: return v == 8 || v == 16 || v == 32;
     case kTuneDbShardTables: return v == 1 || v == 2;
     case kTuneLookupSchedule: return v == 1 || v == 2;
@@ -41,7 +41,7 @@ uint32_t tuneDefault(TuneParam p)
 {
     switch (p) {
     case kTuneAssignCtasPerSm: return 6;
-    case kTuneAssignFCtasPerSm: return 3;
+    case kTuneAssignFCtasPerSm: return 4;
     case kTuneScatterRows: return 16;
     case kTuneDbShardTables: return 1;
     case kTuneLookupSchedule: return 1;

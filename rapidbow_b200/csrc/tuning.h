@@ -8,7 +8,8 @@ namespace rbw {
 
 enum TuneParam : uint32_t {
     kTuneAssignCtasPerSm = 0,  // uint8 k-means assign: resident CTAs per SM, 1..8 (default 6; at most 5 fit)
-    kTuneAssignFCtasPerSm = 1, // float-center assign: resident CTAs per SM, 1..3 (default 3)
+    kTuneAssignFCtasPerSm = 1, // float-center assign: resident CTAs per SM, 1..4 (default 4; at most 3 for centers
+                               // outside [0, 256))
     kTuneScatterRows = 2,      // lookup regroup scatter: rows per thread, 8 | 16 | 32 (default 16)
     kTuneDbShardTables = 3,    // inverted file: 1 one CSR per 2,560-document shard while small (default), 2 one CSR
     kTuneLookupSchedule = 4,   // tensor-core lookup of RBW_LOOKUP_AUTO: 1 sorted schedule (default), 2 ring

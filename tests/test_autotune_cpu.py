@@ -74,3 +74,15 @@ def test_library_rejects_bad_values():
     assert at.get_value("scatter_rows", 16, 4, 1 << 20) == 32
     at.set_value("scatter_rows", 16, 4, 20, 0)  # 0 removes the entry
     assert at.get_value("scatter_rows", 16, 4, 1 << 20) == 16
+
+
+def test_float_assign_ctas_are_what_they_say():
+    """One to four CTAs per SM, each its own value: four fit and are the default, three can be asked for."""
+    assert at.CANDIDATES["assign_f32_ctas_per_sm"] == (1, 2, 3, 4)
+    assert at.get_value("assign_f32_ctas_per_sm", 10, 0, 1 << 20) == 4
+    for v in (1, 2, 3, 4):
+        at.set_value("assign_f32_ctas_per_sm", 10, 0, 20, v)
+        assert at.get_value("assign_f32_ctas_per_sm", 10, 0, 1 << 20) == v
+    with pytest.raises(rbw.RbwError) as e:
+        at.set_value("assign_f32_ctas_per_sm", 10, 0, 20, 5)
+    assert e.value.status == rbw.RBW_ERR_INVALID_ARG
