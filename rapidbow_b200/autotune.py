@@ -159,7 +159,9 @@ class Autotuner:
     def tune_build(self, desc, B: int, L: int, float_centers: bool = False, repeats: int = 2, **build_kw) -> dict:
         """Tunes the assign kernel on a build of `desc` (CUDA uint8 [n, 128]); the build itself is
         the workload, timed by the library's assign-kernel events.  uint8 centers: the entry of
-        the CTAs per SM, with that of the center sums (which have one form) under "sums"."""
+        the CTAs per SM (2, 3, 4 and the default, which stands for the five that fit), with that of
+        the center sums under "sums": they have one form, so nothing is timed for them and the
+        entry keeps the default."""
         from . import build_vocabulary, timing_enable, timing_read, timing_reset
 
         n = desc.shape[0]
@@ -175,13 +177,14 @@ class Autotuner:
 
         if float_centers:
             return self.tune("assign_f32_ctas_per_sm", B, 0, n, measure)
-        sums = self.tune("assign_sums", B, 0, n, measure)
-        e = self.tune("assign_ctas_per_sm", B, 0, n, measure)
+        e = self.tune("assign_ctas_per_sm", B, 0, n, measure, candidates=(2, 3, 4, DEFAULTS["assign_ctas_per_sm"]))
+        sums = self.record("assign_sums", B, 0, n, {DEFAULTS["assign_sums"]: e["ms"]})
         return dict(e, sums=sums)
 
     def tune_lookup(self, voc, desc, repeats: int = 3) -> dict:
         """Tunes the tensor-core schedule of algo "auto" on lookups of `desc` through `voc`, timed
-        by the library's pass events."""
+        by the library's pass events: each candidate by its own algorithm, since "auto" takes no
+        tensor-core pass at all for few descriptors of the same bucket."""
         import torch
 
         from . import timing_enable, timing_read, timing_reset
@@ -189,12 +192,14 @@ class Autotuner:
         out = torch.empty(desc.shape[0], dtype=torch.int32, device=desc.device)
 
         def measure() -> float:
-            voc.lookup(desc, out)
+            schedule = get_value("lookup_schedule", voc.branch_factor, voc.nb_levels, desc.shape[0])
+            algo = {1: "tensor_u8", 2: "tensor_u8_ring"}[schedule]
+            voc.lookup(desc, out, algo=algo)
             torch.cuda.synchronize()
             timing_reset()
             timing_enable(True)
             for _ in range(repeats):
-                voc.lookup(desc, out)
+                voc.lookup(desc, out, algo=algo)
             torch.cuda.synchronize()
             timing_enable(False)
             return timing_read("lookup_pass_tc")[0] / repeats
@@ -203,7 +208,7 @@ class Autotuner:
 
     def tune_lookup_regroup(self, voc, desc, repeats: int = 3) -> dict:
         """Tunes the scatter of regroups of more than 1,024 bins (trees with B^(2p+2) > 1,024 at a
-        pass boundary) on lookups of `desc`, timed by the library's regroup events."""
+        pass boundary) on tensor-core lookups of `desc`, timed by the library's regroup events."""
         import torch
 
         from . import timing_enable, timing_read, timing_reset
@@ -211,12 +216,12 @@ class Autotuner:
         out = torch.empty(desc.shape[0], dtype=torch.int32, device=desc.device)
 
         def measure() -> float:
-            voc.lookup(desc, out)
+            voc.lookup(desc, out, algo="tensor_u8")
             torch.cuda.synchronize()
             timing_reset()
             timing_enable(True)
             for _ in range(repeats):
-                voc.lookup(desc, out)
+                voc.lookup(desc, out, algo="tensor_u8")
             torch.cuda.synchronize()
             timing_enable(False)
             return timing_read("lookup_regroup")[0] / repeats

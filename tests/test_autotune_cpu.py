@@ -86,3 +86,66 @@ def test_float_assign_ctas_are_what_they_say():
     with pytest.raises(rbw.RbwError) as e:
         at.set_value("assign_f32_ctas_per_sm", 10, 0, 20, 5)
     assert e.value.status == rbw.RBW_ERR_INVALID_ARG
+
+
+class _Timed:
+    """The library's timing calls over fake work: `ms` per call of what was last run."""
+
+    def __init__(self, monkeypatch, ms):
+        self.ms, self.total, self.on = ms, 0.0, False
+        torch = pytest.importorskip("torch")
+        monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: None)
+        monkeypatch.setattr(rbw, "timing_enable", lambda on: setattr(self, "on", on))
+        monkeypatch.setattr(rbw, "timing_reset", lambda: setattr(self, "total", 0.0))
+        monkeypatch.setattr(rbw, "timing_read", lambda name: (self.total, 1))
+
+    def ran(self, what):
+        if self.on:
+            self.total += self.ms(what)
+
+
+class _Voc:
+    branch_factor, nb_levels = 10, 6
+
+    def __init__(self, timed):
+        self.timed, self.algos = timed, []
+
+    def lookup(self, desc, out=None, algo="auto"):
+        self.algos.append(algo)
+        self.timed.ran(algo)
+
+
+def test_lookup_tunables_are_timed_on_the_tensor_core_passes(monkeypatch):
+    """150,000 rows of six levels go down in one launch under "auto", whatever the schedule: the candidates
+    are timed by their own algorithms, and the chosen one is for the larger lookups of the same bucket."""
+    import torch
+
+    desc = torch.zeros((150_000, 128), dtype=torch.uint8)
+    voc = _Voc(_Timed(monkeypatch, {"tensor_u8": 0.3, "tensor_u8_ring": 0.2}.__getitem__))
+    e = at.Autotuner("x", 148, "unused").tune_lookup(voc, desc, repeats=2)
+    assert set(voc.algos) == {"tensor_u8", "tensor_u8_ring"}
+    assert e["value"] == 2 and e["candidates"] == {"1": 0.3, "2": 0.2}
+    assert at.get_value("lookup_schedule", 10, 6, 250_000) == 2
+    voc = _Voc(_Timed(monkeypatch, lambda algo: 1.0 / at.get_value("scatter_rows", 10, 6, 150_000)))
+    e = at.Autotuner("x", 148, "unused").tune_lookup_regroup(voc, desc, repeats=2)
+    assert set(voc.algos) == {"tensor_u8"} and e["value"] == 32
+
+
+def test_builds_are_timed_once_per_grid(monkeypatch):
+    """The center sums have one form and five CTAs per SM fit: no candidate is timed against itself."""
+    import torch
+
+    ctas = []
+    timed = _Timed(monkeypatch, lambda c: {2: 4.0, 3: 2.0, 4: 3.0, 6: 2.5}[c])
+
+    def build(desc, B, nb_levels, float_centers, **kw):
+        ctas.append(at.get_value("assign_ctas_per_sm", B, 0, desc.shape[0]))
+        timed.ran(ctas[-1])
+
+    monkeypatch.setattr(rbw, "build_vocabulary", build)
+    t = at.Autotuner("x", 148, "unused")
+    e = t.tune_build(torch.zeros((5000, 128), dtype=torch.uint8), 10, 3, repeats=1)
+    assert ctas == [2, 2, 3, 3, 4, 4, 6, 6]  # a warm-up and a timed build each
+    assert e["value"] == 3 and e["default_ms"] == 2.5
+    assert e["sums"]["value"] == at.DEFAULTS["assign_sums"] and e["sums"]["candidates"] == {"1": 2.0}
+    assert {x["param"] for x in t.entries} == {"assign_sums", "assign_ctas_per_sm"}
