@@ -39,6 +39,7 @@ struct Error : std::runtime_error {
 inline void cudaThrow(cudaError_t e, const char* what)
 {
     if (e != cudaSuccess) {
+        cudaGetLastError(); // reported here, not by the next call's check of its launches
         const Status s = (e == cudaErrorMemoryAllocation) ? kOutOfMemory : kCudaError;
         throw Error(s, std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")");
     }

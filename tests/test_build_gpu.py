@@ -208,3 +208,18 @@ def test_build_in_a_context_of_some_of_the_sms_matches_oracle(oracle, n, L):
     ok((driver.cuGreenCtxDestroy(context)[0], None))
     other = rbw.build_vocabulary(rows, B, nb_doc=30, nb_levels=L, max_iterations=9, ieee_division=True)
     _tree_equal(other, ref)  # no error is left behind
+
+
+def test_a_refused_build_leaves_no_error_behind():
+    """A tree too large for any GPU (15^8 words) is refused with RBW_ERR_OUT_OF_MEMORY; the calls after
+    it work."""
+    desc = sift_like(2_000, seed=1, device="cuda")
+    voc = rbw.build_vocabulary(desc, 10, nb_doc=10, nb_levels=2, init="kmeans++", max_iterations=3)
+    want, words = voc.tree()[0], voc.lookup(desc).clone()
+    calls = [lambda: np.array_equal(voc.tree()[0], want), lambda: torch.equal(voc.lookup(desc), words),
+             lambda: rbw.build_vocabulary(desc, 10, nb_doc=10, nb_levels=1).nb_levels == 1]
+    for call in calls:
+        with pytest.raises(rbw.RbwError) as e:
+            rbw.build_vocabulary(desc, 15, nb_doc=10, nb_levels=8)
+        assert e.value.status == rbw.RBW_ERR_OUT_OF_MEMORY
+        assert call()
