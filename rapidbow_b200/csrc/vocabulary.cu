@@ -301,8 +301,14 @@ void copyUnpadded(const void* padded, void* host, uint64_t nodes, uint32_t B, si
     const size_t nodeBytes = B * bytesPerCenter;
     const uint64_t piece = std::min<uint64_t>(nodes, (size_t(32) << 20) / nodeBytes);
     void* tmp = nullptr;
-    RBW_CUDA(cudaMallocFromPoolAsync(&tmp, piece * nodeBytes, libraryPool(), nullptr));
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = cudaMallocFromPoolAsync(&tmp, piece * nodeBytes, libraryPool(), nullptr);
+    if (e == cudaErrorMemoryAllocation) { // no room to pack it: row by row, which needs none
+        cudaGetLastError();
+        RBW_CUDA(cudaMemcpy2D(host, nodeBytes, padded, kMaxBranch * bytesPerCenter, nodeBytes, nodes,
+                              cudaMemcpyDeviceToHost));
+        return;
+    }
+    RBW_CUDA(e);
     for (uint64_t n0 = 0; n0 < nodes && e == cudaSuccess; n0 += piece) {
         const uint64_t count = std::min(piece, nodes - n0);
         packKernel<<<blocksFor(count * nodeBytes / 16, 256), 256>>>(static_cast<const uint4*>(padded),

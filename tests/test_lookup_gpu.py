@@ -229,3 +229,38 @@ def test_centers_come_back_as_they_went_in(B, L, float_centers):
             assert np.array_equal(voc.tree()[0], centers)
         assert voc.device_errors() == (0, 0)
         del voc
+
+
+_FULL_GPU = """
+import numpy as np, torch
+import rapidbow_b200 as rbw
+
+B, L = 10, 5
+nodes = sum(B ** i for i in range(L))
+centers = np.random.default_rng(3).integers(0, 256, (nodes, B, 128), dtype=np.uint8)
+tree = np.full(nodes, 1023, np.uint32), np.ones((nodes, B), np.float32)
+voc = rbw.vocabulary_from_host(B, L, centers, *tree)
+vof = rbw.vocabulary_from_host_f32(B, 3, centers[:111].astype(np.float32), tree[0][:111], tree[1][:111])
+torch.cuda.synchronize()
+hold, size = [], 1 << 34
+while size >= 1 << 20:
+    try:
+        hold.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+    except torch.OutOfMemoryError:
+        size //= 2
+assert np.array_equal(voc.tree()[0], centers)
+assert np.array_equal(vof.centers_f32(), centers[:111].astype(np.float32))
+print("read back")
+"""
+
+
+def test_centers_come_back_without_device_memory_to_spare():
+    """Trees with padded slots are packed on the device first, and copied as they lie where the GPU's
+    memory is all in use (in a process of its own, whose pool is empty)."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _FULL_GPU], capture_output=True, text=True, cwd=root, timeout=300)
+    assert r.returncode == 0 and "read back" in r.stdout, r.stderr
