@@ -70,6 +70,10 @@ constexpr uint32_t kShardDocs = 2560;     // documents per inverted-file shard
 constexpr uint32_t kGroupShards = kSmemDocs / kShardDocs; // shards per group of kSmemDocs documents (8)
 constexpr uint64_t kShardTableMinBytes = 64ull << 20; // per-shard CSR tables always allowed up to this size
 constexpr uint32_t kMaxK = 1024;          // results selected in shared memory; more in global memory
+// Postings of one segment at most.  The scoring kernel steps through lists of pairs by up to kPairStep
+// positions in 32 bits: a list that ended nearer to 2^32 would be stepped past it and never left.
+constexpr uint32_t kPairStep = 256;
+constexpr uint64_t kMaxSegmentPostings = (1ull << 32) - 2 * kPairStep;
 constexpr double kFixScale = 72057594037927936.0; // 2^56
 constexpr uint32_t kDeltaMinDocs = 256;   // the delta may always hold this many documents
 constexpr uint32_t kDeltaFraction = 4;    // ... or up to main / kDeltaFraction
@@ -1077,7 +1081,8 @@ __global__ void __launch_bounds__(kThreads, kThreads >= 1024 ? 1 : 1024 / kThrea
 #pragma unroll
                 for (uint32_t k = 0; k < kListsAtOnce; k++) {
 #pragma unroll 1
-                    for (uint32_t p0 = (la[k] & ~1u) + 64; p0 < lb[k]; p0 += 256) {
+                    for (uint32_t p0 = (la[k] & ~1u) + 64; p0 < lb[k]; p0 += kPairStep) {
+                        static_assert(kPairStep == 4 * 64 && 32 * kUnionDepth <= kPairStep, "pairs per step");
                         uint4 w[4];
 #pragma unroll
                         for (uint32_t c = 0; c < 4; c++) w[c] = loadPairs(pairs, p0 + 64 * c + 2 * lane, lb[k]);
@@ -1790,7 +1795,7 @@ private:
     void buildSegment(Segment& sg, uint32_t s0, uint32_t s1, unsigned long long* leafPost, SegLayout layout)
     {
         const uint64_t pairsUpper = mHostDocOff[s1] - mHostDocOff[s0];
-        if (pairsUpper >= 0xFFFFFFFFull) throw Error(kUnsupported, "more than 2^32 postings in one segment");
+        if (pairsUpper > kMaxSegmentPostings) throw Error(kUnsupported, "more than 2^32 postings in one segment");
         sg.slotBeg = s0;
         sg.slotEnd = s1;
         sg.grouped = false;
