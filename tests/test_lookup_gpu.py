@@ -209,6 +209,18 @@ def test_center_slots_used_again_and_again_hold_their_own_norms(B, L):
     assert voc.device_errors() == (0, 0)
 
 
+def test_sorted_pass_with_more_groups_than_rows_in_several_rounds():
+    """117,649 groups and 100,003 rows: nearly every super-tile holds a few rows, and they are more than
+    one round of CTAs holds the lists of, by the count of groups that can have rows."""
+    centers, masks, weights = random_tree(7, 7, seed=6, dup_rate=0.0)
+    voc = rbw.vocabulary_from_host(7, 7, centers, masks, weights)
+    g = torch.Generator("cuda").manual_seed(2)
+    for n in (100_003, 75_777):
+        desc = torch.randint(0, 256, (n, 128), dtype=torch.uint8, device="cuda", generator=g)
+        assert torch.equal(voc.lookup(desc, algo="tensor_u8"), voc.lookup(desc, algo="simt_f32"))
+    assert voc.device_errors() == (0, 0)
+
+
 @pytest.mark.parametrize("B,L,float_centers", [(16, 3, False), (10, 6, False), (3, 7, False), (16, 2, True), (9, 4, True)])
 def test_centers_come_back_as_they_went_in(B, L, float_centers):
     """Trees above and below one 32 MiB piece of the packed copy, with and without padded slots, and
