@@ -743,6 +743,9 @@ def serving_bench(args, dev, rank):
                 srv.wait(ids[i])
 
         col = threading.Thread(target=collector)
+        # the submitting thread spins between arrivals: with the interpreter's 5 ms between thread
+        # switches the collector can end half a second after the last result
+        sys.setswitchinterval(0.0002)
         srv.reset_stats()
         if timing:
             rbw.timing_reset()
