@@ -171,10 +171,10 @@ cudaMemPool_t vocabularyPool(int dev)
 }
 } // namespace
 
-void VocabularyMemory::allocate(size_t bytes, cudaStream_t s)
+void VocabularyMemory::allocate(size_t bytes, cudaStream_t s, size_t pooledBytes)
 {
     mDevice = currentDevice();
-    mPooled = bytes <= kPooledBytes;
+    mPooled = bytes <= pooledBytes;
     if (mPooled) RBW_CUDA(cudaMallocFromPoolAsync(&mPtr, bytes, vocabularyPool(mDevice), s));
     else RBW_CUDA(cudaMalloc(&mPtr, bytes));
 }
@@ -256,8 +256,8 @@ std::unique_ptr<Vocabulary> Vocabulary::fromHostF32(uint32_t B, uint32_t L, cons
     std::unique_ptr<Vocabulary> v{new Vocabulary};
     v->allocate(B, L, true, nullptr);
     const uint64_t nodes = v->mNbNodes;
-    VocabularyMemory canonMemory; // from the pool, like the tree: a cudaMalloc / cudaFree pair costs up to 0.6 ms
-    canonMemory.allocate(nodes * B * kDims * sizeof(float), nullptr);
+    VocabularyMemory canonMemory;
+    canonMemory.allocate(nodes * B * kDims * sizeof(float), nullptr, VocabularyMemory::kPooledStaging);
     const DeviceArray canon(canonMemory.get(), nodes * B * kDims * sizeof(float));
     RBW_CUDA(cudaMemcpy(canon.get(), centers, canon.bytes(), cudaMemcpyHostToDevice));
     unsigned long long* outside = v->mRefined.as<unsigned long long>(); // zero, and again below
@@ -352,7 +352,7 @@ std::unique_ptr<Vocabulary> Vocabulary::fromHost(uint32_t B, uint32_t L, const u
     v->allocate(B, L, false, nullptr);
     const uint64_t nodes = v->mNbNodes;
     VocabularyMemory canonMemory; // as in fromHostF32
-    canonMemory.allocate(nodes * B * kDims, nullptr);
+    canonMemory.allocate(nodes * B * kDims, nullptr, VocabularyMemory::kPooledStaging);
     const DeviceArray canon(canonMemory.get(), nodes * B * kDims);
     RBW_CUDA(cudaMemcpy(canon.get(), centers, canon.bytes(), cudaMemcpyHostToDevice));
     padKernel<<<blocksFor(nodes * kMaxBranch * 8, 256), 256>>>(canon.as<uint8_t>(), v->mCenters.as<uint8_t>(), nodes, B);

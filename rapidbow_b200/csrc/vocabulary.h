@@ -48,13 +48,16 @@ class VocabularyMemory
 {
 public:
     static constexpr size_t kPooledBytes = size_t(512) << 20;
+    // Copies that an upload needs meanwhile: from the pool while they are small (a cudaMalloc / cudaFree
+    // pair costs 0.6 ms where it maps and unmaps memory), not to push the trees out of it.
+    static constexpr size_t kPooledStaging = size_t(32) << 20;
     VocabularyMemory() = default;
     VocabularyMemory(const VocabularyMemory&) = delete;
     VocabularyMemory& operator=(const VocabularyMemory&) = delete;
     // Waits for the device, as cudaFree would: work in flight on any stream may use the arrays.
     ~VocabularyMemory();
     // The memory may be used on `s` at once, on other streams after `s` is synchronised.
-    void allocate(size_t bytes, cudaStream_t s);
+    void allocate(size_t bytes, cudaStream_t s, size_t pooledBytes = kPooledBytes);
     uint8_t* get() const { return static_cast<uint8_t*>(mPtr); }
 
 private:
