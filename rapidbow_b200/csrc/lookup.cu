@@ -1909,9 +1909,17 @@ CUtensorMap makeRowMap(const uint8_t* desc, uint64_t n, uint32_t boxRows)
     const cuuint64_t strides[1] = {kDims};
     const cuuint32_t box[2] = {kDims, boxRows};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encodeTiledFn()(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(desc), dims, strides,
-                                       box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    auto encode = [&] {
+        return encodeTiledFn()(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(desc), dims, strides, box, estr,
+                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT) {
+        // a thread whose first CUDA call needs a context here: the runtime's calls before gave it none
+        RBW_CUDA(cudaSetDevice(currentDevice()));
+        r = encode();
+    }
     if (r != CUDA_SUCCESS) throw Error(kCudaError, "cuTensorMapEncodeTiled failed (" + std::to_string(int(r)) + ")");
     return m;
 }

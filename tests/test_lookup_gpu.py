@@ -221,6 +221,37 @@ def test_sorted_pass_with_more_groups_than_rows_in_several_rounds():
     assert voc.device_errors() == (0, 0)
 
 
+@pytest.mark.parametrize("algo", ["auto", "tensor_u8", "tensor_u8_ring", "simt_f32", "noalloc"])
+def test_lookup_as_the_first_call_of_a_thread(oracle, algo):
+    """A thread that has made no CUDA call yet looks descriptors up, on a stream of its own."""
+    import threading
+
+    B, L, n = 16, 4, 100_003
+    centers, masks, weights = random_tree(B, L, seed=14)
+    voc = rbw.vocabulary_from_host(B, L, centers, masks, weights)
+    desc = edge_descriptors(centers, n, seed=15)
+    rows, stream = torch.from_numpy(desc).cuda(), torch.cuda.Stream()
+    out = torch.empty(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    failed = []
+
+    def work():
+        try:
+            if algo == "noalloc":
+                voc.lookup_noalloc(rows, out, stream=stream)
+            else:
+                voc.lookup(rows, out, algo=algo, stream=stream)
+        except Exception as e:
+            failed.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert not failed, failed
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), oracle.lookup(centers, B, L, desc, threads=8))
+
+
 @pytest.mark.parametrize("B,L,float_centers", [(16, 3, False), (10, 6, False), (3, 7, False), (16, 2, True), (9, 4, True)])
 def test_centers_come_back_as_they_went_in(B, L, float_centers):
     """Trees above and below one 32 MiB piece of the packed copy, with and without padded slots, and
