@@ -56,10 +56,11 @@ enum {
  * (kmeans.cu:367); RBW_BUILD_IEEE_DIVISION uses the correctly rounded quotient instead.
  * RBW_BUILD_FLOAT_CENTERS (no counterpart in the reference, whose centers are uint8) keeps fp32
  * centers, c = float(double(sum) / double(count)) of the exact integer sums; distances come from
- * the tensor cores with each center as 24-bit fixed point in three bytes (hi + lo bf16 parts for uploaded
- * centers outside [0, 256)), and every descriptor whose best-versus-second margin is within the stated error bound is re-scored
- * in FP64 on the GPU, so assignments equal those of an FP64 evaluation (lowest index on ties).
- * Lookups through such a vocabulary use the same arithmetic. */
+ * the tensor cores with each center as 24-bit fixed point in three bytes (hi + lo bf16 parts for
+ * uploaded centers outside [0, 256)), and every descriptor whose best-versus-second margin is within
+ * the stated error bound is re-scored in FP64 on the GPU, so assignments equal those of an FP64
+ * evaluation (lowest index on ties).  So do the words of lookups through such a vocabulary, which use
+ * the same arithmetic, or squared differences in fp32 for few descriptors. */
 enum { RBW_BUILD_IEEE_DIVISION = 1, RBW_BUILD_FLOAT_CENTERS = 2 };
 
 /* Center storage of a vocabulary. */
@@ -180,8 +181,9 @@ RBW_API int rbw_voc_device_errors(const rbw_vocabulary* voc, uint32_t* code, uin
 
 /* No counterpart in the reference.  rbw_voc_lookup for callers that must not allocate device
  * memory during the call (latency-bound serving loops, plug-ins inside an application that owns
- * the GPU memory, fixed memory budgets): the same tensor-core lookup, with its working memory taken from one
- * 8 MiB device array that the library reserves on each GPU for the life of the process.
+ * the GPU memory, fixed memory budgets): the same words, by the tensor-core passes however few the
+ * descriptors (RBW_LOOKUP_TENSOR_U8), with the working memory taken from one 8 MiB device array that
+ * the library reserves on each GPU for the life of the process.
  * The first call on a device resolves that array's address and must come before any stream
  * capture; the address is kept for the life of the process, so after cudaDeviceReset on that
  * device this entry point must not be used again.  Calls that may overlap on the GPU share the
@@ -198,7 +200,8 @@ RBW_API void rbw_voc_destroy(rbw_vocabulary* voc);
 /* ------------------------------------------------------------------ inverted file
  * Replaces rbow::IDataBase (RapidBoW.h:92-107, DataBase.h:35-64, DataBase.cpp:39-197): an
  * inverted file over the leaf words of a vocabulary, scored with hierarchical tf-idf L1
- * distances.  The index lives on the GPU.  Adds are staged on the host and indexed on the
+ * distances.  The index lives on the GPU.  Adds are staged on the host (batches of 65,536 leaves and
+ * more are copied to the device when the caller's memory is pageable) and indexed on the
  * device at the next query, in work proportional to the documents added (a delta segment,
  * merged into the main segment from time to time), ordered with queries by CUDA events.
  * Documents, queries and max_results have no size limit beyond memory (items above 32768

@@ -1,8 +1,9 @@
 // Device-resident inverted file and hierarchical tf-idf scoring (reference: DataBase.cpp:39-197).
 //
 // Documents (DataBase.cpp:39-69):
-//   * addDoc only stages the host leaf indices; the device work happens at the next query, for
-//     the documents staged since the last one;
+//   * addDoc only stages the host leaf indices (large batches are copied to the device when they
+//     are added); the device work happens at the next query, for the documents added since the
+//     last one;
 //   * docPrepKernel, one CTA per new document: sorts its leaf words in shared memory, computes
 //     the L1 norm of its weight vector over all levels in the reference's order (levels
 //     leaf->root, descriptors in ascending leaf order, double sum; DataBase.cpp:54-68) and
@@ -864,7 +865,7 @@ __device__ __forceinline__ void writeResults(const ScoreParams& P, uint32_t q, c
 }
 
 // One CTA per (query, range of shardDocs documents).  The accumulators of the range live in
-// shared memory (9 B per document).  Grouped segments hand the CTA the leaf postings of its
+// shared memory (8 B per document).  Grouped segments hand the CTA the leaf postings of its
 // csrPerCta shards only (one range per leaf word); upper-level words read their group's range
 // and keep the CTA's documents.  A single-layout segment is walked by every CTA of the query,
 // each keeping the postings of its range.  kSharded = false: one range holds every document and

@@ -10,12 +10,13 @@
 //   * error bound: of the bf16 form, |score error| <= 4e-5 (|x||c| + |c|^2) (the split leaves
 //     |c - hi - lo| <= 2^-18 |c|; the products are exact in fp32; at most 127 accumulation roundings
 //     of <= 2^-23 each; |c|^2 and the final subtraction round once more); of the fixed-point form, see
-//     assignKernelX.  A member whose best-versus-second margin is at most
-//     kMarginScale (|x| max|c| + max|c|^2) -- six times the bound for both scores together -- is
-//     re-scored in FP64: the warp computes its squared distance to every center within that margin of
-//     the best in the oracle's fixed order (lane partials of four fused multiply-adds, then a
-//     butterfly of pairwise sums) and keeps the lowest index on ties (kmeans.cu:131-135); every other
-//     center and member is decided by more than the error;
+//     assignKernelX; of few rows' lookups, which sum (x - c)^2 in fp32, see lookupDirectF.  A member whose
+//     best-versus-second margin is at most kMarginScale (|x| max|c| + max|c|^2) -- six times the bf16
+//     form's bound for both scores together -- plus the other forms' own terms is re-scored in FP64: the
+//     warp computes its squared distance to every center within that margin of the best in the
+//     oracle's fixed order (lane partials of four fused multiply-adds, then a butterfly of pairwise
+//     sums) and keeps the lowest index on ties (kmeans.cu:131-135); every other center and member is
+//     decided by more than the error;
 //   * inertia: per node, sum_b (Q_b - 2 c_b.S_b + n_b |c_b|^2) in FP64 from the exact member
 //     sums S_b, counts n_b and sums of squared norms Q_b, with the centers of the assignment.
 #include "kmeans.cuh"

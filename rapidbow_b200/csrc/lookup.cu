@@ -920,7 +920,6 @@ __device__ __forceinline__ TileInfo superTile(const SortSmem& S, const PassParam
                     (i + 1 >= nT ? kLastOfGroup : i + 2 >= nT ? kNextIsLast : 0u) | (i == 0 ? kFirstOfGroup : 0u)};
 }
 
-// mbarWait by a whole warp, with one answer for all its lanes.
 // Whether a phase is complete, without waiting.
 __device__ __forceinline__ bool mbarTest(uint64_t* bar, uint32_t parity)
 {
@@ -940,6 +939,7 @@ __device__ __noinline__ void waitTimedOut(uint32_t abortFlag, DeviceErrors* err,
         err->detail = parity;
     }
 }
+// mbarWait by a whole warp, with one answer for all its lanes.
 __device__ __forceinline__ bool waitWarp(uint64_t* bar, uint32_t parity, volatile uint32_t* abortFlag, DeviceErrors* err,
                                          uint32_t site)
 {
@@ -1392,7 +1392,7 @@ __global__ void __launch_bounds__(kSortThreads, 1)
 }
 
 // ------------------------------------------------------------------ regroup kernels
-// Exclusive scans of the bin histogram: rowOff = scan(count), tileOff = scan(ceil(count/128));
+// Exclusive scans of the bin histogram: rowOff = scan(count), tileOff = scan(ceil(count / tileRows));
 // totals[0] = number of tiles, totals[1] = number of rows.
 __global__ void __launch_bounds__(1024) scanBins(const uint32_t* count, uint32_t nb, uint32_t* rowOff,
                                                  uint32_t* tileOff, uint32_t* totals, uint32_t tileRows)
@@ -1613,7 +1613,7 @@ __global__ void __launch_bounds__(1024) regroupScan(uint32_t* ctaHist, uint32_t 
             total += v;
         }
     }
-    // exclusive scans over bins of total and ceil(total / 128) (threads k == 0 hold the bins)
+    // exclusive scans over bins of total and ceil(total / tileRows) (threads k == 0 hold the bins)
     const bool owner = active && k == 0;
     const uint32_t ca = owner ? total : 0u, cb = owner ? (total + tileRows - 1) / tileRows : 0u;
     uint32_t a = ca, t = cb;

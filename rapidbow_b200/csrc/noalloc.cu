@@ -4,8 +4,9 @@
 // serving loops that must not hit the driver allocator (cudaMalloc can synchronise the device
 // and its latency is unbounded), plug-ins running inside a host application that owns all GPU
 // memory, and hosts that hand this library a fixed memory budget up front.  For them,
-// rbw_voc_lookup_noalloc runs the same tensor-core lookup as rbw_voc_lookup, but its working
-// memory (the regroup permutation, histograms and tile lists between passes) lives in one
+// rbw_voc_lookup_noalloc gives the words of rbw_voc_lookup by the tensor-core passes, however few
+// the descriptors (RBW_LOOKUP_TENSOR_U8; rbw_voc_lookup takes few of them down in one launch), and
+// its working memory (the regroup permutation, histograms and tile lists between passes) lives in one
 // file-scope device array of kNoAllocScratchBytes, reserved on every GPU that loads this
 // library for the life of the process.
 //

@@ -1,8 +1,9 @@
 """GPU parity of the float-center mode against the FP64 oracle.
 
 The reference keeps uint8 centers (kmeans.cu:367); this mode keeps fp32 centers computed in FP64
-from exact integer sums, takes distances from the tensor cores with hi + lo bf16 centers and fp32
-accumulation, and re-scores in FP64 every descriptor whose margin is within the error bound.  So
+from exact integer sums, takes distances from the tensor cores with fixed-point centers (hi + lo bf16
+parts outside [0, 256)) or, for few descriptors, from fp32 differences, and re-scores in FP64 every
+descriptor whose margin is within the error bound of its form.  So
 the assignments -- and therefore the centers, occurrence counts and word IDs -- must be identical
 to the oracle's FP64 evaluation (oracle/rbw_oracle.cpp, orc_build_vocabulary_f32 /
 orc_lookup_f32), and centers within 1e-5 relative of its FP64 means."""
