@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(256) prepareNodesKernel(const float* centers, 
 // The nearest of the centers in `cand` to the row whose dims 4 lane .. 4 lane + 3 are x0 .. x3, in FP64
 // in the oracle's order (orc_dist64: lane partials of four fused multiply-adds, then a butterfly of
 // pairwise sums), the lowest index on ties.  All lanes of the warp call it; cBase is their dims of
-// center 0.
+// center 0.  A distance that is no number is never the smallest, except that of center 0, where a scan of
+// all centers starts (the oracle's).
 __device__ __forceinline__ uint32_t nearestFp64(const float* cBase, uint32_t cand, double x0, double x1, double x2,
                                                 double x3)
 {
@@ -142,6 +143,12 @@ __device__ __forceinline__ uint32_t nearestFp64(const float* cBase, uint32_t can
     };
     double bestD = 0.0;
     uint32_t bb = kMaxBranch;
+    auto take = [&](double p, uint32_t b) {
+        if (bb == kMaxBranch ? p == p || b == 0 : p < bestD) {
+            bestD = p;
+            bb = b;
+        }
+    };
     while (cand != 0) {
         const uint32_t b0 = __ffs(cand) - 1;
         cand &= cand - 1;
@@ -155,16 +162,10 @@ __device__ __forceinline__ uint32_t nearestFp64(const float* cBase, uint32_t can
             p0 = __dadd_rn(p0, __shfl_xor_sync(0xFFFFFFFFu, p0, off));
             p1 = __dadd_rn(p1, __shfl_xor_sync(0xFFFFFFFFu, p1, off));
         }
-        if (bb == kMaxBranch || p0 < bestD) {
-            bestD = p0;
-            bb = b0;
-        }
-        if (p1 < bestD) {
-            bestD = p1;
-            bb = b1;
-        }
+        take(p0, b0);
+        take(p1, b1);
     }
-    return bb;
+    return bb == kMaxBranch ? 0u : bb;
 }
 
 // ------------------------------------------------------------------ assign, any fp32 centers

@@ -239,3 +239,23 @@ def test_float_lookup_of_centers_much_shorter_than_the_rows(oracle, scale, brigh
         got = _lookup(voc, desc[:m])
         assert voc.last_kernels == 1 if m < n else voc.last_kernels > 1
         assert np.array_equal(got, want[:m]), f"{m} rows: {np.count_nonzero(got != want[:m])} differ"
+
+
+@pytest.mark.parametrize("n", [700, 40_001])
+def test_centers_that_are_no_numbers_are_never_nearest(oracle, n):
+    """NaN centers in any slot but the first, among near ties that FP64 settles: every word is that of
+    the nearest of the others, as in the oracle."""
+    rng = np.random.default_rng(n)
+    B, L = 10, 3
+    nodes = level_beg(B, L)
+    data = sift_like(3000, seed=65).numpy()
+    centers = data[rng.integers(0, data.shape[0], nodes * B)].reshape(nodes, B, 128).astype(np.float32)
+    centers[:, 1::2] = centers[:, 0::2] + rng.uniform(0, 0.01, centers[:, 0::2].shape).astype(np.float32)
+    lost = rng.random((nodes, B)) < 0.25
+    lost[:, 0] = False
+    centers[lost] = np.nan
+    voc = rbw.vocabulary_from_host_f32(B, L, centers, np.full(nodes, 1023, np.uint32), np.ones((nodes, B), np.float32))
+    desc = np.ascontiguousarray(data[rng.integers(0, data.shape[0], n)])
+    voc.refined_lookups()
+    assert np.array_equal(_lookup(voc, desc), oracle.lookup_f32(centers, B, L, desc, threads=THREADS))
+    assert voc.refined_lookups() > 0
